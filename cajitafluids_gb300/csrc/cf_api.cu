@@ -347,6 +347,7 @@ int cf_ctx_create(const cf_grid_desc* d, cf_ctx** out) {
     if (!rc) rc = cuda_check(c, cudaMallocHost(&c->hPa, sizeof(SolverState)), "cudaMallocHost");
     if (!rc) rc = alloc_dev(c, c->d_tally, 4);
     if (!rc) rc = cuda_check(c, cudaMallocHost(&c->h_out, 4 * sizeof(double)), "cudaMallocHost");
+    if (!rc && c->precision == CF_PREC_FP64) rc = pcg64_setup(c);
     if (!rc && c->precision == CF_PREC_MIXED) rc = cg32_setup(c);
     for (int k = 0; k < 8 && !rc; ++k) rc = cuda_check(c, cudaEventCreate(&c->ev[k]), "event create");
     if (!rc) rc = sync(c, "context init");

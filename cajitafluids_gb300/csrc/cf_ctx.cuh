@@ -62,6 +62,11 @@ struct cf_ctx {
     double* staging = nullptr;      // FP64 staging for conversions / strided copies
     size_t staging_elems = 0;
 
+    // on-chip Jacobi-PCG (cf_pcg.cu): units per block (0: the grid does not
+    // fit), blocks, and the units' border values
+    int pcg_nu = 0, pcg_blocks = 0;
+    double* pcg_border = nullptr;
+
     // CUDA graphs of batches of solver iterations, rebuilt when the stencil changes
     cudaGraphExec_t g64 = nullptr, g32 = nullptr;
     int g64_batch = 0, g32_batch = 0;
@@ -190,6 +195,9 @@ int project_adjoint_async(cf_ctx* c, double dt, const SolveOpts& o, SolveResult*
 int enqueue_step(cf_ctx* ctx, double dt, int value_order, const SolveOpts& so, SolveResult* r, bool* deferred,
                  bool params_ready);
 int parse_solver_opts(cf_ctx* ctx, const cf_solver_opts* opts, SolveOpts* so);
+// on-chip FP64 Jacobi-PCG (cf_pcg.cu)
+int pcg64_setup(cf_ctx* c);
+cudaError_t pcg64_launch(cf_ctx* c, const Stencil& st, int iters);
 // FP32 TMA inner CG (cf_cg32.cu)
 int cg32_setup(cf_ctx* c);
 void cg32_launch_iteration(cf_ctx* c, const Stencil& st);

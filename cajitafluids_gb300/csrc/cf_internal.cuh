@@ -89,6 +89,9 @@ struct SolverState {
     int test_stall;  // test knob (cf_test_stall_wait): see k_tma_dir_matvec32
     int xsel;        // mixed MG-PCG, fused x update: the x buffer holding the solution
     unsigned int ticket[8];
+    // grid barriers of the on-chip solves: arrivals so far, and their count
+    // when the current launch started (both 0 when a projection starts)
+    unsigned int gcount, gbar;
 };
 
 struct Vec64 {

@@ -1,0 +1,502 @@
+// Jacobi-PCG with the whole solve on chip, for grids whose solver vectors fit
+// the SMs' shared memory.
+//
+// The launch-per-phase kernels (cf_project.cu) give one warp a unit of 64 x 16
+// cells, eight units to a block.  Up to a few hundred units that leaves most
+// of the GPU idle: an SM executes one FP64 warp instruction per sub-partition
+// every 64 cycles (measured; 2 FP64 lanes per cycle and SM), so eight units on
+// one SM take 25-30 us per kernel whatever the grid size, and each iteration
+// adds two launches and two last-block folds.  Here one cooperative launch
+// runs many iterations: a block owns NU units (r, p with its
+// halo and A p / z in shared memory, x in registers), the grid meets at two
+// barriers per iteration, and every block folds the unit partials itself.
+//
+//   A  p <- z + beta p (own cells and halo); q <- A p; unit partials of p.q
+//   -- barrier, fold, alpha
+//   B  r <- r - alpha q; z <- M^-1 r; border z published; unit partials of
+//      r.z and r.r; x <- x + alpha p between arriving and waiting
+//   -- barrier, fold, beta, convergence
+//
+// A unit's partial is the canonical one (cf_internal.cuh): lane l adds its two
+// columns row by row with fused multiply-adds, one warp per unit and sum, from
+// the products' factors staged in shared memory; the cells themselves are
+// computed by the whole block.  Every cell value and every
+// sum is formed by the same operations in the same order as by
+// k_cg_dir_matvec64 and k_cg_update64, so the results are the same bits.
+//
+// What bounds it: with one or two units per SM the serial lane sums (32
+// dependent FMAs of 64 cycles, 1 us each phase), the two grid barriers (about
+// 1.2 us each) and the divisions; at seven units per SM the FP64 pipe (12
+// operations per cell and iteration: 21 of 33 us).  Measured on GB300, time of
+// one iteration, the two launches per iteration before and this: 64^2 39.9 ->
+// 9.7 us, 256^2 49.6 -> 10.4 us, 1024^2 53.8 -> 33.2 us.
+#include <cuda_runtime.h>
+#include <math.h>
+
+#include <algorithm>
+
+#include "cf_ctx.cuh"
+
+namespace cf {
+
+// threads per block: the lane sums and folds of one or two units keep few
+// warps busy; four and seven units have the cells to keep 16 warps issuing
+template <int NU>
+struct PcThreads {
+    static constexpr int value = NU <= 2 ? 256 : 512;
+};
+constexpr int PC_PW = CF_UNIT_COLS + 2;                   // row stride of p with its halo
+constexpr int PC_P = PC_PW * (CF_BAND_ROWS + 2);          // doubles of p per unit
+constexpr int PC_CELLS = CF_UNIT_COLS * CF_BAND_ROWS;     // cells per unit
+constexpr int PC_UNIT = PC_P + 2 * PC_CELLS;              // doubles per unit: p, r, q / z
+constexpr int PC_BORDER = 2 * CF_UNIT_COLS + 2 * CF_BAND_ROWS;  // first / last row, first / last column
+constexpr int PC_MAX_UNITS = 7;                           // units per block (181 KB of shared memory)
+// polls of a grid barrier before the launch gives up (each poll is an L2
+// round trip; a barrier takes a few of them)
+constexpr unsigned PC_WAIT_LIMIT = 1u << 22;
+
+struct Pcg64 {
+    int nx, ny, per_x, per_y, G, U, pitch;
+    Stencil st;
+    double *x, *r, *pa, *pb;
+    double* border;                 // PC_BORDER values of z per unit
+    double *partA, *partB0, *partB1;  // unit partials: p.q; r.z, r.r
+    SolverState* S;
+    int iters;                      // iterations of this launch at most
+};
+
+// Grid barrier in two halves (all blocks co-resident: cooperative launch).
+// The counter only grows: S->gbar is its value when the launch starts.
+__device__ __forceinline__ void grid_arrive(SolverState* S) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&S->gcount) : "memory");
+    }
+}
+// true when every block has arrived target times in all (bounded wait)
+__device__ __forceinline__ bool grid_wait(SolverState* S, unsigned target) {
+    bool ok = true;
+    if (threadIdx.x == 0) {
+        unsigned v, k = 0;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&S->gcount) : "memory");
+        } while ((int)(v - target) < 0 && ++k < PC_WAIT_LIMIT);
+        ok = (int)(v - target) >= 0;
+        if (!ok) atomicExch(&S->status, (int)ST_TIMEOUT);
+    }
+    return __syncthreads_and(ok);
+}
+
+// The strided part of final_tree over n unit partials: thread t of the 256
+// adds partial[t], partial[t + 256], ... in that order.
+__device__ __forceinline__ double strided_sum(const double* part, int n, int t) {
+    double s = 0.0;
+    for (int u = t; u < n; u += CF_RED_THREADS) s = s + __ldcg(part + u);
+    return s;
+}
+
+// A unit's canonical sum of a.b: lane l, columns 2l and 2l + 1, row by row.
+// Cells outside the grid hold b = 0.  The next row is read while this row's
+// products are added.
+__device__ __forceinline__ double unit_dot(const double* a, int sa, const double* b, int lane) {
+    a += 2 * lane;
+    b += 2 * lane;
+    double acc = 0.0;
+    double a0 = a[0], a1 = a[1], b0 = b[0], b1 = b[1];
+#pragma unroll 4
+    for (int j = 0; j < CF_BAND_ROWS; ++j) {
+        double c0 = 0.0, c1 = 0.0, d0 = 0.0, d1 = 0.0;
+        if (j + 1 < CF_BAND_ROWS) {
+            c0 = a[(j + 1) * sa];
+            c1 = a[(j + 1) * sa + 1];
+            d0 = b[(j + 1) * CF_UNIT_COLS];
+            d1 = b[(j + 1) * CF_UNIT_COLS + 1];
+        }
+        acc = fma(a0, b0, acc);
+        acc = fma(a1, b1, acc);
+        a0 = c0;
+        a1 = c1;
+        b0 = d0;
+        b1 = d1;
+    }
+    return warp_fold(acc);
+}
+
+// Lane 0's warp_fold when only the first n lanes hold values and the others
+// are zero: the exchanges that would add a zero to it are left out.
+__device__ __forceinline__ double warp_fold_n(double s, int n) {
+    for (int m = 16; m >= 1; m >>= 1)
+        if (n > m) s = s + __shfl_xor_sync(0xffffffffu, s, m);
+    return s;
+}
+
+template <int NU>
+__global__ void __launch_bounds__(PcThreads<NU>::value, 1) k_pcg64(Pcg64 a) {
+    constexpr int PC_THREADS = PcThreads<NU>::value, PC_CPT = PC_CELLS / PC_THREADS;
+    extern __shared__ __align__(16) double pc_smem[];
+    __shared__ double tab_d[16], tab_m[16];
+    __shared__ double ws0[CF_RED_WARPS], ws1[CF_RED_WARPS];
+    __shared__ double bc_val;
+    __shared__ int bc_stat;
+    SolverState* S = a.S;
+    if (*(volatile int*)&S->status != ST_RUNNING) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int it = S->iter;
+    const int it_end = it + a.iters, max_iter = S->max_iter;
+    double beta = S->beta, rho = S->rho, rr = S->rr, alpha = S->alpha;
+    const unsigned gbase = S->gbar;
+    unsigned arrived = 0;
+    if (tid < 16) {
+        tab_d[tid] = a.st.diag[tid];
+        tab_m[tid] = a.st.minv[tid];
+    }
+    __syncthreads();
+    const double ms = a.st.ms;
+    auto unit_of = [&](int k) { return (int)blockIdx.x + k * (int)gridDim.x; };
+    auto P = [&](int k) { return pc_smem + k * PC_UNIT; };
+    auto R = [&](int k) { return pc_smem + k * PC_UNIT + PC_P; };
+    auto Q = [&](int k) { return pc_smem + k * PC_UNIT + PC_P + PC_CELLS; };
+
+    // Thread t owns cells t, t + 256, ... of each unit (64 to a row: row
+    // t / 64 + 4 m, column t % 64) and, below PC_BORDER, one halo value.
+    // code[k]: 4 wall-adjacency bits per cell, then a valid bit per cell.
+    const int col = tid & (CF_UNIT_COLS - 1), row0 = tid / CF_UNIT_COLS;
+    double xr[NU][PC_CPT];
+    unsigned code[NU];
+    int hsrc[NU], hpos[NU];  // border value this thread reads (-1: none, a wall), and its place in p
+    double zh[NU];
+    const double* pold = (it & 1) ? a.pb : a.pa;
+#pragma unroll
+    for (int k = 0; k < NU; ++k) {
+        const int u = unit_of(k);
+        code[k] = 0;
+        hsrc[k] = -1;
+        hpos[k] = 0;
+        zh[k] = 0.0;
+        if (u >= a.U) continue;
+        const int g = u % a.G, band = u / a.G;
+        const int c0 = g * CF_UNIT_COLS, j0 = band * CF_BAND_ROWS;
+        const int nc = min(CF_UNIT_COLS, a.nx - c0), nr = min(CF_BAND_ROWS, a.ny - j0);
+        double *p = P(k), *r = R(k), *q = Q(k);
+        for (int i = tid; i < PC_P; i += PC_THREADS) p[i] = 0.0;
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < PC_CPT; ++m) {
+            const int row = row0 + m * (PC_THREADS / CF_UNIT_COLS), cell = row * CF_UNIT_COLS + col;
+            double rv = 0.0, z = 0.0;
+            xr[k][m] = 0.0;
+            if (col < nc && row < nr) {
+                const int eb = edge_bits(c0 + col, j0 + row, a.nx, a.ny, a.per_x, a.per_y);
+                code[k] |= (unsigned)eb << (4 * m) | 1u << (16 + m);
+                const size_t o = (size_t)(j0 + row) * a.pitch + c0 + col;
+                rv = a.r[o];
+                z = tab_m[eb] * rv;
+                xr[k][m] = a.x[o];
+                if (it > 0) p[(row + 1) * PC_PW + col + 1] = pold[o];
+            }
+            r[cell] = rv;
+            q[cell] = z;
+        }
+        // halo: row below, row above, column west, column east of the unit's
+        // cells in the grid (wrapped along a periodic axis, 0 beyond a wall)
+        if (tid < PC_BORDER) {
+            int gc, gj, pos, off;
+            bool in;
+            if (tid < 2 * CF_UNIT_COLS) {
+                const int cc = tid & (CF_UNIT_COLS - 1), up = tid / CF_UNIT_COLS;
+                in = cc < nc;
+                gc = c0 + cc;
+                gj = up ? j0 + nr : j0 - 1;
+                pos = (up ? nr + 1 : 0) * PC_PW + cc + 1;
+                off = (up ? 0 : CF_UNIT_COLS) + cc;  // the owner's first row is above us, its last row below
+            } else {
+                const int rr_ = (tid - 2 * CF_UNIT_COLS) % CF_BAND_ROWS, east = (tid - 2 * CF_UNIT_COLS) / CF_BAND_ROWS;
+                in = rr_ < nr;
+                gj = j0 + rr_;
+                gc = east ? c0 + nc : c0 - 1;
+                pos = (rr_ + 1) * PC_PW + (east ? nc + 1 : 0);
+                off = 2 * CF_UNIT_COLS + (east ? 0 : CF_BAND_ROWS) + rr_;
+            }
+            const int wc = wrap_index(gc, a.nx, a.per_x), wj = wrap_index(gj, a.ny, a.per_y);
+            if (in && wc >= 0 && wj >= 0) {
+                const int ou = (wj / CF_BAND_ROWS) * a.G + wc / CF_UNIT_COLS;
+                hsrc[k] = ou * PC_BORDER + off;
+                hpos[k] = pos;
+                const size_t o = (size_t)wj * a.pitch + wc;
+                zh[k] = tab_m[edge_bits(wc, wj, a.nx, a.ny, a.per_x, a.per_y)] * a.r[o];
+                if (it > 0) p[pos] = pold[o];
+            }
+        }
+        __syncthreads();
+    }
+    int status = ST_RUNNING;
+    const int nw = min(CF_RED_WARPS, (a.U + 31) / 32);  // warps whose strided sums are not empty
+    for (;;) {
+        // ---- A: direction, A p, p.q
+        const bool first = it == 0;
+#pragma unroll
+        for (int k = 0; k < NU; ++k) {
+            if (unit_of(k) >= a.U) break;
+            double *p = P(k), *q = Q(k);
+#pragma unroll
+            for (int m = 0; m < PC_CPT; ++m) {
+                const int row = row0 + m * (PC_THREADS / CF_UNIT_COLS);
+                if (code[k] >> (16 + m) & 1u) {
+                    const double z = q[row * CF_UNIT_COLS + col];
+                    double& pv = p[(row + 1) * PC_PW + col + 1];
+                    pv = first ? z : fma(beta, pv, z);
+                }
+            }
+            if (hsrc[k] >= 0) p[hpos[k]] = first ? zh[k] : fma(beta, p[hpos[k]], zh[k]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < NU; ++k) {
+            if (unit_of(k) >= a.U) break;
+            const double* p = P(k);
+            double* q = Q(k);
+#pragma unroll
+            for (int m = 0; m < PC_CPT; ++m) {
+                const int row = row0 + m * (PC_THREADS / CF_UNIT_COLS);
+                const double* c = p + (row + 1) * PC_PW + col + 1;
+                double qv = 0.0;
+                if (code[k] >> (16 + m) & 1u) {
+                    qv = tab_d[code[k] >> (4 * m) & 15u] * c[0];
+                    qv = fma(ms, c[-1], qv);
+                    qv = fma(ms, c[1], qv);
+                    qv = fma(ms, c[-PC_PW], qv);
+                    qv = fma(ms, c[PC_PW], qv);
+                }
+                q[row * CF_UNIT_COLS + col] = qv;
+            }
+        }
+        __syncthreads();
+        if (warp < NU && unit_of(warp) < a.U) {
+            const double s = unit_dot(P(warp) + PC_PW + 1, PC_PW, Q(warp), lane);
+            if (lane == 0) __stcg(a.partA + unit_of(warp), s);
+        }
+        grid_arrive(S);
+        arrived += gridDim.x;
+        if (!grid_wait(S, gbase + arrived)) return;
+        if (warp < nw) {
+            const double s = warp_fold_n(strided_sum(a.partA, a.U, tid), a.U - 32 * warp);
+            if (lane == 0) ws0[warp] = s;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            double pq = ws0[0];
+            for (int k = 1; k < nw; ++k) pq = pq + ws0[k];
+            const double al = rho / pq;
+            if (lane == 0) {
+                bc_stat = !(pq > 0.0) ? (isnan(pq) ? (int)ST_NAN : (int)ST_BREAKDOWN) : (int)ST_RUNNING;
+                bc_val = al;
+            }
+        }
+        __syncthreads();
+        status = bc_stat;
+        if (status != ST_RUNNING) break;
+        alpha = bc_val;
+        // ---- B: residual, z, border, r.z and r.r
+        const double malpha = -alpha;
+#pragma unroll
+        for (int k = 0; k < NU; ++k) {
+            const int u = unit_of(k);
+            if (u >= a.U) break;
+            double *r = R(k), *q = Q(k);
+            double* bo = a.border + (size_t)u * PC_BORDER;
+            const int nc = min(CF_UNIT_COLS, a.nx - (u % a.G) * CF_UNIT_COLS);
+            const int nr = min(CF_BAND_ROWS, a.ny - (u / a.G) * CF_BAND_ROWS);
+#pragma unroll
+            for (int m = 0; m < PC_CPT; ++m) {
+                const int row = row0 + m * (PC_THREADS / CF_UNIT_COLS), cell = row * CF_UNIT_COLS + col;
+                if (!(code[k] >> (16 + m) & 1u)) continue;
+                const double rv = fma(malpha, q[cell], r[cell]);
+                const double z = tab_m[code[k] >> (4 * m) & 15u] * rv;
+                r[cell] = rv;
+                q[cell] = z;
+                if (row == 0) __stcg(bo + col, z);
+                if (row == nr - 1) __stcg(bo + CF_UNIT_COLS + col, z);
+                if (col == 0) __stcg(bo + 2 * CF_UNIT_COLS + row, z);
+                if (col == nc - 1) __stcg(bo + 2 * CF_UNIT_COLS + CF_BAND_ROWS + row, z);
+            }
+        }
+        __syncthreads();
+        for (int c = warp; c < 2 * NU; c += PC_THREADS / 32) {
+            const int k = c >> 1, u = unit_of(k);
+            if (u >= a.U) break;
+            const double s = unit_dot(R(k), CF_UNIT_COLS, (c & 1) ? R(k) : Q(k), lane);
+            if (lane == 0) __stcg(((c & 1) ? a.partB1 : a.partB0) + u, s);
+        }
+        grid_arrive(S);
+        arrived += gridDim.x;
+#pragma unroll
+        for (int k = 0; k < NU; ++k) {
+            if (unit_of(k) >= a.U) break;
+            const double* p = P(k);
+#pragma unroll
+            for (int m = 0; m < PC_CPT; ++m) {
+                const int row = row0 + m * (PC_THREADS / CF_UNIT_COLS);
+                if (code[k] >> (16 + m) & 1u) xr[k][m] = fma(alpha, p[(row + 1) * PC_PW + col + 1], xr[k][m]);
+            }
+        }
+        if (!grid_wait(S, gbase + arrived)) return;
+#pragma unroll
+        for (int k = 0; k < NU; ++k)
+            if (hsrc[k] >= 0) zh[k] = __ldcg(a.border + hsrc[k]);
+        // r.z by warps 0 .. nw - 1, r.r by the next nw (or the same where the
+        // block has too few)
+        const int wr = 2 * nw <= PC_THREADS / 32 ? warp - nw : warp;
+        if (warp < nw) {
+            const double s = warp_fold_n(strided_sum(a.partB0, a.U, tid), a.U - 32 * warp);
+            if (lane == 0) ws0[warp] = s;
+        }
+        if (wr >= 0 && wr < nw) {
+            const double s = warp_fold_n(strided_sum(a.partB1, a.U, wr * 32 + lane), a.U - 32 * wr);
+            if (lane == 0) ws1[wr] = s;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            double rz = ws0[0];
+            for (int k = 1; k < nw; ++k) rz = rz + ws0[k];
+            const double be = rz / rho;
+            if (lane == 0) {
+                bc_val = be;
+                ws0[0] = rz;
+            }
+        } else if (warp == 1) {
+            double t = ws1[0];
+            for (int k = 1; k < nw; ++k) t = t + ws1[k];
+            int st = ST_RUNNING;
+            if (isnan(t))
+                st = ST_NAN;
+            else if (t <= S->tol2 * S->bb || (S->use_abs && t * S->area <= S->abs2))
+                st = ST_CONVERGED;
+            else if (it + 1 >= max_iter)
+                st = ST_MAXIT;
+            if (lane == 0) {
+                bc_stat = st;
+                ws1[0] = t;
+            }
+        }
+        __syncthreads();
+        beta = bc_val;
+        rho = ws0[0];
+        rr = ws1[0];
+        status = bc_stat;
+        ++it;
+        if (status != ST_RUNNING || it >= it_end) break;
+        __syncthreads();  // ws0 and ws1 are read above and written again below
+    }
+    // x always; r and p for the next launch of the same solve
+    double* pnew = (it & 1) ? a.pb : a.pa;
+#pragma unroll
+    for (int k = 0; k < NU; ++k) {
+        const int u = unit_of(k);
+        if (u >= a.U) break;
+        const int c0 = (u % a.G) * CF_UNIT_COLS, j0 = (u / a.G) * CF_BAND_ROWS;
+#pragma unroll
+        for (int m = 0; m < PC_CPT; ++m) {
+            const int row = row0 + m * (PC_THREADS / CF_UNIT_COLS), cell = row * CF_UNIT_COLS + col;
+            if (!(code[k] >> (16 + m) & 1u)) continue;
+            const size_t o = (size_t)(j0 + row) * a.pitch + c0 + col;
+            a.x[o] = xr[k][m];
+            a.r[o] = R(k)[cell];
+            pnew[o] = P(k)[(row + 1) * PC_PW + col + 1];
+        }
+    }
+    if (blockIdx.x == 0 && tid == 0) {
+        S->iter = it;
+        S->alpha = alpha;
+        S->beta = beta;
+        S->rho = rho;
+        S->rr = rr;
+        S->gbar = gbase + arrived;
+        atomicCAS(&S->status, (int)ST_RUNNING, status);  // a block's timeout stays
+    }
+}
+
+// --------------------------------------------------------------------------
+// host side
+
+template <int NU>
+static cudaError_t launch_pcg64(cf_ctx* c, const Pcg64& a, int blocks) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(PcThreads<NU>::value);
+    cfg.dynamicSmemBytes = sizeof(double) * PC_UNIT * NU;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_pcg64<NU>, a);
+}
+
+template <int NU>
+static bool pcg64_fits(int sms, int blocks) {
+    const int smem = (int)(sizeof(double) * PC_UNIT * NU);
+    int occ = 0;
+    if (cudaFuncSetAttribute(k_pcg64<NU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pcg64<NU>, PcThreads<NU>::value, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return occ * sms >= blocks;
+}
+
+// Units per block of the on-chip solve (0: the grid does not fit), and the
+// border buffer.  A block takes as few units as the SMs allow; up to seven
+// (1064 units on 152 SMs) the vectors fit shared memory, and there the solve
+// is faster than the launch-per-phase kernels at every size (1024^2, seven
+// units: 33.2 against 53.8 us per iteration).
+int pcg64_setup(cf_ctx* c) {
+    c->pcg_nu = 0;
+    const int per = (c->n_units + c->sms - 1) / c->sms;
+    if (per > PC_MAX_UNITS) return CF_OK;
+    const int nu = per <= 1 ? 1 : (per <= 2 ? 2 : (per <= 4 ? 4 : PC_MAX_UNITS));
+    c->pcg_blocks = std::min(c->n_units, c->sms);
+    const bool fits = nu == 1   ? pcg64_fits<1>(c->sms, c->pcg_blocks)
+                      : nu == 2 ? pcg64_fits<2>(c->sms, c->pcg_blocks)
+                      : nu == 4 ? pcg64_fits<4>(c->sms, c->pcg_blocks)
+                                : pcg64_fits<PC_MAX_UNITS>(c->sms, c->pcg_blocks);
+    if (!fits) return CF_OK;
+    void* p = nullptr;
+    const size_t bytes = sizeof(double) * PC_BORDER * (size_t)c->n_units;
+    if (cudaMalloc(&p, bytes) != cudaSuccess) return fail(c, CF_ERR_NOMEM, "cudaMalloc of %zu bytes failed", bytes);
+    c->allocs.push_back(p);
+    c->pcg_border = static_cast<double*>(p);
+    c->pcg_nu = nu;
+    return CF_OK;
+}
+
+// up to iters Jacobi-PCG iterations in one launch (context with pcg_nu > 0)
+cudaError_t pcg64_launch(cf_ctx* c, const Stencil& st, int iters) {
+    Pcg64 a{};
+    a.nx = c->ph.nx;
+    a.ny = c->ph.ny;
+    a.per_x = c->ph.per_x;
+    a.per_y = c->ph.per_y;
+    a.G = c->G;
+    a.U = c->n_units;
+    a.pitch = c->vpitch;
+    a.st = st;
+    a.x = c->x.a;
+    a.r = c->r.a;
+    a.pa = c->pa.a;
+    a.pb = c->pb.a;
+    a.border = c->pcg_border;
+    a.partA = c->partials;
+    a.partB0 = c->partials + c->n_units;
+    a.partB1 = c->partials + 2 * (size_t)c->n_units;
+    a.S = c->S;
+    a.iters = iters;
+    switch (c->pcg_nu) {
+        case 1: return launch_pcg64<1>(c, a, c->pcg_blocks);
+        case 2: return launch_pcg64<2>(c, a, c->pcg_blocks);
+        case 4: return launch_pcg64<4>(c, a, c->pcg_blocks);
+        default: return launch_pcg64<PC_MAX_UNITS>(c, a, c->pcg_blocks);
+    }
+}
+
+}  // namespace cf

@@ -1573,10 +1573,18 @@ static int launch_mixed_mg_step(cf_ctx* c, const Stencil& st) {
 static const int kBatch = CF_CG_BATCH;  // CG iterations per graph launch
 static const int kBatchMG = 4;          // MG-PCG iterations per graph launch
 
-// kBatch Jacobi-PCG iterations (the body of the batch graph)
-static void batch_cg(cf_ctx* c, const Stencil& st, bool mixed) {
+// The FP64 Jacobi-PCG runs on chip (cf_pcg.cu) where the grid fits; with
+// graphs off (cf_set_graphs) every phase stays a launch of its own.
+static bool onchip64(const cf_ctx* c) { return c->pcg_nu > 0 && !c->direct; }
+
+// kBatch Jacobi-PCG iterations (the body of the batch graph); returns the
+// kernels launched
+static int batch_cg(cf_ctx* c, const Stencil& st, bool mixed) {
     if (mixed) {
         for (int i = 0; i < kBatch; ++i) cg32_launch_iteration(c, st);
+    } else if (onchip64(c)) {
+        pcg64_launch(c, st, kBatch);
+        return 1;
     } else {
         const int nb = red_blocks(c);
         Cg64 a = cg64_args(c, st);
@@ -1585,6 +1593,7 @@ static void batch_cg(cf_ctx* c, const Stencil& st, bool mixed) {
             k_cg_update64<<<nb, CF_RED_THREADS, 0, c->stream>>>(a);
         }
     }
+    return 2 * kBatch;
 }
 
 // kBatchMG MG-PCG iterations: K1 (z-mode), K2, V-cycle, r.z (mixed: the
@@ -1718,6 +1727,9 @@ static int read_state(cf_ctx* c) {
 //   tail : [mixed: double-float x to FP64], gradient subtraction, ||div u||,
 //          copies of the solver state and the norms to pinned host memory
 static const int kResidentBatch = 16;    // Jacobi-PCG iterations per trip
+// the same of the on-chip solve, one launch per trip (bounds one launch to a
+// few milliseconds; loading and storing the vectors costs about one iteration)
+static const int kResidentBatchOnchip = 512;
 static const int kResidentBatchMG = 1;   // MG-PCG iterations per trip
 
 // after each resident projection: count the solves that did not converge
@@ -1749,6 +1761,10 @@ static int launch_iterations(cf_ctx* c, const Stencil& st, bool mixed, bool mg, 
     const int nb = red_blocks(c);
     const double scale = -st.ms;
     int k = 0;
+    if (!mixed && !mg && onchip64(c)) {
+        pcg64_launch(c, st, kResidentBatchOnchip);
+        return 1;
+    }
     Cg64 a = cg64_args(c, st);
     if (mg && !mixed) {
         a.mg = 1;
@@ -2175,7 +2191,7 @@ int project_grids(cf_ctx* c, double dt, const SolveOpts& o, SolveResult* res, Gr
         if (warm) c->launches += launch_warm_init(c, st, false);
         const int batch = mg ? kBatchMG : kBatch;
         cudaGraphExec_t ge = mg ? c->gmg : c->g64;
-        const int per_batch = mg ? c->gmg_per_iter * kBatchMG : 2 * kBatch;
+        const int per_batch = mg ? c->gmg_per_iter * kBatchMG : (onchip64(c) ? 1 : 2 * kBatch);
         if (mg) {
             if ((rc = launch_batch(c, c->gmg_pre, [&] { batch_mg_pre(c, st); }))) return rc;
             c->launches += c->gmg_pre_launches;
