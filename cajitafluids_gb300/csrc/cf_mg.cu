@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <vector>
 
@@ -69,9 +70,9 @@ __device__ __forceinline__ float mg_fma(float a, float b, float c) { return fmaf
 __device__ __forceinline__ bool block_live(const SolverState* S, int inner) {
     __shared__ int live;
     if (threadIdx.x == 0 && threadIdx.y == 0) {
-        int ok = *(volatile const int*)&S->status == ST_RUNNING;
-        if (inner) ok = ok && *(volatile const int*)&S->inner_status == ST_RUNNING;
-        live = ok;
+        // both words at once: one trip to L2, not two in turn
+        const int st = *(volatile const int*)&S->status, ist = *(volatile const int*)&S->inner_status;
+        live = st == ST_RUNNING && (!inner || ist == ST_RUNNING);
     }
     __syncthreads();
     return live != 0;
@@ -1025,179 +1026,7 @@ struct FtRows<double> {
     static constexpr int value = 24;
 };
 
-// ---------------------------------------------------------------------------
-// Bottom of the V-cycle in one CTA: every level with at most MgBottomMax
-// cells, from the restricted right-hand side of the first of them down to the
-// coarsest and back, in shared memory.  The per-cell arithmetic is the same as
-// in the grid kernels above (same formulas and order), so the result is the
-// same as that of the level-by-level launches; each phase ends at a barrier.
-// Levels up to 32^2 go to the one CTA: a 64^2 level's eleven phases there
-// (2048 cells per half sweep on one SM) took longer than its two tile
-// launches (8 CTAs each), in FP32 as in FP64.
-template <typename T>
-struct MgBottomMax {
-    static constexpr int value = 1024;
-};
-constexpr int MG_BOTTOM_LEVELS = 6;
-constexpr int MG_BOTTOM_THREADS = 1024;
-
-template <typename T>
-struct MgBottom {
-    MgLev<T> lev[MG_BOTTOM_LEVELS];  // lev[0]: b read from and x written to global memory
-    int off[MG_BOTTOM_LEVELS];       // shared-memory offsets (elements) of x, b, r: off, off + n, off + 2n
-    int nlev;
-};
-
-template <typename T>
-__device__ __forceinline__ T gs_cell(const MgBc& p, const T* x, int nx, int ny, int gi, int gj, T bval, T scale,
-                                     const T* invd, bool first) {
-    T s;
-    if (first) {
-        s = T(0);
-    } else {
-        s = mg_at(p, x, nx, nx, ny, gi - 1, gj) + mg_at(p, x, nx, nx, ny, gi + 1, gj);
-        s = s + mg_at(p, x, nx, nx, ny, gi, gj - 1);
-        s = s + mg_at(p, x, nx, nx, ny, gi, gj + 1);
-    }
-    T t = mg_fma(scale, s, bval);
-    return t * invd[mg_bits(p, nx, ny, gi, gj)];
-}
-
-template <typename T>
-__global__ void __launch_bounds__(MG_BOTTOM_THREADS) k_mg_bottom(MgBottom<T> P, MgBc p, SolverState* S, int inner) {
-    if (!block_live(S, inner)) return;
-    extern __shared__ __align__(16) unsigned char mg_smem[];
-    T* sm = reinterpret_cast<T*>(mg_smem);
-    // 32 x 32 threads: tx walks columns (or column pairs), ty rows
-    const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
-    auto X = [&](int l) { return sm + P.off[l]; };
-    auto B = [&](int l) { return sm + P.off[l] + P.lev[l].nx * P.lev[l].ny; };
-    auto R = [&](int l) { return sm + P.off[l] + 2 * P.lev[l].nx * P.lev[l].ny; };
-    {
-        const MgLev<T>& G = P.lev[0];
-        T* b = B(0);
-        for (int gj = ty; gj < G.ny; gj += 32)
-            for (int gi = tx; gi < G.nx; gi += 32) b[gj * G.nx + gi] = G.b[(size_t)gj * G.pitch + gi];
-    }
-    __syncthreads();
-    auto half = [&](int l, int color, bool first) {
-        const MgLev<T>& L = P.lev[l];
-        T* x = X(l);
-        const T* b = B(l);
-        const int pairs = (L.nx + 1) / 2;
-        for (int gj = ty; gj < L.ny; gj += 32) {
-            const int par = (gj + color) & 1;
-            for (int pr = tx; pr < pairs; pr += 32) {
-                const int gi = 2 * pr + par, go = 2 * pr + 1 - par;
-                if (gi < L.nx)
-                    x[gj * L.nx + gi] = gs_cell(p, x, L.nx, L.ny, gi, gj, b[gj * L.nx + gi], L.scale, L.invd, first);
-                if (first && go < L.nx) x[gj * L.nx + go] = T(0);
-            }
-        }
-        __syncthreads();
-    };
-    auto residual = [&](int l) {
-        const MgLev<T>& L = P.lev[l];
-        const T* x = X(l);
-        const T* b = B(l);
-        T* r = R(l);
-        for (int gj = ty; gj < L.ny; gj += 32)
-            for (int gi = tx; gi < L.nx; gi += 32) {
-                const int k = gj * L.nx + gi;
-                T ax = L.diag[mg_bits(p, L.nx, L.ny, gi, gj)] * x[k];
-                ax = mg_fma(L.ms, mg_at(p, x, L.nx, L.nx, L.ny, gi - 1, gj), ax);
-                ax = mg_fma(L.ms, mg_at(p, x, L.nx, L.nx, L.ny, gi + 1, gj), ax);
-                ax = mg_fma(L.ms, mg_at(p, x, L.nx, L.nx, L.ny, gi, gj - 1), ax);
-                ax = mg_fma(L.ms, mg_at(p, x, L.nx, L.nx, L.ny, gi, gj + 1), ax);
-                r[k] = b[k] - ax;
-            }
-        __syncthreads();
-    };
-    auto restrict_to = [&](int l) {
-        const MgLev<T>& F = P.lev[l];
-        const MgLev<T>& C = P.lev[l + 1];
-        const T* fr = R(l);
-        T* cb = B(l + 1);
-        for (int J = ty; J < C.ny; J += 32)
-            for (int I = tx; I < C.nx; I += 32) {
-                T acc = T(0);
-                for (int fy0 = 2 * J - 1; fy0 <= 2 * J + 2; ++fy0) {
-                    int fy = fy0;
-                    if (fy < 0 || fy >= F.ny) {
-                        if (!p.per_y) continue;
-                        fy = fy < 0 ? fy + F.ny : fy - F.ny;
-                    }
-                    const T wy = (T)mg_pwq(fy, J, C.ny, p.per_y, p.bc[1], p.bc[3]) * T(0.25);
-                    T rs = T(0);
-                    for (int fx0 = 2 * I - 1; fx0 <= 2 * I + 2; ++fx0) {
-                        int fx = fx0;
-                        if (fx < 0 || fx >= F.nx) {
-                            if (!p.per_x) continue;
-                            fx = fx < 0 ? fx + F.nx : fx - F.nx;
-                        }
-                        const T wx = (T)mg_pwq(fx, I, C.nx, p.per_x, p.bc[0], p.bc[2]) * T(0.25);
-                        rs = mg_fma(wx, fr[fy * F.nx + fx], rs);
-                    }
-                    acc = mg_fma(wy, rs, acc);
-                }
-                cb[J * C.nx + I] = T(0.25) * acc;
-            }
-        __syncthreads();
-    };
-    auto prolong_from = [&](int l) {  // x_l += P x_{l+1}
-        const MgLev<T>& F = P.lev[l];
-        const MgLev<T>& C = P.lev[l + 1];
-        const T* cx = X(l + 1);
-        T* fxs = X(l);
-        for (int fy = ty; fy < F.ny; fy += 32)
-            for (int fx = tx; fx < F.nx; fx += 32) {
-                int I, NI, J, NJ;
-                T wxI, wxN, wyJ, wyN;
-                mg_axis<T>(fx, C.nx, p.per_x, p.bc[0], p.bc[2], I, NI, wxI, wxN);
-                mg_axis<T>(fy, C.ny, p.per_y, p.bc[1], p.bc[3], J, NJ, wyJ, wyN);
-                T row0 = wxI * cx[J * C.nx + I];
-                if (NI >= 0) row0 = mg_fma(wxN, cx[J * C.nx + NI], row0);
-                T v = wyJ * row0;
-                if (NJ >= 0) {
-                    T row1 = wxI * cx[NJ * C.nx + I];
-                    if (NI >= 0) row1 = mg_fma(wxN, cx[NJ * C.nx + NI], row1);
-                    v = mg_fma(wyN, row1, v);
-                }
-                fxs[fy * F.nx + fx] = fxs[fy * F.nx + fx] + v;
-            }
-        __syncthreads();
-    };
-    const int nb = P.nlev;
-    for (int l = 0; l < nb - 1; ++l) {
-        for (int k = 0; k < MG_NU; ++k) {
-            half(l, 0, k == 0);
-            half(l, 1, false);
-        }
-        residual(l);
-        restrict_to(l);
-    }
-    for (int k = 0; k < MG_NC; ++k) {
-        half(nb - 1, 0, k == 0);
-        half(nb - 1, 1, false);
-    }
-    for (int k = 0; k < MG_NC; ++k) {
-        half(nb - 1, 1, false);
-        half(nb - 1, 0, false);
-    }
-    for (int l = nb - 2; l >= 0; --l) {
-        prolong_from(l);
-        for (int k = 0; k < MG_NU; ++k) {
-            half(l, 1, false);
-            half(l, 0, false);
-        }
-    }
-    {
-        const MgLev<T>& G = P.lev[0];
-        const T* x = X(0);
-        for (int gj = ty; gj < G.ny; gj += 32)
-            for (int gi = tx; gi < G.nx; gi += 32) G.x[(size_t)gj * G.pitch + gi] = x[gj * G.nx + gi];
-    }
-}
+#include "cf_mgc.cuh"
 
 // --------------------------------------------------------------------------
 // host side: hierarchy and the V-cycle launch sequence
@@ -1217,22 +1046,6 @@ static void level_tables(const cf_ctx* c, double scale, MgLev<T>& L) {
     L.ms = (T)(-1.0 * scale);
 }
 
-// first level handled by the one-CTA bottom solver (nlev when none is small
-// enough) and the bytes of shared memory it needs
-template <typename T>
-static int bottom_level(const MgLev<T>* lev, int nlev, size_t* smem) {
-    int lb = nlev;
-    for (int l = 0; l < nlev; ++l)
-        if ((long long)lev[l].nx * lev[l].ny <= MgBottomMax<T>::value && nlev - l <= MG_BOTTOM_LEVELS) {
-            lb = l;
-            break;
-        }
-    size_t n = 0;
-    for (int l = lb; l < nlev; ++l) n += 3 * (size_t)lev[l].nx * lev[l].ny;
-    *smem = n * sizeof(T);
-    return lb;
-}
-
 struct MgHierarchy {
     int nlev = 0;
     int fused = -1;  // 1: all levels fused, 0: none, -1: by level (see vcycle)
@@ -1242,6 +1055,11 @@ struct MgHierarchy {
     MgLev<float> f[16];
     double* z64 = nullptr;
     float* r32s = nullptr;  // level-0 residual scratch (mixed)
+    // the cluster launch of the coarse levels (cf_mgc.cuh): its first level
+    // (nlev: none, the coarsest level is too large for one CTA), CTAs, bytes of
+    // shared memory
+    int lc = 0, cluster = 0;
+    size_t csmem = 0;
     std::vector<void*> allocs;
 };
 
@@ -1250,6 +1068,83 @@ static int mg_alloc(cf_ctx* c, MgHierarchy* H, void** p, size_t bytes) {
     if (e != cudaSuccess) return fail(c, CF_ERR_NOMEM, "multigrid: cudaMalloc of %zu bytes failed", bytes);
     H->allocs.push_back(*p);
     return cuda_check(c, cudaMemsetAsync(*p, 0, bytes, c->stream), "multigrid memset");
+}
+
+constexpr size_t MC_SMEM_MAX = 200 * 1024;
+constexpr int MC_CLUSTER = 16;  // CTAs (opt-in size; 8, the portable size, where 16 do not fit)
+
+template <typename T>
+static cudaError_t launch_coarse(const MgCoarse<T>& P, const MgBc& p, SolverState* S, int inner, int cluster,
+                                 size_t smem, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(cluster);
+    cfg.blockDim = dim3(MC_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cluster;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_mg_coarse<T>, P, p, S, inner);
+}
+
+// whether a cluster of that many CTAs with that much shared memory can run
+template <typename T>
+static bool cluster_fits(int cluster, size_t smem) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(cluster);
+    cfg.blockDim = dim3(MC_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cluster;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_mg_coarse<T>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return n >= 1;
+}
+
+// The first level of the cluster launch: the first of at most McMax::first
+// cells whose bands fit shared memory (with CF_MG_FUSED=0 the first of at
+// most 1024 cells).  The finest FP32 level stays a tile launch, whose epilogue
+// forms r.z.  No such launch when the coarsest level has more than 1024 cells.
+template <typename T>
+static int coarse_setup(cf_ctx* c, MgHierarchy* H, const MgLev<T>* lev) {
+    const int nlev = H->nlev;
+    H->lc = nlev;
+    if ((long long)lev[nlev - 1].nx * lev[nlev - 1].ny > MC_COARSEST) return CF_OK;
+    int rc = cuda_check(c, cudaFuncSetAttribute(k_mg_coarse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)MC_SMEM_MAX),
+                        "multigrid coarse levels: shared memory");
+    if (!rc)
+        rc = cuda_check(c, cudaFuncSetAttribute(k_mg_coarse<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
+                        "multigrid coarse levels: cluster size");
+    const long long most = H->fused == 0 ? MC_COARSEST : McMax<T>::first;
+    for (int l = 0; l < nlev && !rc; ++l) {
+        const long long cells = (long long)lev[l].nx * lev[l].ny;
+        if (cells > most || nlev - l > MC_LEVELS) continue;
+        if (sizeof(T) == 4 && l == 0 && nlev > 1) continue;
+        for (int cl : {MC_CLUSTER, MC_CLUSTER / 2}) {
+            MgCoarse<T> P{};
+            const size_t smem = mg_coarse_layout(lev + l, nlev - l, cl, &P);
+            const int n = P.ns > 0 ? cl : 1;
+            if (!smem || smem > MC_SMEM_MAX || !cluster_fits<T>(n, smem)) continue;
+            H->lc = l;
+            H->cluster = n;
+            H->csmem = smem;
+            return CF_OK;
+        }
+    }
+    return rc;
 }
 
 // Halve a level while both axes are even and at least 16, and the halved
@@ -1302,18 +1197,7 @@ int mg_setup(cf_ctx* c) {
         nx /= 2;
         ny /= 2;
     }
-    if (!rc) {
-        size_t smem = 0;
-        if (mixed)
-            bottom_level(H->f, H->nlev, &smem);
-        else
-            bottom_level(H->d, H->nlev, &smem);
-        cudaError_t e = mixed ? cudaFuncSetAttribute(k_mg_bottom<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)smem)
-                              : cudaFuncSetAttribute(k_mg_bottom<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)smem);
-        rc = cuda_check(c, e, "multigrid bottom solver shared memory");
-    }
+    if (!rc) rc = mixed ? coarse_setup(c, H, H->f) : coarse_setup(c, H, H->d);
     return rc;
 }
 
@@ -1387,8 +1271,9 @@ int mg_strip_geometry(int nx, int ny, int tw, int th, int strip_rows, int pre, i
 }
 
 template <typename T>
-static int vcycle(cf_ctx* c, MgLev<T>* lev, int nlev, double scale0, int inner, int fused, int strip_rows,
+static int vcycle(cf_ctx* c, const MgHierarchy* H, MgLev<T>* lev, double scale0, int inner, int strip_rows,
                   double* epi_part, bool* epi_done) {
+    const int nlev = H->nlev, fused = H->fused;
     MgBc p{c->ph.per_x, c->ph.per_y, {c->ph.bc[0], c->ph.bc[1], c->ph.bc[2], c->ph.bc[3]}};
     double s = scale0;
     for (int l = 0; l < nlev; ++l) {
@@ -1404,8 +1289,7 @@ static int vcycle(cf_ctx* c, MgLev<T>* lev, int nlev, double scale0, int inner, 
         k_mg_smooth<T><<<grid2((L.nx + 1) / 2, L.ny), blk, 0, c->stream>>>(L, p, color, first, c->S, inner);
         ++launches;
     };
-    size_t smem = 0;
-    const int lb = bottom_level(lev, nlev, &smem);
+    const int lb = H->lc;
     const int top_end = lb < nlev ? lb : nlev - 1;  // levels smoothed by grid kernels on the way down
     constexpr int TH = FtRows<T>::value;
     auto big = [&](const MgLev<T>& L) { return (long long)((L.nx + 63) / 64) * ((L.ny + TH - 1) / TH) >= 1024; };
@@ -1438,15 +1322,25 @@ static int vcycle(cf_ctx* c, MgLev<T>* lev, int nlev, double scale0, int inner, 
         launches += 2;
     }
     if (lb < nlev) {
-        MgBottom<T> P{};
-        P.nlev = nlev - lb;
-        int off = 0;
+        MgCoarse<T> P{};
+        mg_coarse_layout(lev + lb, nlev - lb, H->cluster, &P);
+        P.solid = (p.bc[0] == CF_BC_SOLID ? 1 : 0) | (p.bc[2] == CF_BC_SOLID ? 2 : 0) |
+                  (p.bc[1] == CF_BC_SOLID ? 4 : 0) | (p.bc[3] == CF_BC_SOLID ? 8 : 0);
         for (int l = 0; l < P.nlev; ++l) {
-            P.lev[l] = lev[lb + l];
-            P.off[l] = off;
-            off += 3 * lev[lb + l].nx * lev[lb + l].ny;
+            const MgLev<T>& L = lev[lb + l];
+            P.scale[l] = L.scale;
+            P.ms[l] = L.ms;
+            // (level_tables subtracts the scale once per SOLID side)
+            for (int b = 0; b < 16; ++b) {
+                const int k = __builtin_popcount(b & P.solid);
+                P.dv[l][k] = L.diag[b];
+                P.dv[l][5 + k] = L.invd[b];
+            }
         }
-        k_mg_bottom<T><<<1, MG_BOTTOM_THREADS, smem, c->stream>>>(P, p, c->S, inner);
+        P.gb = lev[lb].b;
+        P.gx = lev[lb].x;
+        P.gpitch = lev[lb].pitch;
+        launch_coarse(P, p, c->S, inner, H->cluster, H->csmem, c->stream);
         ++launches;
     } else {
         // coarsest level too large for one CTA: sweeps by grid kernels
@@ -1496,10 +1390,10 @@ int mg_vcycle(cf_ctx* c, double scale0, bool* rz_done) {
     bool done = false;
     int n;
     if (c->precision == CF_PREC_MIXED)
-        n = vcycle<float>(c, H->f, H->nlev, scale0, 1, H->fused, H->strip_rows,
+        n = vcycle<float>(c, H, H->f, scale0, 1, H->strip_rows,
                           rz_done && H->rz_fused ? c->partials : nullptr, &done);
     else
-        n = vcycle<double>(c, H->d, H->nlev, scale0, 0, H->fused, 0, nullptr, &done);
+        n = vcycle<double>(c, H, H->d, scale0, 0, 0, nullptr, &done);
     if (rz_done) *rz_done = done;
     return n;
 }
