@@ -197,6 +197,87 @@ __device__ __forceinline__ double final_max(const double* partial, int n) {
     return tot;
 }
 
+// FP64 kernels take one reduction unit per block of 256 threads: an SM executes
+// one FP64 warp instruction per sub-partition every 64 cycles, so a unit per
+// warp (eight units, 8192 cells, on one SM) takes 25 us however small the grid.
+// Measured, unit per warp and unit per block: the direction and matvec kernel
+// 26.6 and 10.5 us at 192x160 (30 units), 33.3 and 25.8 us at 1024^2, the update
+// 17.9 and 9.0, 20.9 and 23.1 us; at 4096^2 246 and 269 us, 182 and 147 us (the
+// update without r.z under multigrid), bound by the FP64 pipe either way.
+// Thread t owns column t % 64 of rows t / 64 + 4 m, m = 0 .. 3; the lane sums
+// of the canonical order are added by one warp from the factors staged in
+// shared memory.
+constexpr int UNIT_CELLS = CF_UNIT_COLS * CF_BAND_ROWS;
+constexpr int UNIT_PW = CF_UNIT_COLS + 2;              // row stride of a unit with its halo
+constexpr int UNIT_P = UNIT_PW * (CF_BAND_ROWS + 2);
+constexpr int UNIT_BORDER = 2 * CF_UNIT_COLS + 2 * CF_BAND_ROWS;  // halo cells
+constexpr int UNIT_CPT = UNIT_CELLS / CF_RED_THREADS;  // cells per thread
+constexpr int UNIT_BLOCKS = 8;  // resident blocks per SM the unit kernels are compiled for (the update: half)
+constexpr int UNIT_ROWSTEP = CF_RED_THREADS / CF_UNIT_COLS;
+
+// The warp that adds a unit's lane sums.  The units an SM works on at a time (a
+// multiple of the SM count apart) put their serial sums on different
+// sub-partitions.
+__device__ __forceinline__ int unit_warp(int unit) { return (unit + (unit >> 3)) & 3; }
+
+struct UnitPos {
+    int c0, j0, nc, nr;  // first column and row; columns and rows in the grid
+};
+__device__ __forceinline__ UnitPos unit_pos(int unit, int G, int nx, int ny) {
+    UnitPos u;
+    u.c0 = (unit % G) * CF_UNIT_COLS;
+    u.j0 = (unit / G) * CF_BAND_ROWS;
+    u.nc = min(CF_UNIT_COLS, nx - u.c0);
+    u.nr = min(CF_BAND_ROWS, ny - u.j0);
+    return u;
+}
+
+// Halo cell t < UNIT_BORDER of a unit: the row below, the row above, the column
+// to the west, the column to the east.  False when the unit has no such cell;
+// (gc, gj) may lie outside the grid.  pos: its place in the unit with its halo
+// (row r, column c of the unit at (r + 1) UNIT_PW + c + 1).
+__device__ __forceinline__ bool unit_halo(const UnitPos& u, int t, int& gc, int& gj, int& pos) {
+    if (t < 2 * CF_UNIT_COLS) {
+        const int cc = t & (CF_UNIT_COLS - 1), up = t / CF_UNIT_COLS;
+        gc = u.c0 + cc;
+        gj = up ? u.j0 + u.nr : u.j0 - 1;
+        pos = (up ? u.nr + 1 : 0) * UNIT_PW + cc + 1;
+        return cc < u.nc;
+    }
+    const int r = (t - 2 * CF_UNIT_COLS) % CF_BAND_ROWS, east = (t - 2 * CF_UNIT_COLS) / CF_BAND_ROWS;
+    gj = u.j0 + r;
+    gc = east ? u.c0 + u.nc : u.c0 - 1;
+    pos = (r + 1) * UNIT_PW + (east ? u.nc + 1 : 0);
+    return r < u.nr;
+}
+
+// A unit's canonical sum of a b, lane l adding its columns 2l and 2l + 1 row by
+// row (row strides sa, sb); cells outside the grid hold b = 0 and a finite a.
+// The next row is read while this row's products are added.
+__device__ __forceinline__ double unit_dot(const double* a, int sa, const double* b, int sb, int lane) {
+    a += 2 * lane;
+    b += 2 * lane;
+    double acc = 0.0;
+    double a0 = a[0], a1 = a[1], b0 = b[0], b1 = b[1];
+#pragma unroll 4
+    for (int j = 0; j < CF_BAND_ROWS; ++j) {
+        double c0 = 0.0, c1 = 0.0, d0 = 0.0, d1 = 0.0;
+        if (j + 1 < CF_BAND_ROWS) {
+            c0 = a[(j + 1) * sa];
+            c1 = a[(j + 1) * sa + 1];
+            d0 = b[(j + 1) * sb];
+            d1 = b[(j + 1) * sb + 1];
+        }
+        acc = fma(a0, b0, acc);
+        acc = fma(a1, b1, acc);
+        a0 = c0;
+        a1 = c1;
+        b0 = d0;
+        b1 = d1;
+    }
+    return warp_fold(acc);
+}
+
 // Wall-adjacency bits of cell (gi, gj); periodic axes have no walls.
 __device__ __forceinline__ int edge_bits(int gi, int gj, int nx, int ny, int per_x, int per_y) {
     int b = 0;

@@ -45,11 +45,8 @@ template <int NU>
 struct PcThreads {
     static constexpr int value = NU <= 2 ? 256 : 512;
 };
-constexpr int PC_PW = CF_UNIT_COLS + 2;                   // row stride of p with its halo
-constexpr int PC_P = PC_PW * (CF_BAND_ROWS + 2);          // doubles of p per unit
-constexpr int PC_CELLS = CF_UNIT_COLS * CF_BAND_ROWS;     // cells per unit
-constexpr int PC_UNIT = PC_P + 2 * PC_CELLS;              // doubles per unit: p, r, q / z
-constexpr int PC_BORDER = 2 * CF_UNIT_COLS + 2 * CF_BAND_ROWS;  // first / last row, first / last column
+constexpr int PC_PW = UNIT_PW, PC_P = UNIT_P, PC_CELLS = UNIT_CELLS, PC_BORDER = UNIT_BORDER;
+constexpr int PC_UNIT = PC_P + 2 * PC_CELLS;  // doubles per unit: p with its halo, r, q / z
 constexpr int PC_MAX_UNITS = 7;                           // units per block (181 KB of shared memory)
 // polls of a grid barrier before the launch gives up (each poll is an L2
 // round trip; a barrier takes a few of them)
@@ -93,33 +90,6 @@ __device__ __forceinline__ double strided_sum(const double* part, int n, int t) 
     double s = 0.0;
     for (int u = t; u < n; u += CF_RED_THREADS) s = s + __ldcg(part + u);
     return s;
-}
-
-// A unit's canonical sum of a.b: lane l, columns 2l and 2l + 1, row by row.
-// Cells outside the grid hold b = 0.  The next row is read while this row's
-// products are added.
-__device__ __forceinline__ double unit_dot(const double* a, int sa, const double* b, int lane) {
-    a += 2 * lane;
-    b += 2 * lane;
-    double acc = 0.0;
-    double a0 = a[0], a1 = a[1], b0 = b[0], b1 = b[1];
-#pragma unroll 4
-    for (int j = 0; j < CF_BAND_ROWS; ++j) {
-        double c0 = 0.0, c1 = 0.0, d0 = 0.0, d1 = 0.0;
-        if (j + 1 < CF_BAND_ROWS) {
-            c0 = a[(j + 1) * sa];
-            c1 = a[(j + 1) * sa + 1];
-            d0 = b[(j + 1) * CF_UNIT_COLS];
-            d1 = b[(j + 1) * CF_UNIT_COLS + 1];
-        }
-        acc = fma(a0, b0, acc);
-        acc = fma(a1, b1, acc);
-        a0 = c0;
-        a1 = c1;
-        b0 = d0;
-        b1 = d1;
-    }
-    return warp_fold(acc);
 }
 
 // Lane 0's warp_fold when only the first n lanes hold values and the others
@@ -200,23 +170,14 @@ __global__ void __launch_bounds__(PcThreads<NU>::value, 1) k_pcg64(Pcg64 a) {
         // halo: row below, row above, column west, column east of the unit's
         // cells in the grid (wrapped along a periodic axis, 0 beyond a wall)
         if (tid < PC_BORDER) {
-            int gc, gj, pos, off;
-            bool in;
-            if (tid < 2 * CF_UNIT_COLS) {
-                const int cc = tid & (CF_UNIT_COLS - 1), up = tid / CF_UNIT_COLS;
-                in = cc < nc;
-                gc = c0 + cc;
-                gj = up ? j0 + nr : j0 - 1;
-                pos = (up ? nr + 1 : 0) * PC_PW + cc + 1;
-                off = (up ? 0 : CF_UNIT_COLS) + cc;  // the owner's first row is above us, its last row below
-            } else {
-                const int rr_ = (tid - 2 * CF_UNIT_COLS) % CF_BAND_ROWS, east = (tid - 2 * CF_UNIT_COLS) / CF_BAND_ROWS;
-                in = rr_ < nr;
-                gj = j0 + rr_;
-                gc = east ? c0 + nc : c0 - 1;
-                pos = (rr_ + 1) * PC_PW + (east ? nc + 1 : 0);
-                off = 2 * CF_UNIT_COLS + (east ? 0 : CF_BAND_ROWS) + rr_;
-            }
+            int gc, gj, pos;
+            const bool in = unit_halo(UnitPos{c0, j0, nc, nr}, tid, gc, gj, pos);
+            // in the owner's border: its last row lies below us, its first row
+            // above, its last column west, its first column east
+            const int off = tid < CF_UNIT_COLS         ? CF_UNIT_COLS + tid
+                            : tid < 2 * CF_UNIT_COLS   ? tid - CF_UNIT_COLS
+                            : tid < 2 * CF_UNIT_COLS + CF_BAND_ROWS ? tid + CF_BAND_ROWS
+                                                                    : tid - CF_BAND_ROWS;
             const int wc = wrap_index(gc, a.nx, a.per_x), wj = wrap_index(gj, a.ny, a.per_y);
             if (in && wc >= 0 && wj >= 0) {
                 const int ou = (wj / CF_BAND_ROWS) * a.G + wc / CF_UNIT_COLS;
@@ -272,7 +233,7 @@ __global__ void __launch_bounds__(PcThreads<NU>::value, 1) k_pcg64(Pcg64 a) {
         }
         __syncthreads();
         if (warp < NU && unit_of(warp) < a.U) {
-            const double s = unit_dot(P(warp) + PC_PW + 1, PC_PW, Q(warp), lane);
+            const double s = unit_dot(P(warp) + PC_PW + 1, PC_PW, Q(warp), CF_UNIT_COLS, lane);
             if (lane == 0) __stcg(a.partA + unit_of(warp), s);
         }
         grid_arrive(S);
@@ -324,7 +285,7 @@ __global__ void __launch_bounds__(PcThreads<NU>::value, 1) k_pcg64(Pcg64 a) {
         for (int c = warp; c < 2 * NU; c += PC_THREADS / 32) {
             const int k = c >> 1, u = unit_of(k);
             if (u >= a.U) break;
-            const double s = unit_dot(R(k), CF_UNIT_COLS, (c & 1) ? R(k) : Q(k), lane);
+            const double s = unit_dot(R(k), CF_UNIT_COLS, (c & 1) ? R(k) : Q(k), CF_UNIT_COLS, lane);
             if (lane == 0) __stcg(((c & 1) ? a.partB1 : a.partB0) + u, s);
         }
         grid_arrive(S);

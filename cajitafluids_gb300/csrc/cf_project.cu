@@ -61,98 +61,77 @@ __device__ __forceinline__ bool converged(const SolverState* S, double rr) {
     return rr <= S->tol2 * S->bb || (S->use_abs && rr * S->area <= S->abs2);
 }
 
-// new search direction at one cell (0 outside a wall)
-__device__ __forceinline__ double pn1(const Cg64& a, const double* pold, int c, int j, bool first, double beta) {
-    int cc = wrap_index(c, a.nx, a.per_x), jj = wrap_index(j, a.ny, a.per_y);
-    if (cc < 0 || jj < 0) return 0.0;
-    size_t k = (size_t)jj * a.pitch + cc;
-    double z = a.mg ? __ldg(a.z + k) : a.st.minv[ebits(a, cc, jj)] * __ldg(a.r + k);
-    return first ? z : fma(beta, __ldg(pold + k), z);
-}
-
-// new search direction at columns c0, c0+1 of row j
-__device__ __forceinline__ double2 pn2(const Cg64& a, const double* pold, int c0, int j, bool first, double beta) {
-    int jj = wrap_index(j, a.ny, a.per_y);
-    if (jj < 0) return make_double2(0.0, 0.0);
-    if (c0 + 1 < a.nx) {
-        size_t k = (size_t)jj * a.pitch + c0;
-        double z0, z1;
-        if (a.mg) {
-            double2 zv = __ldg(reinterpret_cast<const double2*>(a.z + k));
-            z0 = zv.x;
-            z1 = zv.y;
-        } else {
-            double2 rv = __ldg(reinterpret_cast<const double2*>(a.r + k));
-            z0 = a.st.minv[ebits(a, c0, jj)] * rv.x;
-            z1 = a.st.minv[ebits(a, c0 + 1, jj)] * rv.y;
-        }
-        if (first) return make_double2(z0, z1);
-        double2 po = __ldg(reinterpret_cast<const double2*>(pold + k));
-        return make_double2(fma(beta, po.x, z0), fma(beta, po.y, z1));
-    }
-    return make_double2(pn1(a, pold, c0, jj, first, beta), pn1(a, pold, c0 + 1, jj, first, beta));
-}
-
 // K1: direction update + stencil apply + partial p.q
-__global__ void __launch_bounds__(CF_RED_THREADS) k_cg_dir_matvec64(Cg64 a) {
+__global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_cg_dir_matvec64(Cg64 a) {
+    __shared__ double P[UNIT_P], Q[UNIT_CELLS];
+    __shared__ int s_it;
+    __shared__ double s_beta;
     SolverState* S = a.S;
-    if (*(volatile int*)&S->status != ST_RUNNING) return;
-    const int it = S->iter;
+    const int tid = threadIdx.x;
+    if (tid == 0) {
+        s_it = *(volatile int*)&S->status == ST_RUNNING ? S->iter : -1;
+        s_beta = S->beta;
+    }
+    __syncthreads();
+    const int it = s_it;
+    if (it < 0) return;
     const bool first = it == 0;
-    const double beta = S->beta;
+    const double beta = s_beta, ms = a.st.ms;
     const double* pold = (it & 1) ? a.pb : a.pa;
     double* pnew = (it & 1) ? a.pa : a.pb;
-    const double ms = a.st.ms;
-    const int lane = threadIdx.x & 31;
-    const int unit = blockIdx.x * CF_RED_WARPS + (threadIdx.x >> 5);
-    double acc = 0.0;
-    if (unit < a.U) {
-        const int g = unit % a.G, band = unit / a.G;
-        const int c0 = g * CF_UNIT_COLS + 2 * lane;
-        const int j0 = band * CF_BAND_ROWS;
-        const int j1 = min(j0 + CF_BAND_ROWS, a.ny);
-        double2 pm = pn2(a, pold, c0, j0 - 1, first, beta);
-        double2 pc = pn2(a, pold, c0, j0, first, beta);
-        for (int j = j0; j < j1; ++j) {
-            double2 pp = pn2(a, pold, c0, j + 1, first, beta);
-            double left = __shfl_up_sync(FULLMASK, pc.y, 1);
-            double right = __shfl_down_sync(FULLMASK, pc.x, 1);
-            // the two cells just outside the warp's 64 columns, in one branch
-            if (lane == 0 || lane == 31) {
-                double ext = pn1(a, pold, lane == 0 ? c0 - 1 : c0 + 2, j, first, beta);
-                if (lane == 0)
-                    left = ext;
-                else
-                    right = ext;
+    for (int unit = blockIdx.x; unit < a.U; unit += gridDim.x) {
+        if (unit != (int)blockIdx.x) __syncthreads();  // the last unit's sums are done with shared memory
+        const UnitPos u = unit_pos(unit, a.G, a.nx, a.ny);
+        const int col = tid & (CF_UNIT_COLS - 1), row0 = tid / CF_UNIT_COLS;
+        // new search direction at a cell of the grid
+        auto dir = [&](int c, int j) {
+            const size_t k = (size_t)j * a.pitch + c;
+            const double z = a.mg ? __ldg(a.z + k) : a.st.minv[ebits(a, c, j)] * __ldg(a.r + k);
+            return first ? z : fma(beta, __ldg(pold + k), z);
+        };
+#pragma unroll
+        for (int m = 0; m < UNIT_CPT; ++m) {
+            const int row = row0 + m * UNIT_ROWSTEP;
+            double p = 0.0;
+            if (col < u.nc && row < u.nr) {
+                p = dir(u.c0 + col, u.j0 + row);
+                pnew[(size_t)(u.j0 + row) * a.pitch + u.c0 + col] = p;
             }
-            if (c0 < a.nx) {
-                size_t k = (size_t)j * a.pitch + c0;
-                double q0 = a.st.diag[ebits(a, c0, j)] * pc.x;
-                q0 = fma(ms, left, q0);
-                q0 = fma(ms, pc.y, q0);
-                q0 = fma(ms, pm.x, q0);
-                q0 = fma(ms, pp.x, q0);
-                acc = fma(pc.x, q0, acc);
-                if (c0 + 1 < a.nx) {
-                    double q1 = a.st.diag[ebits(a, c0 + 1, j)] * pc.y;
-                    q1 = fma(ms, pc.x, q1);
-                    q1 = fma(ms, right, q1);
-                    q1 = fma(ms, pm.y, q1);
-                    q1 = fma(ms, pp.y, q1);
-                    acc = fma(pc.y, q1, acc);
-                    *reinterpret_cast<double2*>(pnew + k) = pc;
-                    *reinterpret_cast<double2*>(a.qv + k) = make_double2(q0, q1);
-                } else {
-                    pnew[k] = pc.x;
-                    a.qv[k] = q0;
-                }
+            P[(row + 1) * UNIT_PW + col + 1] = p;
+        }
+        double h = 0.0;
+        int gc, gj, pos = 0;
+        const bool halo = tid < UNIT_BORDER && unit_halo(u, tid, gc, gj, pos);
+        if (halo) {
+            gc = wrap_index(gc, a.nx, a.per_x);
+            gj = wrap_index(gj, a.ny, a.per_y);
+            if (gc >= 0 && gj >= 0) h = dir(gc, gj);
+        }
+        // the halo of a unit cut by the grid's edge lies among its cells
+        if (u.nc < CF_UNIT_COLS || u.nr < CF_BAND_ROWS) __syncthreads();
+        if (halo) P[pos] = h;
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < UNIT_CPT; ++m) {
+            const int row = row0 + m * UNIT_ROWSTEP;
+            const double* c = P + (row + 1) * UNIT_PW + col + 1;
+            double q = 0.0;
+            if (col < u.nc && row < u.nr) {
+                q = a.st.diag[ebits(a, u.c0 + col, u.j0 + row)] * c[0];
+                q = fma(ms, c[-1], q);
+                q = fma(ms, c[1], q);
+                q = fma(ms, c[-UNIT_PW], q);
+                q = fma(ms, c[UNIT_PW], q);
+                a.qv[(size_t)(u.j0 + row) * a.pitch + u.c0 + col] = q;
             }
-            pm = pc;
-            pc = pp;
+            Q[row * CF_UNIT_COLS + col] = q;
+        }
+        __syncthreads();
+        if (tid / 32 == unit_warp(unit)) {
+            const double s = unit_dot(P + UNIT_PW + 1, UNIT_PW, Q, CF_UNIT_COLS, tid & 31);
+            if ((tid & 31) == 0) a.part0[unit] = s;
         }
     }
-    acc = warp_fold(acc);
-    if (unit < a.U && lane == 0) a.part0[unit] = acc;
     if (last_block_arrive(&S->ticket[0])) {
         double pq = final_tree(a.part0, a.U);
         if (threadIdx.x == 0) {
@@ -165,62 +144,66 @@ __global__ void __launch_bounds__(CF_RED_THREADS) k_cg_dir_matvec64(Cg64 a) {
     }
 }
 
-// K2: solution / residual update + partial r.z and r.r
-__global__ void __launch_bounds__(CF_RED_THREADS) k_cg_update64(Cg64 a) {
+// K2: solution / residual update + partial r.z (not with the multigrid
+// preconditioner, whose r.z follows its V-cycle) and r.r
+__global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS / 2) k_cg_update64(Cg64 a) {
+    __shared__ double R[UNIT_CELLS], Z[UNIT_CELLS];
+    __shared__ int s_it;
+    __shared__ double s_alpha;
     SolverState* S = a.S;
-    if (*(volatile int*)&S->status != ST_RUNNING) return;
-    const int it = S->iter;
+    const int tid = threadIdx.x;
+    if (tid == 0) {
+        s_it = *(volatile int*)&S->status == ST_RUNNING ? S->iter : -1;
+        s_alpha = S->alpha;
+    }
+    __syncthreads();
+    const int it = s_it;
+    if (it < 0) return;
     const double* pv = (it & 1) ? a.pa : a.pb;
-    const double alpha = S->alpha, malpha = -alpha;
-    const int lane = threadIdx.x & 31;
-    const int unit = blockIdx.x * CF_RED_WARPS + (threadIdx.x >> 5);
-    double arz = 0.0, arr = 0.0;
-    if (unit < a.U) {
-        const int g = unit % a.G, band = unit / a.G;
-        const int c0 = g * CF_UNIT_COLS + 2 * lane;
-        const int j0 = band * CF_BAND_ROWS;
-        const int j1 = min(j0 + CF_BAND_ROWS, a.ny);
-        if (c0 + 1 < a.nx) {
-            for (int j = j0; j < j1; ++j) {
-                size_t k = (size_t)j * a.pitch + c0;
-                double2 xv = *reinterpret_cast<const double2*>(a.x + k);
-                double2 p2 = __ldg(reinterpret_cast<const double2*>(pv + k));
-                double2 rv = *reinterpret_cast<const double2*>(a.r + k);
-                double2 qv = __ldg(reinterpret_cast<const double2*>(a.qv + k));
-                xv.x = fma(alpha, p2.x, xv.x);
-                xv.y = fma(alpha, p2.y, xv.y);
-                rv.x = fma(malpha, qv.x, rv.x);
-                rv.y = fma(malpha, qv.y, rv.y);
-                double z0 = a.st.minv[ebits(a, c0, j)] * rv.x;
-                double z1 = a.st.minv[ebits(a, c0 + 1, j)] * rv.y;
-                arz = fma(rv.x, z0, arz);
-                arr = fma(rv.x, rv.x, arr);
-                arz = fma(rv.y, z1, arz);
-                arr = fma(rv.y, rv.y, arr);
-                *reinterpret_cast<double2*>(a.x + k) = xv;
-                *reinterpret_cast<double2*>(a.r + k) = rv;
-            }
-        } else if (c0 < a.nx) {
-            for (int j = j0; j < j1; ++j) {
-                size_t k = (size_t)j * a.pitch + c0;
-                double xv = fma(alpha, pv[k], a.x[k]);
-                double rv = fma(malpha, a.qv[k], a.r[k]);
-                double z0 = a.st.minv[ebits(a, c0, j)] * rv;
-                arz = fma(rv, z0, arz);
-                arr = fma(rv, rv, arr);
-                a.x[k] = xv;
-                a.r[k] = rv;
+    const double alpha = s_alpha, malpha = -alpha;
+    for (int unit = blockIdx.x; unit < a.U; unit += gridDim.x) {
+        if (unit != (int)blockIdx.x) __syncthreads();  // the last unit's sums are done with shared memory
+        const UnitPos u = unit_pos(unit, a.G, a.nx, a.ny);
+        const int col = tid & (CF_UNIT_COLS - 1), row0 = tid / CF_UNIT_COLS;
+        double xv[UNIT_CPT], pp[UNIT_CPT], rv[UNIT_CPT], qv[UNIT_CPT];
+#pragma unroll
+        for (int m = 0; m < UNIT_CPT; ++m) {
+            const int row = row0 + m * UNIT_ROWSTEP;
+            xv[m] = pp[m] = rv[m] = qv[m] = 0.0;
+            if (col < u.nc && row < u.nr) {
+                const size_t k = (size_t)(u.j0 + row) * a.pitch + u.c0 + col;
+                xv[m] = a.x[k];
+                pp[m] = __ldg(pv + k);
+                rv[m] = a.r[k];
+                qv[m] = __ldg(a.qv + k);
             }
         }
-    }
-    arz = warp_fold(arz);
-    arr = warp_fold(arr);
-    if (unit < a.U && lane == 0) {
-        a.part0[unit] = arz;
-        a.part1[unit] = arr;
+#pragma unroll
+        for (int m = 0; m < UNIT_CPT; ++m) {
+            const int row = row0 + m * UNIT_ROWSTEP, cell = row * CF_UNIT_COLS + col;
+            double r = 0.0, z = 0.0;
+            if (col < u.nc && row < u.nr) {
+                const size_t k = (size_t)(u.j0 + row) * a.pitch + u.c0 + col;
+                a.x[k] = fma(alpha, pp[m], xv[m]);
+                r = fma(malpha, qv[m], rv[m]);
+                a.r[k] = r;
+                if (!a.mg) z = a.st.minv[ebits(a, u.c0 + col, u.j0 + row)] * r;
+            }
+            R[cell] = r;
+            if (!a.mg) Z[cell] = z;
+        }
+        __syncthreads();
+        const int warp = tid / 32, lane = tid & 31;
+        if (warp == unit_warp(unit)) {
+            const double s = unit_dot(R, CF_UNIT_COLS, R, CF_UNIT_COLS, lane);
+            if (lane == 0) a.part1[unit] = s;
+        } else if (!a.mg && warp == unit_warp(unit + 1)) {
+            const double s = unit_dot(R, CF_UNIT_COLS, Z, CF_UNIT_COLS, lane);
+            if (lane == 0) a.part0[unit] = s;
+        }
     }
     if (last_block_arrive(&S->ticket[1])) {
-        double rz = final_tree(a.part0, a.U);
+        double rz = a.mg ? 0.0 : final_tree(a.part0, a.U);
         double rr = final_tree(a.part1, a.U);
         if (threadIdx.x == 0) {
             S->ticket[1] = 0;
@@ -242,34 +225,35 @@ __global__ void __launch_bounds__(CF_RED_THREADS) k_cg_update64(Cg64 a) {
 
 // MG-PCG: rho_new = r.z after the V-cycle, beta = rho_new / rho (init = 1:
 // rho only).  Runs only while the solve is live.
-__global__ void __launch_bounds__(CF_RED_THREADS) k_mg_rz64(Cg64 a, int init) {
+__global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_mg_rz64(Cg64 a, int init) {
+    __shared__ double R[UNIT_CELLS], Z[UNIT_CELLS];
+    __shared__ int s_live;
     SolverState* S = a.S;
-    if (*(volatile int*)&S->status != ST_RUNNING) return;
-    const int lane = threadIdx.x & 31;
-    const int unit = blockIdx.x * CF_RED_WARPS + (threadIdx.x >> 5);
-    double arz = 0.0;
-    if (unit < a.U) {
-        const int g = unit % a.G, band = unit / a.G;
-        const int c0 = g * CF_UNIT_COLS + 2 * lane;
-        const int j0 = band * CF_BAND_ROWS;
-        const int j1 = min(j0 + CF_BAND_ROWS, a.ny);
-        if (c0 + 1 < a.nx) {
-            for (int j = j0; j < j1; ++j) {
-                size_t k = (size_t)j * a.pitch + c0;
-                double2 rv = __ldg(reinterpret_cast<const double2*>(a.r + k));
-                double2 zv = __ldg(reinterpret_cast<const double2*>(a.z + k));
-                arz = fma(rv.x, zv.x, arz);
-                arz = fma(rv.y, zv.y, arz);
+    const int tid = threadIdx.x;
+    if (tid == 0) s_live = *(volatile int*)&S->status == ST_RUNNING;
+    for (int unit = blockIdx.x; unit < a.U; unit += gridDim.x) {
+        if (unit != (int)blockIdx.x) __syncthreads();
+        const UnitPos u = unit_pos(unit, a.G, a.nx, a.ny);
+        const int col = tid & (CF_UNIT_COLS - 1), row0 = tid / CF_UNIT_COLS;
+#pragma unroll
+        for (int m = 0; m < UNIT_CPT; ++m) {
+            const int row = row0 + m * UNIT_ROWSTEP, cell = row * CF_UNIT_COLS + col;
+            double r = 0.0, z = 0.0;
+            if (col < u.nc && row < u.nr) {
+                const size_t k = (size_t)(u.j0 + row) * a.pitch + u.c0 + col;
+                r = __ldg(a.r + k);
+                z = __ldg(a.z + k);
             }
-        } else if (c0 < a.nx) {
-            for (int j = j0; j < j1; ++j) {
-                size_t k = (size_t)j * a.pitch + c0;
-                arz = fma(a.r[k], a.z[k], arz);
-            }
+            R[cell] = r;
+            Z[cell] = z;
+        }
+        __syncthreads();
+        if (!s_live) return;  // (the same answer for every unit)
+        if (tid / 32 == unit_warp(unit)) {
+            const double s = unit_dot(R, CF_UNIT_COLS, Z, CF_UNIT_COLS, tid & 31);
+            if ((tid & 31) == 0) a.part0[unit] = s;
         }
     }
-    arz = warp_fold(arz);
-    if (unit < a.U && lane == 0) a.part0[unit] = arz;
     if (last_block_arrive(&S->ticket[7])) {
         double rz = final_tree(a.part0, a.U);
         if (threadIdx.x == 0) {
@@ -280,67 +264,74 @@ __global__ void __launch_bounds__(CF_RED_THREADS) k_mg_rz64(Cg64 a, int init) {
     }
 }
 
+// the state a solve starts from (||b||^2 in S->bb)
+__device__ __forceinline__ void start_solve64(SolverState* S, double rr, double rz) {
+    S->rr = rr;
+    S->rho = rz;
+    S->beta = 0.0;
+    S->iter = 0;
+    if (S->bb == 0.0 || converged(S, rr))
+        S->status = ST_CONVERGED;
+    else if (S->max_iter <= 0)
+        S->status = ST_MAXIT;
+    else if (isnan(rr))
+        S->status = ST_NAN;
+    else
+        S->status = ST_RUNNING;
+}
+
 // Warm start (FP64): r = b - A x from the previous solution, with A x in the
 // matvec's order (diag x_C, then the W, E, S, N legs), canonical r.z and r.r,
 // and the solver state as the cold init sets it (||b||^2 from k_div_init64).
-__global__ void __launch_bounds__(CF_RED_THREADS) k_warm_resid64(Cg64 a) {
+__global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_warm_resid64(Cg64 a) {
+    __shared__ double R[UNIT_CELLS], Z[UNIT_CELLS];
     SolverState* S = a.S;
-    const int lane = threadIdx.x & 31;
-    const int unit = blockIdx.x * CF_RED_WARPS + (threadIdx.x >> 5);
-    const double ms = a.st.ms;
-    double arz = 0.0, arr = 0.0;
-    if (unit < a.U) {
-        const int g = unit % a.G, band = unit / a.G;
-        const int c0 = g * CF_UNIT_COLS + 2 * lane;
-        const int j0 = band * CF_BAND_ROWS;
-        const int j1 = min(j0 + CF_BAND_ROWS, a.ny);
+    const int tid = threadIdx.x;
+    for (int unit = blockIdx.x; unit < a.U; unit += gridDim.x) {
+        if (unit != (int)blockIdx.x) __syncthreads();  // the last unit's sums are done with shared memory
+        const UnitPos u = unit_pos(unit, a.G, a.nx, a.ny);
+        const int col = tid & (CF_UNIT_COLS - 1), row0 = tid / CF_UNIT_COLS;
+        const double ms = a.st.ms;
         auto xv = [&](int c, int j) -> double {
             int cc = wrap_index(c, a.nx, a.per_x), jj = wrap_index(j, a.ny, a.per_y);
             if (cc < 0 || jj < 0) return 0.0;
             return a.x[(size_t)jj * a.pitch + cc];
         };
-        for (int j = j0; j < j1; ++j)
 #pragma unroll
-            for (int s = 0; s < 2; ++s) {
-                const int c = c0 + s;
-                if (c >= a.nx) continue;
-                const int eb = ebits(a, c, j);
+        for (int m = 0; m < UNIT_CPT; ++m) {
+            const int row = row0 + m * UNIT_ROWSTEP, cell = row * CF_UNIT_COLS + col;
+            double r = 0.0, z = 0.0;
+            if (col < u.nc && row < u.nr) {
+                const int c = u.c0 + col, j = u.j0 + row, eb = ebits(a, c, j);
                 double ax = a.st.diag[eb] * xv(c, j);
                 ax = fma(ms, xv(c - 1, j), ax);
                 ax = fma(ms, xv(c + 1, j), ax);
                 ax = fma(ms, xv(c, j - 1), ax);
                 ax = fma(ms, xv(c, j + 1), ax);
                 const size_t k = (size_t)j * a.pitch + c;
-                const double r = a.r[k] - ax;
+                r = a.r[k] - ax;
                 a.r[k] = r;
-                const double z = a.st.minv[eb] * r;
-                arz = fma(r, z, arz);
-                arr = fma(r, r, arr);
+                z = a.st.minv[eb] * r;
             }
-    }
-    arz = warp_fold(arz);
-    arr = warp_fold(arr);
-    if (unit < a.U && lane == 0) {
-        a.part0[unit] = arz;
-        a.part1[unit] = arr;
+            R[cell] = r;
+            Z[cell] = z;
+        }
+        __syncthreads();
+        const int warp = tid / 32, lane = tid & 31;
+        if (warp == unit_warp(unit)) {
+            const double s = unit_dot(R, CF_UNIT_COLS, R, CF_UNIT_COLS, lane);
+            if (lane == 0) a.part1[unit] = s;
+        } else if (warp == unit_warp(unit + 1)) {
+            const double s = unit_dot(R, CF_UNIT_COLS, Z, CF_UNIT_COLS, lane);
+            if (lane == 0) a.part0[unit] = s;
+        }
     }
     if (last_block_arrive(&S->ticket[3])) {
         double rz = final_tree(a.part0, a.U);
         double rr = final_tree(a.part1, a.U);
         if (threadIdx.x == 0) {
             S->ticket[3] = 0;
-            S->rr = rr;
-            S->rho = rz;
-            S->beta = 0.0;
-            S->iter = 0;
-            if (S->bb == 0.0 || converged(S, rr))
-                S->status = ST_CONVERGED;
-            else if (S->max_iter <= 0)
-                S->status = ST_MAXIT;
-            else if (isnan(rr))
-                S->status = ST_NAN;
-            else
-                S->status = ST_RUNNING;
+            start_solve64(S, rr, rz);
         }
     }
 }
@@ -358,7 +349,6 @@ struct DivArgs {
     double* out;
     SolverState* S;
     int warm;  // keep x from the previous solve (warm start) instead of x = 0
-    int mixed;        // k_div_norms: squares and magnitudes in FP32
     float mscale32;   // -(1/dx) in FP32
     float2 mscale2;   // -(1/dx) as a double-float pair
     // k_div_init_mixed (when set): the faces k_apply_pairs_norms cannot read
@@ -405,35 +395,38 @@ __device__ __forceinline__ void put_r32(float* o, int pitch, int nx, int ny, int
 // (df_add, df_mul, df_split and df_value: cf_internal.cuh)
 
 // FP64 init: b, r = b, x = 0, partial r.z and r.r
-__global__ void __launch_bounds__(CF_RED_THREADS) k_div_init64(DivArgs a) {
+__global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_div_init64(DivArgs a) {
+    __shared__ double R[UNIT_CELLS], Z[UNIT_CELLS];
     SolverState* S = a.S;
-    const int lane = threadIdx.x & 31;
-    const int unit = blockIdx.x * CF_RED_WARPS + (threadIdx.x >> 5);
-    double arz = 0.0, arr = 0.0;
-    if (unit < a.U) {
-        const int g = unit % a.G, band = unit / a.G;
-        const int c0 = g * CF_UNIT_COLS + 2 * lane;
-        const int j0 = band * CF_BAND_ROWS;
-        const int j1 = min(j0 + CF_BAND_ROWS, a.ny);
-        for (int j = j0; j < j1; ++j)
+    const int tid = threadIdx.x;
+    for (int unit = blockIdx.x; unit < a.U; unit += gridDim.x) {
+        if (unit != (int)blockIdx.x) __syncthreads();  // the last unit's sums are done with shared memory
+        const UnitPos u = unit_pos(unit, a.G, a.nx, a.ny);
+        const int col = tid & (CF_UNIT_COLS - 1), row0 = tid / CF_UNIT_COLS;
 #pragma unroll
-            for (int s = 0; s < 2; ++s) {
-                int c = c0 + s;
-                if (c >= a.nx) continue;
-                double b = div_b(a, c, j);
-                size_t k = (size_t)j * a.pitch + c;
+        for (int m = 0; m < UNIT_CPT; ++m) {
+            const int row = row0 + m * UNIT_ROWSTEP, cell = row * CF_UNIT_COLS + col;
+            double b = 0.0, z = 0.0;
+            if (col < u.nc && row < u.nr) {
+                const int c = u.c0 + col, j = u.j0 + row;
+                b = div_b(a, c, j);
+                const size_t k = (size_t)j * a.pitch + c;
                 a.r[k] = b;
                 if (!a.warm) a.x[k] = 0.0;
-                double z = a.st.minv[edge_bits(c, j, a.nx, a.ny, a.per_x, a.per_y)] * b;
-                arz = fma(b, z, arz);
-                arr = fma(b, b, arr);
+                z = a.st.minv[edge_bits(c, j, a.nx, a.ny, a.per_x, a.per_y)] * b;
             }
-    }
-    arz = warp_fold(arz);
-    arr = warp_fold(arr);
-    if (unit < a.U && lane == 0) {
-        a.part0[unit] = arz;
-        a.part1[unit] = arr;
+            R[cell] = b;
+            Z[cell] = z;
+        }
+        __syncthreads();
+        const int warp = tid / 32, lane = tid & 31;
+        if (warp == unit_warp(unit)) {
+            const double s = unit_dot(R, CF_UNIT_COLS, R, CF_UNIT_COLS, lane);
+            if (lane == 0) a.part1[unit] = s;
+        } else if (warp == unit_warp(unit + 1)) {
+            const double s = unit_dot(R, CF_UNIT_COLS, Z, CF_UNIT_COLS, lane);
+            if (lane == 0) a.part0[unit] = s;
+        }
     }
     if (last_block_arrive(&S->ticket[2])) {
         double rz = final_tree(a.part0, a.U);
@@ -441,18 +434,7 @@ __global__ void __launch_bounds__(CF_RED_THREADS) k_div_init64(DivArgs a) {
         if (threadIdx.x == 0) {
             S->ticket[2] = 0;
             S->bb = rr;
-            S->rr = rr;
-            S->rho = rz;
-            S->beta = 0.0;
-            S->iter = 0;
-            if (rr == 0.0 || converged(S, rr))
-                S->status = ST_CONVERGED;
-            else if (S->max_iter <= 0)
-                S->status = ST_MAXIT;
-            else if (isnan(rr))
-                S->status = ST_NAN;
-            else
-                S->status = ST_RUNNING;
+            start_solve64(S, rr, rz);
         }
     }
 }
@@ -1349,40 +1331,62 @@ __global__ void __launch_bounds__(CF_RED_THREADS, 4) k_apply_pairs_norms(Press a
 }
 
 // ||div u||: canonical sum of b^2 and max |b|
+__global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_div_norms64(DivArgs a) {
+    __shared__ double B[UNIT_CELLS], mx[CF_RED_WARPS];
+    SolverState* S = a.S;
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid & 31;
+    for (int unit = blockIdx.x; unit < a.U; unit += gridDim.x) {
+        if (unit != (int)blockIdx.x) __syncthreads();  // the last unit's sums are done with shared memory
+        const UnitPos u = unit_pos(unit, a.G, a.nx, a.ny);
+        const int col = tid & (CF_UNIT_COLS - 1), row0 = tid / CF_UNIT_COLS;
+        double amx = 0.0;
+#pragma unroll
+        for (int m = 0; m < UNIT_CPT; ++m) {
+            const int row = row0 + m * UNIT_ROWSTEP;
+            double b = 0.0;
+            if (col < u.nc && row < u.nr) b = div_b(a, u.c0 + col, u.j0 + row);
+            B[row * CF_UNIT_COLS + col] = b;
+            amx = fmax(amx, fabs(b));
+        }
+        amx = warp_max(amx);
+        if (lane == 0) mx[warp] = amx;
+        __syncthreads();
+        if (warp == unit_warp(unit)) {
+            const double s = unit_dot(B, CF_UNIT_COLS, B, CF_UNIT_COLS, lane);
+            if (lane == 0) a.part0[unit] = s;
+        } else if (tid == 32 * unit_warp(unit + 1)) {
+            double t = mx[0];
+#pragma unroll
+            for (int k = 1; k < CF_RED_WARPS; ++k) t = fmax(t, mx[k]);
+            a.part1[unit] = t;
+        }
+    }
+    if (last_block_arrive(&S->ticket[3])) {
+        double ss = final_tree(a.part0, a.U);
+        double mxx = final_max(a.part1, a.U);
+        if (threadIdx.x == 0) {
+            S->ticket[3] = 0;
+            a.out[0] = ss;
+            a.out[1] = mxx;
+        }
+    }
+}
+
+// the same of a mixed context: the divergence of the pairs, then its square and
+// magnitude in FP32, a unit per warp
 __global__ void __launch_bounds__(CF_RED_THREADS) k_div_norms(DivArgs a) {
     SolverState* S = a.S;
     const int lane = threadIdx.x & 31;
     const int unit = blockIdx.x * CF_RED_WARPS + (threadIdx.x >> 5);
-    double ass = 0.0, amx = 0.0;
     float fss = 0.f, fmx = 0.f;
-    if (unit < a.U && a.mixed) {
-        // the divergence of the pairs, then its square and magnitude in FP32
+    if (unit < a.U)
         div_pairs_unit(a, unit % a.G, unit / a.G, lane, [&](int, int, float2 t) {
             const float bf = t.x * a.mscale32;
             fss = fmaf(bf, bf, fss);
             fmx = fmaxf(fmx, fabsf(bf));
         });
-    } else if (unit < a.U) {
-        const int g = unit % a.G, band = unit / a.G;
-        const int c0 = g * CF_UNIT_COLS + 2 * lane;
-        const int j0 = band * CF_BAND_ROWS;
-        const int j1 = min(j0 + CF_BAND_ROWS, a.ny);
-        for (int j = j0; j < j1; ++j)
-#pragma unroll
-            for (int s = 0; s < 2; ++s) {
-                int c = c0 + s;
-                if (c >= a.nx) continue;
-                double b = div_b(a, c, j);
-                ass = fma(b, b, ass);
-                amx = fmax(amx, fabs(b));
-            }
-    }
-    if (a.mixed) {
-        ass = (double)fss;
-        amx = (double)fmx;
-    }
-    ass = warp_fold(ass);
-    amx = warp_max(amx);
+    const double ass = warp_fold((double)fss);
+    const double amx = warp_max((double)fmx);
     if (unit < a.U && lane == 0) {
         a.part0[unit] = ass;
         a.part1[unit] = amx;
@@ -1413,7 +1417,6 @@ static DivArgs div_args(cf_ctx* c, const Stencil& st) {
     a.u = c->u[c->cur];
     a.v = c->v[c->cur];
     a.mscale = -(1.0 / c->ph.dx);
-    a.mixed = c->precision == CF_PREC_MIXED;
     a.mscale32 = (float)a.mscale;
     a.mscale2 = make_float2(a.mscale32, (float)(a.mscale - (double)a.mscale32));
     a.st = st;
@@ -1469,6 +1472,18 @@ static Cg64 cg64_args(cf_ctx* c, const Stencil& st) {
 }
 
 static int red_blocks(const cf_ctx* c) { return (c->n_units + CF_RED_WARPS - 1) / CF_RED_WARPS; }
+
+// blocks of the FP64 unit kernels: one per unit, at most as many as are resident
+// at once (each then walks several units: a block's arrival at the fold costs
+// about 1 us, and a second wave would leave the GPU part empty)
+static int unit_blocks(const cf_ctx* c) { return std::min(c->n_units, UNIT_BLOCKS * c->sms); }
+
+static void launch_norms(cf_ctx* c, const DivArgs& a) {
+    if (c->precision == CF_PREC_MIXED)
+        k_div_norms<<<red_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a);
+    else
+        k_div_norms64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a);
+}
 
 // The mixed projection of a grid periodic along both axes takes its
 // divergence norms inside the gradient (k_apply_pairs_norms), from faces
@@ -1545,7 +1560,7 @@ static int launch_warm_init(cf_ctx* c, const Stencil& st, bool mixed) {
         k_outer_resid<false><<<red_blocks(c), CF_RED_THREADS, 0, c->stream>>>(oa);
     } else {
         Cg64 a = cg64_args(c, st);
-        k_warm_resid64<<<red_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a);
+        k_warm_resid64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a);
     }
     return 1;
 }
@@ -1586,11 +1601,10 @@ static int batch_cg(cf_ctx* c, const Stencil& st, bool mixed) {
         pcg64_launch(c, st, kBatch);
         return 1;
     } else {
-        const int nb = red_blocks(c);
         Cg64 a = cg64_args(c, st);
         for (int i = 0; i < kBatch; ++i) {
-            k_cg_dir_matvec64<<<nb, CF_RED_THREADS, 0, c->stream>>>(a);
-            k_cg_update64<<<nb, CF_RED_THREADS, 0, c->stream>>>(a);
+            k_cg_dir_matvec64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a);
+            k_cg_update64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a);
         }
     }
     return 2 * kBatch;
@@ -1600,7 +1614,6 @@ static int batch_cg(cf_ctx* c, const Stencil& st, bool mixed) {
 // gated reliable update too); returns the kernels of one iteration
 static int batch_mg(cf_ctx* c, const Stencil& st) {
     const bool mixed = c->precision == CF_PREC_MIXED;
-    const int nb = red_blocks(c);
     const double scale = -st.ms;
     Cg64 a = cg64_args(c, st);
     a.mg = 1;
@@ -1611,10 +1624,10 @@ static int batch_mg(cf_ctx* c, const Stencil& st) {
             per = launch_mixed_mg_step(c, st);
             per += cg32_mg_precondition(c, scale);
         } else {
-            k_cg_dir_matvec64<<<nb, CF_RED_THREADS, 0, c->stream>>>(a);
-            k_cg_update64<<<nb, CF_RED_THREADS, 0, c->stream>>>(a);
+            k_cg_dir_matvec64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a);
+            k_cg_update64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a);
             per = 3 + mg_vcycle(c, scale);
-            k_mg_rz64<<<nb, CF_RED_THREADS, 0, c->stream>>>(a, 0);
+            k_mg_rz64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a, 0);
         }
     }
     return per;
@@ -1629,7 +1642,7 @@ static int batch_mg_pre(cf_ctx* c, const Stencil& st) {
     a.mg = 1;
     a.z = mg_z64(c);
     const int pre = 1 + mg_vcycle(c, scale);
-    k_mg_rz64<<<red_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a, 1);
+    k_mg_rz64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a, 1);
     return pre;
 }
 
@@ -1758,7 +1771,6 @@ __global__ void k_loop_cond(SolverState* S, cudaGraphConditionalHandle h) {
 
 // kernels of one iteration (per trip: batch of them); returns launches
 static int launch_iterations(cf_ctx* c, const Stencil& st, bool mixed, bool mg, int n) {
-    const int nb = red_blocks(c);
     const double scale = -st.ms;
     int k = 0;
     if (!mixed && !mg && onchip64(c)) {
@@ -1786,12 +1798,12 @@ static int launch_iterations(cf_ctx* c, const Stencil& st, bool mixed, bool mg, 
                 }
             }
         } else {
-            k_cg_dir_matvec64<<<nb, CF_RED_THREADS, 0, c->stream>>>(a);
-            k_cg_update64<<<nb, CF_RED_THREADS, 0, c->stream>>>(a);
+            k_cg_dir_matvec64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a);
+            k_cg_update64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a);
             k += 2;
             if (mg) {
                 k += 1 + mg_vcycle(c, scale);
-                k_mg_rz64<<<nb, CF_RED_THREADS, 0, c->stream>>>(a, 0);
+                k_mg_rz64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a, 0);
             }
         }
     }
@@ -1838,7 +1850,7 @@ static int build_resident(cf_ctx* c, const Stencil& st, double dt, bool mixed, b
             if (mixed)
                 k_div_init_mixed<<<nb, CF_RED_THREADS, 0, c->stream>>>(da);
             else
-                k_div_init64<<<nb, CF_RED_THREADS, 0, c->stream>>>(da);
+                k_div_init64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(da);
             nhead = 1;
             if (warm) nhead += launch_warm_init(c, st, mixed);
             if (mg) {
@@ -1849,7 +1861,7 @@ static int build_resident(cf_ctx* c, const Stencil& st, double dt, bool mixed, b
                     a.mg = 1;
                     a.z = mg_z64(c);
                     nhead += 1 + mg_vcycle(c, scale);
-                    k_mg_rz64<<<nb, CF_RED_THREADS, 0, c->stream>>>(a, 1);
+                    k_mg_rz64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a, 1);
                 }
             }
         });
@@ -1898,7 +1910,7 @@ static int build_resident(cf_ctx* c, const Stencil& st, double dt, bool mixed, b
             }
             // (the adjoint's projections report no divergence norms)
             if (!adjoint && !fuse_n) {
-                k_div_norms<<<nb, CF_RED_THREADS, 0, c->stream>>>(dn);
+                launch_norms(c, dn);
                 ntail += 1;
             }
             k_step_tally<<<1, 1, 0, c->stream>>>(c->S, c->d_tally);
@@ -2135,7 +2147,7 @@ static int read_norms(cf_ctx* c, double* l2, double* linf) {
 int div_norms(cf_ctx* c, double* l2, double* linf) {
     Stencil st{};
     DivArgs a = div_args(c, st);
-    k_div_norms<<<red_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a);
+    launch_norms(c, a);
     c->launches += 1;
     return read_norms(c, l2, linf);
 }
@@ -2186,7 +2198,7 @@ int project_grids(cf_ctx* c, double dt, const SolveOpts& o, SolveResult* res, Gr
     da.warm = warm;
     if (c->prof) cudaEventRecord(c->ev[4], c->stream);
     if (!mixed) {
-        k_div_init64<<<nb, CF_RED_THREADS, 0, c->stream>>>(da);
+        k_div_init64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(da);
         c->launches += 1;
         if (warm) c->launches += launch_warm_init(c, st, false);
         const int batch = mg ? kBatchMG : kBatch;
