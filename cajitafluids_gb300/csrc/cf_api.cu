@@ -284,6 +284,9 @@ int cf_ctx_create(const cf_grid_desc* d, cf_ctx** out) {
     p.per_y = d->periodic[1] ? 1 : 0;
     p.dx = dx;
     p.rdx = 1.0 / dx;
+    p.rsh = -1;
+    for (int k = 0; k <= 64; ++k)
+        if (p.rdx == ldexp(1.0, k)) p.rsh = k;
     static const double off[3][2] = {{0.5, 0.5}, {0.0, 0.5}, {0.5, 0.0}};
     for (int k = 0; k < 2; ++k) p.gl[k] = d->lo[k] - 3.0 * dx;
     for (int e = 0; e < 3; ++e)

@@ -63,24 +63,19 @@ __global__ void k_fill_ghosts(Grid<T> g, int nox, int noy, int per_x, int per_y)
 
 // --------------------------------------------------------------------------
 // FP64 spline sample (Cajita B-spline order 1 / 3, evaluated separably);
-// the coordinate clamp and integer part come from the integer-pipe helpers
-// (cf_internal.cuh).
+// the coordinate clamp, the cell and the linear weights come from the
+// integer-pipe helpers (cf_internal.cuh).
 template <int ORDER>
 __device__ __forceinline__ void weights64(double xi, int ext, int& k0, double* w) {
+    int k;
+    double t, s;
     if (ORDER == 1) {
-        xi = clamp_bits(xi, 0.0, exact_double(ext - 1));
-        int k = trunc_bits(xi);
-        if (k > ext - 2) k = ext - 2;
-        double t = xi - exact_double(k);
-        w[0] = 1.0 - t;
+        cell_fraction(clamp_bits(xi, 0.0, exact_double(ext - 1)), ext - 2, k, t, s);
+        w[0] = s;
         w[1] = t;
         k0 = k;
     } else {
-        xi = clamp_bits(xi, 1.0, exact_double(ext - 2));
-        int k = trunc_bits(xi);
-        if (k > ext - 3) k = ext - 3;
-        double t = xi - exact_double(k);
-        double s = 1.0 - t;
+        cell_fraction(clamp_bits(xi, 1.0, exact_double(ext - 2)), ext - 3, k, t, s);
         double t2 = t * t;
         double t3 = t2 * t;
         double s3 = (s * s) * s;
@@ -93,10 +88,10 @@ __device__ __forceinline__ void weights64(double xi, int ext, int& k0, double* w
 }
 
 template <int ORDER>
-__device__ double sample64(const Grid<double>& g, double lx, double ly, double rdx, double x, double y) {
+__device__ double sample64(const Phys& p, const Grid<double>& g, double lx, double ly, double x, double y) {
     constexpr int n = ORDER == 1 ? 2 : 4;
-    double xi = (x - lx) * rdx;
-    double yi = (y - ly) * rdx;
+    double xi = times_rdx(x - lx, p.rdx, p.rsh);
+    double yi = times_rdx(y - ly, p.rdx, p.rsh);
     int kx, ky;
     double wx[n], wy[n];
     weights64<ORDER>(xi, g.ex, kx, wx);
@@ -118,25 +113,24 @@ __device__ __forceinline__ double entity_coord(const Phys& p, int ent, int axis,
     return p.gl[axis] + t * p.dx;
 }
 
-// rk3 backtrace (src/TimeIntegrator.hpp:36-77), linear velocity samples.
-__device__ void rk3_64(const Phys& p, const Grid<double>& u, const Grid<double>& v, double dt,
-                       double x0, double y0, double& tx, double& ty) {
+// rk3 backtrace (src/TimeIntegrator.hpp:36-77) after its first velocity sample
+// (v0x, v0y), linear velocity samples.
+__device__ __forceinline__ void rk3_64_from(const Phys& p, const Grid<double>& u, const Grid<double>& v, double dt,
+                                            double x0, double y0, double v0x, double v0y, double& tx, double& ty) {
     const double ulx = p.low[E_FACEI][0], uly = p.low[E_FACEI][1];
     const double vlx = p.low[E_FACEJ][0], vly = p.low[E_FACEJ][1];
-    double v0x = sample64<1>(u, ulx, uly, p.rdx, x0, y0);
-    double v0y = sample64<1>(v, vlx, vly, p.rdx, x0, y0);
     // the reference's stage expressions as written, one rounding per
     // operation: x0 - 0.5 * dt * v0 is x0 - ((0.5 * dt) * v0)
     double h1 = 0.5 * dt;
     double x1 = __dsub_rn(x0, __dmul_rn(h1, v0x)), y1 = __dsub_rn(y0, __dmul_rn(h1, v0y));
-    double v1x = sample64<1>(u, ulx, uly, p.rdx, x1, y1);
-    double v1y = sample64<1>(v, vlx, vly, p.rdx, x1, y1);
+    double v1x = sample64<1>(p, u, ulx, uly, x1, y1);
+    double v1y = sample64<1>(p, v, vlx, vly, x1, y1);
     double h2 = 0.75 * dt;
     bool ralston = (p.quirks & 2u) != 0;
     double sx = ralston ? v1x : v0x, sy = ralston ? v1y : v0y;
     double x2 = __dsub_rn(x0, __dmul_rn(h2, sx)), y2 = __dsub_rn(y0, __dmul_rn(h2, sy));
-    double v2x = sample64<1>(u, ulx, uly, p.rdx, x2, y2);
-    double v2y = sample64<1>(v, vlx, vly, p.rdx, x2, y2);
+    double v2x = sample64<1>(p, u, ulx, uly, x2, y2);
+    double v2y = sample64<1>(p, v, vlx, vly, x2, y2);
     // x0 - dt * ((2/9) v0 + (3/9) v1 + (4/9) v2), summed left to right
     double ax = __dadd_rn(__dmul_rn(2.0 / 9.0, v0x), __dmul_rn(3.0 / 9.0, v1x));
     ax = __dadd_rn(ax, __dmul_rn(4.0 / 9.0, v2x));
@@ -144,6 +138,13 @@ __device__ void rk3_64(const Phys& p, const Grid<double>& u, const Grid<double>&
     ay = __dadd_rn(ay, __dmul_rn(4.0 / 9.0, v2y));
     tx = __dsub_rn(x0, __dmul_rn(dt, ax));
     ty = __dsub_rn(y0, __dmul_rn(dt, ay));
+}
+
+__device__ void rk3_64(const Phys& p, const Grid<double>& u, const Grid<double>& v, double dt,
+                       double x0, double y0, double& tx, double& ty) {
+    const double v0x = sample64<1>(p, u, p.low[E_FACEI][0], p.low[E_FACEI][1], x0, y0);
+    const double v0y = sample64<1>(p, v, p.low[E_FACEJ][0], p.low[E_FACEJ][1], x0, y0);
+    rk3_64_from(p, u, v, dt, x0, y0, v0x, v0y, tx, ty);
 }
 
 // --------------------------------------------------------------------------
@@ -174,16 +175,12 @@ __device__ __forceinline__ double inputs_cell(const Phys& p, double q, double x,
     return q;
 }
 
-// axis 0: I-face (u), axis 1: J-face (v); rho is used only with a density-scaled force.
-__device__ __forceinline__ double inputs_face_in(const Phys& p, int axis, double w, bool inbox, double dt, int gidx,
-                                                 double rho) {
+// Fused form (constant force; fdt = force * dt, one rounding, made on the host):
+// axis 0: I-face (u), axis 1: J-face (v).
+__device__ __forceinline__ double inputs_face_in(const Phys& p, int axis, double w, bool inbox, double fdt, int gidx) {
     if (inbox && fabs(w) < fabs(p.src_vel[axis])) w = p.src_vel[axis];
-    // ux += _force[0] * delta_t (src/BodyForce.hpp:52, 61); the density-scaled
-    // form (extension) scales the force first
-    if (p.force_density)
-        w = __dadd_rn(w, __dmul_rn(__dmul_rn(p.force[axis], rho), dt));
-    else
-        w = __dadd_rn(w, __dmul_rn(p.force[axis], dt));
+    // ux += _force[0] * delta_t (src/BodyForce.hpp:52, 61)
+    w = __dadd_rn(w, fdt);
     int per = axis == 0 ? p.per_x : p.per_y;
     int n = axis == 0 ? p.nx : p.ny;
     if (!per) {
@@ -193,6 +190,7 @@ __device__ __forceinline__ double inputs_face_in(const Phys& p, int axis, double
     return w;
 }
 
+// axis 0: I-face (u), axis 1: J-face (v); rho is used only with a density-scaled force.
 __device__ __forceinline__ double inputs_face(const Phys& p, int axis, double w, double x, double y,
                                               double dt, int gidx, double rho) {
     if (in_box(p, x, y) && fabs(w) < fabs(p.src_vel[axis])) w = p.src_vel[axis];
@@ -220,34 +218,97 @@ struct Adv64 {
     double dt;
     int fuse;
     int ent0;  // entity of blockIdx.z == 0 (a launch may cover a subset)
+    double fdt[2];  // force * dt (fused inputs: the force is constant there)
 };
 
-template <int ORDER>
+// What an entity's own coordinates fix depends on its column or its row alone:
+// the coordinate, and the cells and weights of the first RK stage's samples of
+// u and v.  Two warps work them out for the block's tile.
+struct AdvAxis {
+    double x0[32];
+    double su[32], tu[32], sv[32], tv[32];
+    int ku[32], kv[32];
+    int u0, v0;  // every tu (tv) is zero: the samples sit on the grid's own points
+};
+
+// The linear sample with weights (sx, tx), (sy, ty) of the cell at q; zx, zy:
+// tx, ty are zero and sx, sy one along the whole tile, so a product with a
+// finite tap drops out exactly.
+__device__ __forceinline__ double stage0_64(const double* q, int pitch, double sx, double tx, double sy, double ty, bool zx,
+                                            bool zy) {
+    const double a0 = __ldg(q), a1 = __ldg(q + 1), b0 = __ldg(q + pitch), b1 = __ldg(q + pitch + 1);
+    if (zx || zy) {
+        auto mag = [](double d) { return __double2hiint(d) & 0x7fffffff; };
+        if (max(max(mag(a0), mag(a1)), max(mag(b0), mag(b1))) < 0x7ff00000) {
+            const double ra = zx ? a0 : fma(tx, a1, sx * a0);
+            if (zy) return ra;
+            const double rb = zx ? b0 : fma(tx, b1, sx * b0);
+            return fma(ty, rb, sy * ra);
+        }
+    }
+    return fma(ty, fma(tx, b1, sx * b0), sy * fma(tx, a1, sx * a0));
+}
+
+// Tiles of 32 columns x 8 ROWS rows.  Bound by the FP64 pipe (two operations
+// per cycle and SM; 86 % busy): of 164 FP64 operations per entity of the plain
+// form, the per-axis tables take 22 (and the samples that need no product 7
+// more), the integer fractions 20, the power-of-two scale 10.  15.7 -> 10.8 ms
+// at 4096^2, 259 -> 185 us at 512^2, 40 -> 31 us at 192x160.
+template <int ORDER, int ROWS>
 __global__ void __launch_bounds__(256) k_advect64(Adv64 a) {
+    __shared__ AdvAxis X, Y;
     const Phys& p = a.p;
-    int ent = blockIdx.z + a.ent0;
-    int gi = blockIdx.x * blockDim.x + threadIdx.x;
-    int gj = blockIdx.y * blockDim.y + threadIdx.y;
-    int ox = p.nx + ((ent == E_FACEI && !p.per_x) ? 1 : 0);
-    int oy = p.ny + ((ent == E_FACEJ && !p.per_y) ? 1 : 0);
-    if (gi >= ox || gj >= oy) return;
+    const int ent = blockIdx.z + a.ent0;
+    const int gi0 = blockIdx.x * 32, gj0 = blockIdx.y * 8 * ROWS;
+    const int lane = threadIdx.x, wrow = threadIdx.y;
+    if (wrow < 2) {
+        AdvAxis& A = wrow ? Y : X;
+        const double x = entity_coord(p, ent, wrow, (wrow ? gj0 : gi0) + lane + CF_HALO);
+        double w[2];
+        int k;
+        A.x0[lane] = x;
+        weights64<1>(times_rdx(x - p.low[E_FACEI][wrow], p.rdx, p.rsh), wrow ? a.u.ey : a.u.ex, k, w);
+        A.su[lane] = w[0];
+        A.tu[lane] = w[1];
+        A.ku[lane] = k;
+        const bool u0 = __all_sync(0xffffffffu, w[1] == 0.0);
+        weights64<1>(times_rdx(x - p.low[E_FACEJ][wrow], p.rdx, p.rsh), wrow ? a.v.ey : a.v.ex, k, w);
+        A.sv[lane] = w[0];
+        A.tv[lane] = w[1];
+        A.kv[lane] = k;
+        const bool v0 = __all_sync(0xffffffffu, w[1] == 0.0);
+        if (lane == 0) {
+            A.u0 = u0;
+            A.v0 = v0;
+        }
+    }
+    __syncthreads();
+    const int gi = gi0 + lane;
+    const int ox = p.nx + ((ent == E_FACEI && !p.per_x) ? 1 : 0);
+    const int oy = p.ny + ((ent == E_FACEJ && !p.per_y) ? 1 : 0);
     const Grid<double>& f = ent == E_CELL ? a.q : (ent == E_FACEI ? a.u : a.v);
     const Grid<double>& fn = ent == E_CELL ? a.qn : (ent == E_FACEI ? a.un : a.vn);
-    double x0 = entity_coord(p, ent, 0, gi + CF_HALO);
-    double y0 = entity_coord(p, ent, 1, gj + CF_HALO);
-    double tx, ty;
-    rk3_64(p, a.u, a.v, a.dt, x0, y0, tx, ty);
-    double val = sample64<ORDER>(f, p.low[ent][0], p.low[ent][1], p.rdx, tx, ty);
-    if (a.fuse) {
-        const bool inbox = in_box_idx(p, ent, gi + CF_HALO, gj + CF_HALO);
-        if (ent == E_CELL)
-            val = inputs_cell_in(p, val, inbox, a.dt);
-        else if (ent == E_FACEI)
-            val = inputs_face_in(p, 0, val, inbox, a.dt, gi, 0.0);
-        else
-            val = inputs_face_in(p, 1, val, inbox, a.dt, gj, 0.0);
+    if (gi >= ox) return;
+#pragma unroll 1
+    for (int m = 0; m < ROWS; ++m) {
+        const int r = wrow + 8 * m, gj = gj0 + r;
+        if (gj >= oy) return;
+        const double v0x = stage0_64(a.u.o + (size_t)Y.ku[r] * a.u.pitch + X.ku[lane], a.u.pitch, X.su[lane], X.tu[lane],
+                                     Y.su[r], Y.tu[r], X.u0, Y.u0);
+        const double v0y = stage0_64(a.v.o + (size_t)Y.kv[r] * a.v.pitch + X.kv[lane], a.v.pitch, X.sv[lane], X.tv[lane],
+                                     Y.sv[r], Y.tv[r], X.v0, Y.v0);
+        double tx, ty;
+        rk3_64_from(p, a.u, a.v, a.dt, X.x0[lane], Y.x0[r], v0x, v0y, tx, ty);
+        double val = sample64<ORDER>(p, f, p.low[ent][0], p.low[ent][1], tx, ty);
+        if (a.fuse) {
+            const bool inbox = in_box_idx(p, ent, gi + CF_HALO, gj + CF_HALO);
+            if (ent == E_CELL)
+                val = inputs_cell_in(p, val, inbox, a.dt);
+            else
+                val = inputs_face_in(p, ent - E_FACEI, val, inbox, a.fdt[ent - E_FACEI], ent == E_FACEI ? gi : gj);
+        }
+        fn.at(gi + CF_HALO, gj + CF_HALO) = val;
     }
-    fn.at(gi + CF_HALO, gj + CF_HALO) = val;
 }
 
 // --------------------------------------------------------------------------
@@ -492,8 +553,8 @@ __global__ void k_interp_points(Pts a) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.n) return;
     double x = a.xy[2 * k], y = a.xy[2 * k + 1];
-    a.out[k] = a.order == 1 ? sample64<1>(a.f, a.p.low[a.ent][0], a.p.low[a.ent][1], a.p.rdx, x, y)
-                            : sample64<3>(a.f, a.p.low[a.ent][0], a.p.low[a.ent][1], a.p.rdx, x, y);
+    a.out[k] = a.order == 1 ? sample64<1>(a.p, a.f, a.p.low[a.ent][0], a.p.low[a.ent][1], x, y)
+                            : sample64<3>(a.p, a.f, a.p.low[a.ent][0], a.p.low[a.ent][1], x, y);
 }
 
 __global__ void k_trace_points(Pts a) {
@@ -514,8 +575,8 @@ __global__ void k_cell_velocity(Phys p, Grid<double> u, Grid<double> v, double* 
     if (gi >= p.nx || gj >= p.ny) return;
     const double x = entity_coord(p, E_CELL, 0, gi + CF_HALO), y = entity_coord(p, E_CELL, 1, gj + CF_HALO);
     const size_t k = (size_t)gj * p.nx + gi;
-    uc[k] = sample64<1>(u, p.low[E_FACEI][0], p.low[E_FACEI][1], p.rdx, x, y);
-    vc[k] = sample64<1>(v, p.low[E_FACEJ][0], p.low[E_FACEJ][1], p.rdx, x, y);
+    uc[k] = sample64<1>(p, u, p.low[E_FACEI][0], p.low[E_FACEI][1], x, y);
+    vc[k] = sample64<1>(p, v, p.low[E_FACEJ][0], p.low[E_FACEJ][1], x, y);
 }
 
 // max |w| over the owned faces of one axis; non-negative doubles order like
@@ -586,11 +647,21 @@ cudaError_t launch_advect(cf_ctx* c, double dt, int order, int fuse_inputs, int 
     dim3 blk(32, 8);
     dim3 grd = grid2(p.nx + 1, p.ny + 1, blk, nent);
     if (c->precision == CF_PREC_FP64) {
-        Adv64 a{p, c->q64[s], c->u[s], c->v[s], c->q64[n], c->u[n], c->v[n], dt, fuse_inputs, ent0};
-        if (order == 1)
-            k_advect64<1><<<grd, blk, 0, c->stream>>>(a);
-        else
-            k_advect64<3><<<grd, blk, 0, c->stream>>>(a);
+        Adv64 a{p, c->q64[s], c->u[s], c->v[s], c->q64[n], c->u[n], c->v[n], dt, fuse_inputs, ent0, {}};
+        for (int k = 0; k < 2; ++k) a.fdt[k] = p.force[k] * dt;
+        // four rows a thread (fewer tables) once that leaves eight blocks per SM
+        const dim3 tall((p.nx + 1 + 31) / 32, (p.ny + 1 + 31) / 32, nent);
+        if ((long long)tall.x * tall.y * tall.z >= 8ll * c->sms) {
+            if (order == 1)
+                k_advect64<1, 4><<<tall, blk, 0, c->stream>>>(a);
+            else
+                k_advect64<3, 4><<<tall, blk, 0, c->stream>>>(a);
+        } else {
+            if (order == 1)
+                k_advect64<1, 1><<<grd, blk, 0, c->stream>>>(a);
+            else
+                k_advect64<3, 1><<<grd, blk, 0, c->stream>>>(a);
+        }
     } else {
         // fused inputs with a density-scaled force are applied by the
         // standalone inputs kernels after the advection

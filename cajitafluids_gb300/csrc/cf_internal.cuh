@@ -41,6 +41,7 @@ struct Phys {
     int nx, ny;
     int per_x, per_y;
     double dx, rdx;
+    int rsh;            // rdx = 2^rsh exactly, 0 <= rsh <= 64, else -1
     double gl[2];       // low corner of the ghosted local mesh
     double low[3][2];   // coordinate of local index 0 per entity (spline origin)
     int bc[4];          // left, bottom, right, top
@@ -396,6 +397,45 @@ __device__ __forceinline__ int trunc_bits(double x) {
     if (e < 0) return 0;
     const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
     return (int)(m >> (52 - e));
+}
+
+// The cell k = min(floor(xi), kmax), the fraction t = xi - k and s = 1 - t of a
+// spline coordinate xi in [0, kmax + 1].  For xi >= 1 both are multiples of
+// 2^-52 no larger than 1, so they are exact, and they come from the significand
+// on the integer pipe instead of two FP64 subtractions: xi's significand shifted
+// left by its exponent leaves the 52 fraction bits F, t = F 2^-52 and s =
+// (2^52 - F) 2^-52, each normalised by its leading zeros.  The rest (xi < 1, a
+// fraction or its complement below 2^-20, the upper end) takes the subtractions.
+__device__ __forceinline__ double fix52(unsigned hi, unsigned lo) {  // (hi 2^32 + lo) 2^-52, 0 < hi <= 2^20
+    const int n = __clz((int)hi) - 11;
+    return __hiloint2double((int)(((unsigned)(1022 - n) << 20) + __funnelshift_l(lo, hi, n)), (int)(lo << n));
+}
+__device__ __forceinline__ void cell_fraction(double xi, int kmax, int& k, double& t, double& s) {
+    const unsigned hi = (unsigned)__double2hiint(xi), lo = (unsigned)__double2loint(xi);
+    const unsigned e = (hi >> 20) - 1023u;  // xi is not negative
+    if (e <= 20u) {
+        const unsigned m = (hi & 0xfffffu) | 0x100000u;
+        const unsigned fh = __funnelshift_l(lo, m, e) & 0xfffffu, fl = lo << e;
+        const unsigned gl = 0u - fl, gh = 0x100000u - fh - (fl != 0u ? 1u : 0u);
+        k = (int)(m >> (20u - e));
+        if (fh != 0u && gh != 0u && k <= kmax) {
+            t = fix52(fh, fl);
+            s = fix52(gh, gl);
+            return;
+        }
+    }
+    k = trunc_bits(xi);
+    if (k > kmax) k = kmax;
+    t = xi - exact_double(k);
+    s = 1.0 - t;
+}
+
+// d * rdx for the mesh's 1 / dx: where that is a power of two (sh its exponent,
+// else -1) an addition to the exponent, the same value exactly
+__device__ __forceinline__ double times_rdx(double d, double rdx, int sh) {
+    const unsigned hi = (unsigned)__double2hiint(d), e = hi & 0x7ff00000u;
+    if (sh >= 0 && e - 0x00100000u < 0x60000000u) return __hiloint2double((int)(hi + ((unsigned)sh << 20)), __double2loint(d));
+    return d * rdx;
 }
 
 // Double-float (hi + lo FP32 pair) error-free sums (Knuth two-sum, Dekker
