@@ -29,7 +29,9 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
-#include "cf_ctx.cuh"
+#include <algorithm>
+
+#include "cf_grid.cuh"
 
 namespace cf {
 
@@ -478,6 +480,394 @@ __global__ void __launch_bounds__(kThreads, 2)
 }
 
 // --------------------------------------------------------------------------
+// The same iteration with the whole solve on chip, for grids of at most four
+// tiles per SM (about 1.2 million cells): one cooperative launch runs many
+// iterations, a block keeping its tiles' r, x and A p in registers and p with its
+// halo in shared memory, the grid meeting at two barriers per iteration
+// (cf_grid.cuh).  The launches above cost 22 us per iteration at 501 x 333 (84
+// tiles), most of it launch, TMA and fold latency; this form 8.1 us, half of it
+// the two barriers and half the FP64 sums and divisions between them.  Every cell value, thread sum,
+// block sum and fold is formed as by those kernels (tile k of block b is tile
+// b + k gridDim; the thread sums of tiles that one of their blocks walks in turn
+// run on in the same order), so the results are the same bits.
+constexpr int kHalo = 2 * kTW + 2 * kTH;  // halo (and border) values of a tile
+constexpr int kMaxTiles = 4;              // tiles per block
+// the stalled wait of the timeout-path test: a grid barrier that cannot complete
+constexpr unsigned kGridStallLimit = 1u << 10;
+
+template <int NT>
+__global__ void __launch_bounds__(kThreads, 1) k_pcg32(Cg32T a, float* border, int ga, int gb, int iters) {
+    extern __shared__ __align__(16) float Ps[];  // NT tiles of kBY rows of kBX columns, owned (c, r) at [r + 1][c + 4]
+    __shared__ float tab_d[16], tab_m[16];
+    __shared__ double red[2][NT][kThreads / 32], ws0[kThreads / 32], ws1[kThreads / 32];
+    __shared__ double bc_a, bc_b, bc_c;
+    __shared__ float bc_f;  // alpha, then beta, in FP32 (one conversion)
+    __shared__ int bc_stat;
+    SolverState* S = a.S;
+    if (!running(S)) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nb = gridDim.x;
+    int it = S->inner_iter, iter = S->iter;
+    const int it_end = it + iters, max_iter = S->max_iter;
+    bool first = it == 0 || S->restart;
+    double rho = S->rho_in, rho_prev = S->rho_prev, rr = S->rr_in, rr0 = S->rr_in0, alpha64 = S->alpha_in,
+           beta64 = S->beta_in;
+    const bool stall = S->test_stall != 0 && blockIdx.x == 0;
+    const unsigned gbase = S->gbar;
+    unsigned arrived = 0;
+    if (tid < 16) {
+        tab_d[tid] = a.st.diag32[tid];
+        tab_m[tid] = a.st.minv32[tid];
+    }
+    for (int k = tid; k < NT * kBY * kBX; k += kThreads) Ps[k] = 0.f;
+    __syncthreads();
+    const float ms = a.st.ms32;
+    auto tile_of = [&](int k) { return (int)blockIdx.x + k * nb; };
+    auto P = [&](int k) { return Ps + k * kBY * kBX; };
+    // the lane's cells: columns 4 lane .. 4 lane + 3 of rows 2 warp, 2 warp + 1
+    float2 x[NT][2][4];
+    float4 r[NT][2], q[NT][2];
+    unsigned code[NT];    // 4 wall-adjacency bits per cell
+    unsigned valid[NT];   // a bit per cell in the grid; bit 31: no wall near the tile
+    int hsrc[NT][2];      // border values this thread reads (-1: none, a wall)
+    short hpos[NT][2];    // and their places in the tile
+    float zh[NT][2];
+    const float* pold = (it & 1) ? a.pb : a.pa;
+#pragma unroll
+    for (int k = 0; k < NT; ++k) {
+        const int t = tile_of(k), i0 = (t % a.tiles_x) * kTW, j0 = (t / a.tiles_x) * kTH;
+        const bool on = t < a.tiles;
+        const int nc = min(kTW, a.nx - i0), nr = min(kTH, a.ny - j0);
+        code[k] = 0;
+        valid[k] = on && interior_tile(a, i0, j0) ? 1u << 31 : 0u;
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+            const int row = 2 * warp + y, j = j0 + row;
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int i = i0 + 4 * lane + c;
+                x[k][y][c] = make_float2(0.f, 0.f);
+                if (on && i < a.nx && j < a.ny) {
+                    code[k] |= (unsigned)edge_bits(i, j, a.nx, a.ny, a.per_x, a.per_y) << (4 * (4 * y + c));
+                    valid[k] |= 1u << (4 * y + c);
+                    v[c] = a.r[(ptrdiff_t)j * a.pitch + i];
+                    x[k][y][c] = a.x[(size_t)j * a.xpitch + i];
+                    if (!first) P(k)[(row + 1) * kBX + 4 + 4 * lane + c] = pold[(ptrdiff_t)j * a.pitch + i];
+                }
+            }
+            r[k][y] = make_float4(v[0], v[1], v[2], v[3]);
+            q[k][y] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        // halo: the row below and above, the column west and east of the tile's
+        // cells in the grid; in the owner's border they are its last row, first
+        // row, last column, first column
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int e = tid + h * kThreads;
+            hsrc[k][h] = -1;
+            hpos[k][h] = 0;
+            zh[k][h] = 0.f;
+            if (!on || e >= kHalo) continue;
+            int gc, gj, pos, off;
+            bool in;
+            if (e < 2 * kTW) {
+                const int c = e % kTW, up = e / kTW;
+                in = c < nc;
+                gc = i0 + c;
+                gj = up ? j0 + nr : j0 - 1;
+                pos = (up ? nr + 1 : 0) * kBX + 4 + c;
+                off = (up ? 0 : kTW) + c;
+            } else {
+                const int y = (e - 2 * kTW) % kTH, east = (e - 2 * kTW) / kTH;
+                in = y < nr;
+                gj = j0 + y;
+                gc = east ? i0 + nc : i0 - 1;
+                pos = (y + 1) * kBX + 4 + (east ? nc : -1);
+                off = 2 * kTW + (east ? 0 : kTH) + y;
+            }
+            const int wc = wrap_index(gc, a.nx, a.per_x), wj = wrap_index(gj, a.ny, a.per_y);
+            if (!in || wc < 0 || wj < 0) continue;
+            hsrc[k][h] = ((wj / kTH) * a.tiles_x + wc / kTW) * kHalo + off;
+            hpos[k][h] = (short)pos;
+            const ptrdiff_t o = (ptrdiff_t)wj * a.pitch + wc;
+            zh[k][h] = tab_m[edge_bits(wc, wj, a.nx, a.ny, a.per_x, a.per_y)] * a.r[o];
+            if (!first) P(k)[pos] = pold[o];
+        }
+    }
+    __syncthreads();
+    // tiles of one block of the launch-per-phase kernels (ga and gb blocks there)
+    // add their thread sums up in turn
+    const int na = ga < a.tiles ? ga / nb : NT, nbb = gb < a.tiles ? gb / nb : NT;
+    auto add_to = [&](float (&acc)[NT], int k, int n, float v) {
+#pragma unroll
+        for (int g = 0; g < NT; ++g)
+            if (k % n == g) acc[g] = acc[g] + v;
+    };
+    auto warp_sums = [&](const float (&acc)[NT], int n, double (*out)[kThreads / 32]) {
+#pragma unroll
+        for (int g = 0; g < NT; ++g)
+            if (g < n && tile_of(g) < a.tiles) {
+                const double v = warp_fold((double)acc[g]);
+                if (lane == 0) out[g][warp] = v;
+            }
+    };
+    auto put_partial = [&](const double (*w)[kThreads / 32], int g, int n, double* part) {
+        if (g < n && tile_of(g) < a.tiles && lane == 0) {
+            double t = w[g][0];
+            for (int k = 1; k < kThreads / 32; ++k) t = t + w[g][k];
+            __stcg(part + tile_of(g), t);
+        }
+    };
+    double* const partA = a.part0;
+    double* const partB0 = a.part0 + a.tiles;
+    double* const partB1 = partB0 + a.tiles;
+    const int nwa = min(kThreads / 32, (ga + 31) / 32), nwb = min(kThreads / 32, (gb + 31) / 32);
+    int status = ST_RUNNING, inner = ST_RUNNING;
+    float beta = (float)beta64;
+    for (;;) {
+        // ---- A: direction, A p, p.q
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+            float* p = P(k);
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+                float4* pv = reinterpret_cast<float4*>(p + (2 * warp + y + 1) * kBX + 4 + 4 * lane);
+                const unsigned cd = code[k] >> (16 * y), vd = valid[k] >> (4 * y);
+                float4 o = *pv, z = r[k][y];
+                z.x = tab_m[cd & 15u] * z.x;
+                z.y = tab_m[cd >> 4 & 15u] * z.y;
+                z.z = tab_m[cd >> 8 & 15u] * z.z;
+                z.w = tab_m[cd >> 12 & 15u] * z.w;
+                if (!first) {
+                    z.x = fmaf(beta, o.x, z.x);
+                    z.y = fmaf(beta, o.y, z.y);
+                    z.z = fmaf(beta, o.z, z.z);
+                    z.w = fmaf(beta, o.w, z.w);
+                }
+                // (beyond the grid's edge the halo values stay)
+                if ((vd & 15u) == 15u) {
+                    *pv = z;
+                } else {
+                    float* f = reinterpret_cast<float*>(pv);
+                    if (vd & 1u) f[0] = z.x;
+                    if (vd & 2u) f[1] = z.y;
+                    if (vd & 4u) f[2] = z.z;
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (hsrc[k][h] >= 0) {
+                    float& v = p[hpos[k][h]];
+                    v = first ? zh[k][h] : fmaf(beta, v, zh[k][h]);
+                }
+        }
+        first = false;
+        __syncthreads();
+        float acc[NT];
+#pragma unroll
+        for (int k = 0; k < NT; ++k) acc[k] = 0.f;
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+            float part = 0.f;
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+                const float* rc = P(k) + (2 * warp + y + 1) * kBX + 4 + 4 * lane;
+                const float4 pc = *reinterpret_cast<const float4*>(rc);
+                const float4 pu = *reinterpret_cast<const float4*>(rc - kBX);
+                const float4 pd = *reinterpret_cast<const float4*>(rc + kBX);
+                const float left = rc[-1], right = rc[4];
+                const unsigned cd = code[k] >> (16 * y), vd = valid[k] >> (4 * y);
+                float4 v;
+                v.x = fmaf(ms, pd.x, fmaf(ms, pu.x, fmaf(ms, pc.y, fmaf(ms, left, tab_d[cd & 15u] * pc.x))));
+                v.y = fmaf(ms, pd.y, fmaf(ms, pu.y, fmaf(ms, pc.z, fmaf(ms, pc.x, tab_d[cd >> 4 & 15u] * pc.y))));
+                v.z = fmaf(ms, pd.z, fmaf(ms, pu.z, fmaf(ms, pc.w, fmaf(ms, pc.y, tab_d[cd >> 8 & 15u] * pc.z))));
+                v.w = fmaf(ms, pd.w, fmaf(ms, pu.w, fmaf(ms, right, fmaf(ms, pc.z, tab_d[cd >> 12 & 15u] * pc.w))));
+                if (vd & 1u) part = fmaf(pc.x, v.x, part);
+                if (vd & 2u) part = fmaf(pc.y, v.y, part);
+                if (vd & 4u) part = fmaf(pc.z, v.z, part);
+                if (vd & 8u) part = fmaf(pc.w, v.w, part);
+                q[k][y] = v;
+            }
+            add_to(acc, k, na, part);
+        }
+        warp_sums(acc, na, red[0]);
+        __syncthreads();
+        put_partial(red[0], warp, min(na, NT), partA);
+        grid_arrive(S);
+        arrived += nb;
+        if (!grid_wait(S, gbase + arrived + (stall ? 1u << 30 : 0u), stall ? kGridStallLimit : PC_WAIT_LIMIT)) return;
+        if (warp < nwa) {
+            const double s = warp_fold_n(strided_sum(partA, ga, tid), ga - 32 * warp);
+            if (lane == 0) ws0[warp] = s;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            double pq = ws0[0];
+            for (int k = 1; k < nwa; ++k) pq = pq + ws0[k];
+            const double al = rho / pq;
+            if (lane == 0) {
+                bc_stat = isnan(pq) ? (int)ST_NAN : (!(pq > 0.0) ? (int)ST_BREAKDOWN : (int)ST_RUNNING);
+                bc_a = al;
+                bc_f = (float)al;
+            }
+        }
+        __syncthreads();
+        if (bc_stat == ST_NAN) status = ST_NAN;
+        if (bc_stat == ST_BREAKDOWN) inner = ST_BREAKDOWN;  // FP32 noise floor: refine and restart
+        if (bc_stat != ST_RUNNING) break;
+        alpha64 = bc_a;
+        const float alpha = bc_f, malpha = -alpha;
+        // ---- B: residual, z, border, r.z and r.r
+        float az[NT], ar[NT];
+#pragma unroll
+        for (int k = 0; k < NT; ++k) az[k] = ar[k] = 0.f;
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+            const int t = tile_of(k);
+            const int nc = min(kTW, a.nx - (t % a.tiles_x) * kTW), nr = min(kTH, a.ny - (t / a.tiles_x) * kTH);
+            float* bo = border + (size_t)t * kHalo;
+            float prz = 0.f, prr = 0.f;
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+                float4 rv = r[k][y];
+                rv.x = fmaf(malpha, q[k][y].x, rv.x);
+                rv.y = fmaf(malpha, q[k][y].y, rv.y);
+                rv.z = fmaf(malpha, q[k][y].z, rv.z);
+                rv.w = fmaf(malpha, q[k][y].w, rv.w);
+                r[k][y] = rv;
+                const int row = 2 * warp + y;
+                const unsigned cd = code[k] >> (16 * y), vd = valid[k] >> (4 * y);
+                const float zs[4] = {tab_m[cd & 15u] * rv.x, tab_m[cd >> 4 & 15u] * rv.y, tab_m[cd >> 8 & 15u] * rv.z,
+                                     tab_m[cd >> 12 & 15u] * rv.w};
+                const float rs[4] = {rv.x, rv.y, rv.z, rv.w};
+                if (valid[k] >> 31) {
+                    const float s2 = fmaf(rv.w, rv.w, fmaf(rv.z, rv.z, fmaf(rv.y, rv.y, rv.x * rv.x)));
+                    prr += s2;
+                    prz = fmaf(tab_m[0], s2, prz);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (vd >> c & 1u) {
+                            prz = fmaf(rs[c], zs[c], prz);
+                            prr = fmaf(rs[c], rs[c], prr);
+                        }
+                }
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    if (!(vd >> c & 1u)) continue;
+                    const int cc = 4 * lane + c;
+                    if (row == 0) __stcg(bo + cc, zs[c]);
+                    if (row == nr - 1) __stcg(bo + kTW + cc, zs[c]);
+                    if (cc == 0) __stcg(bo + 2 * kTW + row, zs[c]);
+                    if (cc == nc - 1) __stcg(bo + 2 * kTW + kTH + row, zs[c]);
+                }
+            }
+            add_to(az, k, nbb, prz);
+            add_to(ar, k, nbb, prr);
+        }
+        warp_sums(az, nbb, red[0]);
+        warp_sums(ar, nbb, red[1]);
+        __syncthreads();
+        if (warp < kThreads / 64)
+            put_partial(red[0], warp, min(nbb, NT), partB0);
+        else
+            put_partial(red[1], warp - kThreads / 64, min(nbb, NT), partB1);
+        grid_arrive(S);
+        arrived += nb;
+#pragma unroll
+        for (int k = 0; k < NT; ++k)
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+                const float4 pc = *reinterpret_cast<const float4*>(P(k) + (2 * warp + y + 1) * kBX + 4 + 4 * lane);
+                x[k][y][0] = df_add_f(x[k][y][0], alpha * pc.x);
+                x[k][y][1] = df_add_f(x[k][y][1], alpha * pc.y);
+                x[k][y][2] = df_add_f(x[k][y][2], alpha * pc.z);
+                x[k][y][3] = df_add_f(x[k][y][3], alpha * pc.w);
+            }
+        if (!grid_wait(S, gbase + arrived)) return;
+#pragma unroll
+        for (int k = 0; k < NT; ++k)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (hsrc[k][h] >= 0) zh[k][h] = __ldcg(border + hsrc[k][h]);
+        const int wr = 2 * nwb <= kThreads / 32 ? warp - nwb : warp;
+        if (warp < nwb) {
+            const double s = warp_fold_n(strided_sum(partB0, gb, tid), gb - 32 * warp);
+            if (lane == 0) ws0[warp] = s;
+        }
+        if (wr >= 0 && wr < nwb) {
+            const double s = warp_fold_n(strided_sum(partB1, gb, wr * 32 + lane), gb - 32 * wr);
+            if (lane == 0) ws1[wr] = s;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            double rz = ws0[0];
+            for (int k = 1; k < nwb; ++k) rz = rz + ws0[k];
+            const double be = rz / rho;
+            if (lane == 0) {
+                bc_a = be;
+                bc_b = rz;
+                bc_f = (float)be;
+            }
+        } else if (warp == 1) {
+            double t = ws1[0];
+            for (int k = 1; k < nwb; ++k) t = t + ws1[k];
+            if (lane == 0) bc_c = t;
+        }
+        __syncthreads();
+        beta64 = bc_a;
+        beta = bc_f;
+        rho_prev = rho;
+        rho = bc_b;
+        rr = bc_c;
+        if (rr > rr0) rr0 = rr;
+        ++it;
+        ++iter;
+        // reliable update when the recursive residual fell by delta since the
+        // last one, or already looks converged
+        if (isnan(rr))
+            status = ST_NAN;
+        else if (rr <= S->tau2 * rr0 || rr <= S->target2)
+            inner = ST_CONVERGED;
+        else if (iter >= max_iter)
+            inner = ST_MAXIT;
+        if (status != ST_RUNNING || inner != ST_RUNNING || it >= it_end) break;
+    }
+    float* pnew = (it & 1) ? a.pb : a.pa;
+#pragma unroll
+    for (int k = 0; k < NT; ++k) {
+        const int t = tile_of(k), i0 = (t % a.tiles_x) * kTW, j0 = (t / a.tiles_x) * kTH;
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+            const int row = 2 * warp + y, j = j0 + row;
+            const float rs[4] = {r[k][y].x, r[k][y].y, r[k][y].z, r[k][y].w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                if (!(valid[k] >> (4 * y + c) & 1u)) continue;
+                const int i = i0 + 4 * lane + c;
+                a.x[(size_t)j * a.xpitch + i] = x[k][y][c];
+                a.r[(ptrdiff_t)j * a.pitch + i] = rs[c];
+                pnew[(ptrdiff_t)j * a.pitch + i] = P(k)[(row + 1) * kBX + 4 + 4 * lane + c];
+            }
+        }
+    }
+    if (blockIdx.x == 0 && tid == 0) {
+        S->inner_iter = it;
+        S->iter = iter;
+        S->restart = 0;
+        S->alpha_in = alpha64;
+        S->beta_in = beta64;
+        S->rho_prev = rho_prev;
+        S->rho_in = rho;
+        S->rr_in = rr;
+        S->rr_in0 = rr0;
+        S->gbar = gbase + arrived;
+        S->inner_status = inner;
+        atomicCAS(&S->status, (int)ST_RUNNING, status);  // a block's timeout stays
+    }
+}
+
+// --------------------------------------------------------------------------
 // Mixed MG-PCG helpers.  z = V-cycle(r) is written to the owned cells of z32;
 // along periodic axes its ghost ring is refreshed here (wall ghosts stay 0).
 __global__ void k_z32_ghosts(float* z, int nx, int ny, int pitch, int per_x, int per_y) {
@@ -566,6 +956,8 @@ static int make_map(cf_ctx* c, CUtensorMap* m, float* base) {
     return CF_OK;
 }
 
+static int pcg32_setup(cf_ctx* c);
+
 int cg32_setup(cf_ctx* c) {
     int rc = make_map(c, &c->map_r, c->r32b);
     if (!rc) rc = make_map(c, &c->map_pa, c->pa32b);
@@ -598,7 +990,36 @@ int cg32_setup(cf_ctx* c) {
     occ2 = occ2 < 1 ? 1 : occ2;
     c->cta32 = c->tiles < occ1 * sms ? c->tiles : occ1 * sms;
     c->cta32b = c->tiles < occ2 * sms ? c->tiles : occ2 * sms;
-    return rc;
+    return pcg32_setup(c);
+}
+
+template <int NT>
+static constexpr size_t pcg32_smem() { return sizeof(float) * NT * kBY * kBX; }
+template <int NT>
+static bool pcg32_fits(const cf_ctx* c) {
+    return all_fit(k_pcg32<NT>, c->pcg_blocks, kThreads, pcg32_smem<NT>(), c->sms);
+}
+
+// Tiles per block of the on-chip inner solve (0: the grid does not fit) and the
+// border buffer.  Up to four tiles per SM; more than one of the launch-per-phase
+// kernels' block would walk in turn only where those fill every SM alike, so that
+// one block here holds them all.
+static int pcg32_setup(cf_ctx* c) {
+    c->pcg_nu = 0;
+    const int per = (c->tiles + c->sms - 1) / c->sms;
+    if (per > kMaxTiles) return CF_OK;
+    if ((c->cta32 < c->tiles && c->cta32 % c->sms) || (c->cta32b < c->tiles && c->cta32b % c->sms)) return CF_OK;
+    const int nt = per <= 1 ? 1 : (per <= 2 ? 2 : kMaxTiles);
+    c->pcg_blocks = std::min(c->tiles, c->sms);
+    const bool fits = nt == 1 ? pcg32_fits<1>(c) : (nt == 2 ? pcg32_fits<2>(c) : pcg32_fits<kMaxTiles>(c));
+    if (!fits) return CF_OK;
+    void* p = nullptr;
+    const size_t bytes = sizeof(float) * kHalo * (size_t)c->tiles;
+    if (cudaMalloc(&p, bytes) != cudaSuccess) return fail(c, CF_ERR_NOMEM, "cudaMalloc of %zu bytes failed", bytes);
+    c->allocs.push_back(p);
+    c->pcg_border = p;
+    c->pcg_nu = nt;
+    return CF_OK;
 }
 
 // z32 (ghosted, zero) and its tensor map, for the mixed MG-PCG
@@ -641,6 +1062,20 @@ void cg32_launch_iteration(cf_ctx* c, const Stencil& st) {
     k_tma_dir_matvec32<<<c->cta32, kThreads, kStages * 2 * kSlot + 128, c->stream>>>(c->map_r, c->map_pa, c->map_pb, a);
     k_tma_update32<<<c->cta32b, kThreads, kStages * 2 * kSlot + 128, c->stream>>>(c->map_r, c->map_pa, c->map_pb,
                                                                             a);
+}
+
+// up to iters inner iterations in one launch (context with pcg_nu > 0)
+cudaError_t pcg32_launch(cf_ctx* c, const Stencil& st, int iters) {
+    const Cg32T a = cg32_args(c, st);
+    float* border = static_cast<float*>(c->pcg_border);
+    const int n = c->pcg_blocks;
+    switch (c->pcg_nu) {
+        case 1: return launch_all(k_pcg32<1>, n, kThreads, pcg32_smem<1>(), c->stream, a, border, c->cta32, c->cta32b, iters);
+        case 2: return launch_all(k_pcg32<2>, n, kThreads, pcg32_smem<2>(), c->stream, a, border, c->cta32, c->cta32b, iters);
+        default:
+            return launch_all(k_pcg32<kMaxTiles>, n, kThreads, pcg32_smem<kMaxTiles>(), c->stream, a, border, c->cta32,
+                              c->cta32b, iters);
+    }
 }
 
 // z = V-cycle(r32), its periodic ghosts, rho = r.z; returns kernels launched

@@ -62,10 +62,10 @@ struct cf_ctx {
     double* staging = nullptr;      // FP64 staging for conversions / strided copies
     size_t staging_elems = 0;
 
-    // on-chip Jacobi-PCG (cf_pcg.cu): units per block (0: the grid does not
-    // fit), blocks, and the units' border values
+    // on-chip Jacobi-PCG (cf_pcg.cu, cf_cg32.cu): units or tiles per block (0:
+    // the grid does not fit), blocks, and their border values
     int pcg_nu = 0, pcg_blocks = 0;
-    double* pcg_border = nullptr;
+    void* pcg_border = nullptr;
 
     // CUDA graphs of batches of solver iterations, rebuilt when the stencil changes
     cudaGraphExec_t g64 = nullptr, g32 = nullptr;
@@ -195,9 +195,11 @@ int project_adjoint_async(cf_ctx* c, double dt, const SolveOpts& o, SolveResult*
 int enqueue_step(cf_ctx* ctx, double dt, int value_order, const SolveOpts& so, SolveResult* r, bool* deferred,
                  bool params_ready);
 int parse_solver_opts(cf_ctx* ctx, const cf_solver_opts* opts, SolveOpts* so);
-// on-chip FP64 Jacobi-PCG (cf_pcg.cu)
+// on-chip Jacobi-PCG: FP64 (cf_pcg.cu) and the mixed solve's inner iteration
+// (cf_cg32.cu, set up with it)
 int pcg64_setup(cf_ctx* c);
 cudaError_t pcg64_launch(cf_ctx* c, const Stencil& st, int iters);
+cudaError_t pcg32_launch(cf_ctx* c, const Stencil& st, int iters);
 // FP32 TMA inner CG (cf_cg32.cu)
 int cg32_setup(cf_ctx* c);
 void cg32_launch_iteration(cf_ctx* c, const Stencil& st);

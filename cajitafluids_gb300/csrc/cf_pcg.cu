@@ -35,7 +35,7 @@
 
 #include <algorithm>
 
-#include "cf_ctx.cuh"
+#include "cf_grid.cuh"
 
 namespace cf {
 
@@ -48,10 +48,6 @@ struct PcThreads {
 constexpr int PC_PW = UNIT_PW, PC_P = UNIT_P, PC_CELLS = UNIT_CELLS, PC_BORDER = UNIT_BORDER;
 constexpr int PC_UNIT = PC_P + 2 * PC_CELLS;  // doubles per unit: p with its halo, r, q / z
 constexpr int PC_MAX_UNITS = 7;                           // units per block (181 KB of shared memory)
-// polls of a grid barrier before the launch gives up (each poll is an L2
-// round trip; a barrier takes a few of them)
-constexpr unsigned PC_WAIT_LIMIT = 1u << 22;
-
 struct Pcg64 {
     int nx, ny, per_x, per_y, G, U, pitch;
     Stencil st;
@@ -62,42 +58,14 @@ struct Pcg64 {
     int iters;                      // iterations of this launch at most
 };
 
-// Grid barrier in two halves (all blocks co-resident: cooperative launch).
-// The counter only grows: S->gbar is its value when the launch starts.
-__device__ __forceinline__ void grid_arrive(SolverState* S) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&S->gcount) : "memory");
-    }
-}
-// true when every block has arrived target times in all (bounded wait)
-__device__ __forceinline__ bool grid_wait(SolverState* S, unsigned target) {
-    bool ok = true;
-    if (threadIdx.x == 0) {
-        unsigned v, k = 0;
-        do {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&S->gcount) : "memory");
-        } while ((int)(v - target) < 0 && ++k < PC_WAIT_LIMIT);
-        ok = (int)(v - target) >= 0;
-        if (!ok) atomicExch(&S->status, (int)ST_TIMEOUT);
-    }
-    return __syncthreads_and(ok);
-}
-
-// The strided part of final_tree over n unit partials: thread t of the 256
-// adds partial[t], partial[t + 256], ... in that order.
-__device__ __forceinline__ double strided_sum(const double* part, int n, int t) {
-    double s = 0.0;
-    for (int u = t; u < n; u += CF_RED_THREADS) s = s + __ldcg(part + u);
-    return s;
-}
-
-// Lane 0's warp_fold when only the first n lanes hold values and the others
-// are zero: the exchanges that would add a zero to it are left out.
-__device__ __forceinline__ double warp_fold_n(double s, int n) {
-    for (int m = 16; m >= 1; m >>= 1)
-        if (n > m) s = s + __shfl_xor_sync(0xffffffffu, s, m);
-    return s;
+// halo cell t of a unit in the border its owner publishes (first row, last row,
+// first column, last column): the owner's last row lies below the unit, its
+// first row above, its last column west, its first column east
+__device__ __forceinline__ int border_of(int t) {
+    return t < CF_UNIT_COLS                      ? CF_UNIT_COLS + t
+           : t < 2 * CF_UNIT_COLS                ? t - CF_UNIT_COLS
+           : t < 2 * CF_UNIT_COLS + CF_BAND_ROWS ? t + CF_BAND_ROWS
+                                                 : t - CF_BAND_ROWS;
 }
 
 template <int NU>
@@ -172,12 +140,7 @@ __global__ void __launch_bounds__(PcThreads<NU>::value, 1) k_pcg64(Pcg64 a) {
         if (tid < PC_BORDER) {
             int gc, gj, pos;
             const bool in = unit_halo(UnitPos{c0, j0, nc, nr}, tid, gc, gj, pos);
-            // in the owner's border: its last row lies below us, its first row
-            // above, its last column west, its first column east
-            const int off = tid < CF_UNIT_COLS         ? CF_UNIT_COLS + tid
-                            : tid < 2 * CF_UNIT_COLS   ? tid - CF_UNIT_COLS
-                            : tid < 2 * CF_UNIT_COLS + CF_BAND_ROWS ? tid + CF_BAND_ROWS
-                                                                    : tid - CF_BAND_ROWS;
+            const int off = border_of(tid);
             const int wc = wrap_index(gc, a.nx, a.per_x), wj = wrap_index(gj, a.ny, a.per_y);
             if (in && wc >= 0 && wj >= 0) {
                 const int ou = (wj / CF_BAND_ROWS) * a.G + wc / CF_UNIT_COLS;
@@ -380,30 +343,10 @@ __global__ void __launch_bounds__(PcThreads<NU>::value, 1) k_pcg64(Pcg64 a) {
 // host side
 
 template <int NU>
-static cudaError_t launch_pcg64(cf_ctx* c, const Pcg64& a, int blocks) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(PcThreads<NU>::value);
-    cfg.dynamicSmemBytes = sizeof(double) * PC_UNIT * NU;
-    cfg.stream = c->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_pcg64<NU>, a);
-}
-
+static constexpr size_t pcg64_smem() { return sizeof(double) * PC_UNIT * NU; }
 template <int NU>
-static bool pcg64_fits(int sms, int blocks) {
-    const int smem = (int)(sizeof(double) * PC_UNIT * NU);
-    int occ = 0;
-    if (cudaFuncSetAttribute(k_pcg64<NU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pcg64<NU>, PcThreads<NU>::value, smem) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return occ * sms >= blocks;
+static bool pcg64_fits(const cf_ctx* c) {
+    return all_fit(k_pcg64<NU>, c->pcg_blocks, PcThreads<NU>::value, pcg64_smem<NU>(), c->sms);
 }
 
 // Units per block of the on-chip solve (0: the grid does not fit), and the
@@ -417,16 +360,16 @@ int pcg64_setup(cf_ctx* c) {
     if (per > PC_MAX_UNITS) return CF_OK;
     const int nu = per <= 1 ? 1 : (per <= 2 ? 2 : (per <= 4 ? 4 : PC_MAX_UNITS));
     c->pcg_blocks = std::min(c->n_units, c->sms);
-    const bool fits = nu == 1   ? pcg64_fits<1>(c->sms, c->pcg_blocks)
-                      : nu == 2 ? pcg64_fits<2>(c->sms, c->pcg_blocks)
-                      : nu == 4 ? pcg64_fits<4>(c->sms, c->pcg_blocks)
-                                : pcg64_fits<PC_MAX_UNITS>(c->sms, c->pcg_blocks);
+    const bool fits = nu == 1   ? pcg64_fits<1>(c)
+                      : nu == 2 ? pcg64_fits<2>(c)
+                      : nu == 4 ? pcg64_fits<4>(c)
+                                : pcg64_fits<PC_MAX_UNITS>(c);
     if (!fits) return CF_OK;
     void* p = nullptr;
     const size_t bytes = sizeof(double) * PC_BORDER * (size_t)c->n_units;
     if (cudaMalloc(&p, bytes) != cudaSuccess) return fail(c, CF_ERR_NOMEM, "cudaMalloc of %zu bytes failed", bytes);
     c->allocs.push_back(p);
-    c->pcg_border = static_cast<double*>(p);
+    c->pcg_border = p;
     c->pcg_nu = nu;
     return CF_OK;
 }
@@ -446,17 +389,19 @@ cudaError_t pcg64_launch(cf_ctx* c, const Stencil& st, int iters) {
     a.r = c->r.a;
     a.pa = c->pa.a;
     a.pb = c->pb.a;
-    a.border = c->pcg_border;
+    a.border = static_cast<double*>(c->pcg_border);
     a.partA = c->partials;
     a.partB0 = c->partials + c->n_units;
     a.partB1 = c->partials + 2 * (size_t)c->n_units;
     a.S = c->S;
     a.iters = iters;
+    const int n = c->pcg_blocks;
     switch (c->pcg_nu) {
-        case 1: return launch_pcg64<1>(c, a, c->pcg_blocks);
-        case 2: return launch_pcg64<2>(c, a, c->pcg_blocks);
-        case 4: return launch_pcg64<4>(c, a, c->pcg_blocks);
-        default: return launch_pcg64<PC_MAX_UNITS>(c, a, c->pcg_blocks);
+        case 1: return launch_all(k_pcg64<1>, n, PcThreads<1>::value, pcg64_smem<1>(), c->stream, a);
+        case 2: return launch_all(k_pcg64<2>, n, PcThreads<2>::value, pcg64_smem<2>(), c->stream, a);
+        case 4: return launch_all(k_pcg64<4>, n, PcThreads<4>::value, pcg64_smem<4>(), c->stream, a);
+        default:
+            return launch_all(k_pcg64<PC_MAX_UNITS>, n, PcThreads<PC_MAX_UNITS>::value, pcg64_smem<PC_MAX_UNITS>(), c->stream, a);
     }
 }
 

@@ -1588,18 +1588,20 @@ static int launch_mixed_mg_step(cf_ctx* c, const Stencil& st) {
 static const int kBatch = CF_CG_BATCH;  // CG iterations per graph launch
 static const int kBatchMG = 4;          // MG-PCG iterations per graph launch
 
-// The FP64 Jacobi-PCG runs on chip (cf_pcg.cu) where the grid fits; with
-// graphs off (cf_set_graphs) every phase stays a launch of its own.
-static bool onchip64(const cf_ctx* c) { return c->pcg_nu > 0 && !c->direct; }
+// The Jacobi-PCG (the mixed form's inner iterations) runs on chip where the grid
+// fits (pcg_nu > 0); with graphs off (cf_set_graphs) every phase stays a launch
+// of its own.  The same bits either way.
+static bool onchip(const cf_ctx* c) { return c->pcg_nu > 0 && !c->direct; }
 
 // kBatch Jacobi-PCG iterations (the body of the batch graph); returns the
 // kernels launched
 static int batch_cg(cf_ctx* c, const Stencil& st, bool mixed) {
+    if (onchip(c)) {
+        mixed ? pcg32_launch(c, st, kBatch) : pcg64_launch(c, st, kBatch);
+        return 1;
+    }
     if (mixed) {
         for (int i = 0; i < kBatch; ++i) cg32_launch_iteration(c, st);
-    } else if (onchip64(c)) {
-        pcg64_launch(c, st, kBatch);
-        return 1;
     } else {
         Cg64 a = cg64_args(c, st);
         for (int i = 0; i < kBatch; ++i) {
@@ -1773,9 +1775,14 @@ __global__ void k_loop_cond(SolverState* S, cudaGraphConditionalHandle h) {
 static int launch_iterations(cf_ctx* c, const Stencil& st, bool mixed, bool mg, int n) {
     const double scale = -st.ms;
     int k = 0;
-    if (!mixed && !mg && onchip64(c)) {
-        pcg64_launch(c, st, kResidentBatchOnchip);
-        return 1;
+    if (!mg && onchip(c)) {
+        if (!mixed) {
+            pcg64_launch(c, st, kResidentBatchOnchip);
+            return 1;
+        }
+        pcg32_launch(c, st, kResidentBatchOnchip);
+        launch_outer(c, st, 1);
+        return 2;
     }
     Cg64 a = cg64_args(c, st);
     if (mg && !mixed) {
@@ -2203,7 +2210,7 @@ int project_grids(cf_ctx* c, double dt, const SolveOpts& o, SolveResult* res, Gr
         if (warm) c->launches += launch_warm_init(c, st, false);
         const int batch = mg ? kBatchMG : kBatch;
         cudaGraphExec_t ge = mg ? c->gmg : c->g64;
-        const int per_batch = mg ? c->gmg_per_iter * kBatchMG : (onchip64(c) ? 1 : 2 * kBatch);
+        const int per_batch = mg ? c->gmg_per_iter * kBatchMG : (onchip(c) ? 1 : 2 * kBatch);
         if (mg) {
             if ((rc = launch_batch(c, c->gmg_pre, [&] { batch_mg_pre(c, st); }))) return rc;
             c->launches += c->gmg_pre_launches;
@@ -2260,7 +2267,7 @@ int project_grids(cf_ctx* c, double dt, const SolveOpts& o, SolveResult* res, Gr
                     if (c->prof) cudaEventRecord(c->ev[0], c->stream);
                     if ((rc = launch_batch(c, c->g32, [&] { batch_cg(c, st, true); }))) return rc;
                     if (c->prof) cudaEventRecord(c->ev[1], c->stream);
-                    c->launches += 2 * kBatch;
+                    c->launches += onchip(c) ? 1 : 2 * kBatch;
                     if ((rc = read_state(c))) return rc;
                     batch_profile(c, c->hS->iter - prev_iter);
                 }
