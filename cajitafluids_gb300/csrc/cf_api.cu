@@ -340,7 +340,7 @@ int cf_ctx_create(const cf_grid_desc* d, cf_ctx** out) {
     c->G = (nx + CF_UNIT_COLS - 1) / CF_UNIT_COLS;
     c->B = (ny + CF_BAND_ROWS - 1) / CF_BAND_ROWS;
     c->n_units = c->G * c->B;
-    if (!rc) rc = alloc_dev(c, c->partials, 4 * (size_t)c->n_units);
+    if (!rc) rc = alloc_dev(c, c->partials, std::max<size_t>(4 * (size_t)c->n_units, c->sms));
     if (!rc) rc = alloc_dev(c, c->S, 1);
     if (!rc) rc = alloc_dev(c, c->d_out, 4);
     c->staging_elems = (size_t)(nx + 1) * (ny + 1);

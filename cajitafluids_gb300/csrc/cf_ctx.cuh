@@ -49,7 +49,7 @@ struct cf_ctx {
     int p32 = 0;
     CUtensorMap map_r{}, map_pa{}, map_pb{};
     int tiles_x = 0, tiles = 0, cta32 = 0, cta32b = 0;
-    double* partials = nullptr;  // 4 * n_units
+    double* partials = nullptr;  // 4 * n_units, and one per SM at least
     int G = 0, B = 0, n_units = 0;
     int sms = 1;  // multiprocessors of the device (launch sizing)
     cf::SolverState* S = nullptr;   // device

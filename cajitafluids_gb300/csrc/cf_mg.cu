@@ -260,13 +260,8 @@ __global__ void __launch_bounds__(MG_BX* MG_BY) k_mg_prolong(MgLev<T> C, MgLev<T
 // k_mg_post reads it from there and writes x: a CTA of k_mg_post reads its
 // halo from other tiles, which must not be written by the same launch.
 constexpr int FT_THREADS = 256;
-// Resident blocks per SM the level kernels are compiled for: the FP32
-// 32x16 tiles fit 4 (64 registers, measured faster: 21.5 vs 24.5 us at 1024^2
-// post), the register strips and FP64 tiles keep 3 (the strips spill at 64).
-template <typename T, int TW>
-struct FtBlocks {
-    static constexpr int value = (sizeof(T) == 4 && TW == 32) ? 4 : 3;
-};
+constexpr int FT_W = 64, FT_H = 32;  // tile of the large FP32 levels
+constexpr int FT_BLOCKS = 3;         // resident blocks per SM (the strips spill at four)
 
 // index along an axis after the periodic wrap; -1 beyond a wall
 __device__ __forceinline__ int mg_dom(int g, int n, int per) {
@@ -424,20 +419,21 @@ struct RzEpi {
     double* part;
 };
 
+__device__ __forceinline__ void rz_scalars(SolverState* S, double rz) {
+    S->ticket[7] = 0;
+    const double den = S->refreshed ? S->rho_prev : S->rho_in;
+    S->refreshed = 0;
+    S->beta_in = den != 0.0 ? rz / den : 0.0;
+    S->rho_in = rz;
+    if (isnan(rz))
+        S->status = ST_NAN;
+    else if (!(rz > 0.0))
+        S->inner_status = ST_BREAKDOWN;  // FP32 noise floor: refine and restart
+}
 __device__ __forceinline__ void rz_finish(const RzEpi& E, SolverState* S, int nparts) {
     if (last_block_arrive(&S->ticket[7])) {
         const double rz = final_tree(E.part, nparts);
-        if (threadIdx.x == 0) {
-            S->ticket[7] = 0;
-            const double den = S->refreshed ? S->rho_prev : S->rho_in;
-            S->refreshed = 0;
-            S->beta_in = den != 0.0 ? rz / den : 0.0;
-            S->rho_in = rz;
-            if (isnan(rz))
-                S->status = ST_NAN;
-            else if (!(rz > 0.0))
-                S->inner_status = ST_BREAKDOWN;  // FP32 noise floor: refine and restart
-        }
+        if (threadIdx.x == 0) rz_scalars(S, rz);
     }
 }
 
@@ -753,7 +749,7 @@ __device__ __forceinline__ float strip_post(const MgLev<float>& C, const MgLev<f
 }
 
 template <typename T, int TW, int TH>
-__global__ void __launch_bounds__(FT_THREADS, FtBlocks<T, TW>::value) k_mg_pre(MgLev<T> F, MgLev<T> C, MgBc p,
+__global__ void __launch_bounds__(FT_THREADS, FT_BLOCKS) k_mg_pre(MgLev<T> F, MgLev<T> C, MgBc p,
                                                                         SolverState* S, int inner,
                                                        StripMap m) {
     if (!block_live(S, inner)) return;
@@ -870,7 +866,7 @@ __global__ void __launch_bounds__(FT_THREADS, FtBlocks<T, TW>::value) k_mg_pre(M
 }
 
 template <typename T, int TW, int TH>
-__global__ void __launch_bounds__(FT_THREADS, FtBlocks<T, TW>::value) k_mg_post(MgLev<T> C, MgLev<T> F, MgBc p,
+__global__ void __launch_bounds__(FT_THREADS, FT_BLOCKS) k_mg_post(MgLev<T> C, MgLev<T> F, MgBc p,
                                                                          SolverState* S, int inner,
                                                            StripMap m, RzEpi E) {
     if (!block_live(S, inner)) return;
@@ -1014,19 +1010,8 @@ __global__ void __launch_bounds__(FT_THREADS, FtBlocks<T, TW>::value) k_mg_post(
     if (E.on) post_epilogue(E, S, nparts, (double)rz);
 }
 
-// tile shapes: 64 x 32 (FP64: 64 x 24, both arrays in 48 KB of shared
-// memory) on large levels; 32 x 16 on levels with fewer than 1024 large tiles,
-// where more, smaller CTAs shorten the latency-bound passes
-template <typename T>
-struct FtRows {
-    static constexpr int value = 32;
-};
-template <>
-struct FtRows<double> {
-    static constexpr int value = 24;
-};
-
 #include "cf_mgc.cuh"
+#include "cf_mgt.cuh"
 
 // --------------------------------------------------------------------------
 // host side: hierarchy and the V-cycle launch sequence
@@ -1197,6 +1182,10 @@ int mg_setup(cf_ctx* c) {
         nx /= 2;
         ny /= 2;
     }
+    if (!rc && !mixed)
+        rc = cuda_check(c, cudaFuncSetAttribute(k_mg_post_rows<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)MT_POST_SMEM<double>),
+                        "multigrid level kernels: shared memory");
     if (!rc) rc = mixed ? coarse_setup(c, H, H->f) : coarse_setup(c, H, H->d);
     return rc;
 }
@@ -1291,23 +1280,29 @@ static int vcycle(cf_ctx* c, const MgHierarchy* H, MgLev<T>* lev, double scale0,
     };
     const int lb = H->lc;
     const int top_end = lb < nlev ? lb : nlev - 1;  // levels smoothed by grid kernels on the way down
-    constexpr int TH = FtRows<T>::value;
-    auto big = [&](const MgLev<T>& L) { return (long long)((L.nx + 63) / 64) * ((L.ny + TH - 1) / TH) >= 1024; };
+    // FP32 levels of at least 1024 tiles take the register strips, which recompute
+    // fewer rows but need many of them to fill the SMs (pre-smoothing, us: 2048^2 19
+    // against about 29 as windows, three times the waves of 1024^2, where the windows
+    // take 10 and the frame tiles alone took 18)
+    auto big = [&](const MgLev<T>& L) {
+        return sizeof(T) == 4 && (long long)((L.nx + FT_W - 1) / FT_W) * ((L.ny + FT_H - 1) / FT_H) >= 1024;
+    };
     auto fuse_level = [&](int l) {
         if (fused >= 0) return fused != 0;
         return sizeof(T) == 4 || (long long)lev[l].nx * lev[l].ny <= (1ll << 20);
     };
-    const int srows = sizeof(T) == 4 ? strip_rows : 0;
     for (int l = 0; l < top_end; ++l) {
         if (fuse_level(l)) {
             if (big(lev[l])) {
-                const StripMap m = strip_map(lev[l].nx, lev[l].ny, 64, TH, srows, true);
-                k_mg_pre<T, 64, TH><<<launch_blocks(m), FT_THREADS, 0, c->stream>>>(lev[l], lev[l + 1], p, c->S,
-                                                                                   inner, m);
+                if constexpr (sizeof(T) == 4) {
+                    const StripMap m = strip_map(lev[l].nx, lev[l].ny, FT_W, FT_H, strip_rows, true);
+                    k_mg_pre<T, FT_W, FT_H><<<launch_blocks(m), FT_THREADS, 0, c->stream>>>(lev[l], lev[l + 1], p, c->S,
+                                                                                          inner, m);
+                }
             } else {
-                const StripMap m = strip_map(lev[l].nx, lev[l].ny, 32, 16, 0, true);
-                k_mg_pre<T, 32, 16><<<launch_blocks(m), FT_THREADS, 0, c->stream>>>(lev[l], lev[l + 1], p, c->S,
-                                                                                   inner, m);
+                const MtGrid m = mt_grid<T>(lev[l].nx, lev[l].ny, c->sms, true);
+                k_mg_pre_rows<T><<<std::min(m.tiles, c->sms), 32 * m.rows, 0, c->stream>>>(
+                    lev[l], lev[l + 1].b, lev[l + 1].pitch, p, c->S, inner, m.tx, m.tiles);
             }
             ++launches;
             continue;
@@ -1361,13 +1356,15 @@ static int vcycle(cf_ctx* c, const MgHierarchy* H, MgLev<T>* lev, double scale0,
                 *epi_done = true;
             }
             if (big(lev[l])) {
-                const StripMap m = strip_map(lev[l].nx, lev[l].ny, 64, TH, srows, false);
-                k_mg_post<T, 64, TH><<<launch_blocks(m), FT_THREADS, 0, c->stream>>>(lev[l + 1], lev[l], p, c->S,
-                                                                                    inner, m, E);
+                if constexpr (sizeof(T) == 4) {
+                    const StripMap m = strip_map(lev[l].nx, lev[l].ny, FT_W, FT_H, strip_rows, false);
+                    k_mg_post<T, FT_W, FT_H><<<launch_blocks(m), FT_THREADS, 0, c->stream>>>(lev[l + 1], lev[l], p, c->S,
+                                                                                            inner, m, E);
+                }
             } else {
-                const StripMap m = strip_map(lev[l].nx, lev[l].ny, 32, 16, 0, false);
-                k_mg_post<T, 32, 16><<<launch_blocks(m), FT_THREADS, 0, c->stream>>>(lev[l + 1], lev[l], p, c->S,
-                                                                                    inner, m, E);
+                const MtGrid m = mt_grid<T>(lev[l].nx, lev[l].ny, c->sms, false);
+                k_mg_post_rows<T><<<std::min(m.tiles, c->sms), 32 * m.rows, MT_POST_SMEM<T>, c->stream>>>(
+                    lev[l + 1].x, lev[l + 1].pitch, lev[l], p, c->S, inner, m.tx, m.tiles, E);
             }
             ++launches;
             continue;
