@@ -218,8 +218,10 @@ __device__ void abandon(SolverState* S, const uint64_t* bars, int kfirst, int kt
     __syncthreads();
 }
 
-// K1: new direction (with halo) in shared memory, stencil, p.q
-__global__ void __launch_bounds__(kThreads, 2)
+// K1: new direction (with halo) in shared memory, stencil, p.q.  MG: on z, whose
+// preconditioner is the identity.
+template <bool MG>
+__global__ void __launch_bounds__(kThreads, MG ? 4 : 2)
     k_tma_dir_matvec32(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_pa,
                        const __grid_constant__ CUtensorMap map_pb, Cg32T a) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -227,24 +229,26 @@ __global__ void __launch_bounds__(kThreads, 2)
     // test knob: an mbarrier that nothing arrives on (cf_test_stall_wait)
     __shared__ __align__(8) uint64_t never;
     __shared__ double red[kThreads / 32];
+    __shared__ SolverState Z;  // the state on entry
     SolverState* S = a.S;
-    if (!running(S)) return;
-    const int it = S->inner_iter;
-    const bool first = it == 0 || S->restart;
-    const bool stall = S->test_stall != 0 && blockIdx.x == 0;
-    const float beta = (float)S->beta_in;
+    copy_state(&Z, S);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kStages; ++s) mbar_init(smem_u32(&bars[s]), 1);
+        mbar_init(smem_u32(&never), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (Z.status != ST_RUNNING || Z.inner_status != ST_RUNNING) return;
+    const int it = Z.inner_iter;
+    const bool first = it == 0 || Z.restart;
+    const bool stall = Z.test_stall != 0 && blockIdx.x == 0;
+    const float beta = (float)Z.beta_in;
     const CUtensorMap* map_old = (it & 1) ? &map_pb : &map_pa;
     float* pnew = (it & 1) ? a.pa : a.pb;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ntile = (a.tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
     unsigned char* sb = smem + ((128u - (smem_u32(smem) & 127u)) & 127u);  // TMA wants 128-byte slots
     auto stage_ptr = [&](int s, int arr) { return reinterpret_cast<float*>(sb + (s * 2 + arr) * kSlot); };
-    if (tid == 0) {
-        for (int s = 0; s < kStages; ++s) mbar_init(smem_u32(&bars[s]), 1);
-        mbar_init(smem_u32(&never), 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
     auto issue = [&](int k) {
         int t = (int)blockIdx.x + k * (int)gridDim.x;
         int s = k % kStages;
@@ -278,7 +282,9 @@ __global__ void __launch_bounds__(kThreads, 2)
             float4 rv = reinterpret_cast<float4*>(R)[v];
             float4 pv = reinterpret_cast<float4*>(P)[v];
             float4 o;
-            if (inner) {
+            if (MG) {
+                o = rv;
+            } else if (inner) {
                 const float m0 = a.st.minv32[0];
                 o.x = m0 * rv.x;
                 o.y = m0 * rv.y;
@@ -321,10 +327,19 @@ __global__ void __launch_bounds__(kThreads, 2)
         __syncthreads();
         if (tid == 0 && k + kStages < ntile) issue(k + kStages);
     }
-    double tot = block_sum((double)acc, red);
-    if (tid == 0) a.part0[blockIdx.x] = tot;
-    if (last_block_arrive(&S->ticket[5])) {
-        double pq = final_tree(a.part0, gridDim.x);
+    double pq;
+    bool finish;
+    if (MG) {
+        double v[1] = {warp_fold((double)acc)};
+        finish = grid_totals<1, kThreads / 32>(v, a.part0, nullptr, &S->ticket[5]);
+        pq = v[0];
+    } else {
+        const double tot = block_sum((double)acc, red);
+        if (tid == 0) a.part0[blockIdx.x] = tot;
+        finish = last_block_arrive(&S->ticket[5]);
+        if (finish) pq = final_tree(a.part0, gridDim.x);
+    }
+    if (finish) {
         if (tid == 0) {
             S->ticket[5] = 0;
             S->restart = 0;
@@ -333,7 +348,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             else if (!(pq > 0.0))
                 S->inner_status = ST_BREAKDOWN;  // FP32 noise floor: refine and restart
             else
-                S->alpha_in = S->rho_in / pq;
+                S->alpha_in = Z.rho_in / pq;
         }
     }
 }
@@ -958,6 +973,26 @@ static int make_map(cf_ctx* c, CUtensorMap* m, float* base) {
 
 static int pcg32_setup(cf_ctx* c);
 
+// K1's grid for the MG-PCG.  One tile to a CTA, with the buffers of one stage, where
+// the chip holds them all (1024^2: 512 tiles; with three stages 456 CTAs fit and 56
+// of them walk two tiles, 6.5 of 16 us); else the persistent grid.
+static int mg_k1_grid(cf_ctx* c, int sms) {
+    int occ = 0;
+    for (int stages : {1, (int)kStages}) {
+        const int smem = stages * 2 * kSlot + 128;
+        int rc = cuda_check(c, cudaFuncSetAttribute(k_tma_dir_matvec32<true>,
+                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attribute");
+        if (!rc)
+            rc = cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tma_dir_matvec32<true>, kThreads, smem),
+                            "occupancy");
+        if (rc) return rc;
+        c->cta32mg = std::min(c->tiles, std::max(occ, 1) * sms);
+        c->smem32mg = smem;
+        if (c->cta32mg == c->tiles) break;
+    }
+    return CF_OK;
+}
+
 int cg32_setup(cf_ctx* c) {
     int rc = make_map(c, &c->map_r, c->r32b);
     if (!rc) rc = make_map(c, &c->map_pa, c->pa32b);
@@ -968,7 +1003,7 @@ int cg32_setup(cf_ctx* c) {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     c->tiles_x = (c->ph.nx + kTW - 1) / kTW;
     c->tiles = c->tiles_x * ((c->ph.ny + kTH - 1) / kTH);
-    rc = cuda_check(c, cudaFuncSetAttribute(k_tma_dir_matvec32, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    rc = cuda_check(c, cudaFuncSetAttribute(k_tma_dir_matvec32<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             kStages * 2 * kSlot + 128),
                     "smem attribute");
     if (!rc)
@@ -978,7 +1013,7 @@ int cg32_setup(cf_ctx* c) {
     // persistent grids: as many CTAs as fit on the GPU at once
     int occ1 = 0, occ2 = 0;
     if (!rc)
-        rc = cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ1, k_tma_dir_matvec32, kThreads,
+        rc = cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ1, k_tma_dir_matvec32<false>, kThreads,
                                                                          kStages * 2 * kSlot + 128),
                         "occupancy");
     if (!rc)
@@ -990,6 +1025,7 @@ int cg32_setup(cf_ctx* c) {
     occ2 = occ2 < 1 ? 1 : occ2;
     c->cta32 = c->tiles < occ1 * sms ? c->tiles : occ1 * sms;
     c->cta32b = c->tiles < occ2 * sms ? c->tiles : occ2 * sms;
+    if ((rc = mg_k1_grid(c, sms))) return rc;
     return pcg32_setup(c);
 }
 
@@ -1059,7 +1095,7 @@ static Cg32T cg32_args(cf_ctx* c, const Stencil& st) {
 
 void cg32_launch_iteration(cf_ctx* c, const Stencil& st) {
     Cg32T a = cg32_args(c, st);
-    k_tma_dir_matvec32<<<c->cta32, kThreads, kStages * 2 * kSlot + 128, c->stream>>>(c->map_r, c->map_pa, c->map_pb, a);
+    k_tma_dir_matvec32<false><<<c->cta32, kThreads, kStages * 2 * kSlot + 128, c->stream>>>(c->map_r, c->map_pa, c->map_pb, a);
     k_tma_update32<<<c->cta32b, kThreads, kStages * 2 * kSlot + 128, c->stream>>>(c->map_r, c->map_pa, c->map_pb,
                                                                             a);
 }
@@ -1103,7 +1139,7 @@ void cg32_launch_pair_mg(cf_ctx* c, const Stencil& st) {
     for (int b = 0; b < 16; ++b) stz.minv32[b] = 1.0f;
     Cg32T a = cg32_args(c, stz);
     a.mg = 1;
-    k_tma_dir_matvec32<<<c->cta32, kThreads, kStages * 2 * kSlot + 128, c->stream>>>(c->map_z, c->map_pa, c->map_pb, a);
+    k_tma_dir_matvec32<true><<<c->cta32mg, kThreads, c->smem32mg, c->stream>>>(c->map_z, c->map_pa, c->map_pb, a);
     if (!c->x_only) {
         k_tma_update32<<<c->cta32b, kThreads, kStages * 2 * kSlot + 128, c->stream>>>(c->map_r, c->map_pa, c->map_pb,
                                                                                 a);

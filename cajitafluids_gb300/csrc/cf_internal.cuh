@@ -175,6 +175,78 @@ __device__ __forceinline__ double final_tree(const double* partial, int n) {
     return tot;
 }
 
+// Grid totals of NQ sums (1 or 2), where the sum order is free: v holds the warp's
+// totals in lane 0; returns true in the last block to arrive, whose warp 0 then
+// holds the grid's totals in v.  WARPS: the most warps of a block.
+// An FP64 instruction takes 64 cycles of its sub-partition and a barrier or a
+// fence by every thread waits for the block's other stores, so as little as
+// possible is done by as few warps as possible: one warp folds the block's totals
+// and arrives, four (one to a sub-partition) fold the blocks'.  The mixed
+// preconditioned CG's kernels spent 7400 (one sum) and 11500 (two) of 16000-19000
+// cycles at 64^2 in block sums, an arrival by all threads and a final_tree per sum.
+template <int NQ, int WARPS>
+__device__ __forceinline__ bool grid_totals(double (&v)[NQ], double* part0, double* part1, unsigned int* ticket) {
+    static_assert(NQ * WARPS <= 32 && (NQ == 1 || NQ == 2), "one warp folds the block's totals");
+    __shared__ double gs[32];
+    __shared__ int last;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+    if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) gs[q * WARPS + warp] = v[q];
+    }
+    __syncthreads();
+    if (warp == 0) {
+        double t = lane < NQ * WARPS && lane % WARPS < nwarp ? gs[lane] : 0.0;
+#pragma unroll
+        for (int m = WARPS / 2; m >= 1; m >>= 1) t = t + __shfl_xor_sync(0xffffffffu, t, m);
+        if (lane == 0) part0[blockIdx.x] = t;
+        if (NQ == 2 && lane == WARPS) part1[blockIdx.x] = t;
+        __syncwarp();
+        if (lane == 0) {
+            __threadfence();
+            last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    if (!last) return false;
+    constexpr int WQ = 4 / NQ;  // warps to a sum
+    const int n = gridDim.x;
+    if (warp < 4) {
+        const double* p = NQ == 2 && warp >= WQ ? part1 : part0;
+        double s = 0.0;
+        for (int k = (warp % WQ) * 32 + lane; k < n; k += CF_FOLD_BATCH * WQ * 32) {
+            double w[CF_FOLD_BATCH];
+#pragma unroll
+            for (int i = 0; i < CF_FOLD_BATCH; ++i) w[i] = k + i * WQ * 32 < n ? __ldcg(p + k + i * WQ * 32) : 0.0;
+            s = s + w[0];
+#pragma unroll
+            for (int i = 1; i < CF_FOLD_BATCH; ++i)
+                if (k + i * WQ * 32 < n) s = s + w[i];
+        }
+        s = warp_fold(s);
+        if (lane == 0) gs[warp] = s;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        double t = gs[lane & 3];
+#pragma unroll
+        for (int m = WQ / 2; m >= 1; m >>= 1) t = t + __shfl_xor_sync(0xffffffffu, t, m);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) v[q] = __shfl_sync(0xffffffffu, t, q * WQ);
+        if (lane == 0) *ticket = 0;
+    }
+    return true;
+}
+
+// The solver state copied into shared memory by the block (one trip to L2 for all
+// of it); valid after the caller's barrier.
+__device__ __forceinline__ void copy_state(SolverState* dst, const SolverState* S) {
+    static_assert(sizeof(SolverState) % 4 == 0, "copied by words");
+    if (threadIdx.x < sizeof(SolverState) / 4)
+        reinterpret_cast<int*>(dst)[threadIdx.x] = reinterpret_cast<const volatile int*>(S)[threadIdx.x];
+}
+
 __device__ __forceinline__ double final_max(const double* partial, int n) {
     __shared__ double ws[CF_RED_WARPS];
     double s = 0.0;

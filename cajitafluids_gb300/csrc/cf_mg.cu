@@ -419,9 +419,7 @@ struct RzEpi {
     double* part;
 };
 
-__device__ __forceinline__ void rz_scalars(SolverState* S, double rz) {
-    S->ticket[7] = 0;
-    const double den = S->refreshed ? S->rho_prev : S->rho_in;
+__device__ __forceinline__ void rz_scalars(SolverState* S, double rz, double den) {
     S->refreshed = 0;
     S->beta_in = den != 0.0 ? rz / den : 0.0;
     S->rho_in = rz;
@@ -433,7 +431,10 @@ __device__ __forceinline__ void rz_scalars(SolverState* S, double rz) {
 __device__ __forceinline__ void rz_finish(const RzEpi& E, SolverState* S, int nparts) {
     if (last_block_arrive(&S->ticket[7])) {
         const double rz = final_tree(E.part, nparts);
-        if (threadIdx.x == 0) rz_scalars(S, rz);
+        if (threadIdx.x == 0) {
+            S->ticket[7] = 0;
+            rz_scalars(S, rz, S->refreshed ? S->rho_prev : S->rho_in);
+        }
     }
 }
 

@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mg_post_rows(const T* cx, int
                     for (int k = 0; k < 4; ++k)
                         if (r.c0 + k < F.nx) row[r.c0 + k] = r.x[k];
                 }
-                if (E.on) {
+                if (sizeof(T) == 4 && E.on) {
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
                         const int gi = r.c0 + k, gj = r.g;
@@ -377,21 +377,18 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mg_post_rows(const T* cx, int
             }
         }
     }
-    if (E.on) {
-        __shared__ double ws[MT_THREADS / 32];
-        const double v = warp_fold((double)rz + (double)rze);
-        if (lane == 0) ws[warp] = v;
-        __syncthreads();
-        if (warp == 0) {
-            const double t = warp_fold(lane < nrow ? ws[lane] : 0.0);
-            if (lane == 0) E.part[blockIdx.x] = t;
+    if (sizeof(T) == 4 && E.on) {
+        // FP64 additions by 32 warps would take 2600 cycles: pairs until the warp's total
+#pragma unroll
+        for (int m = 16; m >= 1; m >>= 1) {
+            const T a = __shfl_xor_sync(0xffffffffu, rz, m), b = __shfl_xor_sync(0xffffffffu, rze, m);
+            const T s = rz + a, d = s - rz;
+            rze = (rze + b) + ((rz - (s - d)) + (a - d));
+            rz = s;
         }
-        if (last_block_arrive(&S->ticket[7]) && warp == 0) {
-            double t = 0.0;
-            for (int k = lane; k < (int)gridDim.x; k += 32) t = t + __ldcg(E.part + k);
-            t = warp_fold(t);
-            if (lane == 0) rz_scalars(S, t);
-        }
+        double v[1] = {(double)rz + (double)rze};
+        const double den = S->refreshed ? S->rho_prev : S->rho_in;
+        if (grid_totals<1, MT_ROWS>(v, E.part, nullptr, &S->ticket[7]) && threadIdx.x == 0) rz_scalars(S, v[0], den);
     }
 }
 

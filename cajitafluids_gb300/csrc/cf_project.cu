@@ -599,6 +599,9 @@ struct Outer {
     double *part0, *part1;
     SolverState* S;
     int gated;  // inside the MG-PCG graph: run only while the refinement is due
+    // rows of a warp's unit (U counts units of that many rows); mg: one partial per
+    // block, else one per unit of CF_BAND_ROWS rows (the Jacobi solver's sum order)
+    int rows, mg;
 };
 
 // The solution values the residual is taken of: x itself, or (fused, upd)
@@ -703,13 +706,23 @@ __device__ __forceinline__ DF2 df2_neg(DF2 x) {
     const float2 m = make_float2(-1.f, -1.f);
     return DF2{f2_mul(m, x.h), f2_mul(m, x.l)};
 }
-// df_resid_int for a lane's two cells: the residuals' high parts
-__device__ __forceinline__ float2 df2_resid_int(float2 scale, DF2 b, DF2 c, DF2 w, DF2 e, DF2 s, DF2 n) {
+// df_resid for a lane's two cells: the residuals' high parts.  d: the diagonal
+// factors; without walls next to the unit 4, and 4 x is exact.
+template <bool WALL>
+__device__ __forceinline__ float2 df2_resid(float2 scale, float2 d, DF2 b, DF2 c, DF2 w, DF2 e, DF2 s, DF2 n) {
     DF2 nb = df2_add_s(w, e);
     nb = df2_add_s(nb, s);
     nb = df2_add_s(nb, n);
-    const float2 four = make_float2(4.f, 4.f);
-    const DF2 t = df2_add_s(DF2{f2_mul(four, c.h), f2_mul(four, c.l)}, df2_neg(nb));
+    DF2 dc;
+    if (WALL) {  // df_mul((d, 0), c)
+        const float2 p = f2_mul(d, c.h);
+        const float2 er = f2_fma(d, c.h, f2_mul(make_float2(-1.f, -1.f), p));
+        dc = df2_quick(p, f2_fma(d, c.l, er));
+    } else {
+        const float2 four = make_float2(4.f, 4.f);
+        dc = DF2{f2_mul(four, c.h), f2_mul(four, c.l)};
+    }
+    const DF2 t = df2_add_s(dc, df2_neg(nb));
     // df_mul(scale, t)
     const float2 sh = make_float2(scale.x, scale.x), sl = make_float2(scale.y, scale.y);
     const float2 p = f2_mul(sh, t.h);
@@ -721,10 +734,12 @@ __device__ __forceinline__ float2 df2_resid_int(float2 scale, DF2 b, DF2 c, DF2 
     return r.h;
 }
 
-// Interior unit (no wall next to any of its cells, whole 64-column group):
-// the same arithmetic without the boundary logic.  Along a periodic axis the
-// halo rows and columns are fetched from their wrapped positions, so every
-// full unit of a periodic domain takes this path.  The rows arrive
+// A unit whose lanes hold two cells or none: WALL = false, the interior unit (no
+// wall next to any of its cells, whole 64-column group); WALL = true, a unit next
+// to a wall or at the end of a row (nx even, and not 2 more than whole groups,
+// where one lane would hold both edges): rows and columns beyond a wall are zero,
+// the diagonal factor follows the cell.  Along a periodic axis the halo rows and
+// columns are fetched from their wrapped positions.  The rows arrive
 // through a per-warp cp.async ring OR_RING - 1 rows ahead (group k: x (and,
 // fused, p) of row j0 - 1 + k, and for the unit's own rows b; the outer
 // columns' neighbours of lanes 0 and 31); each lane reads back only what it
@@ -735,25 +750,28 @@ template <bool FUSED>
 struct OrSlot {
     static constexpr int value = FUSED ? 332 : 264;  // 16-byte multiples
 };
-template <bool FUSED>
-__device__ __forceinline__ void outer_unit_interior(const Outer& a, const XSrc& xs, float2* xo, float* ring, int lane,
+template <bool FUSED, bool WALL>
+__device__ __forceinline__ void outer_unit_ring(const Outer& a, const XSrc& xs, float2* xo, float* ring, int lane,
                                                     int c0, int j0, int j1, float& arz, float& arr) {
     constexpr int SLOT = OrSlot<FUSED>::value;
     const bool upd = FUSED && xs.upd;
     const float m0 = a.minv32[0];
-    const bool edge = lane == 0 || lane == 31;
-    int ec = lane == 0 ? c0 - 1 : c0 + 2;  // outer neighbour column of lanes 0 and 31 (wrapped)
+    const bool act = !WALL || c0 < a.nx;
+    const bool east = WALL ? act && (lane == 31 || c0 + 2 == a.nx) : lane == 31;
+    int ec = lane == 0 ? c0 - 1 : c0 + 2;  // outer neighbour column of the edge lanes (wrapped)
+    const bool edge = (lane == 0 || east) && (!WALL || a.per_x || (ec >= 0 && ec < a.nx));
     ec = ec < 0 ? ec + a.nx : (ec >= a.nx ? ec - a.nx : ec);
+    auto row_in = [&](int row) { return !WALL || a.per_y || (row >= 0 && row < a.ny); };
     // periodic ghost copies of r: columns 0 and nx - 1, rows 0 and ny - 1
     const bool gx0 = a.per_x && c0 == 0, gx1 = a.per_x && c0 + 2 == a.nx;
     const bool ghosts = __any_sync(FULLMASK, gx0 || gx1) || (a.per_y && (j0 == 0 || j1 == a.ny));
-    const int eo = 256 + (lane == 31 ? 2 : 0);
-    const int eop = 328 + (lane == 31 ? 1 : 0);
+    const int eo = 256 + (lane == 0 ? 0 : 2);
+    const int eop = 328 + (lane == 0 ? 0 : 1);
     const int last = j1;                         // groups cover rows j0 - 1 .. j1
     auto issue = [&](int k) {
         const int row = j0 - 1 + k;
         float* sl = ring + (k % OR_RING) * SLOT;
-        if (row <= last) {
+        if (row <= last && act && row_in(row)) {
             const int pr = row < 0 ? row + a.ny : (row >= a.ny ? row - a.ny : row);  // wrapped halo row
             const size_t o = (size_t)pr * a.pitch;
             cpa16(sl + 4 * lane, xs.x + o + c0);
@@ -767,6 +785,7 @@ __device__ __forceinline__ void outer_unit_interior(const Outer& a, const XSrc& 
         cpa_commit();
     };
     auto xrow = [&](int k) {
+        if (!act || !row_in(j0 - 1 + k)) return make_float4(0.f, 0.f, 0.f, 0.f);
         const float* sl = ring + (k % OR_RING) * SLOT;
         float4 v = *reinterpret_cast<const float4*>(sl + 4 * lane);
         if (upd) {
@@ -781,7 +800,7 @@ __device__ __forceinline__ void outer_unit_interior(const Outer& a, const XSrc& 
         return *reinterpret_cast<const float4*>(ring + (k % OR_RING) * SLOT + 128 + 4 * lane);
     };
     auto erow = [&](int k) {
-        if (!edge) return make_float2(0.f, 0.f);
+        if (!edge || !row_in(j0 - 1 + k)) return make_float2(0.f, 0.f);
         const float* sl = ring + (k % OR_RING) * SLOT;
         float2 v = *reinterpret_cast<const float2*>(sl + eo);
         if (upd) v = df_add_f(v, xs.alpha * sl[eop]);
@@ -798,7 +817,7 @@ __device__ __forceinline__ void outer_unit_interior(const Outer& a, const XSrc& 
     float2 ev = erow(1);
     for (int j = j0; j < j1; ++j) {
         const int k = j - j0 + 2;  // group of row j + 1
-        if (upd) *reinterpret_cast<float4*>(xo + (size_t)j * a.pitch + c0) = xc;
+        if (upd && act) *reinterpret_cast<float4*>(xo + (size_t)j * a.pitch + c0) = xc;
         issue(k + OR_RING - 1);
         cpa_wait<OR_RING - 1>();
         const float4 xp = xrow(k), bn = brow(k);
@@ -806,34 +825,43 @@ __device__ __forceinline__ void outer_unit_interior(const Outer& a, const XSrc& 
         float2 left = make_float2(__shfl_up_sync(FULLMASK, xc.z, 1), __shfl_up_sync(FULLMASK, xc.w, 1));
         float2 right = make_float2(__shfl_down_sync(FULLMASK, xc.x, 1), __shfl_down_sync(FULLMASK, xc.y, 1));
         if (lane == 0) left = ev;
-        if (lane == 31) right = ev;
+        if (east) right = ev;
         // cell c0: W = left, E = the lane's second cell; cell c0 + 1: W = the
         // first cell, E = right
-        const float2 rr2 = df2_resid_int(a.scale, DF2{make_float2(bv.x, bv.z), make_float2(bv.y, bv.w)},
+        float2 d = make_float2(4.f, 4.f), m = make_float2(m0, m0);
+        if (WALL && act) {
+            const int e0 = edge_bits(c0, j, a.nx, a.ny, a.per_x, a.per_y);
+            const int e1 = edge_bits(c0 + 1, j, a.nx, a.ny, a.per_x, a.per_y);
+            d = make_float2(a.dfac[e0], a.dfac[e1]);
+            m = make_float2(a.minv32[e0], a.minv32[e1]);
+        }
+        const float2 rr2 = df2_resid<WALL>(a.scale, d, DF2{make_float2(bv.x, bv.z), make_float2(bv.y, bv.w)},
                                          DF2{make_float2(xc.x, xc.z), make_float2(xc.y, xc.w)},
                                          DF2{make_float2(left.x, xc.x), make_float2(left.y, xc.y)},
                                          DF2{make_float2(xc.z, right.x), make_float2(xc.w, right.y)},
                                          DF2{make_float2(xm.x, xm.z), make_float2(xm.y, xm.w)},
                                          DF2{make_float2(xp.x, xp.z), make_float2(xp.y, xp.w)});
-        const float2 r0 = make_float2(rr2.x, 0.f), r1 = make_float2(rr2.y, 0.f);
-        *reinterpret_cast<float2*>(a.r32 + (ptrdiff_t)j * a.pitch32 + c0) = make_float2(r0.x, r1.x);
-        if (ghosts) {  // periodic copies of boundary cells, as put_r32 writes them
-            float* row = a.r32 + (ptrdiff_t)j * a.pitch32;
-            if (gx0) row[a.nx] = r0.x;
-            if (gx1) row[-1] = r1.x;
-            if (a.per_y && j == 0) {
-                a.r32[(ptrdiff_t)a.ny * a.pitch32 + c0] = r0.x;
-                a.r32[(ptrdiff_t)a.ny * a.pitch32 + c0 + 1] = r1.x;
+        const float r0 = rr2.x, r1 = rr2.y;
+        if (act) {
+            *reinterpret_cast<float2*>(a.r32 + (ptrdiff_t)j * a.pitch32 + c0) = rr2;
+            if (ghosts) {  // periodic copies of boundary cells, as put_r32 writes them
+                float* row = a.r32 + (ptrdiff_t)j * a.pitch32;
+                if (gx0) row[a.nx] = r0;
+                if (gx1) row[-1] = r1;
+                if (a.per_y && j == 0) {
+                    a.r32[(ptrdiff_t)a.ny * a.pitch32 + c0] = r0;
+                    a.r32[(ptrdiff_t)a.ny * a.pitch32 + c0 + 1] = r1;
+                }
+                if (a.per_y && j == a.ny - 1) {
+                    a.r32[-(ptrdiff_t)a.pitch32 + c0] = r0;
+                    a.r32[-(ptrdiff_t)a.pitch32 + c0 + 1] = r1;
+                }
             }
-            if (a.per_y && j == a.ny - 1) {
-                a.r32[-(ptrdiff_t)a.pitch32 + c0] = r0.x;
-                a.r32[-(ptrdiff_t)a.pitch32 + c0 + 1] = r1.x;
-            }
+            arz = fmaf(r0, m.x * r0, arz);
+            arr = fmaf(r0, r0, arr);
+            arz = fmaf(r1, m.y * r1, arz);
+            arr = fmaf(r1, r1, arr);
         }
-        arz = fmaf(r0.x, m0 * r0.x, arz);
-        arr = fmaf(r0.x, r0.x, arr);
-        arz = fmaf(r1.x, m0 * r1.x, arz);
-        arr = fmaf(r1.x, r1.x, arr);
         xm = xc;
         xc = xp;
         bv = bn;
@@ -849,33 +877,25 @@ __device__ __forceinline__ void outer_unit_interior(const Outer& a, const XSrc& 
 template <bool FUSED>
 __global__ void __launch_bounds__(CF_RED_THREADS) k_outer_resid(Outer a) {
     SolverState* S = a.S;
-    __shared__ int mode_s, sel_s, it_s;
-    __shared__ float alpha_s;
-    if (threadIdx.x == 0) {
-        const int st = *(volatile const int*)&S->status, ist = *(volatile const int*)&S->inner_status;
-        int mode;  // 0: nothing to do, 1: residual of x, 2: x update and residual
-        if (FUSED)
-            mode = st != ST_RUNNING ? 0 : (ist == ST_RUNNING ? 2 : 1);
-        else
-            mode = (!a.gated || (st == ST_RUNNING && ist != ST_RUNNING)) ? 1 : 0;
-        mode_s = mode;
-        sel_s = S->xsel;
-        it_s = S->inner_iter;
-        alpha_s = (float)S->alpha_in;
-    }
+    __shared__ SolverState Z;  // the state on entry
+    copy_state(&Z, S);
     __syncthreads();
-    const int mode = mode_s;
+    int mode;  // 0: nothing to do, 1: residual of x, 2: x update and residual
+    if (FUSED)
+        mode = Z.status != ST_RUNNING ? 0 : (Z.inner_status == ST_RUNNING ? 2 : 1);
+    else
+        mode = (!a.gated || (Z.status == ST_RUNNING && Z.inner_status != ST_RUNNING)) ? 1 : 0;
     if (mode == 0) return;
-    const int sel = sel_s, it = it_s;
-    const XSrc xs{a.xbuf[sel], (it & 1) ? a.pa : a.pb, alpha_s, FUSED && mode == 2};
+    const int sel = Z.xsel, it = Z.inner_iter;
+    const XSrc xs{a.xbuf[sel], (it & 1) ? a.pa : a.pb, (float)Z.alpha_in, FUSED && mode == 2};
     float2* xo = a.xbuf[sel ^ 1];
     const int lane = threadIdx.x & 31;
     const int unit = blockIdx.x * CF_RED_WARPS + (threadIdx.x >> 5);
     float arz = 0.f, arr = 0.f;
-    // Units next to a wall along x (column groups 0 and G - 1) take the
-    // general path, several times slower than the interior one: they are
-    // numbered first, two per row band, so that they fill blocks of their own
-    // and no interior warp waits for one at the end-of-block barrier.
+    // Units next to a wall along x (column groups 0 and G - 1) are slower than
+    // interior ones (an odd nx: several times): they are numbered first, two per
+    // row band, so that they fill blocks of their own and no interior warp waits
+    // for one at the end-of-block barrier.
     int g, band;
     if (!a.per_x && a.G > 2) {
         const int nb = 2 * (a.U / a.G);
@@ -890,7 +910,7 @@ __global__ void __launch_bounds__(CF_RED_THREADS) k_outer_resid(Outer a) {
         g = unit % a.G;
         band = unit / a.G;
     }
-    const int j0u = band * CF_BAND_ROWS, j1u = min(j0u + CF_BAND_ROWS, a.ny);
+    const int j0u = band * a.rows, j1u = min(j0u + a.rows, a.ny);
     // rows j0u - 1 .. j1u and columns g * 64 - 1 .. g * 64 + 64 are read:
     // inside the domain, or wrapped along a periodic axis
     const bool full_x = (g + 1) * CF_UNIT_COLS <= a.nx;
@@ -899,8 +919,11 @@ __global__ void __launch_bounds__(CF_RED_THREADS) k_outer_resid(Outer a) {
                           (a.per_y || (j0u >= 1 && j1u + 2 <= a.ny));
     __shared__ __align__(16) float ring[CF_RED_WARPS * OR_RING * OrSlot<FUSED>::value];
     if (interior) {
-        outer_unit_interior<FUSED>(a, xs, xo, ring + (threadIdx.x >> 5) * OR_RING * OrSlot<FUSED>::value, lane,
-                                   g * CF_UNIT_COLS + 2 * lane, j0u, j1u, arz, arr);
+        outer_unit_ring<FUSED, false>(a, xs, xo, ring + (threadIdx.x >> 5) * OR_RING * OrSlot<FUSED>::value, lane,
+                                      g * CF_UNIT_COLS + 2 * lane, j0u, j1u, arz, arr);
+    } else if (unit < a.U && (a.nx & 1) == 0 && a.nx % CF_UNIT_COLS != 2) {
+        outer_unit_ring<FUSED, true>(a, xs, xo, ring + (threadIdx.x >> 5) * OR_RING * OrSlot<FUSED>::value, lane,
+                                     g * CF_UNIT_COLS + 2 * lane, j0u, j1u, arz, arr);
     } else if (unit < a.U) {
         const int c0 = g * CF_UNIT_COLS + 2 * lane;
         const int j0 = j0u;
@@ -943,49 +966,57 @@ __global__ void __launch_bounds__(CF_RED_THREADS) k_outer_resid(Outer a) {
             xp = xpp;
         }
     }
-    const double drz = (double)warp_fold_f(arz), drr = (double)warp_fold_f(arr);
-    if (unit < a.U && lane == 0) {
-        a.part0[unit] = drr;
-        a.part1[unit] = drz;
+    double v[2] = {(double)warp_fold_f(arr), (double)warp_fold_f(arz)};  // r.r, r.z
+    if (a.mg) {
+        if (!grid_totals<2, CF_RED_WARPS>(v, a.part0, a.part1, &S->ticket[4])) return;
+    } else {
+        if (unit < a.U && lane == 0) {
+            a.part0[unit] = v[0];
+            a.part1[unit] = v[1];
+        }
+        if (!last_block_arrive(&S->ticket[4])) return;
+        v[0] = final_tree(a.part0, a.U);
+        v[1] = final_tree(a.part1, a.U);
+        if (threadIdx.x == 0) S->ticket[4] = 0;
     }
-    if (last_block_arrive(&S->ticket[4])) {
-        const double rr64 = final_tree(a.part0, a.U);
-        const double rz = final_tree(a.part1, a.U);
-        const double rr = rr64;
-        if (threadIdx.x == 0) {
-            S->ticket[4] = 0;
-            if (FUSED && mode == 2) {
-                // the end of the inner step (as K2 ends it)
-                S->rho_prev = S->rho_in;
-                S->inner_iter = it + 1;
-                S->iter = S->iter + 1;
-                S->inner_status = ST_CONVERGED;
-                S->xsel = sel ^ 1;
+    if (threadIdx.x == 0) {
+        const double rr64 = v[0], rz = v[1];
+        int iter = Z.iter, ist = Z.inner_status;
+        double rho = Z.rho_prev;
+        if (FUSED && mode == 2) {
+            // the end of the inner step (as K2 ends it)
+            rho = Z.rho_in;
+            iter += 1;
+            ist = ST_CONVERGED;
+            S->rho_prev = rho;
+            S->inner_iter = it + 1;
+            S->iter = iter;
+            S->inner_status = ist;
+            S->xsel = sel ^ 1;
+        }
+        S->outer_iter = Z.outer_iter + 1;
+        S->rr = rr64;
+        S->rr_out = rr64;
+        if (isnan(rr64))
+            S->status = ST_NAN;
+        else if (converged(&Z, rr64))
+            S->status = ST_CONVERGED;
+        else if (iter >= Z.max_iter || Z.outer_iter + 1 >= Z.max_outer)
+            S->status = ST_MAXIT;
+        else {
+            // residual replacement: keep the search direction, rescale beta
+            // to the replaced residual (restart only after an FP32 breakdown)
+            if (ist == ST_BREAKDOWN) {
+                S->restart = 1;
+                S->beta_in = 0.0;
+            } else {
+                S->beta_in = rz / rho;
             }
-            S->outer_iter += 1;
-            S->rr = rr64;
-            S->rr_out = rr64;
-            if (isnan(rr64))
-                S->status = ST_NAN;
-            else if (converged(S, rr64))
-                S->status = ST_CONVERGED;
-            else if (S->iter >= S->max_iter || S->outer_iter >= S->max_outer)
-                S->status = ST_MAXIT;
-            else {
-                // residual replacement: keep the search direction, rescale beta
-                // to the replaced residual (restart only after an FP32 breakdown)
-                if (S->inner_status == ST_BREAKDOWN) {
-                    S->restart = 1;
-                    S->beta_in = 0.0;
-                } else {
-                    S->beta_in = rz / S->rho_prev;
-                }
-                S->rho_in = rz;
-                S->rr_in0 = rr;
-                S->rr_in = rr;
-                S->refreshed = 1;
-                S->inner_status = ST_RUNNING;
-            }
+            S->rho_in = rz;
+            S->rr_in0 = rr64;
+            S->rr_in = rr64;
+            S->refreshed = 1;
+            S->inner_status = ST_RUNNING;
         }
     }
 }
@@ -1517,7 +1548,7 @@ static int launch_apply(cf_ctx* c, const Press& pa, const DivArgs* norms = nullp
     return 1;
 }
 
-static Outer outer_args(cf_ctx* c, const Stencil& st, int gated) {
+static Outer outer_args(cf_ctx* c, const Stencil& st, int gated, int mg) {
     Outer oa{};
     oa.nx = c->ph.nx;
     oa.ny = c->ph.ny;
@@ -1549,15 +1580,26 @@ static Outer outer_args(cf_ctx* c, const Stencil& st, int gated) {
     oa.part1 = c->partials + c->n_units;
     oa.S = c->S;
     oa.gated = gated;
+    oa.rows = CF_BAND_ROWS;
+    oa.mg = mg;
+    if (mg) {
+        // 16 rows to a warp leave most of the chip idle on small grids: fewer while the
+        // warps are at most 16 to an SM (a 1024^2 step: 0.88 ms with 16 rows, 0.77 with
+        // 8, 0.78 with 4, whose units read half as many rows again for their halo)
+        while (oa.rows > 4 && (long long)oa.G * ((oa.ny + oa.rows / 2 - 1) / (oa.rows / 2)) <= 16ll * c->sms) oa.rows /= 2;
+        oa.U = oa.G * ((oa.ny + oa.rows - 1) / oa.rows);
+    }
     return oa;
 }
+
+static int outer_blocks(const Outer& oa) { return (oa.U + CF_RED_WARPS - 1) / CF_RED_WARPS; }
 
 // warm start: the initial residual from the previous solution (after the
 // divergence kernel), FP64 or double-float; returns kernels launched
 static int launch_warm_init(cf_ctx* c, const Stencil& st, bool mixed) {
     if (mixed) {
-        Outer oa = outer_args(c, st, 0);
-        k_outer_resid<false><<<red_blocks(c), CF_RED_THREADS, 0, c->stream>>>(oa);
+        Outer oa = outer_args(c, st, 0, 0);
+        k_outer_resid<false><<<outer_blocks(oa), CF_RED_THREADS, 0, c->stream>>>(oa);
     } else {
         Cg64 a = cg64_args(c, st);
         k_warm_resid64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a);
@@ -1565,10 +1607,10 @@ static int launch_warm_init(cf_ctx* c, const Stencil& st, bool mixed) {
     return 1;
 }
 
-// the outer refinement; gated = 1 inside the MG-PCG graph
-static void launch_outer(cf_ctx* c, const Stencil& st, int gated) {
-    Outer oa = outer_args(c, st, gated);
-    k_outer_resid<false><<<red_blocks(c), CF_RED_THREADS, 0, c->stream>>>(oa);
+// the outer refinement; gated = 1 inside a graph, mg = 1 with the MG-PCG
+static void launch_outer(cf_ctx* c, const Stencil& st, int gated, int mg) {
+    Outer oa = outer_args(c, st, gated, mg);
+    k_outer_resid<false><<<outer_blocks(oa), CF_RED_THREADS, 0, c->stream>>>(oa);
 }
 
 // one mixed MG-PCG inner iteration before its V-cycle: K1, then the x update
@@ -1577,11 +1619,11 @@ static void launch_outer(cf_ctx* c, const Stencil& st, int gated) {
 static int launch_mixed_mg_step(cf_ctx* c, const Stencil& st) {
     cg32_launch_pair_mg(c, st);
     if (c->x_only) {
-        Outer oa = outer_args(c, st, 1);
-        k_outer_resid<true><<<red_blocks(c), CF_RED_THREADS, 0, c->stream>>>(oa);
+        Outer oa = outer_args(c, st, 1, 1);
+        k_outer_resid<true><<<outer_blocks(oa), CF_RED_THREADS, 0, c->stream>>>(oa);
         return 2;
     }
-    launch_outer(c, st, 1);
+    launch_outer(c, st, 1, 1);
     return 3;
 }
 
@@ -1781,7 +1823,7 @@ static int launch_iterations(cf_ctx* c, const Stencil& st, bool mixed, bool mg, 
             return 1;
         }
         pcg32_launch(c, st, kResidentBatchOnchip);
-        launch_outer(c, st, 1);
+        launch_outer(c, st, 1, 0);
         return 2;
     }
     Cg64 a = cg64_args(c, st);
@@ -1800,7 +1842,7 @@ static int launch_iterations(cf_ctx* c, const Stencil& st, bool mixed, bool mg, 
                 cg32_launch_iteration(c, st);
                 k += 2;
                 if (i == n - 1) {
-                    launch_outer(c, st, 1);
+                    launch_outer(c, st, 1, 0);
                     k += 1;
                 }
             }
@@ -2272,7 +2314,7 @@ int project_grids(cf_ctx* c, double dt, const SolveOpts& o, SolveResult* res, Gr
                     batch_profile(c, c->hS->iter - prev_iter);
                 }
                 if (c->hS->status != ST_RUNNING) break;
-                launch_outer(c, st, 0);
+                launch_outer(c, st, 0, 0);
                 c->launches += 1;
                 if ((rc = read_state(c))) return rc;
                 if (++launches > max_launch) return fail(c, CF_ERR_NUMERIC, "mixed solver did not stop");
