@@ -49,6 +49,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include <algorithm>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -61,12 +62,37 @@ namespace cf {
 static __constant__ double ADJ_OFF[3][2] = {{0.5, 0.5}, {0.0, 0.5}, {0.5, 0.0}};
 
 struct RecKind {
-    int2* base;   // stencil start on the destination grid (local ghosted index)
     double* cx;   // x weights times the scattered value, cx[a * nt + t]
     double* wy;   // y weights, wy[b * nt + t]
     int n;        // weights per axis (2 or 4)
-    int nt, tex;  // target slots and target grid x extent
+    int nt;       // target slots
 };
+// Where a target's samples start, relative to the target: eight bits a sample (x and
+// y, four each, plus 4), the u samples of the three stages, the v samples, the
+// advected field's.  All ones: no target.
+using RecCode = unsigned long long;
+struct RecWhere {
+    RecCode* code;
+    int ex, ey;  // target grid extents
+};
+enum { REC_U = 0, REC_V = 3, REC_F = 6 };
+
+// Along an axis where the target lies o = TWO_O / 2 past a point of the destination
+// grid, a position less than a cell away has its linear sample start in [lo, hi] and
+// its taps in [lo, lo + n).
+template <int TWO_O>
+struct AjSpan {
+    static constexpr int lo = TWO_O < 0 ? -2 : -1;
+    static constexpr int hi = TWO_O > 0 ? 1 : 0;
+    static constexpr int n = TWO_O == 0 ? 3 : 4;
+};
+// twice the offsets of an entity's position from the u and v grids' points
+__host__ __device__ constexpr int off2_u(int ent, int axis) {
+    return axis == 0 ? (ent == E_FACEI ? 0 : 1) : (ent == E_FACEJ ? -1 : 0);
+}
+__host__ __device__ constexpr int off2_v(int ent, int axis) {
+    return axis == 0 ? (ent == E_FACEI ? -1 : 0) : (ent == E_FACEJ ? 0 : 1);
+}
 
 struct Samp {
     int kx, ky;
@@ -149,17 +175,38 @@ struct AdjRec {
     double dt;
     int order;
     RecKind F[3], Su[3][3], Sv[3][3];
+    RecWhere w[3];
     int* err;
     double* qclamp;  // clamp-form source: per box cell, the adjoint where the clamp fired, else 0
 };
 
-__device__ __forceinline__ void put_rec(const RecKind& R, int t, int kx, int ky, double val, const double* wx,
-                                        const double* wy, int n) {
-    R.base[t] = make_int2(kx, ky);
-    for (int a = 0; a < n; ++a) {
+// A sample a whole cell away starts one past [lo, hi] with its outermost weight zero
+// (or, for the rounding of a position, next to it): that weight is dropped, so that
+// the taps stay in the gather's window.
+template <int N>
+__device__ __forceinline__ int rec_fit(int rel, double* w, int lo, int hi) {
+    if (rel > hi) {
+#pragma unroll
+        for (int a = N - 1; a > 0; --a) w[a] = w[a - 1];
+        w[0] = 0.0;
+    } else if (rel < lo) {
+#pragma unroll
+        for (int a = 0; a < N - 1; ++a) w[a] = w[a + 1];
+        w[N - 1] = 0.0;
+    }
+    return min(max(rel, lo), hi);
+}
+template <int N>
+__device__ __forceinline__ RecCode put_rec(const RecKind& R, int t, int sample, int rx, int ry, double val, double* wx,
+                                           double* wy, int xlo, int xhi, int ylo, int yhi) {
+    rx = rec_fit<N>(rx, wx, xlo, xhi);
+    ry = rec_fit<N>(ry, wy, ylo, yhi);
+#pragma unroll
+    for (int a = 0; a < N; ++a) {
         R.cx[a * R.nt + t] = val * wx[a];
         R.wy[a * R.nt + t] = wy[a];
     }
+    return (RecCode)((rx + 4) | (ry + 4) << 4) << (8 * sample);
 }
 
 // The adjoint of an advected value through the inputs that replace it:
@@ -185,6 +232,7 @@ __device__ __forceinline__ double inputs_adjoint_gate(const Phys& p, int ent, in
 }
 
 // pass 1: one thread per owned target entity (blockIdx.z = entity type)
+template <int ORDER>
 __global__ void k_adj_records(AdjRec a) {
     const Phys& p = a.p;
     const int ent = blockIdx.z;
@@ -222,10 +270,7 @@ __global__ void k_adj_records(AdjRec a) {
     double ay = __dadd_rn(__dmul_rn(2.0 / 9.0, s0v.val), __dmul_rn(3.0 / 9.0, s1v.val));
     ay = __dadd_rn(ay, __dmul_rn(4.0 / 9.0, s2v.val));
     double tx = __dsub_rn(x0, __dmul_rn(dt, ax)), ty = __dsub_rn(y0, __dmul_rn(dt, ay));
-    if (a.order == 1)
-        samp<1>(f, p.low[ent][0], p.low[ent][1], p.rdx, tx, ty, sf);
-    else
-        samp<3>(f, p.low[ent][0], p.low[ent][1], p.rdx, tx, ty, sf);
+    samp<ORDER>(f, p.low[ent][0], p.low[ent][1], p.rdx, tx, ty, sf);
     // the gather window assumes every position moved at most one cell
     double lim = p.dx;
     if (fabs(tx - x0) > lim || fabs(ty - y0) > lim || fabs(x1 - x0) > lim || fabs(y1 - y0) > lim ||
@@ -236,15 +281,27 @@ __global__ void k_adj_records(AdjRec a) {
     // sensitivity to it there: the clamp q = max(q, Q) (the adjoint goes to
     // dL/dQ instead) and the velocity inflow (src/InflowSource.hpp:39-77)
     const double fb = inputs_adjoint_gate(p, ent, li, lj, sf.val, fbar, a.qclamp);
-    put_rec(a.F[ent], t, sf.kx, sf.ky, fb, sf.wx, sf.wy, a.order == 1 ? 2 : 4);
+    // taps within two columns and two rows of the target
+    const int nx2 = off2_u(ent, 0), ny2 = off2_u(ent, 1), mx2 = off2_v(ent, 0), my2 = off2_v(ent, 1);
+    auto lo = [](int o2) { return o2 < 0 ? -2 : -1; };
+    auto hi = [](int o2) { return o2 > 0 ? 1 : 0; };
+    auto put_u = [&](int stage, Samp& s, double val) {
+        return put_rec<2>(a.Su[ent][stage], t, REC_U + stage, s.kx - li, s.ky - lj, val, s.wx, s.wy, lo(nx2), hi(nx2),
+                          lo(ny2), hi(ny2));
+    };
+    auto put_v = [&](int stage, Samp& s, double val) {
+        return put_rec<2>(a.Sv[ent][stage], t, REC_V + stage, s.kx - li, s.ky - lj, val, s.wx, s.wy, lo(mx2), hi(mx2),
+                          lo(my2), hi(my2));
+    };
+    RecCode code = ORDER == 1 ? put_rec<2>(a.F[ent], t, REC_F, sf.kx - li, sf.ky - lj, fb, sf.wx, sf.wy, -1, 0, -1, 0)
+                              : put_rec<4>(a.F[ent], t, REC_F, sf.kx - li, sf.ky - lj, fb, sf.wx, sf.wy, -2, -1, -2, -1);
     double tbx = fb * sf.gx, tby = fb * sf.gy;
     double abx = -dt * tbx, aby = -dt * tby;
     double v0x = (2.0 / 9.0) * abx, v0y = (2.0 / 9.0) * aby;
     double v1x = (3.0 / 9.0) * abx, v1y = (3.0 / 9.0) * aby;
     double v2x = (4.0 / 9.0) * abx, v2y = (4.0 / 9.0) * aby;
     // stage 2 at (x2, y2)
-    put_rec(a.Su[ent][2], t, s2u.kx, s2u.ky, v2x, s2u.wx, s2u.wy, 2);
-    put_rec(a.Sv[ent][2], t, s2v.kx, s2v.ky, v2y, s2v.wx, s2v.wy, 2);
+    code |= put_u(2, s2u, v2x) | put_v(2, s2v, v2y);
     double x2bx = s2u.gx * v2x + s2v.gx * v2y, x2by = s2u.gy * v2x + s2v.gy * v2y;
     if (ralston) {
         v1x -= h2 * x2bx;
@@ -254,43 +311,81 @@ __global__ void k_adj_records(AdjRec a) {
         v0y -= h2 * x2by;
     }
     // stage 1 at (x1, y1)
-    put_rec(a.Su[ent][1], t, s1u.kx, s1u.ky, v1x, s1u.wx, s1u.wy, 2);
-    put_rec(a.Sv[ent][1], t, s1v.kx, s1v.ky, v1y, s1v.wx, s1v.wy, 2);
+    code |= put_u(1, s1u, v1x) | put_v(1, s1v, v1y);
     double x1bx = s1u.gx * v1x + s1v.gx * v1y, x1by = s1u.gy * v1x + s1v.gy * v1y;
     v0x -= h1 * x1bx;
     v0y -= h1 * x1by;
     // stage 0 at (x0, y0)
-    put_rec(a.Su[ent][0], t, s0u.kx, s0u.ky, v0x, s0u.wx, s0u.wy, 2);
-    put_rec(a.Sv[ent][0], t, s0v.kx, s0v.ky, v0y, s0v.wx, s0v.wy, 2);
+    code |= put_u(0, s0u, v0x) | put_v(0, s0v, v0y);
+    a.w[ent].code[t] = code;
 }
 
 struct AdjGather {
-    Grid<double> out;
-    RecKind k[10];
-    int nk;
+    Grid<double> out[3];
+    RecKind F[3], Su[3][3], Sv[3][3];
+    RecWhere w[3];
 };
 
-// pass 2: one thread per destination entity (ghosted index space)
-__global__ void k_adj_gather(AdjGather a) {
+// The contributions of target entity ENT to the destination (di, dj): of its linear
+// samples R of the destination's field (samples m0 .. m0 + 2 of the code) and, when
+// OWN, of its sample of the advected field F.  Every target whose taps can reach the
+// destination is looked at (AjSpan; the first stage's samples lie at the target
+// itself), in a fixed order.
+template <int ENT, int O2X, int O2Y, bool OWN, int NF>
+__device__ __forceinline__ double gather_ent(double acc, const RecWhere& w, const RecKind* R, int m0, const RecKind& F,
+                                             int di, int dj) {
+    constexpr int XL = AjSpan<O2X>::lo, XN = AjSpan<O2X>::n, YL = AjSpan<O2Y>::lo, YN = AjSpan<O2Y>::n;
+    constexpr int FL = NF == 4 ? -2 : -1, FN = NF == 4 ? 5 : 3;
+    constexpr int x0 = OWN ? FL : XL, x1 = OWN ? FL + FN : XL + XN, y0 = OWN ? FL : YL, y1 = OWN ? FL + FN : YL + YN;
+#pragma unroll
+    for (int ey = y0; ey < y1; ++ey)
+#pragma unroll
+        for (int ex = x0; ex < x1; ++ex) {
+            const int ti = di - ex, tj = dj - ey;
+            if ((unsigned)ti >= (unsigned)w.ex || (unsigned)tj >= (unsigned)w.ey) continue;
+            const int t = tj * w.ex + ti;
+            const RecCode code = __ldg(w.code + t);
+            auto add = [&](const RecKind& K, int sample, int n) {
+                const unsigned c = (unsigned)(code >> (8 * sample));
+                const unsigned ox = (unsigned)(ex + 4) - (c & 15u), oy = (unsigned)(ey + 4) - (c >> 4 & 15u);
+                if (ox < (unsigned)n && oy < (unsigned)n)
+                    acc = fma(__ldg(K.cx + (size_t)ox * K.nt + t), __ldg(K.wy + (size_t)oy * K.nt + t), acc);
+            };
+            if (OWN) add(F, REC_F, NF);
+            if (R && ex >= XL && ex < XL + XN && ey >= YL && ey < YL + YN) {
+                constexpr int bx = O2X < 0 ? -1 : 0, by = O2Y < 0 ? -1 : 0;  // where a half offset's own sample starts
+                const bool at0 = (O2X == 0 || ex == bx || ex == bx + 1) && (O2Y == 0 || ey == by || ey == by + 1);
+                if (at0) add(R[0], m0, 2);
+                add(R[1], m0 + 1, 2);
+                add(R[2], m0 + 2, 2);
+            }
+        }
+    return acc;
+}
+
+// pass 2: one thread per destination entity (ghosted index space; blockIdx.z = field).
+// A destination looks at the 111 samples that can reach it (u, v; q: 25) and loads a
+// target's places once for all of them: 7 x 7 targets for each of ten kinds of record,
+// each with a place of its own, took 199 us for u or v at 512^2.
+template <int NF>
+__global__ void __launch_bounds__(256) k_adj_gather(const __grid_constant__ AdjGather a) {
     const int di = blockIdx.x * blockDim.x + threadIdx.x;
     const int dj = blockIdx.y * blockDim.y + threadIdx.y;
-    if (di >= a.out.ex || dj >= a.out.ey) return;
+    const Grid<double>& out = a.out[blockIdx.z];
+    if (di >= out.ex || dj >= out.ey) return;
     double acc = 0.0;
-    for (int k = 0; k < a.nk; ++k) {
-        const RecKind& R = a.k[k];
-        const int tey = R.nt / R.tex;
-        const int j0 = max(dj - 3, 0), j1 = min(dj + 3, tey - 1);
-        const int i0 = max(di - 3, 0), i1 = min(di + 3, R.tex - 1);
-        for (int tj = j0; tj <= j1; ++tj)
-            for (int ti = i0; ti <= i1; ++ti) {
-                const int t = tj * R.tex + ti;
-                const int2 b = R.base[t];
-                const int ox = di - b.x, oy = dj - b.y;
-                if ((unsigned)ox < (unsigned)R.n && (unsigned)oy < (unsigned)R.n)
-                    acc = fma(R.cx[ox * R.nt + t], R.wy[oy * R.nt + t], acc);
-            }
+    if (blockIdx.z == 0) {
+        acc = gather_ent<E_CELL, 0, 0, true, NF>(acc, a.w[0], nullptr, 0, a.F[0], di, dj);
+    } else if (blockIdx.z == 1) {
+        acc = gather_ent<E_CELL, off2_u(E_CELL, 0), off2_u(E_CELL, 1), false, NF>(acc, a.w[0], a.Su[0], REC_U, a.F[1], di, dj);
+        acc = gather_ent<E_FACEI, 0, 0, true, NF>(acc, a.w[1], a.Su[1], REC_U, a.F[1], di, dj);
+        acc = gather_ent<E_FACEJ, off2_u(E_FACEJ, 0), off2_u(E_FACEJ, 1), false, NF>(acc, a.w[2], a.Su[2], REC_U, a.F[1], di, dj);
+    } else {
+        acc = gather_ent<E_CELL, off2_v(E_CELL, 0), off2_v(E_CELL, 1), false, NF>(acc, a.w[0], a.Sv[0], REC_V, a.F[2], di, dj);
+        acc = gather_ent<E_FACEI, off2_v(E_FACEI, 0), off2_v(E_FACEI, 1), false, NF>(acc, a.w[1], a.Sv[1], REC_V, a.F[2], di, dj);
+        acc = gather_ent<E_FACEJ, 0, 0, true, NF>(acc, a.w[2], a.Sv[2], REC_V, a.F[2], di, dj);
     }
-    a.out.at(di, dj) = acc;
+    out.at(di, dj) = acc;
 }
 
 // --------------------------------------------------------------------------
@@ -345,16 +440,8 @@ __device__ __forceinline__ void aj_outer(float* P, float s, const float* WX, con
 #pragma unroll
         for (int k = 0; k < 5; ++k) P[r * 5 + k] = fmaf(WY[r], x[k], P[r * 5 + k]);
 }
-// A linear sample at a position p = o + d of the target (o in {-1/2, 0,
-// 1/2} per axis, |d| < 1) has its stencil cell in [floor(o - 1) + 1 ..
-// floor(o + 1)] and its taps in columns [XLO, XLO + XN): o = 0: [-1, 2),
-// o = 1/2: [-1, 3), o = -1/2: [-2, 2).  Only that block of the tile is
-// touched (the same products as the full tile, without the zero terms).
-template <int TWO_O>
-struct AjSpan {
-    static constexpr int lo = TWO_O < 0 ? -2 : -1;
-    static constexpr int n = TWO_O == 0 ? 3 : 4;
-};
+// A linear sample touches only the block of the tile that AjSpan gives (the same
+// products as the full tile, without the zero terms).
 template <int TWO_OX, int TWO_OY>
 __device__ __forceinline__ void aj_lin(float* P, float s, const Lin32& l) {
     constexpr int XL = AjSpan<TWO_OX>::lo, XN = AjSpan<TWO_OX>::n;
@@ -800,6 +887,7 @@ struct AdjState {
     cudaEvent_t ev_adv[2] = {nullptr, nullptr};  // profiling: around the reverse advection
     Grid<float> aq32{}, oq32{};
     RecKind F[3], Su[3][3], Sv[3][3];
+    RecWhere rw[3];
     int* d_err = nullptr;
     double* d_rbar = nullptr;  // dL/d(rate), accumulated on the device
     double* xa = nullptr;      // the adjoint pressure between reverse steps (the warm start)
@@ -905,20 +993,20 @@ int setup_records(cf_ctx* c, AdjState* A) {
     auto mk = [&](RecKind& R, int ent, int n) {
         const Grid<double>& tg = *shapes[ent];
         R.n = n;
-        R.tex = tg.ex;
         R.nt = tg.ex * tg.ey;
-        void *b = nullptr, *x = nullptr, *y = nullptr;
-        if (!rc) rc = dalloc(c, A, &b, sizeof(int2) * R.nt);
+        void *x = nullptr, *y = nullptr;
         if (!rc) rc = dalloc(c, A, &x, sizeof(double) * n * R.nt);
         if (!rc) rc = dalloc(c, A, &y, sizeof(double) * n * R.nt);
         if (rc) return;
-        cudaMemsetAsync(b, 0x80, sizeof(int2) * R.nt, c->stream);  // empty slots: far-away stencil start
-        R.base = (int2*)b;
         R.cx = (double*)x;
         R.wy = (double*)y;
     };
     for (int e = 0; e < 3; ++e) {
         mk(A->F[e], e, 4);
+        A->rw[e] = RecWhere{nullptr, shapes[e]->ex, shapes[e]->ey};
+        const size_t nc = sizeof(RecCode) * (size_t)A->F[e].nt;
+        if (!rc) rc = dalloc(c, A, (void**)&A->rw[e].code, nc);
+        if (!rc) cudaMemsetAsync(A->rw[e].code, 0xff, nc, c->stream);  // slots without a target
         for (int s = 0; s < 3; ++s) {
             mk(A->Su[e][s], e, 2);
             mk(A->Sv[e][s], e, 2);
@@ -1184,7 +1272,6 @@ int adjoint_step(cf_ctx* c, AdjState* A, const SolveOpts& so, bool params_ready,
     // A^T at the forward state of this step
     const StateView sv = state_view(c, fwd);
     if ((rc = fill_view_ghosts(c, sv))) return rc;
-    for (int e = 0; e < 3; ++e) A->F[e].n = A->order == 1 ? 2 : 4;
     AdjRec ar;
     ar.p = p;
     ar.q = sv.q64;
@@ -1197,6 +1284,7 @@ int adjoint_step(cf_ctx* c, AdjState* A, const SolveOpts& so, bool params_ready,
     ar.order = A->order;
     for (int e = 0; e < 3; ++e) {
         ar.F[e] = A->F[e];
+        ar.w[e] = A->rw[e];
         for (int s = 0; s < 3; ++s) {
             ar.Su[e][s] = A->Su[e][s];
             ar.Sv[e][s] = A->Sv[e][s];
@@ -1204,22 +1292,31 @@ int adjoint_step(cf_ctx* c, AdjState* A, const SolveOpts& so, bool params_ready,
     }
     ar.err = A->d_err;
     ar.qclamp = A->qclamp;
-    k_adj_records<<<dim3((p.nx + 1 + 31) / 32, (p.ny + 1 + 7) / 8, 3), blk, 0, c->stream>>>(ar);
+    const dim3 grr((p.nx + 1 + 31) / 32, (p.ny + 1 + 7) / 8, 3);
+    if (A->order == 1)
+        k_adj_records<1><<<grr, blk, 0, c->stream>>>(ar);
+    else
+        k_adj_records<3><<<grr, blk, 0, c->stream>>>(ar);
     clamp_sum(c, A);
-    for (int gsel = 0; gsel < 3; ++gsel) {
-        AdjGather ag{};
-        ag.out = A->bg[gsel];
-        if (gsel == 0) {
-            ag.k[0] = A->F[0];
-            ag.nk = 1;
-        } else {
-            ag.k[0] = A->F[gsel];
-            int m = 1;
-            for (int e = 0; e < 3; ++e)
-                for (int s = 0; s < 3; ++s) ag.k[m++] = gsel == 1 ? A->Su[e][s] : A->Sv[e][s];
-            ag.nk = m;
+    AdjGather ag{};
+    int ex = 0, ey = 0;
+    for (int g = 0; g < 3; ++g) {
+        ag.out[g] = A->bg[g];
+        ex = std::max(ex, ag.out[g].ex);
+        ey = std::max(ey, ag.out[g].ey);
+        ag.F[g] = A->F[g];
+        ag.w[g] = A->rw[g];
+        for (int st = 0; st < 3; ++st) {
+            ag.Su[g][st] = A->Su[g][st];
+            ag.Sv[g][st] = A->Sv[g][st];
         }
-        k_adj_gather<<<dim3((ag.out.ex + 31) / 32, (ag.out.ey + 7) / 8), blk, 0, c->stream>>>(ag);
+    }
+    const dim3 grg((ex + 31) / 32, (ey + 7) / 8, 3);
+    if (A->order == 1)
+        k_adj_gather<2><<<grg, blk, 0, c->stream>>>(ag);
+    else
+        k_adj_gather<4><<<grg, blk, 0, c->stream>>>(ag);
+    for (int gsel = 0; gsel < 3; ++gsel) {
         int nox = p.nx + ((gsel == 1 && !p.per_x) ? 1 : 0);
         int noy = p.ny + ((gsel == 2 && !p.per_y) ? 1 : 0);
         if (p.per_x || p.per_y)
@@ -1227,7 +1324,7 @@ int adjoint_step(cf_ctx* c, AdjState* A, const SolveOpts& so, bool params_ready,
                                                                                      p.per_y);
         std::swap(A->ag[gsel], A->bg[gsel]);
     }
-    c->launches += 4 + (p.per_x || p.per_y ? 3 : 0);
+    c->launches += 2 + (p.per_x || p.per_y ? 3 : 0);
     return cuda_check(c, cudaGetLastError(), "adjoint advection");
 }
 
