@@ -55,11 +55,10 @@
 #include <vector>
 
 #include "cf_adv32.cuh"
+#include "cf_adv64.cuh"
 #include "cf_ctx.cuh"
 
 namespace cf {
-
-static __constant__ double ADJ_OFF[3][2] = {{0.5, 0.5}, {0.0, 0.5}, {0.5, 0.0}};
 
 struct RecKind {
     double* cx;   // x weights times the scattered value, cx[a * nt + t]
@@ -94,78 +93,119 @@ __host__ __device__ constexpr int off2_v(int ent, int axis) {
     return axis == 0 ? (ent == E_FACEI ? -1 : 0) : (ent == E_FACEJ ? 0 : 1);
 }
 
-struct Samp {
+// A linear sample: the cell, its weights, the value (the forward's bits) and the
+// gradient (zero along an axis where the position was clamped).
+struct Lin64 {
     int kx, ky;
-    double wx[4], wy[4];
+    double wx[2], wy[2];
     double val, gx, gy;
 };
+__device__ __forceinline__ void lin64_taps(const Phys& p, const Grid<double>& g, Lin64& s) {
+    const double* q = g.o + (size_t)s.ky * g.pitch + s.kx;
+    const double a0 = __ldg(q), a1 = __ldg(q + 1), b0 = __ldg(q + g.pitch), b1 = __ldg(q + g.pitch + 1);
+    const double ra = fma(s.wx[1], a1, s.wx[0] * a0), rb = fma(s.wx[1], b1, s.wx[0] * b0);
+    s.val = fma(s.wy[1], rb, s.wy[0] * ra);
+    s.gx = times_rdx(fma(s.wy[1], b1 - b0, s.wy[0] * (a1 - a0)), p.rdx, p.rsh);
+    s.gy = times_rdx(rb - ra, p.rdx, p.rsh);
+}
+__device__ __forceinline__ void lin64(const Phys& p, const Grid<double>& g, double lx, double ly, double x, double y,
+                                      Lin64& s) {
+    const double xi = times_rdx(x - lx, p.rdx, p.rsh), yi = times_rdx(y - ly, p.rdx, p.rsh);
+    weights64<1>(xi, g.ex, s.kx, s.wx);
+    weights64<1>(yi, g.ey, s.ky, s.wy);
+    lin64_taps(p, g, s);
+    if (outside_bits(xi, 0.0, exact_double(g.ex - 1))) s.gx = 0.0;
+    if (outside_bits(yi, 0.0, exact_double(g.ey - 1))) s.gy = 0.0;
+}
+// the sample of the first stage, at the entity itself (AdvAxis; zx, zy: the position
+// is on the grid's own points along the axis)
+__device__ __forceinline__ void lin64_at(const Phys& p, const Grid<double>& g, int kx, int ky, double sx, double tx,
+                                         double sy, double ty, bool zx, bool zy, Lin64& s) {
+    s.kx = kx;
+    s.ky = ky;
+    s.wx[0] = sx;
+    s.wx[1] = tx;
+    s.wy[0] = sy;
+    s.wy[1] = ty;
+    if (zx || zy) {
+        const double* q = g.o + (size_t)ky * g.pitch + kx;
+        const double a0 = __ldg(q), a1 = __ldg(q + 1), b0 = __ldg(q + g.pitch), b1 = __ldg(q + g.pitch + 1);
+        auto mag = [](double d) { return __double2hiint(d) & 0x7fffffff; };
+        if (max(max(mag(a0), mag(a1)), max(mag(b0), mag(b1))) < 0x7ff00000) {
+            const double ra = zx ? a0 : fma(tx, a1, sx * a0), rb = zx ? b0 : fma(tx, b1, sx * b0);
+            const double da = a1 - a0;
+            s.val = zy ? ra : fma(ty, rb, sy * ra);
+            s.gx = times_rdx(zy ? da : fma(ty, b1 - b0, sy * da), p.rdx, p.rsh);
+            s.gy = times_rdx(rb - ra, p.rdx, p.rsh);
+            return;
+        }
+    }
+    lin64_taps(p, g, s);
+}
 
-// Weights, derivative weights and the sample value / gradient, in the same
-// arithmetic as the forward sample (cf_fields.cu; clamps, integer parts and
-// int-to-double conversions on the integer pipe, exact).
+// The sample of the advected field at the trace's foot.
 template <int ORDER>
-__device__ void samp(const Grid<double>& g, double lx, double ly, double rdx, double x, double y, Samp& s) {
-    constexpr int n = ORDER == 1 ? 2 : 4;
-    double xi[2] = {(x - lx) * rdx, (y - ly) * rdx};
-    int ext[2] = {g.ex, g.ey};
-    double w[2][4], dw[2][4];
-    int k0[2];
-    bool clamped[2];
-    for (int d = 0; d < 2; ++d) {
-        double v = xi[d];
-        if (ORDER == 1) {
-            double lo = 0.0, hi = exact_double(ext[d] - 1);
-            clamped[d] = outside_bits(v, lo, hi);
-            v = clamp_bits(v, lo, hi);
-            int k = trunc_bits(v);
-            if (k > ext[d] - 2) k = ext[d] - 2;
-            double t = v - exact_double(k);
-            w[d][0] = 1.0 - t;
-            w[d][1] = t;
-            dw[d][0] = -1.0;
-            dw[d][1] = 1.0;
-            k0[d] = k;
-        } else {
-            double lo = 1.0, hi = exact_double(ext[d] - 2);
-            clamped[d] = outside_bits(v, lo, hi);
-            v = clamp_bits(v, lo, hi);
-            int k = trunc_bits(v);
-            if (k > ext[d] - 3) k = ext[d] - 3;
-            double t = v - exact_double(k);
-            double sm = 1.0 - t, t2 = t * t, t3 = t2 * t, s3 = (sm * sm) * sm;
-            w[d][0] = s3 * (1.0 / 6.0);
-            w[d][1] = fma(0.5, t3, -t2) + (2.0 / 3.0);
-            w[d][2] = fma(0.5, (t + t2) - t3, 1.0 / 6.0);
-            w[d][3] = t3 * (1.0 / 6.0);
-            dw[d][0] = -0.5 * sm * sm;
-            dw[d][1] = 1.5 * t2 - 2.0 * t;
-            dw[d][2] = -1.5 * t2 + t + 0.5;
-            dw[d][3] = 0.5 * t2;
-            k0[d] = k - 1;
-        }
+struct Foot64 {
+    static constexpr int n = ORDER == 1 ? 2 : 4;
+    int kx, ky;
+    double wx[n], wy[n];
+    double val, gx, gy;
+};
+// cubic weights (weights64's bits) and their derivatives
+__device__ __forceinline__ bool cubic64(double xi, int ext, int& k0, double* w, double* d) {
+    int k;
+    double t, s;
+    const double hi = exact_double(ext - 2);
+    cell_fraction(clamp_bits(xi, 1.0, hi), ext - 3, k, t, s);
+    const double t2 = t * t, t3 = t2 * t, s2 = s * s;
+    w[0] = (s2 * s) * (1.0 / 6.0);
+    w[1] = fma(0.5, t3, -t2) + (2.0 / 3.0);
+    w[2] = fma(0.5, (t + t2) - t3, 1.0 / 6.0);
+    w[3] = t3 * (1.0 / 6.0);
+    d[0] = -0.5 * s2;
+    d[1] = fma(1.5, t2, -2.0 * t);
+    d[2] = fma(-1.5, t2, t + 0.5);
+    d[3] = 0.5 * t2;
+    k0 = k - 1;
+    return outside_bits(xi, 1.0, hi);
+}
+__device__ __forceinline__ void foot64(const Phys& p, const Grid<double>& g, double lx, double ly, double x, double y,
+                                       Foot64<1>& f) {
+    Lin64 s;
+    lin64(p, g, lx, ly, x, y, s);
+    f.kx = s.kx;
+    f.ky = s.ky;
+    for (int a = 0; a < 2; ++a) {
+        f.wx[a] = s.wx[a];
+        f.wy[a] = s.wy[a];
     }
+    f.val = s.val;
+    f.gx = s.gx;
+    f.gy = s.gy;
+}
+__device__ __forceinline__ void foot64(const Phys& p, const Grid<double>& g, double lx, double ly, double x, double y,
+                                       Foot64<3>& f) {
+    double dx[4], dy[4];
+    const bool cx = cubic64(times_rdx(x - lx, p.rdx, p.rsh), g.ex, f.kx, f.wx, dx);
+    const bool cy = cubic64(times_rdx(y - ly, p.rdx, p.rsh), g.ey, f.ky, f.wy, dy);
     double val = 0.0, gx = 0.0, gy = 0.0;
-    for (int b = 0; b < n; ++b) {
-        const double* row = g.o + (size_t)(k0[1] + b) * g.pitch + k0[0];
-        double rs = 0.0, rd = 0.0;
-        for (int a = 0; a < n; ++a) {
-            double f = row[a];
-            rs = fma(w[0][a], f, rs);
-            rd = fma(dw[0][a], f, rd);
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        const double* row = g.o + (size_t)(f.ky + b) * g.pitch + f.kx;
+        double v = __ldg(row), rs = f.wx[0] * v, rd = dx[0] * v;
+#pragma unroll
+        for (int a = 1; a < 4; ++a) {
+            v = __ldg(row + a);
+            rs = fma(f.wx[a], v, rs);
+            rd = fma(dx[a], v, rd);
         }
-        val = fma(w[1][b], rs, val);
-        gx = fma(w[1][b], rd, gx);
-        gy = fma(dw[1][b], rs, gy);
+        val = b == 0 ? f.wy[0] * rs : fma(f.wy[b], rs, val);
+        gx = b == 0 ? f.wy[0] * rd : fma(f.wy[b], rd, gx);
+        gy = b == 0 ? dy[0] * rs : fma(dy[b], rs, gy);
     }
-    s.kx = k0[0];
-    s.ky = k0[1];
-    for (int a = 0; a < n; ++a) {
-        s.wx[a] = w[0][a];
-        s.wy[a] = w[1][a];
-    }
-    s.val = val;
-    s.gx = clamped[0] ? 0.0 : gx * rdx;
-    s.gy = clamped[1] ? 0.0 : gy * rdx;
+    f.val = val;
+    f.gx = cx ? 0.0 : times_rdx(gx, p.rdx, p.rsh);
+    f.gy = cy ? 0.0 : times_rdx(gy, p.rdx, p.rsh);
 }
 
 struct AdjRec {
@@ -231,13 +271,22 @@ __device__ __forceinline__ double inputs_adjoint_gate(const Phys& p, int ent, in
     return fabs((double)val) < fabs(p.src_vel[ent - 1]) ? 0.0 : fbar;
 }
 
-// pass 1: one thread per owned target entity (blockIdx.z = entity type)
+// pass 1: one thread per owned target entity (blockIdx.z = entity type).  Bound by the
+// FP64 pipe.  Of 306 FP64 operations a target, cells and fractions on the integer
+// pipe, the first stage's places from per-axis tables, differences instead of
+// derivative weights and the reach test on the displacements' bits leave about 200:
+// 500 -> 385 us at 512^2 (422 with one block to an SM).
 template <int ORDER>
-__global__ void k_adj_records(AdjRec a) {
+__global__ void __launch_bounds__(256, 2) k_adj_records(const __grid_constant__ AdjRec a) {
+    __shared__ AdvAxis X, Y;
     const Phys& p = a.p;
     const int ent = blockIdx.z;
-    const int gi = blockIdx.x * blockDim.x + threadIdx.x;
-    const int gj = blockIdx.y * blockDim.y + threadIdx.y;
+    const int lane = threadIdx.x, r = threadIdx.y;
+    const int gi = blockIdx.x * 32 + lane, gj = blockIdx.y * 8 + r;
+    if (r < 2)
+        fill_axis(r ? Y : X, p, ent, r, (r ? blockIdx.y * 8 : blockIdx.x * 32) + lane + CF_HALO, lane, r ? a.u.ey : a.u.ex,
+                  r ? a.v.ey : a.v.ex);
+    __syncthreads();
     const int ox = p.nx + ((ent == E_FACEI && !p.per_x) ? 1 : 0);
     const int oy = p.ny + ((ent == E_FACEJ && !p.per_y) ? 1 : 0);
     if (gi >= ox || gj >= oy) return;
@@ -246,36 +295,48 @@ __global__ void k_adj_records(AdjRec a) {
     const Grid<double>& fa = ent == E_CELL ? a.aq : (ent == E_FACEI ? a.au : a.av);
     const int t = lj * f.ex + li;
     const double fbar = fa.at(li, lj);
-    const double x0 = p.gl[0] + ((double)li + ADJ_OFF[ent][0]) * p.dx;
-    const double y0 = p.gl[1] + ((double)lj + ADJ_OFF[ent][1]) * p.dx;
+    const double x0 = X.x0[lane], y0 = Y.x0[r];
     const double dt = a.dt;
     // forward trace (src/TimeIntegrator.hpp:36-77)
-    Samp s0u, s0v, s1u, s1v, s2u, s2v, sf;
+    Lin64 s0u, s0v, s1u, s1v, s2u, s2v;
+    Foot64<ORDER> sf;
     const double ulx = p.low[E_FACEI][0], uly = p.low[E_FACEI][1];
     const double vlx = p.low[E_FACEJ][0], vly = p.low[E_FACEJ][1];
-    samp<1>(a.u, ulx, uly, p.rdx, x0, y0, s0u);
-    samp<1>(a.v, vlx, vly, p.rdx, x0, y0, s0v);
+    lin64_at(p, a.u, X.ku[lane], Y.ku[r], X.su[lane], X.tu[lane], Y.su[r], Y.tu[r], X.u0, Y.u0, s0u);
+    lin64_at(p, a.v, X.kv[lane], Y.kv[r], X.sv[lane], X.tv[lane], Y.sv[r], Y.tv[r], X.v0, Y.v0, s0v);
     const double h1 = 0.5 * dt, h2 = 0.75 * dt;
+    // the gather window assumes every position moved at most one cell; only a
+    // displacement whose bits come near a cell takes the subtraction
+    const double lim = p.dx;
+    const int near = __double2hiint(lim) - 1;
+    bool far = false;
+    auto moved = [&](double d, double x, double from) {
+        if ((__double2hiint(d) & 0x7fffffff) >= near) far = far || fabs(x - from) > lim;
+    };
     // the forward's operation order (one rounding per operation)
-    double x1 = __dsub_rn(x0, __dmul_rn(h1, s0u.val)), y1 = __dsub_rn(y0, __dmul_rn(h1, s0v.val));
-    samp<1>(a.u, ulx, uly, p.rdx, x1, y1, s1u);
-    samp<1>(a.v, vlx, vly, p.rdx, x1, y1, s1v);
+    const double d1x = __dmul_rn(h1, s0u.val), d1y = __dmul_rn(h1, s0v.val);
+    const double x1 = __dsub_rn(x0, d1x), y1 = __dsub_rn(y0, d1y);
+    moved(d1x, x1, x0);
+    moved(d1y, y1, y0);
+    lin64(p, a.u, ulx, uly, x1, y1, s1u);
+    lin64(p, a.v, vlx, vly, x1, y1, s1v);
     const bool ralston = (p.quirks & 2u) != 0;
-    double sx = ralston ? s1u.val : s0u.val, sy = ralston ? s1v.val : s0v.val;
-    double x2 = __dsub_rn(x0, __dmul_rn(h2, sx)), y2 = __dsub_rn(y0, __dmul_rn(h2, sy));
-    samp<1>(a.u, ulx, uly, p.rdx, x2, y2, s2u);
-    samp<1>(a.v, vlx, vly, p.rdx, x2, y2, s2v);
+    const double d2x = __dmul_rn(h2, ralston ? s1u.val : s0u.val), d2y = __dmul_rn(h2, ralston ? s1v.val : s0v.val);
+    const double x2 = __dsub_rn(x0, d2x), y2 = __dsub_rn(y0, d2y);
+    moved(d2x, x2, x0);
+    moved(d2y, y2, y0);
+    lin64(p, a.u, ulx, uly, x2, y2, s2u);
+    lin64(p, a.v, vlx, vly, x2, y2, s2v);
     double ax = __dadd_rn(__dmul_rn(2.0 / 9.0, s0u.val), __dmul_rn(3.0 / 9.0, s1u.val));
     ax = __dadd_rn(ax, __dmul_rn(4.0 / 9.0, s2u.val));
     double ay = __dadd_rn(__dmul_rn(2.0 / 9.0, s0v.val), __dmul_rn(3.0 / 9.0, s1v.val));
     ay = __dadd_rn(ay, __dmul_rn(4.0 / 9.0, s2v.val));
-    double tx = __dsub_rn(x0, __dmul_rn(dt, ax)), ty = __dsub_rn(y0, __dmul_rn(dt, ay));
-    samp<ORDER>(f, p.low[ent][0], p.low[ent][1], p.rdx, tx, ty, sf);
-    // the gather window assumes every position moved at most one cell
-    double lim = p.dx;
-    if (fabs(tx - x0) > lim || fabs(ty - y0) > lim || fabs(x1 - x0) > lim || fabs(y1 - y0) > lim ||
-        fabs(x2 - x0) > lim || fabs(y2 - y0) > lim)
-        atomicOr(a.err, 1);
+    const double dx = __dmul_rn(dt, ax), dy = __dmul_rn(dt, ay);
+    const double tx = __dsub_rn(x0, dx), ty = __dsub_rn(y0, dy);
+    moved(dx, tx, x0);
+    moved(dy, ty, y0);
+    if (far) atomicOr(a.err, 1);
+    foot64(p, f, p.low[ent][0], p.low[ent][1], tx, ty, sf);
     // reverse
     // inputs that replace the advected value where they fire carry no
     // sensitivity to it there: the clamp q = max(q, Q) (the adjoint goes to
@@ -285,36 +346,36 @@ __global__ void k_adj_records(AdjRec a) {
     const int nx2 = off2_u(ent, 0), ny2 = off2_u(ent, 1), mx2 = off2_v(ent, 0), my2 = off2_v(ent, 1);
     auto lo = [](int o2) { return o2 < 0 ? -2 : -1; };
     auto hi = [](int o2) { return o2 > 0 ? 1 : 0; };
-    auto put_u = [&](int stage, Samp& s, double val) {
+    auto put_u = [&](int stage, Lin64& s, double val) {
         return put_rec<2>(a.Su[ent][stage], t, REC_U + stage, s.kx - li, s.ky - lj, val, s.wx, s.wy, lo(nx2), hi(nx2),
                           lo(ny2), hi(ny2));
     };
-    auto put_v = [&](int stage, Samp& s, double val) {
+    auto put_v = [&](int stage, Lin64& s, double val) {
         return put_rec<2>(a.Sv[ent][stage], t, REC_V + stage, s.kx - li, s.ky - lj, val, s.wx, s.wy, lo(mx2), hi(mx2),
                           lo(my2), hi(my2));
     };
-    RecCode code = ORDER == 1 ? put_rec<2>(a.F[ent], t, REC_F, sf.kx - li, sf.ky - lj, fb, sf.wx, sf.wy, -1, 0, -1, 0)
-                              : put_rec<4>(a.F[ent], t, REC_F, sf.kx - li, sf.ky - lj, fb, sf.wx, sf.wy, -2, -1, -2, -1);
-    double tbx = fb * sf.gx, tby = fb * sf.gy;
-    double abx = -dt * tbx, aby = -dt * tby;
+    constexpr int flo = ORDER == 1 ? -1 : -2;
+    RecCode code = put_rec<Foot64<ORDER>::n>(a.F[ent], t, REC_F, sf.kx - li, sf.ky - lj, fb, sf.wx, sf.wy, flo, flo + 1,
+                                             flo, flo + 1);
+    const double sb = -dt * fb, abx = sb * sf.gx, aby = sb * sf.gy;
     double v0x = (2.0 / 9.0) * abx, v0y = (2.0 / 9.0) * aby;
     double v1x = (3.0 / 9.0) * abx, v1y = (3.0 / 9.0) * aby;
-    double v2x = (4.0 / 9.0) * abx, v2y = (4.0 / 9.0) * aby;
+    const double v2x = (4.0 / 9.0) * abx, v2y = (4.0 / 9.0) * aby;
     // stage 2 at (x2, y2)
     code |= put_u(2, s2u, v2x) | put_v(2, s2v, v2y);
-    double x2bx = s2u.gx * v2x + s2v.gx * v2y, x2by = s2u.gy * v2x + s2v.gy * v2y;
+    const double x2bx = fma(s2v.gx, v2y, s2u.gx * v2x), x2by = fma(s2v.gy, v2y, s2u.gy * v2x);
     if (ralston) {
-        v1x -= h2 * x2bx;
-        v1y -= h2 * x2by;
+        v1x = fma(-h2, x2bx, v1x);
+        v1y = fma(-h2, x2by, v1y);
     } else {
-        v0x -= h2 * x2bx;
-        v0y -= h2 * x2by;
+        v0x = fma(-h2, x2bx, v0x);
+        v0y = fma(-h2, x2by, v0y);
     }
     // stage 1 at (x1, y1)
     code |= put_u(1, s1u, v1x) | put_v(1, s1v, v1y);
-    double x1bx = s1u.gx * v1x + s1v.gx * v1y, x1by = s1u.gy * v1x + s1v.gy * v1y;
-    v0x -= h1 * x1bx;
-    v0y -= h1 * x1by;
+    const double x1bx = fma(s1v.gx, v1y, s1u.gx * v1x), x1by = fma(s1v.gy, v1y, s1u.gy * v1x);
+    v0x = fma(-h1, x1bx, v0x);
+    v0y = fma(-h1, x1by, v0y);
     // stage 0 at (x0, y0)
     code |= put_u(0, s0u, v0x) | put_v(0, s0v, v0y);
     a.w[ent].code[t] = code;

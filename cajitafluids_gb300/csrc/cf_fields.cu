@@ -11,11 +11,11 @@
 #include <math.h>
 
 #include "cf_adv32.cuh"
+#include "cf_adv64.cuh"
 #include "cf_ctx.cuh"
 
 namespace cf {
 
-static __constant__ double ENT_OFF_D[3][2] = {{0.5, 0.5}, {0.0, 0.5}, {0.5, 0.0}};
 
 // --------------------------------------------------------------------------
 // Ghost fill: the one-GPU form of Cajita's advection halo gather
@@ -66,28 +66,6 @@ __global__ void k_fill_ghosts(Grid<T> g, int nox, int noy, int per_x, int per_y)
 // the coordinate clamp, the cell and the linear weights come from the
 // integer-pipe helpers (cf_internal.cuh).
 template <int ORDER>
-__device__ __forceinline__ void weights64(double xi, int ext, int& k0, double* w) {
-    int k;
-    double t, s;
-    if (ORDER == 1) {
-        cell_fraction(clamp_bits(xi, 0.0, exact_double(ext - 1)), ext - 2, k, t, s);
-        w[0] = s;
-        w[1] = t;
-        k0 = k;
-    } else {
-        cell_fraction(clamp_bits(xi, 1.0, exact_double(ext - 2)), ext - 3, k, t, s);
-        double t2 = t * t;
-        double t3 = t2 * t;
-        double s3 = (s * s) * s;
-        w[0] = s3 * (1.0 / 6.0);
-        w[1] = fma(0.5, t3, -t2) + (2.0 / 3.0);
-        w[2] = fma(0.5, (t + t2) - t3, 1.0 / 6.0);
-        w[3] = t3 * (1.0 / 6.0);
-        k0 = k - 1;
-    }
-}
-
-template <int ORDER>
 __device__ double sample64(const Phys& p, const Grid<double>& g, double lx, double ly, double x, double y) {
     constexpr int n = ORDER == 1 ? 2 : 4;
     double xi = times_rdx(x - lx, p.rdx, p.rsh);
@@ -106,11 +84,6 @@ __device__ double sample64(const Phys& p, const Grid<double>& g, double lx, doub
         val = (b == 0) ? wy[0] * rs : fma(wy[b], rs, val);
     }
     return val;
-}
-
-__device__ __forceinline__ double entity_coord(const Phys& p, int ent, int axis, int idx) {
-    double t = exact_double(idx) + ENT_OFF_D[ent][axis];
-    return p.gl[axis] + t * p.dx;
 }
 
 // rk3 backtrace (src/TimeIntegrator.hpp:36-77) after its first velocity sample
@@ -221,16 +194,6 @@ struct Adv64 {
     double fdt[2];  // force * dt (fused inputs: the force is constant there)
 };
 
-// What an entity's own coordinates fix depends on its column or its row alone:
-// the coordinate, and the cells and weights of the first RK stage's samples of
-// u and v.  Two warps work them out for the block's tile.
-struct AdvAxis {
-    double x0[32];
-    double su[32], tu[32], sv[32], tv[32];
-    int ku[32], kv[32];
-    int u0, v0;  // every tu (tv) is zero: the samples sit on the grid's own points
-};
-
 // The linear sample with weights (sx, tx), (sy, ty) of the cell at q; zx, zy:
 // tx, ty are zero and sx, sy one along the whole tile, so a product with a
 // finite tap drops out exactly.
@@ -261,27 +224,8 @@ __global__ void __launch_bounds__(256) k_advect64(Adv64 a) {
     const int ent = blockIdx.z + a.ent0;
     const int gi0 = blockIdx.x * 32, gj0 = blockIdx.y * 8 * ROWS;
     const int lane = threadIdx.x, wrow = threadIdx.y;
-    if (wrow < 2) {
-        AdvAxis& A = wrow ? Y : X;
-        const double x = entity_coord(p, ent, wrow, (wrow ? gj0 : gi0) + lane + CF_HALO);
-        double w[2];
-        int k;
-        A.x0[lane] = x;
-        weights64<1>(times_rdx(x - p.low[E_FACEI][wrow], p.rdx, p.rsh), wrow ? a.u.ey : a.u.ex, k, w);
-        A.su[lane] = w[0];
-        A.tu[lane] = w[1];
-        A.ku[lane] = k;
-        const bool u0 = __all_sync(0xffffffffu, w[1] == 0.0);
-        weights64<1>(times_rdx(x - p.low[E_FACEJ][wrow], p.rdx, p.rsh), wrow ? a.v.ey : a.v.ex, k, w);
-        A.sv[lane] = w[0];
-        A.tv[lane] = w[1];
-        A.kv[lane] = k;
-        const bool v0 = __all_sync(0xffffffffu, w[1] == 0.0);
-        if (lane == 0) {
-            A.u0 = u0;
-            A.v0 = v0;
-        }
-    }
+    if (wrow < 2) fill_axis(wrow ? Y : X, p, ent, wrow, (wrow ? gj0 : gi0) + lane + CF_HALO, lane, wrow ? a.u.ey : a.u.ex,
+                            wrow ? a.v.ey : a.v.ex);
     __syncthreads();
     const int gi = gi0 + lane;
     const int ox = p.nx + ((ent == E_FACEI && !p.per_x) ? 1 : 0);
