@@ -3,6 +3,7 @@
 #pragma once
 
 #include "cf_internal.cuh"
+#include "cf_mul64.cuh"
 
 namespace cf {
 
@@ -21,13 +22,13 @@ __device__ __forceinline__ void weights64(double xi, int ext, int& k0, double* w
         k0 = k;
     } else {
         cell_fraction(clamp_bits(xi, 1.0, exact_double(ext - 2)), ext - 3, k, t, s);
-        double t2 = t * t;
-        double t3 = t2 * t;
-        double s3 = (s * s) * s;
-        w[0] = s3 * (1.0 / 6.0);
+        double t2 = mul64i(t, t);
+        double t3 = mul64i(t2, t);
+        double s3 = mul64i(mul64i(s, s), s);
+        w[0] = mul64i(s3, 1.0 / 6.0);
         w[1] = fma(0.5, t3, -t2) + (2.0 / 3.0);
         w[2] = fma(0.5, (t + t2) - t3, 1.0 / 6.0);
-        w[3] = t3 * (1.0 / 6.0);
+        w[3] = mul64i(t3, 1.0 / 6.0);
         k0 = k - 1;
     }
 }

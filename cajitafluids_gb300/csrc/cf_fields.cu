@@ -78,10 +78,10 @@ __device__ double sample64(const Phys& p, const Grid<double>& g, double lx, doub
 #pragma unroll
     for (int b = 0; b < n; ++b) {
         const double* row = g.o + (size_t)(ky + b) * g.pitch + kx;
-        double rs = wx[0] * __ldg(row);
+        double rs = mul64i(wx[0], __ldg(row));
 #pragma unroll
         for (int a = 1; a < n; ++a) rs = fma(wx[a], __ldg(row + a), rs);
-        val = (b == 0) ? wy[0] * rs : fma(wy[b], rs, val);
+        val = (b == 0) ? mul64i(wy[0], rs) : fma(wy[b], rs, val);
     }
     return val;
 }
@@ -95,22 +95,22 @@ __device__ __forceinline__ void rk3_64_from(const Phys& p, const Grid<double>& u
     // the reference's stage expressions as written, one rounding per
     // operation: x0 - 0.5 * dt * v0 is x0 - ((0.5 * dt) * v0)
     double h1 = 0.5 * dt;
-    double x1 = __dsub_rn(x0, __dmul_rn(h1, v0x)), y1 = __dsub_rn(y0, __dmul_rn(h1, v0y));
+    double x1 = __dsub_rn(x0, mul64i(h1, v0x)), y1 = __dsub_rn(y0, mul64i(h1, v0y));
     double v1x = sample64<1>(p, u, ulx, uly, x1, y1);
     double v1y = sample64<1>(p, v, vlx, vly, x1, y1);
     double h2 = 0.75 * dt;
     bool ralston = (p.quirks & 2u) != 0;
     double sx = ralston ? v1x : v0x, sy = ralston ? v1y : v0y;
-    double x2 = __dsub_rn(x0, __dmul_rn(h2, sx)), y2 = __dsub_rn(y0, __dmul_rn(h2, sy));
+    double x2 = __dsub_rn(x0, mul64i(h2, sx)), y2 = __dsub_rn(y0, mul64i(h2, sy));
     double v2x = sample64<1>(p, u, ulx, uly, x2, y2);
     double v2y = sample64<1>(p, v, vlx, vly, x2, y2);
     // x0 - dt * ((2/9) v0 + (3/9) v1 + (4/9) v2), summed left to right
-    double ax = __dadd_rn(__dmul_rn(2.0 / 9.0, v0x), __dmul_rn(3.0 / 9.0, v1x));
-    ax = __dadd_rn(ax, __dmul_rn(4.0 / 9.0, v2x));
-    double ay = __dadd_rn(__dmul_rn(2.0 / 9.0, v0y), __dmul_rn(3.0 / 9.0, v1y));
-    ay = __dadd_rn(ay, __dmul_rn(4.0 / 9.0, v2y));
-    tx = __dsub_rn(x0, __dmul_rn(dt, ax));
-    ty = __dsub_rn(y0, __dmul_rn(dt, ay));
+    double ax = __dadd_rn(mul64i(2.0 / 9.0, v0x), mul64i(3.0 / 9.0, v1x));
+    ax = __dadd_rn(ax, mul64i(4.0 / 9.0, v2x));
+    double ay = __dadd_rn(mul64i(2.0 / 9.0, v0y), mul64i(3.0 / 9.0, v1y));
+    ay = __dadd_rn(ay, mul64i(4.0 / 9.0, v2y));
+    tx = __dsub_rn(x0, mul64i(dt, ax));
+    ty = __dsub_rn(y0, mul64i(dt, ay));
 }
 
 __device__ void rk3_64(const Phys& p, const Grid<double>& u, const Grid<double>& v, double dt,
@@ -203,20 +203,22 @@ __device__ __forceinline__ double stage0_64(const double* q, int pitch, double s
     if (zx || zy) {
         auto mag = [](double d) { return __double2hiint(d) & 0x7fffffff; };
         if (max(max(mag(a0), mag(a1)), max(mag(b0), mag(b1))) < 0x7ff00000) {
-            const double ra = zx ? a0 : fma(tx, a1, sx * a0);
+            const double ra = zx ? a0 : fma(tx, a1, mul64i(sx, a0));
             if (zy) return ra;
-            const double rb = zx ? b0 : fma(tx, b1, sx * b0);
-            return fma(ty, rb, sy * ra);
+            const double rb = zx ? b0 : fma(tx, b1, mul64i(sx, b0));
+            return fma(ty, rb, mul64i(sy, ra));
         }
     }
-    return fma(ty, fma(tx, b1, sx * b0), sy * fma(tx, a1, sx * a0));
+    return fma(ty, fma(tx, b1, mul64i(sx, b0)), mul64i(sy, fma(tx, a1, mul64i(sx, a0))));
 }
 
 // Tiles of 32 columns x 8 ROWS rows.  Bound by the FP64 pipe (two operations
-// per cycle and SM; 86 % busy): of 164 FP64 operations per entity of the plain
+// per cycle and SM; 78 % busy): of 164 FP64 operations per entity of the plain
 // form, the per-axis tables take 22 (and the samples that need no product 7
-// more), the integer fractions 20, the power-of-two scale 10.  15.7 -> 10.8 ms
-// at 4096^2, 259 -> 185 us at 512^2, 40 -> 31 us at 192x160.
+// more), the integer fractions 20, the power-of-two scale 10: 15.7 -> 10.8 ms
+// at 4096^2, 259 -> 185 us at 512^2, 40 -> 31 us at 192x160.  The plain products
+// of the rest run beside it on the integer pipes (mul64i; half the issue slots
+// then): 10.8 -> 8.0 ms, 185 -> 135 us, 31 -> 24 us.
 template <int ORDER, int ROWS>
 __global__ void __launch_bounds__(256) k_advect64(Adv64 a) {
     __shared__ AdvAxis X, Y;
