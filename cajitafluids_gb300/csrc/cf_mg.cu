@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "cf_ctx.cuh"
+#include "cf_mul64.cuh"
 
 namespace cf {
 
@@ -64,6 +65,16 @@ __device__ __forceinline__ T mg_at(const MgBc& p, const T* a, int pitch, int nx,
 
 __device__ __forceinline__ double mg_fma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float mg_fma(float a, float b, float c) { return fmaf(a, b, c); }
+// plain products: FP64 ones beside the FP64 pipe (cf_mul64.cuh)
+__device__ __forceinline__ double mg_mul(double a, double b) { return mul64i(a, b); }
+__device__ __forceinline__ float mg_mul(float a, float b) { return a * b; }
+// a / 4, exact: in FP64 on the exponent
+__device__ __forceinline__ float mg_quarter(float a) { return 0.25f * a; }
+__device__ __forceinline__ double mg_quarter(double a) {
+    const unsigned hi = (unsigned)__double2hiint(a), e = hi & 0x7ff00000u;
+    if (e - 0x00300000u < 0x7fc00000u) return __hiloint2double((int)(hi - 0x00200000u), __double2loint(a));
+    return e == 0u && ((hi << 1) | (unsigned)__double2loint(a)) == 0u ? a : 0.25 * a;
+}
 
 // Kernels read the solver status once per block (a per-thread read of the one
 // status word serialises every warp of the grid on one L2 slice).
@@ -107,7 +118,7 @@ __global__ void __launch_bounds__(MG_BX* MG_BY) k_mg_smooth(MgLev<T> L, MgBc p, 
                 s = s + mg_at(p, L.x, L.pitch, L.nx, L.ny, gi, gj + 1);
             }
             T t = mg_fma(L.scale, s, L.b[row + gi]);
-            L.x[row + gi] = t * L.invd[mg_bits(p, L.nx, L.ny, gi, gj)];
+            L.x[row + gi] = mg_mul(t, L.invd[mg_bits(p, L.nx, L.ny, gi, gj)]);
         }
         const int go = 2 * pair + (1 - par);
         if (first && go < L.nx) L.x[row + go] = T(0);
@@ -124,7 +135,7 @@ __global__ void __launch_bounds__(MG_BX* MG_BY) k_mg_residual(MgLev<T> L, MgBc p
         const int gj = (blockIdx.y * MG_ROWS + rr) * MG_BY + threadIdx.y;
         if (gj >= L.ny) break;
         const size_t k = (size_t)gj * L.pitch + gi;
-        T ax = L.diag[mg_bits(p, L.nx, L.ny, gi, gj)] * L.x[k];
+        T ax = mg_mul(L.diag[mg_bits(p, L.nx, L.ny, gi, gj)], L.x[k]);
         ax = mg_fma(L.ms, mg_at(p, L.x, L.pitch, L.nx, L.ny, gi - 1, gj), ax);
         ax = mg_fma(L.ms, mg_at(p, L.x, L.pitch, L.nx, L.ny, gi + 1, gj), ax);
         ax = mg_fma(L.ms, mg_at(p, L.x, L.pitch, L.nx, L.ny, gi, gj - 1), ax);
@@ -148,50 +159,49 @@ __device__ __forceinline__ int mg_pwq(int f, int I, int nc, int per, int bclo, i
     return (parent == I ? wp : 0) + ((nb_in && nb == I) ? 1 : 0);
 }
 
-// b_coarse = R r = P^T r / 4 over the 4 x 4 fine cells each coarse cell touches
+// b_coarse = R r = P^T r / 4 over the 4 x 4 fine cells each coarse cell touches.  A
+// thread walks MG_WALK coarse rows down a column: the weighted sum of a fine row's
+// four cells serves two coarse rows.  (FP64, bound by the FP64 pipe: 21 operations a
+// coarse cell as four sums each, 242 us at 4096^2; now 10, 92 us.)
+constexpr int MG_WALK = 4;
 template <typename T>
 __global__ void __launch_bounds__(MG_BX* MG_BY) k_mg_restrict(MgLev<T> F, MgLev<T> C, MgBc p, SolverState* S,
                                                                int inner) {
     if (!block_live(S, inner)) return;
     const int I = blockIdx.x * MG_BX + threadIdx.x;
-    if (I >= C.nx) return;
-    // the x weights do not depend on the row
-    T wxs[4];
-    int fxs[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        int fx = 2 * I - 1 + q;
-        if (fx < 0 || fx >= F.nx) {
-            if (!p.per_x) {
-                fxs[q] = -1;
-                wxs[q] = T(0);
-                continue;
-            }
-            fx = fx < 0 ? fx + F.nx : fx - F.nx;
+    const int J0 = (blockIdx.y * MG_BY + threadIdx.y) * MG_WALK, J1 = min(J0 + MG_WALK, C.ny);
+    if (I >= C.nx || J0 >= C.ny) return;
+    // beside a wall the outer weight falls away and the inner one is the wall's
+    const bool lo = !p.per_x && I == 0, hi = !p.per_x && I == C.nx - 1;
+    const T w1 = lo && p.bc[0] == 0 ? T(1) : T(0.75), w2 = hi && p.bc[2] == 0 ? T(1) : T(0.75);
+    const int fm = I == 0 ? F.nx - 1 : 2 * I - 1, fp = I == C.nx - 1 ? 0 : 2 * I + 2;
+    auto row_sum = [&](int fy0) {
+        const int fy = fy0 < 0 ? fy0 + F.ny : (fy0 >= F.ny ? fy0 - F.ny : fy0);
+        const T* fr = F.r + (size_t)fy * F.pitch;
+        T rs = lo ? T(0) : mg_quarter(fr[fm]);
+        rs = mg_fma(w1, fr[2 * I], rs);
+        rs = mg_fma(w2, fr[2 * I + 1], rs);
+        return hi ? rs : mg_fma(T(0.25), fr[fp], rs);
+    };
+    // the row below a coarse row's own two (none beyond a wall) and those two
+    bool has = p.per_y || J0 > 0;
+    T below = has ? row_sum(2 * J0 - 1) : T(0), r0 = row_sum(2 * J0);
+    for (int J = J0; J < J1; ++J) {
+        const T r1 = row_sum(2 * J + 1);
+        const bool top = !p.per_y && J == C.ny - 1;
+        const T wb = !p.per_y && J == 0 && p.bc[1] == 0 ? T(1) : T(0.75), wt = top && p.bc[3] == 0 ? T(1) : T(0.75);
+        T acc = has ? mg_quarter(below) : T(0);
+        acc = mg_fma(wb, r0, acc);
+        acc = mg_fma(wt, r1, acc);
+        T above = T(0);
+        if (!top) {
+            above = row_sum(2 * J + 2);
+            acc = mg_fma(T(0.25), above, acc);
         }
-        fxs[q] = fx;
-        wxs[q] = (T)mg_pwq(fx, I, C.nx, p.per_x, p.bc[0], p.bc[2]) * T(0.25);
-    }
-#pragma unroll
-    for (int rr = 0; rr < MG_ROWS; ++rr) {
-        const int J = (blockIdx.y * MG_ROWS + rr) * MG_BY + threadIdx.y;
-        if (J >= C.ny) break;
-        T acc = T(0);
-        for (int fy0 = 2 * J - 1; fy0 <= 2 * J + 2; ++fy0) {
-            int fy = fy0;
-            if (fy < 0 || fy >= F.ny) {
-                if (!p.per_y) continue;
-                fy = fy < 0 ? fy + F.ny : fy - F.ny;
-            }
-            const T wy = (T)mg_pwq(fy, J, C.ny, p.per_y, p.bc[1], p.bc[3]) * T(0.25);
-            const T* fr = F.r + (size_t)fy * F.pitch;
-            T rs = T(0);
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (fxs[q] >= 0) rs = mg_fma(wxs[q], fr[fxs[q]], rs);
-            acc = mg_fma(wy, rs, acc);
-        }
-        C.b[(size_t)J * C.pitch + I] = T(0.25) * acc;
+        C.b[(size_t)J * C.pitch + I] = mg_quarter(acc);
+        below = r1;
+        r0 = above;
+        has = true;
     }
 }
 
@@ -216,32 +226,41 @@ __device__ __forceinline__ void mg_axis(int f, int nc, int per, int bclo, int bc
     N = nb;
 }
 
+// x += P x_coarse.  A thread walks 2 MG_WALK fine rows up a column: the weighted sum
+// of a coarse row's two cells serves four fine rows.  (FP64, bound by the FP64 pipe: 8
+// operations a cell with two sums each, 220 us at 4096^2; now 3, 106 us.)
 template <typename T>
 __global__ void __launch_bounds__(MG_BX* MG_BY) k_mg_prolong(MgLev<T> C, MgLev<T> F, MgBc p, SolverState* S,
                                                               int inner) {
     if (!block_live(S, inner)) return;
     const int fx = blockIdx.x * MG_BX + threadIdx.x;
-    if (fx >= F.nx) return;
+    const int J0 = (blockIdx.y * MG_BY + threadIdx.y) * MG_WALK, J1 = min(J0 + MG_WALK, C.ny);
+    if (fx >= F.nx || J0 >= C.ny) return;
     int I, NI;
     T wxI, wxN;
     mg_axis<T>(fx, C.nx, p.per_x, p.bc[0], p.bc[2], I, NI, wxI, wxN);
-#pragma unroll
-    for (int rr = 0; rr < MG_ROWS; ++rr) {
-        const int fy = (blockIdx.y * MG_ROWS + rr) * MG_BY + threadIdx.y;
-        if (fy >= F.ny) break;
-        int J, NJ;
-        T wyJ, wyN;
-        mg_axis<T>(fy, C.ny, p.per_y, p.bc[1], p.bc[3], J, NJ, wyJ, wyN);
-        T row0 = wxI * C.x[(size_t)J * C.pitch + I];
-        if (NI >= 0) row0 = mg_fma(wxN, C.x[(size_t)J * C.pitch + NI], row0);
-        T v = wyJ * row0;
-        if (NJ >= 0) {
-            T row1 = wxI * C.x[(size_t)NJ * C.pitch + I];
-            if (NI >= 0) row1 = mg_fma(wxN, C.x[(size_t)NJ * C.pitch + NI], row1);
-            v = mg_fma(wyN, row1, v);
-        }
-        const size_t k = (size_t)fy * F.pitch + fx;
-        F.x[k] = F.x[k] + v;
+    auto row_sum = [&](int J) {
+        J = J < 0 ? J + C.ny : (J >= C.ny ? J - C.ny : J);
+        const T* cr = C.x + (size_t)J * C.pitch;
+        const T h = mg_mul(wxI, cr[I]);
+        return NI >= 0 ? mg_fma(wxN, cr[NI], h) : h;
+    };
+    bool has = p.per_y || J0 > 0;
+    T below = has ? row_sum(J0 - 1) : T(0), own = row_sum(J0);
+    for (int J = J0; J < J1; ++J) {
+        const bool top = !p.per_y && J == C.ny - 1;
+        T above = T(0);
+        if (!top) above = row_sum(J + 1);
+        T* x = F.x + (size_t)(2 * J) * F.pitch + fx;
+        T v = mg_mul(!has && p.bc[1] == 0 ? T(1) : T(0.75), own);
+        if (has) v = mg_fma(T(0.25), below, v);
+        x[0] = x[0] + v;
+        v = mg_mul(top && p.bc[3] == 0 ? T(1) : T(0.75), own);
+        if (!top) v = mg_fma(T(0.25), above, v);
+        x[F.pitch] = x[F.pitch] + v;
+        below = own;
+        own = above;
+        has = true;
     }
 }
 
@@ -1201,12 +1220,13 @@ void mg_free(cf_ctx* c) {
 
 double* mg_z64(cf_ctx* c) { return static_cast<MgHierarchy*>(c->mg)->z64; }
 
-// fused = 1: levels above the bottom solver run the fused pre/post kernels;
+// fused = 1: levels above the coarse cluster run the fused pre/post kernels;
 // 0: one launch per half sweep, residual, restriction and prolongation (the
 // same arithmetic); -1 (default): fused for FP32 levels, which are bound by
-// memory traffic, and for FP64 levels of at most 2^20 cells, which are bound
+// memory traffic, and for FP64 levels of at most 2^18 cells, which are bound
 // by launch latency; larger FP64 levels are bound by the FP64 pipe, where the
-// fused tiles' halo recomputation costs more than it saves.  CF_MG_FUSED=0/1
+// recomputed halo costs more than it saves (1024^2: pre and post 121 us fused; a
+// 4096^2 step 18.40 ms with 1024^2 level by level, 18.52 fused).  CF_MG_FUSED=0/1
 // in the environment forces one form.
 // Launch geometry of a fused pre (or post) launch: tiles of tw x th over the
 // level; with strip_rows > 0 (FP32 64-wide tiles only), register strips of
@@ -1273,6 +1293,7 @@ static int vcycle(cf_ctx* c, const MgHierarchy* H, MgLev<T>* lev, double scale0,
     const dim3 blk(MG_BX, MG_BY);
     const int rows = MG_BY * MG_ROWS;
     auto grid2 = [&](int nx, int ny) { return dim3((nx + MG_BX - 1) / MG_BX, (ny + rows - 1) / rows); };
+    auto walk = [&](int nx, int rows) { return dim3((nx + MG_BX - 1) / MG_BX, (rows + MG_BY * MG_WALK - 1) / (MG_BY * MG_WALK)); };
     int launches = 0;
     auto smooth = [&](int l, int color, int first) {
         const MgLev<T>& L = lev[l];
@@ -1290,7 +1311,7 @@ static int vcycle(cf_ctx* c, const MgHierarchy* H, MgLev<T>* lev, double scale0,
     };
     auto fuse_level = [&](int l) {
         if (fused >= 0) return fused != 0;
-        return sizeof(T) == 4 || (long long)lev[l].nx * lev[l].ny <= (1ll << 20);
+        return sizeof(T) == 4 || (long long)lev[l].nx * lev[l].ny <= (1ll << 18);
     };
     for (int l = 0; l < top_end; ++l) {
         if (fuse_level(l)) {
@@ -1313,8 +1334,7 @@ static int vcycle(cf_ctx* c, const MgHierarchy* H, MgLev<T>* lev, double scale0,
             smooth(l, 1, 0);
         }
         k_mg_residual<T><<<grid2(lev[l].nx, lev[l].ny), blk, 0, c->stream>>>(lev[l], p, c->S, inner);
-        k_mg_restrict<T><<<grid2(lev[l + 1].nx, lev[l + 1].ny), blk, 0, c->stream>>>(lev[l], lev[l + 1], p, c->S,
-                                                                                      inner);
+        k_mg_restrict<T><<<walk(lev[l + 1].nx, lev[l + 1].ny), blk, 0, c->stream>>>(lev[l], lev[l + 1], p, c->S, inner);
         launches += 2;
     }
     if (lb < nlev) {
@@ -1370,7 +1390,7 @@ static int vcycle(cf_ctx* c, const MgHierarchy* H, MgLev<T>* lev, double scale0,
             ++launches;
             continue;
         }
-        k_mg_prolong<T><<<grid2(lev[l].nx, lev[l].ny), blk, 0, c->stream>>>(lev[l + 1], lev[l], p, c->S, inner);
+        k_mg_prolong<T><<<walk(lev[l].nx, lev[l + 1].ny), blk, 0, c->stream>>>(lev[l + 1], lev[l], p, c->S, inner);
         ++launches;
         for (int k = 0; k < MG_NU; ++k) {
             smooth(l, 1, 0);
