@@ -125,9 +125,15 @@ __device__ __forceinline__ double warp_fold(double s) {
     return s;
 }
 
-__device__ __forceinline__ double warp_max(double s) {
+// max(s, |v|) of s >= 0, a NaN v left out (fmax's answer); on the integer pipe, where
+// magnitudes compare as their bits
+__device__ __forceinline__ double max_mag(double s, double v) {
+    const long long a = __double_as_longlong(s), b = __double_as_longlong(v) & 0x7fffffffffffffffll;
+    return __longlong_as_double(b <= 0x7ff0000000000000ll && b > a ? b : a);
+}
+__device__ __forceinline__ double warp_max(double s) {  // s >= 0
 #pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) s = fmax(s, __shfl_xor_sync(0xffffffffu, s, m));
+    for (int m = 16; m >= 1; m >>= 1) s = max_mag(s, __shfl_xor_sync(0xffffffffu, s, m));
     return s;
 }
 
@@ -256,16 +262,16 @@ __device__ __forceinline__ double final_max(const double* partial, int n) {
 #pragma unroll
         for (int k = 0; k < CF_FOLD_BATCH; ++k) v[k] = __ldcg(partial + u + k * CF_RED_THREADS);
 #pragma unroll
-        for (int k = 0; k < CF_FOLD_BATCH; ++k) s = fmax(s, v[k]);
+        for (int k = 0; k < CF_FOLD_BATCH; ++k) s = max_mag(s, v[k]);
     }
-    for (; u < n; u += CF_RED_THREADS) s = fmax(s, __ldcg(partial + u));
+    for (; u < n; u += CF_RED_THREADS) s = max_mag(s, __ldcg(partial + u));
     s = warp_max(s);
     __syncthreads();
     if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
     __syncthreads();
     double tot = ws[0];
 #pragma unroll
-    for (int k = 1; k < CF_RED_WARPS; ++k) tot = fmax(tot, ws[k]);
+    for (int k = 1; k < CF_RED_WARPS; ++k) tot = max_mag(tot, ws[k]);
     __syncthreads();
     return tot;
 }

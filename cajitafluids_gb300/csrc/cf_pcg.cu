@@ -29,13 +29,14 @@
 // 1.2 us each) and the divisions; at seven units per SM the FP64 pipe (12
 // operations per cell and iteration: 21 of 33 us).  Measured on GB300, time of
 // one iteration, the two launches per iteration before and this: 64^2 39.9 ->
-// 9.7 us, 256^2 49.6 -> 10.4 us, 1024^2 53.8 -> 33.2 us.
+// 9.7 us, 256^2 49.6 -> 10.4 us, 1024^2 53.8 -> 31.1 us.
 #include <cuda_runtime.h>
 #include <math.h>
 
 #include <algorithm>
 
 #include "cf_grid.cuh"
+#include "cf_mul64.cuh"
 
 namespace cf {
 
@@ -45,6 +46,14 @@ template <int NU>
 struct PcThreads {
     static constexpr int value = NU <= 2 ? 256 : 512;
 };
+// Plain products: four and seven units per block are bound by the FP64 pipe, and
+// products on the integer pipes run beside it (1024^2: 33.2 -> 31.1 us an iteration);
+// one or two units wait for results, which the hardware product returns sooner
+// (a 256^2 step: 10.2 ms against 10.4 with integer products).
+template <int NU>
+__device__ __forceinline__ double pcg_mul(double a, double b) {
+    return NU <= 2 ? a * b : mul64i(a, b);
+}
 constexpr int PC_PW = UNIT_PW, PC_P = UNIT_P, PC_CELLS = UNIT_CELLS, PC_BORDER = UNIT_BORDER;
 constexpr int PC_UNIT = PC_P + 2 * PC_CELLS;  // doubles per unit: p with its halo, r, q / z
 constexpr int PC_MAX_UNITS = 7;                           // units per block (181 KB of shared memory)
@@ -128,7 +137,7 @@ __global__ void __launch_bounds__(PcThreads<NU>::value, 1) k_pcg64(Pcg64 a) {
                 code[k] |= (unsigned)eb << (4 * m) | 1u << (16 + m);
                 const size_t o = (size_t)(j0 + row) * a.pitch + c0 + col;
                 rv = a.r[o];
-                z = tab_m[eb] * rv;
+                z = pcg_mul<NU>(tab_m[eb], rv);
                 xr[k][m] = a.x[o];
                 if (it > 0) p[(row + 1) * PC_PW + col + 1] = pold[o];
             }
@@ -185,7 +194,7 @@ __global__ void __launch_bounds__(PcThreads<NU>::value, 1) k_pcg64(Pcg64 a) {
                 const double* c = p + (row + 1) * PC_PW + col + 1;
                 double qv = 0.0;
                 if (code[k] >> (16 + m) & 1u) {
-                    qv = tab_d[code[k] >> (4 * m) & 15u] * c[0];
+                    qv = pcg_mul<NU>(tab_d[code[k] >> (4 * m) & 15u], c[0]);
                     qv = fma(ms, c[-1], qv);
                     qv = fma(ms, c[1], qv);
                     qv = fma(ms, c[-PC_PW], qv);
@@ -235,7 +244,7 @@ __global__ void __launch_bounds__(PcThreads<NU>::value, 1) k_pcg64(Pcg64 a) {
                 const int row = row0 + m * (PC_THREADS / CF_UNIT_COLS), cell = row * CF_UNIT_COLS + col;
                 if (!(code[k] >> (16 + m) & 1u)) continue;
                 const double rv = fma(malpha, q[cell], r[cell]);
-                const double z = tab_m[code[k] >> (4 * m) & 15u] * rv;
+                const double z = pcg_mul<NU>(tab_m[code[k] >> (4 * m) & 15u], rv);
                 r[cell] = rv;
                 q[cell] = z;
                 if (row == 0) __stcg(bo + col, z);
@@ -353,7 +362,7 @@ static bool pcg64_fits(const cf_ctx* c) {
 // border buffer.  A block takes as few units as the SMs allow; up to seven
 // (1064 units on 152 SMs) the vectors fit shared memory, and there the solve
 // is faster than the launch-per-phase kernels at every size (1024^2, seven
-// units: 33.2 against 53.8 us per iteration).
+// units: 31.1 against 53.8 us per iteration).
 int pcg64_setup(cf_ctx* c) {
     c->pcg_nu = 0;
     const int per = (c->n_units + c->sms - 1) / c->sms;

@@ -38,6 +38,7 @@
 #include <cstring>
 
 #include "cf_ctx.cuh"
+#include "cf_mul64.cuh"
 
 namespace cf {
 
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_cg_dir_matvec64
         // new search direction at a cell of the grid
         auto dir = [&](int c, int j) {
             const size_t k = (size_t)j * a.pitch + c;
-            const double z = a.mg ? __ldg(a.z + k) : a.st.minv[ebits(a, c, j)] * __ldg(a.r + k);
+            const double z = a.mg ? __ldg(a.z + k) : mul64i(a.st.minv[ebits(a, c, j)], __ldg(a.r + k));
             return first ? z : fma(beta, __ldg(pold + k), z);
         };
 #pragma unroll
@@ -117,7 +118,7 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_cg_dir_matvec64
             const double* c = P + (row + 1) * UNIT_PW + col + 1;
             double q = 0.0;
             if (col < u.nc && row < u.nr) {
-                q = a.st.diag[ebits(a, u.c0 + col, u.j0 + row)] * c[0];
+                q = mul64i(a.st.diag[ebits(a, u.c0 + col, u.j0 + row)], c[0]);
                 q = fma(ms, c[-1], q);
                 q = fma(ms, c[1], q);
                 q = fma(ms, c[-UNIT_PW], q);
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS / 2) k_cg_update64
                 a.x[k] = fma(alpha, pp[m], xv[m]);
                 r = fma(malpha, qv[m], rv[m]);
                 a.r[k] = r;
-                if (!a.mg) z = a.st.minv[ebits(a, u.c0 + col, u.j0 + row)] * r;
+                if (!a.mg) z = mul64i(a.st.minv[ebits(a, u.c0 + col, u.j0 + row)], r);
             }
             R[cell] = r;
             if (!a.mg) Z[cell] = z;
@@ -303,7 +304,7 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_warm_resid64(Cg
             double r = 0.0, z = 0.0;
             if (col < u.nc && row < u.nr) {
                 const int c = u.c0 + col, j = u.j0 + row, eb = ebits(a, c, j);
-                double ax = a.st.diag[eb] * xv(c, j);
+                double ax = mul64i(a.st.diag[eb], xv(c, j));
                 ax = fma(ms, xv(c - 1, j), ax);
                 ax = fma(ms, xv(c + 1, j), ax);
                 ax = fma(ms, xv(c, j - 1), ax);
@@ -311,7 +312,7 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_warm_resid64(Cg
                 const size_t k = (size_t)j * a.pitch + c;
                 r = a.r[k] - ax;
                 a.r[k] = r;
-                z = a.st.minv[eb] * r;
+                z = mul64i(a.st.minv[eb], r);
             }
             R[cell] = r;
             Z[cell] = z;
@@ -367,7 +368,7 @@ __device__ __forceinline__ double div_b(const DivArgs& a, int gi, int gj) {
     double t = u1 - u0;
     t = t + v1;
     t = t - v0;
-    return a.mscale * t;
+    return mul64i(a.mscale, t);
 }
 
 // FP32 solver vectors carry a ghost ring (cf_cg32.cu); r's periodic ghost
@@ -413,7 +414,7 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_div_init64(DivA
                 const size_t k = (size_t)j * a.pitch + c;
                 a.r[k] = b;
                 if (!a.warm) a.x[k] = 0.0;
-                z = a.st.minv[edge_bits(c, j, a.nx, a.ny, a.per_x, a.per_y)] * b;
+                z = mul64i(a.st.minv[edge_bits(c, j, a.nx, a.ny, a.per_x, a.per_y)], b);
             }
             R[cell] = b;
             Z[cell] = z;
@@ -1087,7 +1088,7 @@ __device__ __forceinline__ double press_update(const Press& a, const float2* xdf
         return __hiloint2double(__float_as_int(r.y), __float_as_int(r.x));  // the pair's 8 bytes
     }
     const double d = pval(a, ci, cj) - pval(a, ni, nj);
-    return __dadd_rn(w, __dmul_rn(a.ms, d));
+    return __dadd_rn(w, mul64i(a.ms, d));
 }
 
 // One face: I face (axis 0) or J face (axis 1) of index (gi, gj), with the
@@ -1377,7 +1378,7 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_div_norms64(Div
             double b = 0.0;
             if (col < u.nc && row < u.nr) b = div_b(a, u.c0 + col, u.j0 + row);
             B[row * CF_UNIT_COLS + col] = b;
-            amx = fmax(amx, fabs(b));
+            amx = max_mag(amx, b);
         }
         amx = warp_max(amx);
         if (lane == 0) mx[warp] = amx;
@@ -1388,7 +1389,7 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_div_norms64(Div
         } else if (tid == 32 * unit_warp(unit + 1)) {
             double t = mx[0];
 #pragma unroll
-            for (int k = 1; k < CF_RED_WARPS; ++k) t = fmax(t, mx[k]);
+            for (int k = 1; k < CF_RED_WARPS; ++k) t = max_mag(t, mx[k]);
             a.part1[unit] = t;
         }
     }
