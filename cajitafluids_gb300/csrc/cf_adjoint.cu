@@ -103,9 +103,9 @@ struct Lin64 {
 __device__ __forceinline__ void lin64_taps(const Phys& p, const Grid<double>& g, Lin64& s) {
     const double* q = g.o + (size_t)s.ky * g.pitch + s.kx;
     const double a0 = __ldg(q), a1 = __ldg(q + 1), b0 = __ldg(q + g.pitch), b1 = __ldg(q + g.pitch + 1);
-    const double ra = fma(s.wx[1], a1, s.wx[0] * a0), rb = fma(s.wx[1], b1, s.wx[0] * b0);
-    s.val = fma(s.wy[1], rb, s.wy[0] * ra);
-    s.gx = times_rdx(fma(s.wy[1], b1 - b0, s.wy[0] * (a1 - a0)), p.rdx, p.rsh);
+    const double ra = fma(s.wx[1], a1, mul64i(s.wx[0], a0)), rb = fma(s.wx[1], b1, mul64i(s.wx[0], b0));
+    s.val = fma(s.wy[1], rb, mul64i(s.wy[0], ra));
+    s.gx = times_rdx(fma(s.wy[1], b1 - b0, mul64i(s.wy[0], a1 - a0)), p.rdx, p.rsh);
     s.gy = times_rdx(rb - ra, p.rdx, p.rsh);
 }
 __device__ __forceinline__ void lin64(const Phys& p, const Grid<double>& g, double lx, double ly, double x, double y,
@@ -132,10 +132,10 @@ __device__ __forceinline__ void lin64_at(const Phys& p, const Grid<double>& g, i
         const double a0 = __ldg(q), a1 = __ldg(q + 1), b0 = __ldg(q + g.pitch), b1 = __ldg(q + g.pitch + 1);
         auto mag = [](double d) { return __double2hiint(d) & 0x7fffffff; };
         if (max(max(mag(a0), mag(a1)), max(mag(b0), mag(b1))) < 0x7ff00000) {
-            const double ra = zx ? a0 : fma(tx, a1, sx * a0), rb = zx ? b0 : fma(tx, b1, sx * b0);
+            const double ra = zx ? a0 : fma(tx, a1, mul64i(sx, a0)), rb = zx ? b0 : fma(tx, b1, mul64i(sx, b0));
             const double da = a1 - a0;
-            s.val = zy ? ra : fma(ty, rb, sy * ra);
-            s.gx = times_rdx(zy ? da : fma(ty, b1 - b0, sy * da), p.rdx, p.rsh);
+            s.val = zy ? ra : fma(ty, rb, mul64i(sy, ra));
+            s.gx = times_rdx(zy ? da : fma(ty, b1 - b0, mul64i(sy, da)), p.rdx, p.rsh);
             s.gy = times_rdx(rb - ra, p.rdx, p.rsh);
             return;
         }
@@ -157,15 +157,15 @@ __device__ __forceinline__ bool cubic64(double xi, int ext, int& k0, double* w, 
     double t, s;
     const double hi = exact_double(ext - 2);
     cell_fraction(clamp_bits(xi, 1.0, hi), ext - 3, k, t, s);
-    const double t2 = t * t, t3 = t2 * t, s2 = s * s;
-    w[0] = (s2 * s) * (1.0 / 6.0);
+    const double t2 = mul64i(t, t), t3 = mul64i(t2, t), s2 = mul64i(s, s);
+    w[0] = mul64i(mul64i(s2, s), 1.0 / 6.0);
     w[1] = fma(0.5, t3, -t2) + (2.0 / 3.0);
     w[2] = fma(0.5, (t + t2) - t3, 1.0 / 6.0);
-    w[3] = t3 * (1.0 / 6.0);
-    d[0] = -0.5 * s2;
-    d[1] = fma(1.5, t2, -2.0 * t);
+    w[3] = mul64i(t3, 1.0 / 6.0);
+    d[0] = mul64i(-0.5, s2);
+    d[1] = fma(1.5, t2, mul64i(-2.0, t));
     d[2] = fma(-1.5, t2, t + 0.5);
-    d[3] = 0.5 * t2;
+    d[3] = mul64i(0.5, t2);
     k0 = k - 1;
     return outside_bits(xi, 1.0, hi);
 }
@@ -192,16 +192,16 @@ __device__ __forceinline__ void foot64(const Phys& p, const Grid<double>& g, dou
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
         const double* row = g.o + (size_t)(f.ky + b) * g.pitch + f.kx;
-        double v = __ldg(row), rs = f.wx[0] * v, rd = dx[0] * v;
+        double v = __ldg(row), rs = mul64i(f.wx[0], v), rd = mul64i(dx[0], v);
 #pragma unroll
         for (int a = 1; a < 4; ++a) {
             v = __ldg(row + a);
             rs = fma(f.wx[a], v, rs);
             rd = fma(dx[a], v, rd);
         }
-        val = b == 0 ? f.wy[0] * rs : fma(f.wy[b], rs, val);
-        gx = b == 0 ? f.wy[0] * rd : fma(f.wy[b], rd, gx);
-        gy = b == 0 ? dy[0] * rs : fma(dy[b], rs, gy);
+        val = b == 0 ? mul64i(f.wy[0], rs) : fma(f.wy[b], rs, val);
+        gx = b == 0 ? mul64i(f.wy[0], rd) : fma(f.wy[b], rd, gx);
+        gy = b == 0 ? mul64i(dy[0], rs) : fma(dy[b], rs, gy);
     }
     f.val = val;
     f.gx = cx ? 0.0 : times_rdx(gx, p.rdx, p.rsh);
@@ -243,7 +243,7 @@ __device__ __forceinline__ RecCode put_rec(const RecKind& R, int t, int sample, 
     ry = rec_fit<N>(ry, wy, ylo, yhi);
 #pragma unroll
     for (int a = 0; a < N; ++a) {
-        R.cx[a * R.nt + t] = val * wx[a];
+        R.cx[a * R.nt + t] = mul64i(val, wx[a]);
         R.wy[a * R.nt + t] = wy[a];
     }
     return (RecCode)((rx + 4) | (ry + 4) << 4) << (8 * sample);
@@ -275,7 +275,9 @@ __device__ __forceinline__ double inputs_adjoint_gate(const Phys& p, int ent, in
 // FP64 pipe.  Of 306 FP64 operations a target, cells and fractions on the integer
 // pipe, the first stage's places from per-axis tables, differences instead of
 // derivative weights and the reach test on the displacements' bits leave about 200:
-// 500 -> 385 us at 512^2 (422 with one block to an SM).
+// 500 -> 375 us at 512^2 (422 with one block to an SM); its plain products run on the
+// integer pipes (cf_mul64.cuh): 315 us, the FP64 pipe 65 % busy, 16 warps to an SM
+// (20 or 24 with fewer registers: no faster).
 template <int ORDER>
 __global__ void __launch_bounds__(256, 2) k_adj_records(const __grid_constant__ AdjRec a) {
     __shared__ AdvAxis X, Y;
@@ -314,24 +316,24 @@ __global__ void __launch_bounds__(256, 2) k_adj_records(const __grid_constant__ 
         if ((__double2hiint(d) & 0x7fffffff) >= near) far = far || fabs(x - from) > lim;
     };
     // the forward's operation order (one rounding per operation)
-    const double d1x = __dmul_rn(h1, s0u.val), d1y = __dmul_rn(h1, s0v.val);
+    const double d1x = mul64i(h1, s0u.val), d1y = mul64i(h1, s0v.val);
     const double x1 = __dsub_rn(x0, d1x), y1 = __dsub_rn(y0, d1y);
     moved(d1x, x1, x0);
     moved(d1y, y1, y0);
     lin64(p, a.u, ulx, uly, x1, y1, s1u);
     lin64(p, a.v, vlx, vly, x1, y1, s1v);
     const bool ralston = (p.quirks & 2u) != 0;
-    const double d2x = __dmul_rn(h2, ralston ? s1u.val : s0u.val), d2y = __dmul_rn(h2, ralston ? s1v.val : s0v.val);
+    const double d2x = mul64i(h2, ralston ? s1u.val : s0u.val), d2y = mul64i(h2, ralston ? s1v.val : s0v.val);
     const double x2 = __dsub_rn(x0, d2x), y2 = __dsub_rn(y0, d2y);
     moved(d2x, x2, x0);
     moved(d2y, y2, y0);
     lin64(p, a.u, ulx, uly, x2, y2, s2u);
     lin64(p, a.v, vlx, vly, x2, y2, s2v);
-    double ax = __dadd_rn(__dmul_rn(2.0 / 9.0, s0u.val), __dmul_rn(3.0 / 9.0, s1u.val));
-    ax = __dadd_rn(ax, __dmul_rn(4.0 / 9.0, s2u.val));
-    double ay = __dadd_rn(__dmul_rn(2.0 / 9.0, s0v.val), __dmul_rn(3.0 / 9.0, s1v.val));
-    ay = __dadd_rn(ay, __dmul_rn(4.0 / 9.0, s2v.val));
-    const double dx = __dmul_rn(dt, ax), dy = __dmul_rn(dt, ay);
+    double ax = __dadd_rn(mul64i(2.0 / 9.0, s0u.val), mul64i(3.0 / 9.0, s1u.val));
+    ax = __dadd_rn(ax, mul64i(4.0 / 9.0, s2u.val));
+    double ay = __dadd_rn(mul64i(2.0 / 9.0, s0v.val), mul64i(3.0 / 9.0, s1v.val));
+    ay = __dadd_rn(ay, mul64i(4.0 / 9.0, s2v.val));
+    const double dx = mul64i(dt, ax), dy = mul64i(dt, ay);
     const double tx = __dsub_rn(x0, dx), ty = __dsub_rn(y0, dy);
     moved(dx, tx, x0);
     moved(dy, ty, y0);
@@ -357,13 +359,13 @@ __global__ void __launch_bounds__(256, 2) k_adj_records(const __grid_constant__ 
     constexpr int flo = ORDER == 1 ? -1 : -2;
     RecCode code = put_rec<Foot64<ORDER>::n>(a.F[ent], t, REC_F, sf.kx - li, sf.ky - lj, fb, sf.wx, sf.wy, flo, flo + 1,
                                              flo, flo + 1);
-    const double sb = -dt * fb, abx = sb * sf.gx, aby = sb * sf.gy;
-    double v0x = (2.0 / 9.0) * abx, v0y = (2.0 / 9.0) * aby;
-    double v1x = (3.0 / 9.0) * abx, v1y = (3.0 / 9.0) * aby;
-    const double v2x = (4.0 / 9.0) * abx, v2y = (4.0 / 9.0) * aby;
+    const double sb = mul64i(-dt, fb), abx = mul64i(sb, sf.gx), aby = mul64i(sb, sf.gy);
+    double v0x = mul64i(2.0 / 9.0, abx), v0y = mul64i(2.0 / 9.0, aby);
+    double v1x = mul64i(3.0 / 9.0, abx), v1y = mul64i(3.0 / 9.0, aby);
+    const double v2x = mul64i(4.0 / 9.0, abx), v2y = mul64i(4.0 / 9.0, aby);
     // stage 2 at (x2, y2)
     code |= put_u(2, s2u, v2x) | put_v(2, s2v, v2y);
-    const double x2bx = fma(s2v.gx, v2y, s2u.gx * v2x), x2by = fma(s2v.gy, v2y, s2u.gy * v2x);
+    const double x2bx = fma(s2v.gx, v2y, mul64i(s2u.gx, v2x)), x2by = fma(s2v.gy, v2y, mul64i(s2u.gy, v2x));
     if (ralston) {
         v1x = fma(-h2, x2bx, v1x);
         v1y = fma(-h2, x2by, v1y);
@@ -373,7 +375,7 @@ __global__ void __launch_bounds__(256, 2) k_adj_records(const __grid_constant__ 
     }
     // stage 1 at (x1, y1)
     code |= put_u(1, s1u, v1x) | put_v(1, s1v, v1y);
-    const double x1bx = fma(s1v.gx, v1y, s1u.gx * v1x), x1by = fma(s1v.gy, v1y, s1u.gy * v1x);
+    const double x1bx = fma(s1v.gx, v1y, mul64i(s1u.gx, v1x)), x1by = fma(s1v.gy, v1y, mul64i(s1u.gy, v1x));
     v0x = fma(-h1, x1bx, v0x);
     v0y = fma(-h1, x1by, v0y);
     // stage 0 at (x0, y0)
