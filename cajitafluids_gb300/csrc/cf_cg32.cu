@@ -973,26 +973,6 @@ static int make_map(cf_ctx* c, CUtensorMap* m, float* base) {
 
 static int pcg32_setup(cf_ctx* c);
 
-// K1's grid for the MG-PCG.  One tile to a CTA, with the buffers of one stage, where
-// the chip holds them all (1024^2: 512 tiles; with three stages 456 CTAs fit and 56
-// of them walk two tiles, 6.5 of 16 us); else the persistent grid.
-static int mg_k1_grid(cf_ctx* c, int sms) {
-    int occ = 0;
-    for (int stages : {1, (int)kStages}) {
-        const int smem = stages * 2 * kSlot + 128;
-        int rc = cuda_check(c, cudaFuncSetAttribute(k_tma_dir_matvec32<true>,
-                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attribute");
-        if (!rc)
-            rc = cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tma_dir_matvec32<true>, kThreads, smem),
-                            "occupancy");
-        if (rc) return rc;
-        c->cta32mg = std::min(c->tiles, std::max(occ, 1) * sms);
-        c->smem32mg = smem;
-        if (c->cta32mg == c->tiles) break;
-    }
-    return CF_OK;
-}
-
 int cg32_setup(cf_ctx* c) {
     int rc = make_map(c, &c->map_r, c->r32b);
     if (!rc) rc = make_map(c, &c->map_pa, c->pa32b);
@@ -1006,6 +986,10 @@ int cg32_setup(cf_ctx* c) {
     rc = cuda_check(c, cudaFuncSetAttribute(k_tma_dir_matvec32<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             kStages * 2 * kSlot + 128),
                     "smem attribute");
+    if (!rc)
+        rc = cuda_check(c, cudaFuncSetAttribute(k_tma_dir_matvec32<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                kStages * 2 * kSlot + 128),
+                        "smem attribute");
     if (!rc)
         rc = cuda_check(c, cudaFuncSetAttribute(k_tma_update32, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 kStages * 2 * kSlot + 128),
@@ -1025,7 +1009,6 @@ int cg32_setup(cf_ctx* c) {
     occ2 = occ2 < 1 ? 1 : occ2;
     c->cta32 = c->tiles < occ1 * sms ? c->tiles : occ1 * sms;
     c->cta32b = c->tiles < occ2 * sms ? c->tiles : occ2 * sms;
-    if ((rc = mg_k1_grid(c, sms))) return rc;
     return pcg32_setup(c);
 }
 
@@ -1139,7 +1122,7 @@ void cg32_launch_pair_mg(cf_ctx* c, const Stencil& st) {
     for (int b = 0; b < 16; ++b) stz.minv32[b] = 1.0f;
     Cg32T a = cg32_args(c, stz);
     a.mg = 1;
-    k_tma_dir_matvec32<true><<<c->cta32mg, kThreads, c->smem32mg, c->stream>>>(c->map_z, c->map_pa, c->map_pb, a);
+    k_tma_dir_matvec32<true><<<c->cta32, kThreads, kStages * 2 * kSlot + 128, c->stream>>>(c->map_z, c->map_pa, c->map_pb, a);
     if (!c->x_only) {
         k_tma_update32<<<c->cta32b, kThreads, kStages * 2 * kSlot + 128, c->stream>>>(c->map_r, c->map_pa, c->map_pb,
                                                                                 a);

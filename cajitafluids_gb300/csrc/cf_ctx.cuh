@@ -49,7 +49,6 @@ struct cf_ctx {
     int p32 = 0;
     CUtensorMap map_r{}, map_pa{}, map_pb{};
     int tiles_x = 0, tiles = 0, cta32 = 0, cta32b = 0;
-    int cta32mg = 0, smem32mg = 0;  // K1 in the MG-PCG: grid and shared memory
     double* partials = nullptr;  // 4 * n_units, and one per SM at least
     int G = 0, B = 0, n_units = 0;
     int sms = 1;  // multiprocessors of the device (launch sizing)

@@ -1372,7 +1372,8 @@ static int vcycle(cf_ctx* c, const MgHierarchy* H, MgLev<T>* lev, double scale0,
     for (int l = top_end - 1; l >= 0; --l) {
         if (fuse_level(l)) {
             RzEpi E{0, epi_part};
-            if (l == 0 && epi_part) {
+            // (grids of at most MC_COARSEST cells: r.z in k_mg_rz32's order)
+            if (l == 0 && epi_part && (long long)lev[0].nx * lev[0].ny > MC_COARSEST) {
                 E.on = 1;
                 *epi_done = true;
             }
@@ -1383,7 +1384,7 @@ static int vcycle(cf_ctx* c, const MgHierarchy* H, MgLev<T>* lev, double scale0,
                                                                                             inner, m, E);
                 }
             } else {
-                const MtGrid m = mt_grid<T>(lev[l].nx, lev[l].ny, c->sms, false);
+                const MtGrid m = mt_grid<T>(lev[l].nx, lev[l].ny, c->sms, false, E.on ? MT_RZ_ROWS : 0);
                 k_mg_post_rows<T><<<std::min(m.tiles, c->sms), 32 * m.rows, MT_POST_SMEM<T>, c->stream>>>(
                     lev[l + 1].x, lev[l + 1].pitch, lev[l], p, c->S, inner, m.tx, m.tiles, E);
             }

@@ -14,7 +14,7 @@
 //
 // Why: tiles of 32 x 16 in shared memory read five neighbours per update there
 // with a stride of two (two wavefronts each) and computed 2.1 cells per cell kept.
-// us, tiles -> rows: FP32 1024^2 pre 17.8 -> 10.6, post with r.z 35.6 -> 17.4;
+// us, tiles -> rows: FP32 1024^2 pre 17.8 -> 10.6, post with r.z 35.6 -> 18.2;
 // FP32 512^2 9.2 -> 4.7 and 8.7 -> 5.6; FP64 (bound by the FP64 pipe) 512^2 30.2
 // -> 19.6 and 37.3 -> 17.8, 256^2 11.4 -> 10.8 and 10.8 -> 10.7.  The height of a
 // window is chosen per level (mt_grid): 32 rows for all left 120 and 36 blocks on
@@ -26,6 +26,7 @@ constexpr int MT_ROWS = 32;                   // most rows of a window (a warp e
 constexpr int MT_COLS = 128;                  // columns of a window, four to a lane
 constexpr int MT_PRE_COLS = 112, MT_POST_COLS = 120;  // columns kept
 constexpr int MT_PRE_HALO = 10, MT_POST_HALO = 8;     // rows of a window not kept
+constexpr int MT_RZ_ROWS = 16 + MT_POST_HALO;         // rows of a post-smoothing window that forms r.z
 
 template <typename T>
 struct MtRow {
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mg_post_rows(const T* cx, int
     if (!block_live(S, inner)) return;
     const T scale = F.scale;
     const int nc = F.nx / 2, mc = F.ny / 2;
-    T rz = T(0), rze = T(0);  // r.z of the lane's cells: sum and what its rounding left out
+    T rz = T(0), rze = T(0);  // the lane's share of r.z: sum and what its rounding left out
     for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
         place(t, r.g, r.c0);
         r.live = (p.per_y || (r.g >= 0 && r.g < F.ny)) && r.g < F.ny + 4;
@@ -360,9 +361,6 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mg_post_rows(const T* cx, int
                     for (int k = 0; k < 4; ++k) {
                         const int gi = r.c0 + k, gj = r.g;
                         if (gi >= F.nx) continue;
-                        const T v = r.b[k] * r.x[k], s = rz + v, d = s - rz;
-                        rze = rze + ((rz - (s - d)) + (v - d));
-                        rz = s;
                         // ghost copies along periodic axes (the finest level's x has a ghost ring)
                         if (p.per_x) {
                             if (gi == 0) row[F.nx] = r.x[k];
@@ -375,6 +373,32 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mg_post_rows(const T* cx, int
                     }
                 }
             }
+        }
+        if (sizeof(T) == 4 && E.on) {
+            // r.z in units of two cells eight rows apart, one fused operation each (the
+            // solver's fixed FP32 order; windows of MT_RZ_ROWS hold whole units), their
+            // sums as pairs
+            constexpr int lo = MT_POST_HALO / 2;
+            const bool own = lane >= 1 && lane < 31 && r.g < F.ny;
+            if (warp >= lo && warp < lo + 8) {
+                T v[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[k] = own && r.c0 + k < F.nx ? mg_fma(r.b[k], r.x[k], T(0)) : T(0);
+                mc_st<4>(hs + (warp - lo) * MT_COLS + 4 * lane, v);
+            }
+            __syncthreads();
+            if (warp >= lo + 8 && warp < lo + 16) {
+                T v[4];
+                mc_ld<4>(v, hs + (warp - lo - 8) * MT_COLS + 4 * lane);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (own && r.c0 + k < F.nx) v[k] = mg_fma(r.b[k], r.x[k], v[k]);
+                    const T s = rz + v[k], d = s - rz;
+                    rze = rze + ((rz - (s - d)) + (v[k] - d));
+                    rz = s;
+                }
+            }
+            __syncthreads();
         }
     }
     if (sizeof(T) == 4 && E.on) {
@@ -403,7 +427,7 @@ struct MtGrid {
     int tx, tiles, rows;
 };
 template <typename T>
-static MtGrid mt_grid(int nx, int ny, int sms, bool pre) {
+static MtGrid mt_grid(int nx, int ny, int sms, bool pre, int fixed_rows = 0) {
     const int w = pre ? MT_PRE_COLS : MT_POST_COLS, halo = pre ? MT_PRE_HALO : MT_POST_HALO;
     const int more = sizeof(T) == 4 ? 16 : 4;
     const int tx = (nx + w - 1) / w;
@@ -412,6 +436,7 @@ static MtGrid mt_grid(int nx, int ny, int sms, bool pre) {
     for (int rows = MT_ROWS; rows >= halo + 2; rows -= 2) {
         const int tiles = tx * ((ny + rows - halo - 1) / (rows - halo));
         const long long c = (long long)((tiles + sms - 1) / sms) * (rows + more);
+        if (fixed_rows > 0 && rows != fixed_rows) continue;
         if (cost < 0 || c < cost) {
             cost = c;
             best = MtGrid{tx, tiles, rows};

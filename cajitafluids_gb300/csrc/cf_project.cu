@@ -600,9 +600,8 @@ struct Outer {
     double *part0, *part1;
     SolverState* S;
     int gated;  // inside the MG-PCG graph: run only while the refinement is due
-    // rows of a warp's unit (U counts units of that many rows); mg: one partial per
-    // block, else one per unit of CF_BAND_ROWS rows (the Jacobi solver's sum order)
-    int rows, mg;
+    int mg;     // the MG-PCG's: a partial per block (the Jacobi solver's are per unit, in its order)
+    int split;  // warps to a unit of CF_BAND_ROWS rows, CF_BAND_ROWS / split rows each
 };
 
 // The solution values the residual is taken of: x itself, or (fused, upd)
@@ -891,41 +890,46 @@ __global__ void __launch_bounds__(CF_RED_THREADS) k_outer_resid(Outer a) {
     const XSrc xs{a.xbuf[sel], (it & 1) ? a.pa : a.pb, (float)Z.alpha_in, FUSED && mode == 2};
     float2* xo = a.xbuf[sel ^ 1];
     const int lane = threadIdx.x & 31;
-    const int unit = blockIdx.x * CF_RED_WARPS + (threadIdx.x >> 5);
+    const int warp = threadIdx.x >> 5;
     float arz = 0.f, arr = 0.f;
     // Units next to a wall along x (column groups 0 and G - 1) are slower than
     // interior ones (an odd nx: several times): they are numbered first, two per
     // row band, so that they fill blocks of their own and no interior warp waits
     // for one at the end-of-block barrier.
-    int g, band;
-    if (!a.per_x && a.G > 2) {
-        const int nb = 2 * (a.U / a.G);
-        if (unit < nb) {
-            band = unit >> 1;
-            g = (unit & 1) ? a.G - 1 : 0;
+    auto place = [&](int unit, int& g, int& band) {
+        if (!a.per_x && a.G > 2) {
+            const int nb = 2 * (a.U / a.G);
+            if (unit < nb) {
+                band = unit >> 1;
+                g = (unit & 1) ? a.G - 1 : 0;
+            } else {
+                band = (unit - nb) / (a.G - 2);
+                g = 1 + (unit - nb) % (a.G - 2);
+            }
         } else {
-            band = (unit - nb) / (a.G - 2);
-            g = 1 + (unit - nb) % (a.G - 2);
+            g = unit % a.G;
+            band = unit / a.G;
         }
-    } else {
-        g = unit % a.G;
-        band = unit / a.G;
-    }
-    const int j0u = band * a.rows, j1u = min(j0u + a.rows, a.ny);
+    };
+    const int part = blockIdx.x * CF_RED_WARPS + warp, unit = part / a.split, rows = CF_BAND_ROWS / a.split;
+    int g, band;
+    place(unit, g, band);
+    const int j0u = band * CF_BAND_ROWS + (part % a.split) * rows, j1u = min(j0u + rows, a.ny);
+    const bool have = unit < a.U && j0u < a.ny;
     // rows j0u - 1 .. j1u and columns g * 64 - 1 .. g * 64 + 64 are read:
     // inside the domain, or wrapped along a periodic axis
     const bool full_x = (g + 1) * CF_UNIT_COLS <= a.nx;
-    const bool interior = unit < a.U && full_x &&
+    const bool interior = have && full_x &&
                           (a.per_x || (g * CF_UNIT_COLS >= 1 && (g + 1) * CF_UNIT_COLS + 1 <= a.nx)) &&
                           (a.per_y || (j0u >= 1 && j1u + 2 <= a.ny));
     __shared__ __align__(16) float ring[CF_RED_WARPS * OR_RING * OrSlot<FUSED>::value];
     if (interior) {
         outer_unit_ring<FUSED, false>(a, xs, xo, ring + (threadIdx.x >> 5) * OR_RING * OrSlot<FUSED>::value, lane,
                                       g * CF_UNIT_COLS + 2 * lane, j0u, j1u, arz, arr);
-    } else if (unit < a.U && (a.nx & 1) == 0 && a.nx % CF_UNIT_COLS != 2) {
+    } else if (have && (a.nx & 1) == 0 && a.nx % CF_UNIT_COLS != 2) {
         outer_unit_ring<FUSED, true>(a, xs, xo, ring + (threadIdx.x >> 5) * OR_RING * OrSlot<FUSED>::value, lane,
                                      g * CF_UNIT_COLS + 2 * lane, j0u, j1u, arz, arr);
-    } else if (unit < a.U) {
+    } else if (have) {
         const int c0 = g * CF_UNIT_COLS + 2 * lane;
         const int j0 = j0u;
         const int j1 = j1u;
@@ -965,6 +969,33 @@ __global__ void __launch_bounds__(CF_RED_THREADS) k_outer_resid(Outer a) {
             xm = xc;
             xc = xp;
             xp = xpp;
+        }
+    }
+    if (a.split > 1) {
+        // the sums in a whole unit's order, from the residuals just written
+        arz = arr = 0.f;
+        __syncthreads();
+        const int nu = CF_RED_WARPS / a.split, u2 = blockIdx.x * nu + warp;
+        if (warp < nu && u2 < a.U) {
+            place(u2, g, band);
+            const int c0 = g * CF_UNIT_COLS + 2 * lane, j0 = band * CF_BAND_ROWS;
+            float2 rv[CF_BAND_ROWS];
+#pragma unroll
+            for (int k = 0; k < CF_BAND_ROWS; ++k)
+                rv[k] = j0 + k < a.ny && c0 < a.nx
+                            ? *reinterpret_cast<const float2*>(a.r32 + (ptrdiff_t)(j0 + k) * a.pitch32 + c0)
+                            : make_float2(0.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < CF_BAND_ROWS; ++k) {
+                if (j0 + k < a.ny && c0 < a.nx) {
+                    arz = fmaf(rv[k].x, a.minv32[edge_bits(c0, j0 + k, a.nx, a.ny, a.per_x, a.per_y)] * rv[k].x, arz);
+                    arr = fmaf(rv[k].x, rv[k].x, arr);
+                }
+                if (j0 + k < a.ny && c0 + 1 < a.nx) {
+                    arz = fmaf(rv[k].y, a.minv32[edge_bits(c0 + 1, j0 + k, a.nx, a.ny, a.per_x, a.per_y)] * rv[k].y, arz);
+                    arr = fmaf(rv[k].y, rv[k].y, arr);
+                }
+            }
         }
     }
     double v[2] = {(double)warp_fold_f(arr), (double)warp_fold_f(arz)};  // r.r, r.z
@@ -1581,19 +1612,17 @@ static Outer outer_args(cf_ctx* c, const Stencil& st, int gated, int mg) {
     oa.part1 = c->partials + c->n_units;
     oa.S = c->S;
     oa.gated = gated;
-    oa.rows = CF_BAND_ROWS;
     oa.mg = mg;
-    if (mg) {
-        // 16 rows to a warp leave most of the chip idle on small grids: fewer while the
-        // warps are at most 16 to an SM (a 1024^2 step: 0.88 ms with 16 rows, 0.77 with
-        // 8, 0.78 with 4, whose units read half as many rows again for their halo)
-        while (oa.rows > 4 && (long long)oa.G * ((oa.ny + oa.rows / 2 - 1) / (oa.rows / 2)) <= 16ll * c->sms) oa.rows /= 2;
-        oa.U = oa.G * ((oa.ny + oa.rows - 1) / oa.rows);
-    }
+    oa.split = 1;
+    // 16 rows to a warp leave most of the chip idle on small grids: two or four warps
+    // to a unit while they are at most 16 to an SM (1024^2: 35 -> 19 us).  A unit's FP32
+    // sums stay one chain over its 16 rows: the inner solve's scalars are taken in FP32,
+    // and another order moves the solution by a part in 1e8.
+    while (mg && oa.split < 4 && 2ll * oa.split * oa.U <= 16ll * c->sms) oa.split *= 2;
     return oa;
 }
 
-static int outer_blocks(const Outer& oa) { return (oa.U + CF_RED_WARPS - 1) / CF_RED_WARPS; }
+static int outer_blocks(const Outer& oa) { return (oa.U * oa.split + CF_RED_WARPS - 1) / CF_RED_WARPS; }
 
 // warm start: the initial residual from the previous solution (after the
 // divergence kernel), FP64 or double-float; returns kernels launched
