@@ -45,6 +45,9 @@ constexpr int kBoxBytes = kBX * kBY * 4; // 9792
 constexpr int kSlot = 9856;              // 128-byte aligned slot
 constexpr int kStages = 3;
 constexpr int kThreads = 256;
+// CTAs to an SM of K1 and K2: the FP32 sums of a CTA's tiles follow the grid, so it is
+// fixed here rather than left to the registers a build happens to need
+constexpr int kCtas1 = 3, kCtas2 = 2;
 constexpr unsigned kWaitLimit = 1u << 22;
 // the drain after a timeout waits longer than any tile wait: a CTA must not
 // exit while one of its bulk copies may still be writing its shared memory
@@ -221,7 +224,7 @@ __device__ void abandon(SolverState* S, const uint64_t* bars, int kfirst, int kt
 // K1: new direction (with halo) in shared memory, stencil, p.q.  MG: on z, whose
 // preconditioner is the identity.
 template <bool MG>
-__global__ void __launch_bounds__(kThreads, MG ? 4 : 2)
+__global__ void __launch_bounds__(kThreads, MG ? 4 : kCtas1)
     k_tma_dir_matvec32(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_pa,
                        const __grid_constant__ CUtensorMap map_pb, Cg32T a) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -355,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, MG ? 4 : 2)
 
 // K2: recompute A p, update x (double-float) and r, r.z and r.r.  x is read
 // with plain loads issued before the tile's copies are awaited.
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, kCtas2)
     k_tma_update32(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_pa,
                    const __grid_constant__ CUtensorMap map_pb, Cg32T a) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -469,8 +472,9 @@ __global__ void __launch_bounds__(kThreads, 2)
         a.part1[blockIdx.x] = trr;
     }
     if (last_block_arrive(&S->ticket[6])) {
-        double rz = final_tree(a.part0, gridDim.x);
-        double rr = final_tree(a.part1, gridDim.x);
+        double sums[2];
+        final_trees<2>(a.part0, a.part1, gridDim.x, sums);
+        const double rz = sums[0], rr = sums[1];
         if (tid == 0) {
             S->ticket[6] = 0;
             S->rho_prev = S->rho_in;
@@ -1005,8 +1009,8 @@ int cg32_setup(cf_ctx* c) {
                                                                          kStages * 2 * kSlot + 128),
                         "occupancy");
     if (rc) return rc;
-    occ1 = occ1 < 1 ? 1 : occ1;
-    occ2 = occ2 < 1 ? 1 : occ2;
+    occ1 = std::clamp(occ1, 1, kCtas1);
+    occ2 = std::clamp(occ2, 1, kCtas2);
     c->cta32 = c->tiles < occ1 * sms ? c->tiles : occ1 * sms;
     c->cta32b = c->tiles < occ2 * sms ? c->tiles : occ2 * sms;
     return pcg32_setup(c);

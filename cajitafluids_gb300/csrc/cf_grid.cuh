@@ -35,19 +35,11 @@ __device__ __forceinline__ bool grid_wait(SolverState* S, unsigned target, unsig
     return __syncthreads_and(ok);
 }
 
-// The strided part of final_tree over n unit partials: thread t of the 256
+// The strided part of final_trees over n unit partials: thread t of the 256
 // adds partial[t], partial[t + 256], ... in that order.
 __device__ __forceinline__ double strided_sum(const double* part, int n, int t) {
     double s = 0.0;
     for (int u = t; u < n; u += CF_RED_THREADS) s = s + __ldcg(part + u);
-    return s;
-}
-
-// Lane 0's warp_fold when only the first n lanes hold values and the others
-// are zero: the exchanges that would add a zero to it are left out.
-__device__ __forceinline__ double warp_fold_n(double s, int n) {
-    for (int m = 16; m >= 1; m >>= 1)
-        if (n > m) s = s + __shfl_xor_sync(0xffffffffu, s, m);
     return s;
 }
 

@@ -137,48 +137,79 @@ __device__ __forceinline__ double warp_max(double s) {  // s >= 0
     return s;
 }
 
-// Returns true in the block that arrives last.  Every thread fences its own
-// global writes before the block takes its ticket.
+// Returns true in the block that arrives last, with every block's global writes
+// before its arrival visible to it.
 __device__ __forceinline__ bool last_block_arrive(unsigned int* ticket) {
     __shared__ bool am_last;
-    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
+        // the barriers order the block's accesses with this thread's, its fences those
+        // with the other blocks' (a fence by every thread waits for all their stores)
+        __threadfence();
         unsigned int t = atomicAdd(ticket, 1u);
         am_last = (t == gridDim.x - 1);
+        __threadfence();
     }
     __syncthreads();
-    if (am_last) __threadfence();
     return am_last;
 }
 
-// Canonical final sum over n partials; blockDim.x must be 256.  All threads
-// return the same value.
-// Each thread adds partial[t], partial[t + 256], ... in that order; the
-// loads go out eight at a time ahead of the additions (one block does this
-// at the end of a launch, so a chain of dependent loads would be its tail).
+// Canonical final sums over n partials; blockDim.x must be 256.  Thread t adds
+// partial[t], partial[t + 256], ... in that order, a butterfly folds each warp and
+// the warp sums are added in order.  Warps without a partial would add zeros and are
+// left out; where half the warps hold all partials, two sums take a half each.
 constexpr int CF_FOLD_BATCH = 8;
-__device__ __forceinline__ double final_tree(const double* partial, int n) {
-    __shared__ double ws[CF_RED_WARPS];
+__device__ __forceinline__ double batched_sum(const double* part, int n, int t) {
     double s = 0.0;
-    int u = threadIdx.x;
+    int u = t;
+    // the loads go out eight at a time ahead of the additions (one block does this
+    // at the end of a launch, so a chain of dependent loads would be its tail)
     for (; u + (CF_FOLD_BATCH - 1) * CF_RED_THREADS < n; u += CF_FOLD_BATCH * CF_RED_THREADS) {
         double v[CF_FOLD_BATCH];
 #pragma unroll
-        for (int k = 0; k < CF_FOLD_BATCH; ++k) v[k] = __ldcg(partial + u + k * CF_RED_THREADS);
+        for (int k = 0; k < CF_FOLD_BATCH; ++k) v[k] = __ldcg(part + u + k * CF_RED_THREADS);
 #pragma unroll
         for (int k = 0; k < CF_FOLD_BATCH; ++k) s = s + v[k];
     }
-    for (; u < n; u += CF_RED_THREADS) s = s + __ldcg(partial + u);
-    s = warp_fold(s);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-    __syncthreads();
-    double tot = ws[0];
+    for (; u < n; u += CF_RED_THREADS) s = s + __ldcg(part + u);
+    return s;
+}
+// Lane 0's warp_fold when only the first n lanes hold values and the others
+// are zero: the exchanges that would add a zero to it are left out.
+__device__ __forceinline__ double warp_fold_n(double s, int n) {
+    for (int m = 16; m >= 1; m >>= 1)
+        if (n > m) s = s + __shfl_xor_sync(0xffffffffu, s, m);
+    return s;
+}
+template <int NQ>
+__device__ __forceinline__ void final_trees(const double* part0, const double* part1, int n, double (&out)[NQ]) {
+    __shared__ double ws[NQ][CF_RED_WARPS], tot[NQ];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nw = min(CF_RED_WARPS, (n + 31) / 32);
+    const bool halves = NQ == 2 && nw <= CF_RED_WARPS / 2;
 #pragma unroll
-    for (int k = 1; k < CF_RED_WARPS; ++k) tot = tot + ws[k];
+    for (int q = 0; q < NQ; ++q) {
+        const int w = halves && q == 1 ? warp - CF_RED_WARPS / 2 : warp;
+        if (w >= 0 && w < nw) {
+            const double s = warp_fold_n(batched_sum(q == 0 ? part0 : part1, n, w * 32 + lane), n - 32 * w);
+            if (lane == 0) ws[q][w] = s;
+        }
+    }
     __syncthreads();
-    return tot;
+    if (warp < NQ) {
+        double t = ws[warp][0];
+        for (int k = 1; k < nw; ++k) t = t + ws[warp][k];
+        if (lane == 0) tot[warp] = t;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) out[q] = tot[q];
+    __syncthreads();
+}
+__device__ __forceinline__ double final_tree(const double* partial, int n) {
+    double v[1];
+    final_trees<1>(partial, nullptr, n, v);
+    return v[0];
 }
 
 // Grid totals of NQ sums (1 or 2), where the sum order is free: v holds the warp's

@@ -65,19 +65,15 @@ __device__ __forceinline__ bool converged(const SolverState* S, double rr) {
 // K1: direction update + stencil apply + partial p.q
 __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_cg_dir_matvec64(Cg64 a) {
     __shared__ double P[UNIT_P], Q[UNIT_CELLS];
-    __shared__ int s_it;
-    __shared__ double s_beta;
+    __shared__ SolverState Z;  // the state on entry
     SolverState* S = a.S;
     const int tid = threadIdx.x;
-    if (tid == 0) {
-        s_it = *(volatile int*)&S->status == ST_RUNNING ? S->iter : -1;
-        s_beta = S->beta;
-    }
+    copy_state(&Z, S);
     __syncthreads();
-    const int it = s_it;
-    if (it < 0) return;
+    if (Z.status != ST_RUNNING) return;
+    const int it = Z.iter;
     const bool first = it == 0;
-    const double beta = s_beta, ms = a.st.ms;
+    const double beta = Z.beta, ms = a.st.ms;
     const double* pold = (it & 1) ? a.pb : a.pa;
     double* pnew = (it & 1) ? a.pa : a.pb;
     for (int unit = blockIdx.x; unit < a.U; unit += gridDim.x) {
@@ -140,7 +136,7 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_cg_dir_matvec64
             if (!(pq > 0.0))
                 S->status = isnan(pq) ? ST_NAN : ST_BREAKDOWN;
             else
-                S->alpha = S->rho / pq;
+                S->alpha = Z.rho / pq;
         }
     }
 }
@@ -149,19 +145,15 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_cg_dir_matvec64
 // preconditioner, whose r.z follows its V-cycle) and r.r
 __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS / 2) k_cg_update64(Cg64 a) {
     __shared__ double R[UNIT_CELLS], Z[UNIT_CELLS];
-    __shared__ int s_it;
-    __shared__ double s_alpha;
+    __shared__ SolverState E;  // the state on entry
     SolverState* S = a.S;
     const int tid = threadIdx.x;
-    if (tid == 0) {
-        s_it = *(volatile int*)&S->status == ST_RUNNING ? S->iter : -1;
-        s_alpha = S->alpha;
-    }
+    copy_state(&E, S);
     __syncthreads();
-    const int it = s_it;
-    if (it < 0) return;
+    if (E.status != ST_RUNNING) return;
+    const int it = E.iter;
     const double* pv = (it & 1) ? a.pa : a.pb;
-    const double alpha = s_alpha, malpha = -alpha;
+    const double alpha = E.alpha, malpha = -alpha;
     for (int unit = blockIdx.x; unit < a.U; unit += gridDim.x) {
         if (unit != (int)blockIdx.x) __syncthreads();  // the last unit's sums are done with shared memory
         const UnitPos u = unit_pos(unit, a.G, a.nx, a.ny);
@@ -204,21 +196,28 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS / 2) k_cg_update64
         }
     }
     if (last_block_arrive(&S->ticket[1])) {
-        double rz = a.mg ? 0.0 : final_tree(a.part0, a.U);
-        double rr = final_tree(a.part1, a.U);
+        double rz = 0.0, rr;
+        if (a.mg) {
+            rr = final_tree(a.part1, a.U);
+        } else {
+            double sums[2];
+            final_trees<2>(a.part0, a.part1, a.U, sums);
+            rz = sums[0];
+            rr = sums[1];
+        }
         if (threadIdx.x == 0) {
             S->ticket[1] = 0;
             if (!a.mg) {
-                S->beta = rz / S->rho;
+                S->beta = rz / E.rho;
                 S->rho = rz;
             }
             S->rr = rr;
             S->iter = it + 1;
             if (isnan(rr))
                 S->status = ST_NAN;
-            else if (converged(S, rr))
+            else if (converged(&E, rr))
                 S->status = ST_CONVERGED;
-            else if (it + 1 >= S->max_iter)
+            else if (it + 1 >= E.max_iter)
                 S->status = ST_MAXIT;
         }
     }
@@ -228,10 +227,10 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS / 2) k_cg_update64
 // rho only).  Runs only while the solve is live.
 __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_mg_rz64(Cg64 a, int init) {
     __shared__ double R[UNIT_CELLS], Z[UNIT_CELLS];
-    __shared__ int s_live;
+    __shared__ SolverState E;  // the state on entry
     SolverState* S = a.S;
     const int tid = threadIdx.x;
-    if (tid == 0) s_live = *(volatile int*)&S->status == ST_RUNNING;
+    copy_state(&E, S);
     for (int unit = blockIdx.x; unit < a.U; unit += gridDim.x) {
         if (unit != (int)blockIdx.x) __syncthreads();
         const UnitPos u = unit_pos(unit, a.G, a.nx, a.ny);
@@ -249,7 +248,7 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_mg_rz64(Cg64 a,
             Z[cell] = z;
         }
         __syncthreads();
-        if (!s_live) return;  // (the same answer for every unit)
+        if (E.status != ST_RUNNING) return;  // (the same answer for every unit)
         if (tid / 32 == unit_warp(unit)) {
             const double s = unit_dot(R, CF_UNIT_COLS, Z, CF_UNIT_COLS, tid & 31);
             if ((tid & 31) == 0) a.part0[unit] = s;
@@ -259,7 +258,7 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_mg_rz64(Cg64 a,
         double rz = final_tree(a.part0, a.U);
         if (threadIdx.x == 0) {
             S->ticket[7] = 0;
-            if (!init) S->beta = rz / S->rho;
+            if (!init) S->beta = rz / E.rho;
             S->rho = rz;
         }
     }
@@ -328,8 +327,9 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_warm_resid64(Cg
         }
     }
     if (last_block_arrive(&S->ticket[3])) {
-        double rz = final_tree(a.part0, a.U);
-        double rr = final_tree(a.part1, a.U);
+        double sums[2];
+        final_trees<2>(a.part0, a.part1, a.U, sums);
+        const double rz = sums[0], rr = sums[1];
         if (threadIdx.x == 0) {
             S->ticket[3] = 0;
             start_solve64(S, rr, rz);
@@ -430,8 +430,9 @@ __global__ void __launch_bounds__(CF_RED_THREADS, UNIT_BLOCKS) k_div_init64(DivA
         }
     }
     if (last_block_arrive(&S->ticket[2])) {
-        double rz = final_tree(a.part0, a.U);
-        double rr = final_tree(a.part1, a.U);
+        double sums[2];
+        final_trees<2>(a.part0, a.part1, a.U, sums);
+        const double rz = sums[0], rr = sums[1];
         if (threadIdx.x == 0) {
             S->ticket[2] = 0;
             S->bb = rr;
@@ -549,8 +550,9 @@ __global__ void __launch_bounds__(CF_RED_THREADS) k_div_init_mixed(DivArgs a) {
         a.part1[unit] = drz;
     }
     if (last_block_arrive(&S->ticket[2])) {
-        const double bb = final_tree(a.part0, a.U);
-        const double rz = final_tree(a.part1, a.U);
+        double sums[2];
+        final_trees<2>(a.part0, a.part1, a.U, sums);
+        const double bb = sums[0], rz = sums[1];
         const double rr = bb;
         if (threadIdx.x == 0) {
             S->ticket[2] = 0;
@@ -1007,8 +1009,7 @@ __global__ void __launch_bounds__(CF_RED_THREADS) k_outer_resid(Outer a) {
             a.part1[unit] = v[1];
         }
         if (!last_block_arrive(&S->ticket[4])) return;
-        v[0] = final_tree(a.part0, a.U);
-        v[1] = final_tree(a.part1, a.U);
+        final_trees<2>(a.part0, a.part1, a.U, v);
         if (threadIdx.x == 0) S->ticket[4] = 0;
     }
     if (threadIdx.x == 0) {
