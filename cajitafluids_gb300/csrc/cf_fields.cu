@@ -318,21 +318,24 @@ __device__ __forceinline__ float max_nan(float x, float y) {
     return r;
 }
 
-// One CTA per 32 x 32 tile and entity kind (blockIdx.x, fastest, so that the
-// kinds of one tile run together and share its windows through L2; tiles
-// along blockIdx.y, blockIdx.z).  The CTA copies the windows of u, v and
+// One CTA per 32 x 32 tile and KINDS entity kinds from ent0 + blockIdx.x on (fastest,
+// so that the kinds of one tile run together and share its windows through L2; tiles
+// along blockIdx.y, blockIdx.z): all three where the tiles alone fill the SMs, which
+// stages the u and v windows once instead of three times and fixes each kind's
+// offsets at compile time (bound by instruction issue, 340 -> 268 an entity: 472 ->
+// 375 us at 4096^2), one where they do not.  The CTA copies the windows of u, v and
 // (cells) q into shared memory, 16-byte rows, and takes the largest |u|, |v|
 // in them, M.  Every RK velocity is a convex combination of window values,
 // so while (dt / dx) M <= 0.99 no position moves a full cell and the traces
 // read only the window; otherwise (or with a NaN, or when a test asks for
 // it) the tile reads global memory with the clamped stencil.  Either way
 // each entity gets the same bits.
-template <int ORDER>
-__global__ void __launch_bounds__(256, 8) k_advect32(Adv32 a) {
+template <int ORDER, int KINDS>
+__global__ void __launch_bounds__(256, KINDS == 3 ? 6 : 8) k_advect32(Adv32 a) {
     __shared__ __align__(16) float sw[3 * AW_N];  // u, v, q windows
     __shared__ float red[8];
     const Phys& p = a.p;
-    const int ent = blockIdx.x + a.ent0;
+    const int ent1 = KINDS == 3 ? (int)E_CELL : blockIdx.x + a.ent0;
     const int gi0 = blockIdx.y * AT_X, gj0 = blockIdx.z * AT_Y;
     const int lane = threadIdx.x & 31, wrow = threadIdx.x >> 5;
     // The window's origin is ghosted (gi0 - 1, gj0 + 1); rows past an array
@@ -357,7 +360,7 @@ __global__ void __launch_bounds__(256, 8) k_advect32(Adv32 a) {
             m = max_nan(m, max_nan(fabsf(w.x), fabsf(w.z)));
         }
     }
-    if (ent == E_CELL) {
+    if (ent1 == E_CELL) {
         constexpr int kRowChunks = AW_X / 4, kChunks = AW_Y * kRowChunks;
         const float* src = a.q.o + (size_t)(gj0 + 1) * a.q.pitch + (gi0 - 1);
         const int nrow = a.q.ey - (gj0 + 1), nc4 = (a.q.pitch - CF_COL0 - gi0 + 1) >> 2;
@@ -378,55 +381,59 @@ __global__ void __launch_bounds__(256, 8) k_advect32(Adv32 a) {
     for (int w = 1; w < 8; ++w) big = max_nan(big, red[w]);
     const bool staged = !a.unstaged && a.c * big <= 0.99f;
 
-    const int ox = p.nx + ((ent == E_FACEI && !p.per_x) ? 1 : 0);
-    const int oy = p.ny + ((ent == E_FACEJ && !p.per_y) ? 1 : 0);
-    const int fa = ent == E_CELL ? 2 : (ent == E_FACEI ? 0 : 1);
-    const GlobalTaps gu{reinterpret_cast<const float*>(a.u.o), a.u.pitch, a.u.ex, a.u.ey, 2},
-        gv{reinterpret_cast<const float*>(a.v.o), a.v.pitch, a.v.ex, a.v.ey, 2};
-    const GlobalTaps gf =
-        ent == E_CELL ? GlobalTaps{a.q.o, a.q.pitch, a.q.ex, a.q.ey, 1} : (ent == E_FACEI ? gu : gv);
+#pragma unroll
+    for (int kind = 0; kind < KINDS; ++kind) {
+        const int ent = ent1 + kind;  // (all three: a constant, so that its offsets and taps fold)
+        const int ox = p.nx + ((ent == E_FACEI && !p.per_x) ? 1 : 0);
+        const int oy = p.ny + ((ent == E_FACEJ && !p.per_y) ? 1 : 0);
+        const int fa = ent == E_CELL ? 2 : (ent == E_FACEI ? 0 : 1);
+        const GlobalTaps gu{reinterpret_cast<const float*>(a.u.o), a.u.pitch, a.u.ex, a.u.ey, 2},
+            gv{reinterpret_cast<const float*>(a.v.o), a.v.pitch, a.v.ex, a.v.ey, 2};
+        const GlobalTaps gf =
+            ent == E_CELL ? GlobalTaps{a.q.o, a.q.pitch, a.q.ex, a.q.ey, 1} : (ent == E_FACEI ? gu : gv);
 #pragma unroll 1
-    for (int k = 0; k < AT_Y / 8; ++k) {
-        const int gi = gi0 + lane, gj = gj0 + wrow + 8 * k;
-        if (gi >= ox || gj >= oy) continue;
-        const int li = gi + CF_HALO, lj = gj + CF_HALO;
-        float val;
-        if (staged) {
-            const WindowTaps U{sw, gi0 - 1, gj0 + 1}, V{sw + AW_N, gi0 - 1, gj0 + 1},
-                F{sw + fa * AW_N, gi0 - 1, gj0 + 1};
-            val = advect_value<ORDER>(a, ent, li, lj, U, V, F);
-        } else {
-            val = advect_value<ORDER>(a, ent, li, lj, gu, gv, gf);
-        }
-        if (ent == E_CELL) {
-            // cell inputs (src/Solver.hpp:181-263): the clamp max(q, Q) rounds to
-            // the same FP32 value when taken in FP32; the rate form in FP64
-            if (a.fuse && in_box_idx(p, E_CELL, li, lj)) {
-                if (p.src_mode == 0) {
-                    const float qf = (float)p.src_q;
-                    if (val < qf) val = qf;
-                } else {
-                    val = (float)__dadd_rn((double)val, __dmul_rn(p.src_q, a.dt));
+        for (int k = 0; k < AT_Y / 8; ++k) {
+            const int gi = gi0 + lane, gj = gj0 + wrow + 8 * k;
+            if (gi >= ox || gj >= oy) continue;
+            const int li = gi + CF_HALO, lj = gj + CF_HALO;
+            float val;
+            if (staged) {
+                const WindowTaps U{sw, gi0 - 1, gj0 + 1}, V{sw + AW_N, gi0 - 1, gj0 + 1},
+                    F{sw + fa * AW_N, gi0 - 1, gj0 + 1};
+                val = advect_value<ORDER>(a, ent, li, lj, U, V, F);
+            } else {
+                val = advect_value<ORDER>(a, ent, li, lj, gu, gv, gf);
+            }
+            if (ent == E_CELL) {
+                // cell inputs (src/Solver.hpp:181-263): the clamp max(q, Q) rounds to
+                // the same FP32 value when taken in FP32; the rate form in FP64
+                if (a.fuse && in_box_idx(p, E_CELL, li, lj)) {
+                    if (p.src_mode == 0) {
+                        const float qf = (float)p.src_q;
+                        if (val < qf) val = qf;
+                    } else {
+                        val = (float)__dadd_rn((double)val, __dmul_rn(p.src_q, a.dt));
+                    }
+                }
+                a.qn.at(li, lj) = val;
+                continue;
+            }
+            // face inputs (src/Solver.hpp:181-263) on the pair (val, 0): the inflow
+            // velocity where it is larger, then the body force, then the walls
+            const int axis = ent == E_FACEI ? 0 : 1;
+            float2 w = make_float2(val, 0.f);
+            if (a.fuse) {
+                if (in_box_idx(p, ent, li, lj) && fabs((double)val) < fabs(p.src_vel[axis])) w = df_split(p.src_vel[axis]);
+                if (a.force_on[axis]) w = df_add(w, a.fdt2[axis]);
+                const int per = axis == 0 ? p.per_x : p.per_y, n = axis == 0 ? p.nx : p.ny, gg = axis == 0 ? gi : gj;
+                if (!per) {
+                    if (gg <= 0 && p.bc[axis] == 0) w = make_float2(0.f, 0.f);
+                    if (gg > n - 1 && p.bc[axis + 2] == 0) w = make_float2(0.f, 0.f);
                 }
             }
-            a.qn.at(li, lj) = val;
-            continue;
+            double& dst = axis == 0 ? a.un.at(li, lj) : a.vn.at(li, lj);
+            reinterpret_cast<float2&>(dst) = w;
         }
-        // face inputs (src/Solver.hpp:181-263) on the pair (val, 0): the inflow
-        // velocity where it is larger, then the body force, then the walls
-        const int axis = ent == E_FACEI ? 0 : 1;
-        float2 w = make_float2(val, 0.f);
-        if (a.fuse) {
-            if (in_box_idx(p, ent, li, lj) && fabs((double)val) < fabs(p.src_vel[axis])) w = df_split(p.src_vel[axis]);
-            if (a.force_on[axis]) w = df_add(w, a.fdt2[axis]);
-            const int per = axis == 0 ? p.per_x : p.per_y, n = axis == 0 ? p.nx : p.ny, gg = axis == 0 ? gi : gj;
-            if (!per) {
-                if (gg <= 0 && p.bc[axis] == 0) w = make_float2(0.f, 0.f);
-                if (gg > n - 1 && p.bc[axis + 2] == 0) w = make_float2(0.f, 0.f);
-            }
-        }
-        double& dst = axis == 0 ? a.un.at(li, lj) : a.vn.at(li, lj);
-        reinterpret_cast<float2&>(dst) = w;
     }
 }
 
@@ -621,10 +628,18 @@ cudaError_t launch_advect(cf_ctx* c, double dt, int order, int fuse_inputs, int 
         }
         (void)prep;
         const dim3 tiles(nent, (p.nx + 1 + AT_X - 1) / AT_X, (p.ny + 1 + AT_Y - 1) / AT_Y);
-        if (order == 1)
-            k_advect32<1><<<tiles, 256, 0, c->stream>>>(a);
+        // the kinds together from four tiles to an SM (an advection with its launch: 512^2
+        // 26.7 against 25.6 us apart, 800^2 35.9 against 36.7, 1500^2 70 against 81)
+        const bool together = nent == 3 && (long long)tiles.y * tiles.z >= 4ll * c->sms;
+        const dim3 one(1, tiles.y, tiles.z);
+        if (together && order == 1)
+            k_advect32<1, 3><<<one, 256, 0, c->stream>>>(a);
+        else if (together)
+            k_advect32<3, 3><<<one, 256, 0, c->stream>>>(a);
+        else if (order == 1)
+            k_advect32<1, 1><<<tiles, 256, 0, c->stream>>>(a);
         else
-            k_advect32<3><<<tiles, 256, 0, c->stream>>>(a);
+            k_advect32<3, 1><<<tiles, 256, 0, c->stream>>>(a);
     }
     c->launches += 1;
     if (advance) {
