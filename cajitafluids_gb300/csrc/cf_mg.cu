@@ -109,15 +109,13 @@ __global__ void __launch_bounds__(MG_BX* MG_BY) k_mg_smooth(MgLev<T> L, MgBc p, 
         if (gj >= L.ny) break;
         const size_t row = (size_t)gj * L.pitch;
         if (gi < L.nx) {
-            T s;
-            if (first) {
-                s = T(0);
-            } else {
-                s = mg_at(p, L.x, L.pitch, L.nx, L.ny, gi - 1, gj) + mg_at(p, L.x, L.pitch, L.nx, L.ny, gi + 1, gj);
+            T t = L.b[row + gi];
+            if (!first) {
+                T s = mg_at(p, L.x, L.pitch, L.nx, L.ny, gi - 1, gj) + mg_at(p, L.x, L.pitch, L.nx, L.ny, gi + 1, gj);
                 s = s + mg_at(p, L.x, L.pitch, L.nx, L.ny, gi, gj - 1);
                 s = s + mg_at(p, L.x, L.pitch, L.nx, L.ny, gi, gj + 1);
+                t = mg_fma(L.scale, s, t);
             }
-            T t = mg_fma(L.scale, s, L.b[row + gi]);
             L.x[row + gi] = mg_mul(t, L.invd[mg_bits(p, L.nx, L.ny, gi, gj)]);
         }
         const int go = 2 * pair + (1 - par);

@@ -295,13 +295,13 @@ struct McRow {
             const T w = FIRST ? T(0) : west();
 #pragma unroll
             for (int i = 0; i < HC; ++i) {
-                T t = T(0);
+                T t = b[2 * i];
                 if (!FIRST) {
                     t = (i == 0 ? w : x[(2 * i + CPL - 1) % CPL]) + x[2 * i + 1];
                     t = t + s[i];
                     t = t + n[i];
+                    t = mg_fma(scale, t, b[2 * i]);
                 }
-                t = mg_fma(scale, t, b[2 * i]);
                 v[i] = x[2 * i] = mask(2 * i, t * ((i == 0 && lane == 0) ? idw : idm));
             }
         } else {
@@ -309,13 +309,13 @@ struct McRow {
 #pragma unroll
             for (int i = 0; i < HC; ++i) {
                 const int k = 2 * i + 1;
-                T t = T(0);
+                T t = b[k];
                 if (!FIRST) {
                     t = x[k - 1] + right(k, e);
                     t = t + s[i];
                     t = t + n[i];
+                    t = mg_fma(scale, t, b[k]);
                 }
-                t = mg_fma(scale, t, b[k]);
                 v[i] = x[k] = mask(k, t * ((!FULL || k == CPL - 1) && end(k) ? ide : idm));
             }
         }
@@ -412,7 +412,7 @@ __device__ __forceinline__ void mc_down(const MgCoarse<T>& P, const MgBc& p, con
             // the inner one the wall's
             const bool lo = i == 0 && lane == 0 && !p.per_x;
             const bool hi = (!FULL || i == HC - 1) && !p.per_x && r.end(2 * i + 1);
-            T t = mg_fma(lo ? T(0) : T(0.25), i == 0 ? qw : q[(2 * i + CPL - 1) % CPL], T(0));
+            T t = lo ? T(0) : mg_quarter(i == 0 ? qw : q[(2 * i + CPL - 1) % CPL]);
             t = mg_fma(lo && p.bc[0] == 0 ? T(1) : T(0.75), q[2 * i], t);
             t = mg_fma(hi && p.bc[2] == 0 ? T(1) : T(0.75), q[2 * i + 1], t);
             v[i] = mg_fma(hi ? T(0) : T(0.25), r.right(2 * i + 1, qe), t);
@@ -433,10 +433,10 @@ __device__ __forceinline__ void mc_down(const MgCoarse<T>& P, const MgBc& p, con
             T v[HC];
             mc_ld<HC>(v, rs + (2 * warp - 1 + a + MC_H) * 32 * HC + lane * HC);
 #pragma unroll
-            for (int i = 0; i < HC; ++i) acc[i] = mg_fma(wy[a], v[i], acc[i]);
+            for (int i = 0; i < HC; ++i) acc[i] = a == 0 ? mg_quarter(v[i]) : mg_fma(wy[a], v[i], acc[i]);
         }
 #pragma unroll
-        for (int i = 0; i < HC; ++i) acc[i] = T(0.25) * acc[i];
+        for (int i = 0; i < HC; ++i) acc[i] = mg_quarter(acc[i]);
         if (l + 1 < K.ns) {
             mc_st<HC>(K.sm + P.bo[l + 1] + (warp + MC_H) * P.sp[l + 1] + lane * HC, acc);
         } else {
@@ -787,14 +787,14 @@ __global__ void __launch_bounds__(MC_THREADS, 1) k_mg_coarse(const __grid_consta
                     if (out) g = g < 0 ? g + ny : g - ny;
                     // (a cell beyond a wall has weight 0 and reads its neighbour)
                     const T* rr = r + (g + 1) * sp + PAD;
-                    T rs = mg_fma(wx[0], rr[fa], T(0));
+                    T rs = I > 0 || p.per_x ? mg_quarter(rr[fa]) : T(0);
                     rs = mg_fma(wx[1], rr[f], rs);
                     rs = mg_fma(wx[2], rr[f + 1], rs);
                     rs = mg_fma(wx[3], rr[fd], rs);
-                    const T v = mg_fma(wy[a], rs, acc);
+                    const T v = a == 0 ? mg_quarter(rs) : mg_fma(wy[a], rs, acc);
                     if (!out || p.per_y) acc = v;
                 }
-                sm[P.bo[l + 1] + J * P.sp[l + 1] + PAD + I] = T(0.25) * acc;
+                sm[P.bo[l + 1] + J * P.sp[l + 1] + PAD + I] = mg_quarter(acc);
             }
             mc_bar(bar, n);
         }

@@ -58,26 +58,26 @@ struct MtRow {
             const T w = FIRST ? T(0) : west();
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                T t = T(0);
+                T t = b[2 * i];
                 if (!FIRST) {
                     t = (i == 0 ? w : x[1]) + x[2 * i + 1];
                     t = t + s[i];
                     t = t + n[i];
+                    t = mg_fma(scale, t, b[2 * i]);
                 }
-                t = mg_fma(scale, t, b[2 * i]);
                 v[i] = x[2 * i] = t * id[2 * i];
             }
         } else {
             const T e = FIRST ? T(0) : east();
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                T t = T(0);
+                T t = b[2 * i + 1];
                 if (!FIRST) {
                     t = x[2 * i] + (i == 1 ? e : x[2]);
                     t = t + s[i];
                     t = t + n[i];
+                    t = mg_fma(scale, t, b[2 * i + 1]);
                 }
-                t = mg_fma(scale, t, b[2 * i + 1]);
                 v[i] = x[2 * i + 1] = t * id[2 * i + 1];
             }
         }
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mg_pre_rows(const __grid_cons
             for (int i = 0; i < 2; ++i) {
                 // beside a wall the outer weight is 0 and the inner one the wall's
                 const bool lo = !p.per_x && r.c0 + 2 * i == 0, hi = !p.per_x && r.c0 + 2 * i + 1 == F.nx - 1;
-                T t2 = mg_fma(lo ? T(0) : T(0.25), i == 0 ? qw : q[1], T(0));
+                T t2 = lo ? T(0) : mg_quarter(i == 0 ? qw : q[1]);
                 t2 = mg_fma(lo && p.bc[0] == 0 ? T(1) : T(0.75), q[2 * i], t2);
                 t2 = mg_fma(hi && p.bc[2] == 0 ? T(1) : T(0.75), q[2 * i + 1], t2);
                 v[i] = mg_fma(hi ? T(0) : T(0.25), i == 0 ? q[2] : qe, t2);
@@ -232,12 +232,12 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mg_pre_rows(const __grid_cons
                 if (!p.per_y && (g < 0 || g >= F.ny)) continue;
                 T v[2];
                 mc_ld<2>(v, rs + (2 * warp + a) * (MT_COLS / 2) + lane * 2);
-                acc[0] = mg_fma(wy[a], v[0], acc[0]);
-                acc[1] = mg_fma(wy[a], v[1], acc[1]);
+                acc[0] = a == 0 ? mg_quarter(v[0]) : mg_fma(wy[a], v[0], acc[0]);
+                acc[1] = a == 0 ? mg_quarter(v[1]) : mg_fma(wy[a], v[1], acc[1]);
             }
             T* o = cb + (size_t)J * cpitch + I;
-            o[0] = T(0.25) * acc[0];
-            if (I + 1 < nc) o[1] = T(0.25) * acc[1];
+            o[0] = mg_quarter(acc[0]);
+            if (I + 1 < nc) o[1] = mg_quarter(acc[1]);
         }
     }
 }
