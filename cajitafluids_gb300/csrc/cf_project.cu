@@ -447,15 +447,68 @@ __device__ __forceinline__ float2 pair_at(const Grid<double>& g, int i, int j) {
 }
 __device__ __forceinline__ float2 df_neg(float2 x) { return make_float2(-x.x, -x.y); }
 
+// Two double-float values side by side, (h.x, l.x) and (h.y, l.y): a lane's
+// two cells, so that each error-free step runs as one packed f32x2
+// instruction for both (each half rounded as the scalar form, hence the bits
+// of df_resid_int cell by cell).
+struct DF2 {
+    float2 h, l;
+};
+__device__ __forceinline__ DF2 df2_two_sum(float2 a, float2 b) {
+    const float2 s = f2_add(a, b);
+    const float2 bb = f2_sub(s, a);
+    return DF2{s, f2_add(f2_sub(a, f2_sub(s, bb)), f2_sub(b, bb))};
+}
+__device__ __forceinline__ DF2 df2_quick(float2 a, float2 b) {
+    const float2 s = f2_add(a, b);
+    return DF2{s, f2_sub(b, f2_sub(s, a))};
+}
+__device__ __forceinline__ DF2 df2_add_s(DF2 x, DF2 y) {
+    DF2 s = df2_two_sum(x.h, y.h);
+    s.l = f2_add(s.l, f2_add(x.l, y.l));
+    return df2_quick(s.h, s.l);
+}
+// the accurate sum and difference (df_add)
+__device__ __forceinline__ DF2 df2_two_diff(float2 a, float2 b) {
+    const float2 s = f2_sub(a, b);
+    const float2 bb = f2_sub(s, a);
+    return DF2{s, f2_sub(f2_sub(a, f2_sub(s, bb)), f2_add(b, bb))};
+}
+__device__ __forceinline__ DF2 df2_join(DF2 s, DF2 t) {
+    s.l = f2_add(s.l, t.h);
+    s = df2_quick(s.h, s.l);
+    s.l = f2_add(s.l, t.l);
+    return df2_quick(s.h, s.l);
+}
+__device__ __forceinline__ DF2 df2_add(DF2 x, DF2 y) { return df2_join(df2_two_sum(x.h, y.h), df2_two_sum(x.l, y.l)); }
+__device__ __forceinline__ DF2 df2_sub(DF2 x, DF2 y) { return df2_join(df2_two_diff(x.h, y.h), df2_two_diff(x.l, y.l)); }
+// df_mul by one pair for both (the leading product as scalar operations: the compiler
+// fuses a packed product and the packed additions that use it)
+__device__ __forceinline__ DF2 df2_scale(float2 c, DF2 x) {
+    const float2 p = make_float2(__fmul_rn(c.x, x.h.x), __fmul_rn(c.x, x.h.y));
+    float2 e = make_float2(fmaf(c.x, x.h.x, -p.x), fmaf(c.x, x.h.y, -p.y));
+    const float2 ch = make_float2(c.x, c.x), cl = make_float2(c.y, c.y);
+    e = f2_fma(ch, x.l, e);
+    e = f2_fma(cl, x.h, e);
+    return df2_quick(p, e);
+}
+// two adjacent pairs of an array as they are stored
+__device__ __forceinline__ DF2 df2_of(float4 v) { return DF2{make_float2(v.x, v.z), make_float2(v.y, v.w)}; }
+__device__ __forceinline__ float4 df2_pairs(DF2 v) { return make_float4(v.h.x, v.l.x, v.h.y, v.l.y); }
+__device__ __forceinline__ DF2 df2_neg(DF2 x) {
+    const float2 m = make_float2(-1.f, -1.f);
+    return DF2{f2_mul(m, x.h), f2_mul(m, x.l)};
+}
 // The divergences of one unit's cells (64 columns x up to 16 rows, lane l
 // on columns c0 = 64 g + 2 l and c0 + 1), row by row: each row loads the
 // lane's two u pairs and two v pairs of row j + 1 as 16-byte vectors (row j's
 // v pairs come from the previous row), the E face of column c0 + 1 from the
 // next lane, and reads directly only the one pair a wrap, the domain's last
 // column or the warp's last lane needs; every load of row j + 1 is issued
-// before row j's divergences are handed to f.  Calls f(c, j, div) for every
-// owned cell, div = ((u_E - u_W) + v_N) - v_S of its face pairs in
-// double-float (E across a periodic wrap is column 0, N row 0).
+// before row j's divergences are handed to f.  Calls f(c0, j, two, div) for the
+// lane's cells of every row (the second one when two), div = ((u_E - u_W) + v_N)
+// - v_S of their face pairs in double-float (E across a periodic wrap is column 0,
+// N row 0).
 template <typename F>
 __device__ __forceinline__ void div_pairs_unit(const DivArgs& a, int g, int band, int lane, F&& f) {
     const int c0 = g * CF_UNIT_COLS + 2 * lane;
@@ -502,16 +555,10 @@ __device__ __forceinline__ void div_pairs_unit(const DivArgs& a, int g, int band
             // column c0: E face c0 + 1 (or column 0 across a periodic wrap)
             float2 ue1 = make_float2(uu.z, uu.w);
             if (e1) ue1 = ex;
-            float2 t = df_add(ue1, df_neg(make_float2(uu.x, uu.y)));
-            t = df_add(t, make_float2(v1.x, v1.y));
-            t = df_add(t, df_neg(make_float2(v0.x, v0.y)));
-            f(c0, j, t);
-            if (two) {
-                float2 t1 = df_add(ue2, df_neg(make_float2(uu.z, uu.w)));
-                t1 = df_add(t1, make_float2(v1.z, v1.w));
-                t1 = df_add(t1, df_neg(make_float2(v0.z, v0.w)));
-                f(c0 + 1, j, t1);
-            }
+            DF2 t = df2_sub(DF2{make_float2(ue1.x, ue2.x), make_float2(ue1.y, ue2.y)}, df2_of(uu));
+            t = df2_add(t, df2_of(v1));
+            t = df2_sub(t, df2_of(v0));
+            f(c0, j, two, t);
         }
         v0 = v1;
     }
@@ -528,18 +575,29 @@ __global__ void __launch_bounds__(CF_RED_THREADS) k_div_init_mixed(DivArgs a) {
     if (unit < a.U) {
         // the divergence of the velocity pairs and its scale -1/dx, in
         // double-float on the FP32 pipe
-        div_pairs_unit(a, unit % a.G, unit / a.G, lane, [&](int c, int j, float2 t) {
+        div_pairs_unit(a, unit % a.G, unit / a.G, lane, [&](int c, int j, bool two, DF2 t) {
             const size_t k = (size_t)j * a.pitch + c;
-            const float2 bs = df_mul(a.mscale2, t);
-            reinterpret_cast<float2*>(a.b)[k] = bs;
+            const DF2 bs = df2_scale(a.mscale2, t);
             // x as a double-float pair: 0, or (warm start) the previous
             // FP64 solution split in place (same 8 bytes per cell)
-            reinterpret_cast<float2*>(a.x)[k] = a.warm ? df_split(a.x[k]) : make_float2(0.f, 0.f);
-            const float r = bs.x;
-            put_r32(a.r32, a.pitch32, a.nx, a.ny, a.per_x, a.per_y, c, j, r);
-            float z = a.st.minv32[edge_bits(c, j, a.nx, a.ny, a.per_x, a.per_y)] * r;
-            abb = fmaf(r, r, abb);
-            arz = fmaf(r, z, arz);
+            float2* x = reinterpret_cast<float2*>(a.x) + k;
+            if (two) {
+                *reinterpret_cast<float4*>(reinterpret_cast<float2*>(a.b) + k) = df2_pairs(bs);
+                if (!a.warm) *reinterpret_cast<float4*>(x) = make_float4(0.f, 0.f, 0.f, 0.f);
+            } else {
+                reinterpret_cast<float2*>(a.b)[k] = make_float2(bs.h.x, bs.l.x);
+                if (!a.warm) *x = make_float2(0.f, 0.f);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                if (i == 1 && !two) break;
+                if (a.warm) x[i] = df_split(a.x[k + i]);
+                const float r = i == 0 ? bs.h.x : bs.h.y;
+                put_r32(a.r32, a.pitch32, a.nx, a.ny, a.per_x, a.per_y, c + i, j, r);
+                const float z = a.st.minv32[edge_bits(c + i, j, a.nx, a.ny, a.per_x, a.per_y)] * r;
+                abb = fmaf(r, r, abb);
+                arz = fmaf(r, z, arz);
+            }
         });
     }
     // inner r.r equals b.b here (the same squares in the same order)
@@ -683,31 +741,6 @@ __device__ __forceinline__ float2 df_resid_int(const Outer& a, float2 b, float2 
     return df_add_s(b, make_float2(-ax.x, -ax.y));
 }
 
-// Two double-float values side by side, (h.x, l.x) and (h.y, l.y): a lane's
-// two cells, so that each error-free step runs as one packed f32x2
-// instruction for both (each half rounded as the scalar form, hence the bits
-// of df_resid_int cell by cell).
-struct DF2 {
-    float2 h, l;
-};
-__device__ __forceinline__ DF2 df2_two_sum(float2 a, float2 b) {
-    const float2 s = f2_add(a, b);
-    const float2 bb = f2_sub(s, a);
-    return DF2{s, f2_add(f2_sub(a, f2_sub(s, bb)), f2_sub(b, bb))};
-}
-__device__ __forceinline__ DF2 df2_quick(float2 a, float2 b) {
-    const float2 s = f2_add(a, b);
-    return DF2{s, f2_sub(b, f2_sub(s, a))};
-}
-__device__ __forceinline__ DF2 df2_add_s(DF2 x, DF2 y) {
-    DF2 s = df2_two_sum(x.h, y.h);
-    s.l = f2_add(s.l, f2_add(x.l, y.l));
-    return df2_quick(s.h, s.l);
-}
-__device__ __forceinline__ DF2 df2_neg(DF2 x) {
-    const float2 m = make_float2(-1.f, -1.f);
-    return DF2{f2_mul(m, x.h), f2_mul(m, x.l)};
-}
 // df_resid for a lane's two cells: the residuals' high parts.  d: the diagonal
 // factors; without walls next to the unit 4, and 4 x is exact.
 template <bool WALL>
@@ -1444,10 +1477,15 @@ __global__ void __launch_bounds__(CF_RED_THREADS) k_div_norms(DivArgs a) {
     const int unit = blockIdx.x * CF_RED_WARPS + (threadIdx.x >> 5);
     float fss = 0.f, fmx = 0.f;
     if (unit < a.U)
-        div_pairs_unit(a, unit % a.G, unit / a.G, lane, [&](int, int, float2 t) {
-            const float bf = t.x * a.mscale32;
+        div_pairs_unit(a, unit % a.G, unit / a.G, lane, [&](int, int, bool two, DF2 t) {
+            float bf = t.h.x * a.mscale32;
             fss = fmaf(bf, bf, fss);
             fmx = fmaxf(fmx, fabsf(bf));
+            if (two) {
+                bf = t.h.y * a.mscale32;
+                fss = fmaf(bf, bf, fss);
+                fmx = fmaxf(fmx, fabsf(bf));
+            }
         });
     const double ass = warp_fold((double)fss);
     const double amx = warp_max((double)fmx);
