@@ -46,7 +46,7 @@ MG_NAMES = ("PFMG", "SMG", "MG")
 # DRAM bytes (read + write) of one mixed MG-PCG inner iteration at 4096^2:
 # dram__bytes_read.sum + dram__bytes_write.sum of this bench's kernels, one
 # kernel per ncu capture (K1, the fused x update and reliable update, the
-# V-cycle's pre- and post-smoothing per level, the bottom solve), summed over
+# V-cycle's pre- and post-smoothing per level, the coarse levels), summed over
 # one iteration
 MEASURED_TRAFFIC_MG_ITER_4096 = 1.234e9
 
@@ -340,7 +340,8 @@ def bench_gb300(args, rank, world, dist, device):
         if mg:
             kname = ("MG-PCG inner iteration: k_tma_dir_matvec32 + k_outer_resid<true> (x update fused with the "
                      "reliable update; at an update threshold below 0.5, k_tma_update32 + gated k_outer_resid) + "
-                     "V-cycle (k_mg_pre/k_mg_post per level with r.z in the finest post-smoothing, k_mg_bottom)")
+                     "V-cycle (k_mg_pre/k_mg_post and k_mg_pre_rows/k_mg_post_rows per level with r.z in the "
+                     "finest post-smoothing, k_mg_coarse)")
             kern_extra = {}
         else:
             kname = "inner CG iteration (k_tma_dir_matvec32 + k_tma_update32)"

@@ -26,8 +26,8 @@
 //
 // What bounds it: with one or two units per SM the serial lane sums (32
 // dependent FMAs of 64 cycles, 1 us each phase), the two grid barriers (about
-// 1.2 us each) and the divisions; at seven units per SM the FP64 pipe (12
-// operations per cell and iteration: 21 of 33 us).  Measured on GB300, time of
+// 1.2 us each) and the divisions; at seven units per SM the FP64 pipe (10
+// operations per cell and iteration: 18 of 31 us).  Measured on GB300, time of
 // one iteration, the two launches per iteration before and this: 64^2 39.9 ->
 // 9.7 us, 256^2 49.6 -> 10.4 us, 1024^2 53.8 -> 31.1 us.
 #include <cuda_runtime.h>
