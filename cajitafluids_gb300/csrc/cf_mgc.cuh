@@ -4,14 +4,14 @@
 // and operation order it repeats, so each value is the one the launch-per-level
 // kernels form).
 //
-// Why: below about 256^2 cells a level is latency.  As launches, each level
-// cost 6.5-7 us per direction in FP32 (9-12 us in FP64) and the one-CTA bottom
-// solver 34 us (45-65 us): 74 us of an FP32 V-cycle and 128 us of an FP64 one
-// at 256^2 and 128^2.  Inside a cluster the levels meet at a hardware barrier
-// (0.2 us) and read each other's rows directly: 28 us (FP32 from 256^2; 41 us
-// between the launches of a 4096^2 cycle, whose traffic leaves the caches cold)
-// and 52 us (FP64 from 128^2), 10 and 17 us when only the levels from 32^2 and
-// 16^2 are there.
+// Why: a small level is latency.  As launches of shared-memory tiles, each level
+// below 256^2 cost 6.5-7 us per direction in FP32 (9-12 us in FP64) and a one-CTA
+// solver of the last ones 34 us (45-65 us): 74 us of an FP32 V-cycle and 128 us of
+// an FP64 one from 256^2 and 128^2.  Inside a cluster the levels meet at a hardware
+// barrier (0.2 us) and read each other's rows directly: 20 us (FP32 from 128^2; 29 us
+// between the launches of a 4096^2 cycle, whose traffic leaves the caches cold) and
+// 33 us (FP64 from 64^2), 10 and 17 us when only the levels from 32^2 and 16^2 are
+// there.
 //
 // Levels [0, ns) are distributed: a CTA owns a band of rows (twice as many on
 // each finer level).  Within a level no CTA waits for another: MC_H halo rows
@@ -35,14 +35,19 @@ constexpr long long MC_COARSEST = 1024;  // cells of the coarsest level at most
 constexpr int MC_WARPS = MC_THREADS / 32;
 
 // Largest first level, its most columns (32 lanes of CPL), and the level size
-// CTA 0 takes alone.  FP32: 256^2.  FP64: 128^2, since an SM executes two FP64
-// operations per cycle and the 256^2 level keeps 128 SMs busy as tiles; alone
-// up to 16^2 for the same reason.
+// CTA 0 takes alone.  A cluster is 16 of the SMs and recomputes its halo rows, so a
+// level goes there only once its launches (cf_mgt.cuh) are latency too.  FP32:
+// 128^2 (a 1024^2 step 0.797 ms, with 256^2 in the cluster 0.806, from 64^2 on 0.807;
+// 4096^2 2.535, 2.549, 2.529).  FP64, where an SM executes two operations per cycle:
+// 64^2 (a 192x160 step 0.682 ms, with 96x80 in the cluster 0.737, without 48x40
+// 0.727; 512^2 adjoint 8.34 + 12.88, 8.58 + 13.15, 8.63 + 13.23); alone up to 16^2 for
+// the same reason.
 template <typename T>
 struct McMax {
-    static constexpr int first = sizeof(T) == 4 ? 65536 : 16384;
+    static constexpr int first = sizeof(T) == 4 ? 16384 : 4096;
     static constexpr int columns = sizeof(T) == 4 ? 256 : 128;
     static constexpr int alone = sizeof(T) == 4 ? 1024 : 256;
+    static_assert(alone <= 2 * MC_THREADS, "a thread of CTA 0 holds one cell pair");
 };
 
 template <typename T>
