@@ -1201,8 +1201,8 @@ int mg_setup(cf_ctx* c) {
         ny /= 2;
     }
     if (!rc && !mixed)
-        rc = cuda_check(c, cudaFuncSetAttribute(k_mg_post_rows<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)MT_POST_SMEM<double>),
+        rc = cuda_check(c, cudaFuncSetAttribute(k_mg_post_rows<double, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)MT_POST_SMEM<double, 4>),
                         "multigrid level kernels: shared memory");
     if (!rc) rc = mixed ? coarse_setup(c, H, H->f) : coarse_setup(c, H, H->d);
     return rc;
@@ -1321,8 +1321,11 @@ static int vcycle(cf_ctx* c, const MgHierarchy* H, MgLev<T>* lev, double scale0,
                 }
             } else {
                 const MtGrid m = mt_grid<T>(lev[l].nx, lev[l].ny, c->sms, true);
-                k_mg_pre_rows<T><<<std::min(m.tiles, c->sms), 32 * m.rows, 0, c->stream>>>(
-                    lev[l], lev[l + 1].b, lev[l + 1].pitch, p, c->S, inner, m.tx, m.tiles);
+                auto* kern = k_mg_pre_rows<T, 4>;
+                if constexpr (sizeof(T) == 8)
+                    if (m.cpl == 2) kern = k_mg_pre_rows<T, 2>;
+                kern<<<std::min(m.tiles, c->sms), 32 * m.rows, 0, c->stream>>>(lev[l], lev[l + 1].b, lev[l + 1].pitch, p, c->S,
+                                                                              inner, m.tx, m.tiles);
             }
             ++launches;
             continue;
@@ -1383,8 +1386,15 @@ static int vcycle(cf_ctx* c, const MgHierarchy* H, MgLev<T>* lev, double scale0,
                 }
             } else {
                 const MtGrid m = mt_grid<T>(lev[l].nx, lev[l].ny, c->sms, false, E.on ? MT_RZ_ROWS : 0);
-                k_mg_post_rows<T><<<std::min(m.tiles, c->sms), 32 * m.rows, MT_POST_SMEM<T>, c->stream>>>(
-                    lev[l + 1].x, lev[l + 1].pitch, lev[l], p, c->S, inner, m.tx, m.tiles, E);
+                auto* kern = k_mg_post_rows<T, 4>;
+                size_t smem = MT_POST_SMEM<T, 4>;
+                if constexpr (sizeof(T) == 8)
+                    if (m.cpl == 2) {
+                        kern = k_mg_post_rows<T, 2>;
+                        smem = MT_POST_SMEM<T, 2>;
+                    }
+                kern<<<std::min(m.tiles, c->sms), 32 * m.rows, smem, c->stream>>>(lev[l + 1].x, lev[l + 1].pitch, lev[l], p, c->S,
+                                                                                inner, m.tx, m.tiles, E);
             }
             ++launches;
             continue;

@@ -39,8 +39,9 @@ constexpr int MC_WARPS = MC_THREADS / 32;
 // level goes there only once its launches (cf_mgt.cuh) are latency too.  FP32:
 // 128^2 (a 1024^2 step 0.797 ms, with 256^2 in the cluster 0.806, from 64^2 on 0.807;
 // 4096^2 2.535, 2.549, 2.529).  FP64, where an SM executes two operations per cycle:
-// 64^2 (a 192x160 step 0.682 ms, with 96x80 in the cluster 0.737, without 48x40
-// 0.727; 512^2 adjoint 8.34 + 12.88, 8.58 + 13.15, 8.63 + 13.23); alone up to 16^2 for
+// 64^2 (a 192x160 step 0.617 ms, without 48x40 0.628; 512^2 adjoint 7.90 + 12.35, 7.95
+// + 12.40; with 96x80 and 128^2 in it, before these levels had narrow windows, 0.737
+// against 0.682 and 8.58 + 13.15 against 8.34 + 12.88); alone up to 16^2 for
 // the same reason.
 template <typename T>
 struct McMax {

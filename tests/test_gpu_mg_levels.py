@@ -10,7 +10,9 @@ from test_gpu_mg_coarse import BCS, _project
 pytestmark = pytest.mark.gpu
 
 SIZES = {"mixed": [(32, 16), (112, 24), (116, 44), (120, 48), (244, 92), (600, 304), (2020, 940)],
-         "fp64": [(272, 64), (224, 88), (228, 92), (240, 96), (244, 200), (600, 304), (1016, 1000)]}
+         "fp64": [(272, 64), (224, 88), (228, 92), (240, 96), (244, 200), (600, 304), (1016, 1000),
+                  # (two columns to a lane: 52 | 56 columns kept)
+                  (104, 80), (106, 44), (112, 96), (114, 100), (156, 64), (192, 160), (256, 256)]}
 
 
 @pytest.mark.parametrize("precision,nx,ny", [(p, *s) for p in SIZES for s in SIZES[p]])
