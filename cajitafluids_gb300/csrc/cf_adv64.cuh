@@ -9,9 +9,15 @@ namespace cf {
 
 static __constant__ double ENT_OFF_D[3][2] = {{0.5, 0.5}, {0.0, 0.5}, {0.5, 0.0}};
 
+// a plain product on the integer pipes (IP) or by the hardware: the same bits
+template <bool IP>
+__device__ __forceinline__ double prod64(double a, double b) {
+    return IP ? mul64i(a, b) : a * b;
+}
+
 // FP64 spline weights (Cajita B-spline order 1 / 3); the coordinate clamp, the cell
 // and the linear weights come from the integer-pipe helpers (cf_internal.cuh).
-template <int ORDER>
+template <int ORDER, bool IP = true>
 __device__ __forceinline__ void weights64(double xi, int ext, int& k0, double* w) {
     int k;
     double t, s;
@@ -22,13 +28,13 @@ __device__ __forceinline__ void weights64(double xi, int ext, int& k0, double* w
         k0 = k;
     } else {
         cell_fraction(clamp_bits(xi, 1.0, exact_double(ext - 2)), ext - 3, k, t, s);
-        double t2 = mul64i(t, t);
-        double t3 = mul64i(t2, t);
-        double s3 = mul64i(mul64i(s, s), s);
-        w[0] = mul64i(s3, 1.0 / 6.0);
+        double t2 = prod64<IP>(t, t);
+        double t3 = prod64<IP>(t2, t);
+        double s3 = prod64<IP>(prod64<IP>(s, s), s);
+        w[0] = prod64<IP>(s3, 1.0 / 6.0);
         w[1] = fma(0.5, t3, -t2) + (2.0 / 3.0);
         w[2] = fma(0.5, (t + t2) - t3, 1.0 / 6.0);
-        w[3] = mul64i(t3, 1.0 / 6.0);
+        w[3] = prod64<IP>(t3, 1.0 / 6.0);
         k0 = k - 1;
     }
 }

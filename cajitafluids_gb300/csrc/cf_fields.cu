@@ -65,23 +65,23 @@ __global__ void k_fill_ghosts(Grid<T> g, int nox, int noy, int per_x, int per_y)
 // FP64 spline sample (Cajita B-spline order 1 / 3, evaluated separably);
 // the coordinate clamp, the cell and the linear weights come from the
 // integer-pipe helpers (cf_internal.cuh).
-template <int ORDER>
+template <int ORDER, bool IP = true>
 __device__ double sample64(const Phys& p, const Grid<double>& g, double lx, double ly, double x, double y) {
     constexpr int n = ORDER == 1 ? 2 : 4;
     double xi = times_rdx(x - lx, p.rdx, p.rsh);
     double yi = times_rdx(y - ly, p.rdx, p.rsh);
     int kx, ky;
     double wx[n], wy[n];
-    weights64<ORDER>(xi, g.ex, kx, wx);
-    weights64<ORDER>(yi, g.ey, ky, wy);
+    weights64<ORDER, IP>(xi, g.ex, kx, wx);
+    weights64<ORDER, IP>(yi, g.ey, ky, wy);
     double val = 0.0;
 #pragma unroll
     for (int b = 0; b < n; ++b) {
         const double* row = g.o + (size_t)(ky + b) * g.pitch + kx;
-        double rs = mul64i(wx[0], __ldg(row));
+        double rs = prod64<IP>(wx[0], __ldg(row));
 #pragma unroll
         for (int a = 1; a < n; ++a) rs = fma(wx[a], __ldg(row + a), rs);
-        val = (b == 0) ? mul64i(wy[0], rs) : fma(wy[b], rs, val);
+        val = (b == 0) ? prod64<IP>(wy[0], rs) : fma(wy[b], rs, val);
     }
     return val;
 }
@@ -502,12 +502,19 @@ struct Pts {
     double dt;
 };
 
+// Plain products of the point samples: few points wait for their own results and for
+// code to be fetched, of which integer products make several times as much; many are
+// bound by the FP64 pipe.  A call, us, hardware / integer products (cubic): 1000
+// points 30.5 / 39, 60000 52 / 53, 100000 172 / 163, 10^6 435 / 410; cell velocities of
+// 33^2 cells 33 / 42, of 200^2 and 300^2 the same.
+constexpr int POINTS_IP = 65536;
+template <bool IP>
 __global__ void k_interp_points(Pts a) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.n) return;
     double x = a.xy[2 * k], y = a.xy[2 * k + 1];
-    a.out[k] = a.order == 1 ? sample64<1>(a.p, a.f, a.p.low[a.ent][0], a.p.low[a.ent][1], x, y)
-                            : sample64<3>(a.p, a.f, a.p.low[a.ent][0], a.p.low[a.ent][1], x, y);
+    a.out[k] = a.order == 1 ? sample64<1, IP>(a.p, a.f, a.p.low[a.ent][0], a.p.low[a.ent][1], x, y)
+                            : sample64<3, IP>(a.p, a.f, a.p.low[a.ent][0], a.p.low[a.ent][1], x, y);
 }
 
 __global__ void k_trace_points(Pts a) {
@@ -522,14 +529,15 @@ __global__ void k_trace_points(Pts a) {
 // SiloWriter::writeFile's cell-centred velocity (src/SiloWriter.hpp:177-191):
 // interpolateVelocity<2, 1> (linear) of u and v at each owned cell centre,
 // written owned-region, x fastest, into uc, vc (pitch nx)
+template <bool IP>
 __global__ void k_cell_velocity(Phys p, Grid<double> u, Grid<double> v, double* uc, double* vc) {
     const int gi = blockIdx.x * blockDim.x + threadIdx.x;
     const int gj = blockIdx.y * blockDim.y + threadIdx.y;
     if (gi >= p.nx || gj >= p.ny) return;
     const double x = entity_coord(p, E_CELL, 0, gi + CF_HALO), y = entity_coord(p, E_CELL, 1, gj + CF_HALO);
     const size_t k = (size_t)gj * p.nx + gi;
-    uc[k] = sample64<1>(p, u, p.low[E_FACEI][0], p.low[E_FACEI][1], x, y);
-    vc[k] = sample64<1>(p, v, p.low[E_FACEJ][0], p.low[E_FACEJ][1], x, y);
+    uc[k] = sample64<1, IP>(p, u, p.low[E_FACEI][0], p.low[E_FACEI][1], x, y);
+    vc[k] = sample64<1, IP>(p, v, p.low[E_FACEJ][0], p.low[E_FACEJ][1], x, y);
 }
 
 // max |w| over the owned faces of one axis; non-negative doubles order like
@@ -740,7 +748,8 @@ cudaError_t launch_interp_points(cf_ctx* c, int field, int order, int n, const d
     if (velocity_f64(c, &gu, &gv)) return cudaErrorMemoryAllocation;
     Grid<double> f = field == CF_FIELD_QUANTITY ? c->q64[s] : (field == CF_FIELD_U ? gu : gv);
     Pts a{c->ph, f, gu, gv, field, order, n, d_xy, d_out, 0.0};
-    k_interp_points<<<(n + 127) / 128, 128, 0, c->stream>>>(a);
+    const auto kern = n >= POINTS_IP ? k_interp_points<true> : k_interp_points<false>;
+    kern<<<(n + 127) / 128, 128, 0, c->stream>>>(a);
     c->launches += 1;
     return cudaGetLastError();
 }
@@ -750,7 +759,8 @@ cudaError_t launch_cell_velocity(cf_ctx* c, double* d_uc, double* d_vc) {
     dim3 blk(32, 8);
     Grid<double> gu, gv;
     if (velocity_f64(c, &gu, &gv)) return cudaErrorMemoryAllocation;
-    k_cell_velocity<<<grid2(p.nx, p.ny, blk), blk, 0, c->stream>>>(p, gu, gv, d_uc, d_vc);
+    const auto kern = (long long)p.nx * p.ny >= POINTS_IP ? k_cell_velocity<true> : k_cell_velocity<false>;
+    kern<<<grid2(p.nx, p.ny, blk), blk, 0, c->stream>>>(p, gu, gv, d_uc, d_vc);
     c->launches += 1;
     return cudaGetLastError();
 }
