@@ -271,6 +271,16 @@ class Context:
                                                  w.ctypes.data_as(ctypes.POINTER(ctypes.c_double))))
         return f, w
 
+    def test_precondition(self, dt: float, r: np.ndarray, levels: bool = False):
+        """cf_test_precondition: one multigrid V-cycle on r; returns z and r.z."""
+        r = np.ascontiguousarray(r, dtype=np.float64)
+        assert r.shape == self.owned_shape("q")
+        z = np.empty_like(r)
+        rz = ctypes.c_double()
+        self._check(self.lib.cf_test_precondition(self.h, float(dt), int(bool(levels)), _dptr(r), _dptr(z),
+                                                  ctypes.byref(rz)))
+        return z, rz.value
+
     def max_velocity(self) -> float:
         a = ctypes.c_double()
         self._check(self.lib.cf_max_velocity(self.h, ctypes.byref(a)))

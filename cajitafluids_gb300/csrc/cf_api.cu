@@ -489,6 +489,14 @@ int cf_test_apply_general(cf_ctx* ctx, int on) {
     return CF_OK;
 }
 
+int cf_test_precondition(cf_ctx* ctx, double dt, int levels, const double* r, double* z, double* rz) {
+    if (!ctx || !r || !z || !rz || !(dt > 0.0)) return CF_ERR_INVALID;
+    CF_GUARD_BEGIN
+    cudaSetDevice(ctx->device);
+    return test_precondition(ctx, dt, levels != 0, r, z, rz);
+    CF_GUARD_END
+}
+
 int cf_set_density(cf_ctx* ctx, double density) {
     if (!ctx) return CF_ERR_INVALID;
     if (!(density > 0.0) || !isfinite(density)) return fail(ctx, CF_ERR_INVALID, "density must be positive");

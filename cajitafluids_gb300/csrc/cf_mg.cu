@@ -1063,6 +1063,7 @@ struct MgHierarchy {
     // shared memory
     int lc = 0, cluster = 0;
     size_t csmem = 0;
+    int test_levels = 0;  // cf_test_precondition: no fused levels and no cluster launch
     std::vector<void*> allocs;
 };
 
@@ -1281,7 +1282,7 @@ int mg_strip_geometry(int nx, int ny, int tw, int th, int strip_rows, int pre, i
 template <typename T>
 static int vcycle(cf_ctx* c, const MgHierarchy* H, MgLev<T>* lev, double scale0, int inner, int strip_rows,
                   double* epi_part, bool* epi_done) {
-    const int nlev = H->nlev, fused = H->fused;
+    const int nlev = H->nlev, fused = H->test_levels ? 0 : H->fused;
     MgBc p{c->ph.per_x, c->ph.per_y, {c->ph.bc[0], c->ph.bc[1], c->ph.bc[2], c->ph.bc[3]}};
     double s = scale0;
     for (int l = 0; l < nlev; ++l) {
@@ -1298,7 +1299,7 @@ static int vcycle(cf_ctx* c, const MgHierarchy* H, MgLev<T>* lev, double scale0,
         k_mg_smooth<T><<<grid2((L.nx + 1) / 2, L.ny), blk, 0, c->stream>>>(L, p, color, first, c->S, inner);
         ++launches;
     };
-    const int lb = H->lc;
+    const int lb = H->test_levels ? nlev : H->lc;
     const int top_end = lb < nlev ? lb : nlev - 1;  // levels smoothed by grid kernels on the way down
     // FP32 levels of at least 1024 tiles take the register strips, which recompute
     // fewer rows but need many of them to fill the SMs (pre-smoothing, us: 2048^2 19
@@ -1424,6 +1425,8 @@ int mg_vcycle(cf_ctx* c, double scale0, bool* rz_done) {
     if (rz_done) *rz_done = done;
     return n;
 }
+
+void mg_test_levels(cf_ctx* c, int on) { static_cast<MgHierarchy*>(c->mg)->test_levels = on; }
 
 int mg_levels(const cf_ctx* c) { return c->mg ? static_cast<const MgHierarchy*>(c->mg)->nlev : 0; }
 

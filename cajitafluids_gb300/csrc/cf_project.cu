@@ -36,6 +36,7 @@
 #include <cstdlib>
 #include <functional>
 #include <cstring>
+#include <vector>
 
 #include "cf_ctx.cuh"
 #include "cf_mul64.cuh"
@@ -2283,6 +2284,52 @@ int div_norms(cf_ctx* c, double* l2, double* linf) {
     launch_norms(c, a);
     c->launches += 1;
     return read_norms(c, l2, linf);
+}
+
+// cf_test_precondition
+int test_precondition(cf_ctx* c, double dt, int levels, const double* r, double* z, double* rz) {
+    const bool mixed = c->precision == CF_PREC_MIXED;
+    const int nx = c->ph.nx, ny = c->ph.ny;
+    int rc = mg_setup(c);
+    if (rc) return rc;
+    Stencil st{};
+    build_stencil(c, dt, 0, &st);
+    settle_pressure(c);  // (the solver state names the buffer it is in)
+    SolverState* h = c->hS;
+    memset(h, 0, sizeof(SolverState));
+    h->status = h->inner_status = ST_RUNNING;
+    cudaMemcpyAsync(c->S, h, sizeof(SolverState), cudaMemcpyHostToDevice, c->stream);
+    std::vector<float> f;
+    if (mixed) {
+        f.assign(r, r + (size_t)nx * ny);
+        cudaMemcpy2DAsync(c->r32.a, sizeof(float) * c->p32, f.data(), sizeof(float) * nx, sizeof(float) * nx, ny,
+                          cudaMemcpyHostToDevice, c->stream);
+    } else {
+        cudaMemcpy2DAsync(c->r.a, sizeof(double) * c->vpitch, r, sizeof(double) * nx, sizeof(double) * nx, ny,
+                          cudaMemcpyHostToDevice, c->stream);
+    }
+    mg_test_levels(c, levels);
+    if (mixed) {
+        c->launches += cg32_mg_precondition(c, -st.ms);
+    } else {
+        Cg64 a = cg64_args(c, st);
+        a.mg = 1;
+        a.z = mg_z64(c);
+        c->launches += 1 + mg_vcycle(c, -st.ms);
+        k_mg_rz64<<<unit_blocks(c), CF_RED_THREADS, 0, c->stream>>>(a, 1);
+    }
+    mg_test_levels(c, 0);
+    if ((rc = cuda_check(c, cudaGetLastError(), "preconditioner"))) return rc;
+    if (mixed)
+        cudaMemcpy2DAsync(f.data(), sizeof(float) * nx, c->z32.a, sizeof(float) * c->p32, sizeof(float) * nx, ny,
+                          cudaMemcpyDeviceToHost, c->stream);
+    else
+        cudaMemcpy2DAsync(z, sizeof(double) * nx, mg_z64(c), sizeof(double) * c->vpitch, sizeof(double) * nx, ny,
+                          cudaMemcpyDeviceToHost, c->stream);
+    if ((rc = read_state(c))) return rc;
+    if (mixed) std::copy(f.begin(), f.end(), z);
+    *rz = mixed ? c->hS->rho_in : c->hS->rho;
+    return CF_OK;
 }
 
 int project(cf_ctx* c, double dt, const SolveOpts& o, SolveResult* res) {

@@ -286,6 +286,13 @@ int cf_test_advect_unstaged(cf_ctx* ctx, int on);
  * instead of the unit-per-warp kernel.  The results are the same bits either
  * way; 0 switches the hook off. */
 int cf_test_apply_general(cf_ctx* ctx, int on);
+/* Test hook: z = M^-1 r of the multigrid preconditioner of a projection with
+ * time step dt, and rz = r.z as the solver forms it.  r, z: nx x ny arrays (x
+ * fastest); a mixed context rounds r to FP32 and works in FP32.  levels = 0:
+ * the launches a solve makes; levels != 0: every level, the coarsest included,
+ * by one launch per half sweep, residual, restriction and prolongation (the
+ * same bits in z).  The fields are left as they are. */
+int cf_test_precondition(cf_ctx* ctx, double dt, int levels, const double* r, double* z, double* rz);
 
 /* ---- output (replaces the device half of SiloWriter::writeFile) ----
  * SiloWriter interpolates the face velocities to cell centres for its
