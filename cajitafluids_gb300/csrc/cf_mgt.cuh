@@ -254,6 +254,40 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mg_pre_rows(const __grid_cons
     }
 }
 
+// A sum of FP32 terms in three words, each holding what the rounding of the one above
+// left out: 72 bits, more than FP64's 53 (two words would hold 48), of FP32's range,
+// as K1's p.q.  In FP64 a window's terms are 32 warp instructions of 64 cycles on four
+// sub-partitions and the warps' totals 40 more: a 1024^2 mixed step 0.817 ms, this way
+// 0.808 (0.813 with the warps' totals alone in FP64).
+struct Sum72 {
+    float h = 0.f, m = 0.f, l = 0.f;
+    // s + v rounded, e what that left out
+    __device__ __forceinline__ static float two_sum(float s, float v, float& e) {
+        const float t = s + v, d = t - s;
+        e = (s - (t - d)) + (v - d);
+        return t;
+    }
+    __device__ __forceinline__ void add(float v) {
+        float e, f;
+        h = two_sum(h, v, e);
+        m = two_sum(m, e, f);
+        l = l + f;
+    }
+    // the warp's total, in every lane
+    __device__ __forceinline__ double warp_total() {
+#pragma unroll
+        for (int k = 16; k >= 1; k >>= 1) {
+            const float oh = __shfl_xor_sync(0xffffffffu, h, k), om = __shfl_xor_sync(0xffffffffu, m, k);
+            const float ol = __shfl_xor_sync(0xffffffffu, l, k);
+            float f;
+            add(oh);
+            m = two_sum(m, om, f);
+            l = (l + ol) + f;
+        }
+        return (double)h + ((double)m + (double)l);
+    }
+};
+
 // x = x_pre + P x_coarse, (black, red) x 2, x written; on the finest FP32 level
 // also r.z and z's periodic ghosts (RzEpi)
 template <typename T, int CPL>
@@ -292,7 +326,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mg_post_rows(const T* cx, int
     if (!block_live(S, inner)) return;
     const T scale = F.scale;
     const int nc = F.nx / 2, mc = F.ny / 2;
-    T rz = T(0), rze = T(0);  // the lane's share of r.z: sum and what its rounding left out
+    Sum72 rz;  // the lane's share of r.z
     for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
         place(t, r.g, r.c0);
         r.live = (p.per_y || (r.g >= 0 && r.g < F.ny)) && r.g < F.ny + 4;
@@ -389,8 +423,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mg_post_rows(const T* cx, int
         }
         if (sizeof(T) == 4 && E.on) {
             // r.z in units of two cells eight rows apart, one fused operation each (the
-            // solver's fixed FP32 order; windows of MT_RZ_ROWS hold whole units), their
-            // sums as pairs
+            // solver's fixed FP32 order; windows of MT_RZ_ROWS hold whole units)
             constexpr int lo = MT_POST_HALO / 2;
             const bool own = lane >= HALO / CPL && lane < 32 - HALO / CPL && r.g < F.ny;
             if (warp >= lo && warp < lo + 8) {
@@ -406,24 +439,16 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mg_post_rows(const T* cx, int
 #pragma unroll
                 for (int k = 0; k < CPL; ++k) {
                     if (own && r.c0 + k < F.nx) v[k] = mg_fma(r.b[k], r.x[k], v[k]);
-                    const T s = rz + v[k], d = s - rz;
-                    rze = rze + ((rz - (s - d)) + (v[k] - d));
-                    rz = s;
+                    rz.add((float)v[k]);
                 }
             }
             __syncthreads();
         }
     }
     if (sizeof(T) == 4 && E.on) {
-        // FP64 additions by 32 warps would take 2600 cycles: pairs until the warp's total
-#pragma unroll
-        for (int m = 16; m >= 1; m >>= 1) {
-            const T a = __shfl_xor_sync(0xffffffffu, rz, m), b = __shfl_xor_sync(0xffffffffu, rze, m);
-            const T s = rz + a, d = s - rz;
-            rze = (rze + b) + ((rz - (s - d)) + (a - d));
-            rz = s;
-        }
-        double v[1] = {(double)rz + (double)rze};
+        double v[1] = {0.0};
+        // (the other warps hold nothing)
+        if (warp >= MT_POST_HALO / 2 + 8 && warp < MT_POST_HALO / 2 + 16) v[0] = rz.warp_total();
         const double den = S->refreshed ? S->rho_prev : S->rho_in;
         if (grid_totals<1, MT_ROWS>(v, E.part, nullptr, &S->ticket[7]) && threadIdx.x == 0) rz_scalars(S, v[0], den);
     }

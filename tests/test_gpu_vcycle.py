@@ -35,3 +35,25 @@ def test_vcycle_equals_levels(built, precision, nx, ny, periodic, bc):
     if precision == "fp64":
         zo, nlev = Oracle(nx, ny, hi=(1.0, ny / nx), periodic=periodic, bc=bc, density=rho, precon_mg=True).mg_apply(dt, r)
         assert nlev >= 2 and np.array_equal(z, zo)
+
+
+@pytest.mark.parametrize("seed", range(8))
+def test_rz_holds_fp64s_bits(built, seed):
+    """r.z of a finest level in row windows: terms of two cells eight rows apart in
+    FP32 (r z + (r z), one rounding each), their sum no less precise than in FP64.  r is four cells of one
+    row, 2^-24 and 2^-28 and 2^-32 times the first, so the sum has bits that a pair of
+    FP32 values (48 bits) cannot hold."""
+    from cajitafluids_gb300 import Context
+    nx, ny = 240, 96
+    rng = np.random.default_rng(seed)
+    i, j = 4 * int(rng.integers(1, nx // 4 - 1)), int(rng.integers(0, ny))
+    r = np.zeros((ny, nx))
+    r[j, i:i + 4] = (rng.uniform(1.0, 2.0, 4) * 2.0 ** np.array([0.0, -24.0, -28.0, -32.0])).astype(np.float32)
+    with Context(nx, ny, hi=(1.0, ny * (1.0 / nx)), precision="mixed") as c:
+        z, rz = c.test_precondition(0.01, r)
+    # the FP32 terms (the other cell of each unit holds r = 0), in exact arithmetic
+    from fractions import Fraction
+    terms = [Fraction(float(np.float32(r[j, k] * z[j, k]))) for k in range(i, i + 4)]  # (products of 48 bits are exact in FP64)
+    exact = sum(terms)
+    # at most three additions of non-zero terms, each off by half a unit of 2^-52
+    assert abs(Fraction(rz) - exact) <= 3 * Fraction(1, 2 ** 53) * sum(abs(t) for t in terms)
