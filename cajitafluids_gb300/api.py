@@ -281,6 +281,13 @@ class Context:
                                                   ctypes.byref(rz)))
         return z, rz.value
 
+    def test_residual(self, dt: float, split: bool = False) -> np.ndarray:
+        """cf_test_residual: b - A p of the current state, in FP32."""
+        r = np.empty(self.owned_shape("q"), dtype=np.float32)
+        self._check(self.lib.cf_test_residual(self.h, float(dt), int(bool(split)),
+                                              r.ctypes.data_as(ctypes.POINTER(ctypes.c_float))))
+        return r
+
     def max_velocity(self) -> float:
         a = ctypes.c_double()
         self._check(self.lib.cf_max_velocity(self.h, ctypes.byref(a)))

@@ -497,6 +497,13 @@ int cf_test_precondition(cf_ctx* ctx, double dt, int levels, const double* r, do
     CF_GUARD_END
 }
 
+int cf_test_residual(cf_ctx* ctx, double dt, int split, float* r) {
+    if (!ctx || !r || !(dt > 0.0)) return CF_ERR_INVALID;
+    if (ctx->precision != CF_PREC_MIXED) return fail(ctx, CF_ERR_UNSUPPORTED, "a mixed context is needed");
+    cudaSetDevice(ctx->device);
+    return test_residual(ctx, dt, split != 0, r);
+}
+
 int cf_set_density(cf_ctx* ctx, double density) {
     if (!ctx) return CF_ERR_INVALID;
     if (!(density > 0.0) || !isfinite(density)) return fail(ctx, CF_ERR_INVALID, "density must be positive");

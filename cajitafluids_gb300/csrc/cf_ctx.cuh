@@ -221,6 +221,7 @@ int mg_vcycle(cf_ctx* c, double scale0, bool* rz_done = nullptr);
 int mg_levels(const cf_ctx* c);
 void mg_test_levels(cf_ctx* c, int on);  // on: every launch of a V-cycle a single phase of one level
 int test_precondition(cf_ctx* c, double dt, int levels, const double* r, double* z, double* rz);
+int test_residual(cf_ctx* c, double dt, int split, float* r);
 int mg_strip_geometry(int nx, int ny, int tw, int th, int strip_rows, int pre, int* fields, int* frame_xy, int cap);
 double* mg_z64(cf_ctx* c);
 }  // namespace cf

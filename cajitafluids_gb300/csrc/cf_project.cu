@@ -2286,6 +2286,31 @@ int div_norms(cf_ctx* c, double* l2, double* linf) {
     return read_norms(c, l2, linf);
 }
 
+// cf_test_residual
+int test_residual(cf_ctx* c, double dt, int split, float* r) {
+    Stencil st{};
+    build_stencil(c, dt, 0, &st);
+    settle_pressure(c);  // (the solver state names the buffer it is in)
+    SolverState* h = c->hS;
+    memset(h, 0, sizeof(SolverState));
+    h->status = h->inner_status = ST_RUNNING;
+    cudaMemcpyAsync(c->S, h, sizeof(SolverState), cudaMemcpyHostToDevice, c->stream);
+    DivArgs da = div_args(c, st);
+    da.warm = 1;
+    k_div_init_mixed<<<red_blocks(c), CF_RED_THREADS, 0, c->stream>>>(da);
+    c->p_df = 1;
+    const Outer oa = outer_args(c, st, 0, split);
+    k_outer_resid<false><<<outer_blocks(oa), CF_RED_THREADS, 0, c->stream>>>(oa);
+    c->launches += 2;
+    int rc = cuda_check(c, cudaGetLastError(), "residual");
+    if (!rc)
+        rc = cuda_check(c, cudaMemcpy2DAsync(r, sizeof(float) * c->ph.nx, c->r32.a, sizeof(float) * c->p32,
+                                             sizeof(float) * c->ph.nx, c->ph.ny, cudaMemcpyDeviceToHost, c->stream),
+                        "residual copy");
+    if (!rc) rc = cuda_check(c, cudaStreamSynchronize(c->stream), "residual");
+    return rc;
+}
+
 // cf_test_precondition
 int test_precondition(cf_ctx* c, double dt, int levels, const double* r, double* z, double* rz) {
     const bool mixed = c->precision == CF_PREC_MIXED;

@@ -293,6 +293,12 @@ int cf_test_apply_general(cf_ctx* ctx, int on);
  * by one launch per half sweep, residual, restriction and prolongation (the
  * same bits in z).  The fields are left as they are. */
 int cf_test_precondition(cf_ctx* ctx, double dt, int levels, const double* r, double* z, double* rz);
+/* Test hook (mixed context): r = b - A p of the current velocities and
+ * pressure with time step dt, as the solver's refinement forms it in
+ * double-float and rounds it to FP32; r: nx x ny (x fastest).  split != 0: as
+ * the multigrid solver launches it, which on small grids gives a unit of 16
+ * rows to several warps (the same bits).  The fields are left as they are. */
+int cf_test_residual(cf_ctx* ctx, double dt, int split, float* r);
 
 /* ---- output (replaces the device half of SiloWriter::writeFile) ----
  * SiloWriter interpolates the face velocities to cell centres for its
