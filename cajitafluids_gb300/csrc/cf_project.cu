@@ -451,7 +451,7 @@ __device__ __forceinline__ float2 df_neg(float2 x) { return make_float2(-x.x, -x
 // Two double-float values side by side, (h.x, l.x) and (h.y, l.y): a lane's
 // two cells, so that each error-free step runs as one packed f32x2
 // instruction for both (each half rounded as the scalar form, hence the bits
-// of df_resid_int cell by cell).
+// of df_add, df_mul and df_resid cell by cell).
 struct DF2 {
     float2 h, l;
 };
@@ -483,10 +483,14 @@ __device__ __forceinline__ DF2 df2_join(DF2 s, DF2 t) {
 }
 __device__ __forceinline__ DF2 df2_add(DF2 x, DF2 y) { return df2_join(df2_two_sum(x.h, y.h), df2_two_sum(x.l, y.l)); }
 __device__ __forceinline__ DF2 df2_sub(DF2 x, DF2 y) { return df2_join(df2_two_diff(x.h, y.h), df2_two_diff(x.l, y.l)); }
-// df_mul by one pair for both (the leading product as scalar operations: the compiler
-// fuses a packed product and the packed additions that use it)
+// A product whose rounding the additions after it rely on, as scalar operations: the
+// compiler may fuse a packed product with the packed additions that use it.
+__device__ __forceinline__ float2 f2_mul_rounded(float2 a, float2 b) {
+    return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
+}
+// df_mul by one pair for both
 __device__ __forceinline__ DF2 df2_scale(float2 c, DF2 x) {
-    const float2 p = make_float2(__fmul_rn(c.x, x.h.x), __fmul_rn(c.x, x.h.y));
+    const float2 p = f2_mul_rounded(make_float2(c.x, c.x), x.h);
     float2 e = make_float2(fmaf(c.x, x.h.x, -p.x), fmaf(c.x, x.h.y, -p.y));
     const float2 ch = make_float2(c.x, c.x), cl = make_float2(c.y, c.y);
     e = f2_fma(ch, x.l, e);
@@ -745,18 +749,6 @@ __device__ __forceinline__ float2 df_resid(const Outer& a, int eb, float2 b, flo
     return df_add_s(b, make_float2(-ax.x, -ax.y));
 }
 
-// interior cell: wall-adjacency bits 0, so the diagonal factor is 4 and
-// 4 x is exact
-__device__ __forceinline__ float2 df_resid_int(const Outer& a, float2 b, float2 c, float2 w, float2 e, float2 s,
-                                               float2 n) {
-    float2 nb = df_add_s(w, e);
-    nb = df_add_s(nb, s);
-    nb = df_add_s(nb, n);
-    float2 t = df_add_s(make_float2(4.f * c.x, 4.f * c.y), make_float2(-nb.x, -nb.y));
-    float2 ax = df_mul(a.scale, t);
-    return df_add_s(b, make_float2(-ax.x, -ax.y));
-}
-
 // df_resid for a lane's two cells: the residuals' high parts.  d: the diagonal
 // factors; without walls next to the unit 4, and 4 x is exact.
 template <bool WALL>
@@ -766,7 +758,7 @@ __device__ __forceinline__ float2 df2_resid(float2 scale, float2 d, DF2 b, DF2 c
     nb = df2_add_s(nb, n);
     DF2 dc;
     if (WALL) {  // df_mul((d, 0), c)
-        const float2 p = f2_mul(d, c.h);
+        const float2 p = f2_mul_rounded(d, c.h);
         const float2 er = f2_fma(d, c.h, f2_mul(make_float2(-1.f, -1.f), p));
         dc = df2_quick(p, f2_fma(d, c.l, er));
     } else {
@@ -774,14 +766,7 @@ __device__ __forceinline__ float2 df2_resid(float2 scale, float2 d, DF2 b, DF2 c
         dc = DF2{f2_mul(four, c.h), f2_mul(four, c.l)};
     }
     const DF2 t = df2_add_s(dc, df2_neg(nb));
-    // df_mul(scale, t)
-    const float2 sh = make_float2(scale.x, scale.x), sl = make_float2(scale.y, scale.y);
-    const float2 p = f2_mul(sh, t.h);
-    float2 er = f2_fma(sh, t.h, f2_mul(make_float2(-1.f, -1.f), p));
-    er = f2_fma(sh, t.l, er);
-    er = f2_fma(sl, t.h, er);
-    const DF2 ax = df2_quick(p, er);
-    const DF2 r = df2_add_s(b, df2_neg(ax));
+    const DF2 r = df2_add_s(b, df2_neg(df2_scale(scale, t)));
     return r.h;
 }
 
