@@ -511,8 +511,6 @@ __global__ void __launch_bounds__(kThreads, kCtas2)
 // run on in the same order), so the results are the same bits.
 constexpr int kHalo = 2 * kTW + 2 * kTH;  // halo (and border) values of a tile
 constexpr int kMaxTiles = 4;              // tiles per block
-// the stalled wait of the timeout-path test: a grid barrier that cannot complete
-constexpr unsigned kGridStallLimit = 1u << 10;
 
 template <int NT>
 __global__ void __launch_bounds__(kThreads, 1) k_pcg32(Cg32T a, float* border, int ga, int gb, int iters) {
@@ -714,7 +712,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg32(Cg32T a, float* border, i
         put_partial(red[0], warp, min(na, NT), partA);
         grid_arrive(S);
         arrived += nb;
-        if (!grid_wait(S, gbase + arrived + (stall ? 1u << 30 : 0u), stall ? kGridStallLimit : PC_WAIT_LIMIT)) return;
+        if (!grid_wait(S, gbase + arrived, stall)) return;
         if (warp < nwa) {
             const double s = warp_fold_n(strided_sum(partA, ga, tid), ga - 32 * warp);
             if (lane == 0) ws0[warp] = s;

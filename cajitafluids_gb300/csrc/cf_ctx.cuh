@@ -114,7 +114,8 @@ struct cf_ctx {
     // host-polled projection); the results are the same bits
     int direct = 0;
     // cf_test_stall_wait: the inner FP32 CG's first tile wait of block 0
-    // waits on an mbarrier nothing arrives on (timeout-path test)
+    // waits on an mbarrier nothing arrives on, an on-chip solve's first grid
+    // barrier there for arrivals that never come (timeout-path test)
     int test_stall = 0;
     // cf_test_advect_unstaged: every FP32 advection tile reads its taps from
     // global memory instead of its shared-memory window (same bits)

@@ -9,6 +9,7 @@ namespace cf {
 // polls of a grid barrier before the launch gives up (each poll is an L2
 // round trip; a barrier takes a few of them)
 constexpr unsigned PC_WAIT_LIMIT = 1u << 22;
+constexpr unsigned PC_STALL_LIMIT = 1u << 10;
 
 // Grid barrier in two halves (all blocks co-resident: cooperative launch).
 // The counter only grows: S->gbar is its value when the launch starts.
@@ -19,10 +20,13 @@ __device__ __forceinline__ void grid_arrive(SolverState* S) {
     }
 }
 // true when the arrivals have reached target; the wait is bounded, and ends
-// early once another block has given up
-__device__ __forceinline__ bool grid_wait(SolverState* S, unsigned target, unsigned limit = PC_WAIT_LIMIT) {
+// early once another block has given up.  stall: the timeout-path test's wait
+// (cf_test_stall_wait), for arrivals that never come.
+__device__ __forceinline__ bool grid_wait(SolverState* S, unsigned target, bool stall = false) {
     bool ok = true;
     if (threadIdx.x == 0) {
+        const unsigned limit = stall ? PC_STALL_LIMIT : PC_WAIT_LIMIT;
+        if (stall) target += 1u << 30;
         unsigned v, k = 0;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&S->gcount) : "memory");

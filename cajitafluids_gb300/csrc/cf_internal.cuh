@@ -87,7 +87,7 @@ struct SolverState {
     int iter, max_iter, status;
     int inner_iter, inner_status;
     int outer_iter, max_outer;
-    int test_stall;  // test knob (cf_test_stall_wait): see k_tma_dir_matvec32
+    int test_stall;  // test knob (cf_test_stall_wait): see k_tma_dir_matvec32, k_pcg64 and k_pcg32
     int xsel;        // mixed MG-PCG, fused x update: the x buffer holding the solution
     unsigned int ticket[8];
     // grid barriers of the on-chip solves: arrivals so far, and their count

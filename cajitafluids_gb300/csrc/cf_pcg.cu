@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(PcThreads<NU>::value, 1) k_pcg64(Pcg64 a) {
     int it = S->iter;
     const int it_end = it + a.iters, max_iter = S->max_iter;
     double beta = S->beta, rho = S->rho, rr = S->rr, alpha = S->alpha;
+    const bool stall = S->test_stall != 0 && blockIdx.x == 0;
     const unsigned gbase = S->gbar;
     unsigned arrived = 0;
     if (tid < 16) {
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(PcThreads<NU>::value, 1) k_pcg64(Pcg64 a) {
         }
         grid_arrive(S);
         arrived += gridDim.x;
-        if (!grid_wait(S, gbase + arrived)) return;
+        if (!grid_wait(S, gbase + arrived, stall)) return;
         if (warp < nw) {
             const double s = warp_fold_n(strided_sum(a.partA, a.U, tid), a.U - 32 * warp);
             if (lane == 0) ws0[warp] = s;

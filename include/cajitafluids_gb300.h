@@ -271,10 +271,10 @@ int cf_test_fail_alloc(int nth);
  * of one CTA of the mixed-precision inner CG waits on an mbarrier that
  * nothing arrives on, with a short limit; it times out, the CTA waits for
  * its own bulk copies in flight and returns, and the projection returns
- * CF_ERR_TIMEOUT.  Where the inner CG runs on chip (grids of up to about
- * a million cells with the diagonal preconditioner) it is that block's
- * first grid barrier that waits for arrivals that never come.  The context
- * stays usable; 0 switches the hook off. */
+ * CF_ERR_TIMEOUT.  Where the Jacobi-PCG runs on chip (grids of up to about
+ * a million cells with the diagonal preconditioner, FP64 too) it is that
+ * block's first grid barrier that waits for arrivals that never come.  The
+ * context stays usable; 0 switches the hook off. */
 int cf_test_stall_wait(cf_ctx* ctx, int on);
 /* Test hook: with on != 0, every tile of the mixed-precision advection reads
  * its stencil taps from global memory (the path a tile takes when a trace
