@@ -1,12 +1,10 @@
 // Jacobi-PCG with the whole solve on chip, for grids whose solver vectors fit
 // the SMs' shared memory.
 //
-// The launch-per-phase kernels (cf_project.cu) give one warp a unit of 64 x 16
-// cells, eight units to a block.  Up to a few hundred units that leaves most
-// of the GPU idle: an SM executes one FP64 warp instruction per sub-partition
-// every 64 cycles (measured; 2 FP64 lanes per cycle and SM), so eight units on
-// one SM take 25-30 us per kernel whatever the grid size, and each iteration
-// adds two launches and two last-block folds.  Here one cooperative launch
+// As launches (cf_project.cu: a block per unit of 64 x 16 cells) an iteration is two
+// kernels, each of which starts, reads its vectors, is folded by its last block and
+// drains: 23 us at 256^2, of which the FP64 work (an SM executes one FP64 warp
+// instruction per sub-partition every 64 cycles) is two.  Here one cooperative launch
 // runs many iterations: a block owns NU units (r, p with its
 // halo and A p / z in shared memory, x in registers), the grid meets at two
 // barriers per iteration, and every block folds the unit partials itself.
@@ -28,8 +26,9 @@
 // dependent FMAs of 64 cycles, 1 us each phase), the two grid barriers (about
 // 1.2 us each) and the divisions; at seven units per SM the FP64 pipe (10
 // operations per cell and iteration: 18 of 31 us).  Measured on GB300, time of
-// one iteration, the two launches per iteration before and this: 64^2 39.9 ->
-// 9.7 us, 256^2 49.6 -> 10.4 us, 1024^2 53.8 -> 31.1 us.
+// one iteration, launches (with eight units to a block, as they were then) and this:
+// 64^2 39.9 -> 9.7 us, 256^2 49.6 -> 10.4 us, 1024^2 53.8 -> 31.3 us; 1072^2, with a unit
+// to a block, 44.4 -> 34.9 us.
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -41,12 +40,12 @@
 namespace cf {
 
 // threads per block: the lane sums and folds of one or two units keep few
-// warps busy; four and seven units have the cells to keep 16 warps issuing
+// warps busy; more have the cells to keep 16 warps issuing
 template <int NU>
 struct PcThreads {
     static constexpr int value = NU <= 2 ? 256 : 512;
 };
-// Plain products: four and seven units per block are bound by the FP64 pipe, and
+// Plain products: more than two units per block are bound by the FP64 pipe, and
 // products on the integer pipes run beside it (1024^2: 33.2 -> 31.1 us an iteration);
 // one or two units wait for results, which the hardware product returns sooner
 // (a 256^2 step: 10.2 ms against 10.4 with integer products).
@@ -56,7 +55,7 @@ __device__ __forceinline__ double pcg_mul(double a, double b) {
 }
 constexpr int PC_PW = UNIT_PW, PC_P = UNIT_P, PC_CELLS = UNIT_CELLS, PC_BORDER = UNIT_BORDER;
 constexpr int PC_UNIT = PC_P + 2 * PC_CELLS;  // doubles per unit: p with its halo, r, q / z
-constexpr int PC_MAX_UNITS = 7;                           // units per block (181 KB of shared memory)
+constexpr int PC_MAX_UNITS = 8;  // units per block: 207 KB of the 227 KB of shared memory a block may have
 struct Pcg64 {
     int nx, ny, per_x, per_y, G, U, pitch;
     Stencil st;
@@ -105,8 +104,8 @@ __global__ void __launch_bounds__(PcThreads<NU>::value, 1) k_pcg64(Pcg64 a) {
     auto R = [&](int k) { return pc_smem + k * PC_UNIT + PC_P; };
     auto Q = [&](int k) { return pc_smem + k * PC_UNIT + PC_P + PC_CELLS; };
 
-    // Thread t owns cells t, t + 256, ... of each unit (64 to a row: row
-    // t / 64 + 4 m, column t % 64) and, below PC_BORDER, one halo value.
+    // Thread t owns cells t, t + PC_THREADS, ... of each unit (64 to a row: row
+    // t / 64 + m PC_THREADS / 64, column t % 64) and, below PC_BORDER, one halo value.
     // code[k]: 4 wall-adjacency bits per cell, then a valid bit per cell.
     const int col = tid & (CF_UNIT_COLS - 1), row0 = tid / CF_UNIT_COLS;
     double xr[NU][PC_CPT];
@@ -360,10 +359,9 @@ static bool pcg64_fits(const cf_ctx* c) {
 }
 
 // Units per block of the on-chip solve (0: the grid does not fit), and the
-// border buffer.  A block takes as few units as the SMs allow; up to seven
-// (1064 units on 152 SMs) the vectors fit shared memory, and there the solve
-// is faster than the launch-per-phase kernels at every size (1024^2, seven
-// units: 31.1 against 53.8 us per iteration).
+// border buffer.  A block takes as few units as the SMs allow, up to the eight whose
+// vectors shared memory holds (1216 units on 152 SMs); the solve is faster than the
+// launches at every such size (above).
 int pcg64_setup(cf_ctx* c) {
     c->pcg_nu = 0;
     const int per = (c->n_units + c->sms - 1) / c->sms;
