@@ -63,7 +63,6 @@ namespace cf {
 struct RecKind {
     double* cx;   // x weights times the scattered value, cx[a * nt + t]
     double* wy;   // y weights, wy[b * nt + t]
-    int n;        // weights per axis (2 or 4)
     int nt;       // target slots
 };
 // Where a target's samples start, relative to the target: eight bits a sample (x and
@@ -213,7 +212,6 @@ struct AdjRec {
     Grid<double> q, u, v;     // forward state of the step (ghosts filled)
     Grid<double> aq, au, av;  // adjoint of the advected values
     double dt;
-    int order;
     RecKind F[3], Su[3][3], Sv[3][3];
     RecWhere w[3];
     int* err;
@@ -1055,7 +1053,6 @@ int setup_records(cf_ctx* c, AdjState* A) {
         }
     auto mk = [&](RecKind& R, int ent, int n) {
         const Grid<double>& tg = *shapes[ent];
-        R.n = n;
         R.nt = tg.ex * tg.ey;
         void *x = nullptr, *y = nullptr;
         if (!rc) rc = dalloc(c, A, &x, sizeof(double) * n * R.nt);
@@ -1344,7 +1341,6 @@ int adjoint_step(cf_ctx* c, AdjState* A, const SolveOpts& so, bool params_ready,
     ar.au = A->ag[1];
     ar.av = A->ag[2];
     ar.dt = A->dt;
-    ar.order = A->order;
     for (int e = 0; e < 3; ++e) {
         ar.F[e] = A->F[e];
         ar.w[e] = A->rw[e];
