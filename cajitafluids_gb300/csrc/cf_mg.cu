@@ -263,8 +263,8 @@ __global__ void __launch_bounds__(MG_BX* MG_BY) k_mg_prolong(MgLev<T> C, MgLev<T
 }
 
 // ---------------------------------------------------------------------------
-// Fused level kernels (temporal blocking in shared memory).  A CTA owns a
-// tile of TW x TH fine cells (both even) and recomputes a shrinking halo, so that the
+// Fused kernels of the large FP32 levels (temporal blocking in shared memory).  A
+// CTA owns a tile of FT_W x FT_H fine cells and recomputes a shrinking halo, so that the
 // MG_NU = 2 sweep pairs of a level need one pass over memory:
 //   k_mg_pre : x = 4 half sweeps from x = 0 (red, black, red, black),
 //              r = b - A x (in shared memory), b_coarse = R r
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(MG_BX* MG_BY) k_mg_prolong(MgLev<T> C, MgLev<T
 // k_mg_post reads it from there and writes x: a CTA of k_mg_post reads its
 // halo from other tiles, which must not be written by the same launch.
 constexpr int FT_THREADS = 256;
-constexpr int FT_W = 64, FT_H = 32;  // tile of the large FP32 levels
+constexpr int FT_W = 64, FT_H = 32;  // tile
 constexpr int FT_BLOCKS = 3;         // resident blocks per SM (the strips spill at four)
 
 // index along an axis after the periodic wrap; -1 beyond a wall
@@ -288,11 +288,11 @@ __device__ __forceinline__ int mg_dom(int g, int n, int per) {
 }
 
 // one half sweep of colour c over the tile grown by h cells; arrays have halo H
-template <typename T, int TW, int TH, int H>
-__device__ __forceinline__ void ft_half(const MgLev<T>& L, const MgBc& p, T* xs, const T* bs, int i0, int j0, int c,
-                                        int h, bool first) {
-    constexpr int W = TW + 2 * H;
-    const int ncol = TW + 2 * h, nrow = TH + 2 * h, hw = ncol / 2;
+template <int H>
+__device__ __forceinline__ void ft_half(const MgLev<float>& L, const MgBc& p, float* xs, const float* bs, int i0, int j0,
+                                        int c, int h, bool first) {
+    constexpr int W = FT_W + 2 * H;
+    const int ncol = FT_W + 2 * h, nrow = FT_H + 2 * h, hw = ncol / 2;
     const int gi0 = i0 - h;
     for (int k = threadIdx.x; k < hw * nrow; k += FT_THREADS) {
         const int rj = k / hw, pk = k % hw;
@@ -302,15 +302,15 @@ __device__ __forceinline__ void ft_half(const MgLev<T>& L, const MgBc& p, T* xs,
         if (wi < 0 || wj < 0) continue;  // beyond a wall: stays 0
         const int li = gi - (i0 - H), lj = gj - (j0 - H);
         const int q = lj * W + li;
-        T s;
+        float s;
         if (first) {
-            s = T(0);
+            s = 0.f;
         } else {
             s = xs[q - 1] + xs[q + 1];
             s = s + xs[q - W];
             s = s + xs[q + W];
         }
-        T t = mg_fma(L.scale, s, bs[q]);
+        float t = mg_fma(L.scale, s, bs[q]);
         xs[q] = t * L.invd[mg_bits(p, L.nx, L.ny, wi, wj)];
     }
     __syncthreads();
@@ -318,14 +318,14 @@ __device__ __forceinline__ void ft_half(const MgLev<T>& L, const MgBc& p, T* xs,
 
 // load x from xsrc (0 when null) and b over the tile with halo H (wrapped; 0
 // beyond walls)
-template <typename T, int TW, int TH, int H>
-__device__ __forceinline__ void ft_load(const MgLev<T>& L, const MgBc& p, T* xs, T* bs, int i0, int j0,
-                                        const T* xsrc) {
-    constexpr int W = TW + 2 * H, HT = TH + 2 * H;
+template <int H>
+__device__ __forceinline__ void ft_load(const MgLev<float>& L, const MgBc& p, float* xs, float* bs, int i0, int j0,
+                                        const float* xsrc) {
+    constexpr int W = FT_W + 2 * H, HT = FT_H + 2 * H;
     for (int q = threadIdx.x; q < W * HT; q += FT_THREADS) {
         const int li = q % W, lj = q / W;
         const int wi = mg_dom(i0 - H + li, L.nx, p.per_x), wj = mg_dom(j0 - H + lj, L.ny, p.per_y);
-        T xv = T(0), bv = T(0);
+        float xv = 0.f, bv = 0.f;
         if (wi >= 0 && wj >= 0) {
             const size_t k = (size_t)wj * L.pitch + wi;
             bv = L.b[k];
@@ -343,26 +343,26 @@ __device__ __forceinline__ void ft_load(const MgLev<T>& L, const MgBc& p, T* xs,
 // wall-adjacency bit is then 0 and every transfer weight the interior one,
 // and those tiles take the index-light paths below, reading their halo
 // through mg_wrap.
-template <int TW, int TH, int H>
+template <int H>
 __device__ __forceinline__ bool ft_interior(int nx, int ny, int i0, int j0, const MgBc& p) {
-    const bool ix = p.per_x ? (i0 + TW <= nx && nx >= H) : (i0 - H >= 1 && i0 + TW + H <= nx - 1);
-    const bool iy = p.per_y ? (j0 + TH <= ny && ny >= H) : (j0 - H >= 1 && j0 + TH + H <= ny - 1);
+    const bool ix = p.per_x ? (i0 + FT_W <= nx && nx >= H) : (i0 - H >= 1 && i0 + FT_W + H <= nx - 1);
+    const bool iy = p.per_y ? (j0 + FT_H <= ny && ny >= H) : (j0 - H >= 1 && j0 + FT_H + H <= ny - 1);
     return ix && iy;
 }
 
 // an index within one period of [0, n): wrapped (interior tiles only)
 __device__ __forceinline__ int mg_wrap(int g, int n) { return g < 0 ? g + n : (g >= n ? g - n : g); }
 
-template <typename T, int TW, int TH, int H>
-__device__ __forceinline__ void ft_load_int(const MgLev<T>& L, T* xs, T* bs, int i0, int j0, const T* xsrc) {
-    constexpr int W = TW + 2 * H, HT = TH + 2 * H;
+template <int H>
+__device__ __forceinline__ void ft_load_int(const MgLev<float>& L, float* xs, float* bs, int i0, int j0, const float* xsrc) {
+    constexpr int W = FT_W + 2 * H, HT = FT_H + 2 * H;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int lj = warp; lj < HT; lj += FT_THREADS / 32) {
         const size_t row = (size_t)mg_wrap(j0 - H + lj, L.ny) * L.pitch;
         for (int li = lane; li < W; li += 32) {
             const size_t k = row + mg_wrap(i0 - H + li, L.nx);
             bs[lj * W + li] = L.b[k];
-            xs[lj * W + li] = xsrc ? xsrc[k] : T(0);
+            xs[lj * W + li] = xsrc ? xsrc[k] : 0.f;
         }
     }
     __syncthreads();
@@ -371,26 +371,26 @@ __device__ __forceinline__ void ft_load_int(const MgLev<T>& L, T* xs, T* bs, int
 // interior half sweep: warp w takes rows w, w + 8, ... (all of one parity, so
 // a lane's cells of the colour sit in one column per row parity); lane l
 // takes the cells 2l (+ 64) of the row's colour
-template <typename T, int TW, int TH, int H>
-__device__ __forceinline__ void ft_half_int(const MgLev<T>& L, T* xs, const T* bs, int i0, int j0, int c, int h,
-                                            bool first) {
-    constexpr int W = TW + 2 * H, RS = FT_THREADS / 32;
-    const int nrow = TH + 2 * h, hw = TW / 2 + h;
+template <int H>
+__device__ __forceinline__ void ft_half_int(const MgLev<float>& L, float* xs, const float* bs, int i0, int j0, int c,
+                                            int h, bool first) {
+    constexpr int W = FT_W + 2 * H, RS = FT_THREADS / 32;
+    const int nrow = FT_H + 2 * h, hw = FT_W / 2 + h;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const T scale = L.scale, id0 = L.invd[0];
+    const float scale = L.scale, id0 = L.invd[0];
     const int off = (c + (j0 - h + warp) + i0 - h) & 1;  // rows step by RS (even): fixed parity
     for (int pk = lane; pk < hw; pk += 32) {
         int q = (warp + H - h) * W + (H - h) + off + 2 * pk;
         for (int rj = warp; rj < nrow; rj += RS, q += RS * W) {
-            T s;
+            float s;
             if (first) {
-                s = T(0);
+                s = 0.f;
             } else {
                 s = xs[q - 1] + xs[q + 1];
                 s = s + xs[q - W];
                 s = s + xs[q + W];
             }
-            T t = mg_fma(scale, s, bs[q]);
+            float t = mg_fma(scale, s, bs[q]);
             xs[q] = t * id0;
         }
     }
@@ -429,8 +429,9 @@ struct StripMap {
 // Epilogue of the finest FP32 post-smoothing (mixed MG-PCG): rho = r.z over
 // the level (r = the level's b, z = its x), the CG scalars updated as by
 // k_mg_rz32, and the periodic ghost copies of z written with the edge cells.
-// Partials: one per frame tile (slot = block) and one per strip (slot =
-// nframe + strip); the last block to finish folds them in a fixed order.
+// Partials: one per frame tile (slot = block) and one per strip (slot = nframe +
+// strip), or one per block of the row windows (k_mg_post_rows); the last block to
+// finish folds them in a fixed order.
 struct RzEpi {
     int on;
     double* part;
@@ -766,44 +767,39 @@ __device__ __forceinline__ float strip_post(const MgLev<float>& C, const MgLev<f
     return rz;
 }
 
-template <typename T, int TW, int TH>
-__global__ void __launch_bounds__(FT_THREADS, FT_BLOCKS) k_mg_pre(MgLev<T> F, MgLev<T> C, MgBc p,
-                                                                        SolverState* S, int inner,
-                                                       StripMap m) {
+__global__ void __launch_bounds__(FT_THREADS, FT_BLOCKS) k_mg_pre(MgLev<float> F, MgLev<float> C, MgBc p,
+                                                                  SolverState* S, int inner, StripMap m) {
     if (!block_live(S, inner)) return;
-    constexpr int H = 5, W = TW + 2 * H, HT = TH + 2 * H;
-    constexpr bool STRIPS = sizeof(T) == 4 && TW == 64;
-    constexpr size_t TILE_B = 2 * sizeof(T) * W * HT;
-    constexpr size_t RING_B = STRIPS ? (FT_THREADS / 32) * SP_RING * 32 * sizeof(float4) : 0;
+    constexpr int H = 5, W = FT_W + 2 * H, HT = FT_H + 2 * H;
+    constexpr size_t TILE_B = 2 * sizeof(float) * W * HT;
+    constexpr size_t RING_B = (FT_THREADS / 32) * SP_RING * 32 * sizeof(float4);
     __shared__ __align__(16) unsigned char smem[TILE_B > RING_B ? TILE_B : RING_B];
-    if constexpr (STRIPS) {
-        if ((int)blockIdx.x >= m.nframe) {
-            const int warp = threadIdx.x >> 5;
-            const int k = ((int)blockIdx.x - m.nframe) * (FT_THREADS / 32) + warp;
-            if (k >= m.ns * m.nr) return;
-            const int sx = k % m.ns, sy = k / m.ns;
-            strip_pre(F, C, reinterpret_cast<float4*>(smem) + warp * SP_RING * 32, m.x0 + SP_PRE_OUT * sx,
-                      m.y0 + m.rh * sy, m.rh);
-            return;
-        }
+    if ((int)blockIdx.x >= m.nframe) {
+        const int warp = threadIdx.x >> 5;
+        const int k = ((int)blockIdx.x - m.nframe) * (FT_THREADS / 32) + warp;
+        if (k >= m.ns * m.nr) return;
+        const int sx = k % m.ns, sy = k / m.ns;
+        strip_pre(F, C, reinterpret_cast<float4*>(smem) + warp * SP_RING * 32, m.x0 + SP_PRE_OUT * sx,
+                  m.y0 + m.rh * sy, m.rh);
+        return;
     }
-    T* xs = reinterpret_cast<T*>(smem);
-    T* bs = xs + W * HT;  // b, then r in place on the residual ring
+    float* xs = reinterpret_cast<float*>(smem);
+    float* bs = xs + W * HT;  // b, then r in place on the residual ring
     int tx, ty;
     frame_tile(m, blockIdx.x, tx, ty);
-    const int i0 = tx * TW, j0 = ty * TH;
-    if (ft_interior<TW, TH, H>(F.nx, F.ny, i0, j0, p)) {
-        ft_load_int<T, TW, TH, H>(F, xs, bs, i0, j0, nullptr);
-        ft_half_int<T, TW, TH, H>(F, xs, bs, i0, j0, 0, 5, true);
-        ft_half_int<T, TW, TH, H>(F, xs, bs, i0, j0, 1, 4, false);
-        ft_half_int<T, TW, TH, H>(F, xs, bs, i0, j0, 0, 3, false);
-        ft_half_int<T, TW, TH, H>(F, xs, bs, i0, j0, 1, 2, false);
+    const int i0 = tx * FT_W, j0 = ty * FT_H;
+    if (ft_interior<H>(F.nx, F.ny, i0, j0, p)) {
+        ft_load_int<H>(F, xs, bs, i0, j0, nullptr);
+        ft_half_int<H>(F, xs, bs, i0, j0, 0, 5, true);
+        ft_half_int<H>(F, xs, bs, i0, j0, 1, 4, false);
+        ft_half_int<H>(F, xs, bs, i0, j0, 0, 3, false);
+        ft_half_int<H>(F, xs, bs, i0, j0, 1, 2, false);
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const T d0 = F.diag[0], ms = F.ms;
-        for (int rj = warp; rj < TH + 2; rj += FT_THREADS / 32)
-            for (int ci = lane; ci < TW + 2; ci += 32) {
+        const float d0 = F.diag[0], ms = F.ms;
+        for (int rj = warp; rj < FT_H + 2; rj += FT_THREADS / 32)
+            for (int ci = lane; ci < FT_W + 2; ci += 32) {
                 const int q = (rj + H - 1) * W + (ci + H - 1);
-                T ax = d0 * xs[q];
+                float ax = d0 * xs[q];
                 ax = mg_fma(ms, xs[q - 1], ax);
                 ax = mg_fma(ms, xs[q + 1], ax);
                 ax = mg_fma(ms, xs[q - W], ax);
@@ -811,42 +807,42 @@ __global__ void __launch_bounds__(FT_THREADS, FT_BLOCKS) k_mg_pre(MgLev<T> F, Mg
                 bs[q] = bs[q] - ax;
             }
         __syncthreads();
-        for (int k = threadIdx.x; k < TW * TH; k += FT_THREADS) {
-            const int li = k % TW, lj = k / TW;
+        for (int k = threadIdx.x; k < FT_W * FT_H; k += FT_THREADS) {
+            const int li = k % FT_W, lj = k / FT_W;
             F.r[(size_t)(j0 + lj) * F.pitch + i0 + li] = xs[(lj + H) * W + li + H];
         }
         // restriction with the interior weights 1/4, 3/4, 3/4, 1/4 per axis
-        const T w4[4] = {T(0.25), T(0.75), T(0.75), T(0.25)};
-        for (int k = threadIdx.x; k < (TW / 2) * (TH / 2); k += FT_THREADS) {
-            const int ci = k % (TW / 2), cj = k / (TW / 2);
+        const float w4[4] = {0.25f, 0.75f, 0.75f, 0.25f};
+        for (int k = threadIdx.x; k < (FT_W / 2) * (FT_H / 2); k += FT_THREADS) {
+            const int ci = k % (FT_W / 2), cj = k / (FT_W / 2);
             const int qr = (2 * cj - 1 + H) * W + (2 * ci - 1 + H);
-            T acc = T(0);
+            float acc = 0.f;
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-                const T* row = bs + qr + a * W;
-                T rs = T(0);
+                const float* row = bs + qr + a * W;
+                float rs = 0.f;
 #pragma unroll
                 for (int b = 0; b < 4; ++b) rs = mg_fma(w4[b], row[b], rs);
                 acc = mg_fma(w4[a], rs, acc);
             }
-            C.b[(size_t)(j0 / 2 + cj) * C.pitch + i0 / 2 + ci] = T(0.25) * acc;
+            C.b[(size_t)(j0 / 2 + cj) * C.pitch + i0 / 2 + ci] = 0.25f * acc;
         }
         return;
     }
-    ft_load<T, TW, TH, H>(F, p, xs, bs, i0, j0, nullptr);
-    ft_half<T, TW, TH, H>(F, p, xs, bs, i0, j0, 0, 5, true);
-    ft_half<T, TW, TH, H>(F, p, xs, bs, i0, j0, 1, 4, false);
-    ft_half<T, TW, TH, H>(F, p, xs, bs, i0, j0, 0, 3, false);
-    ft_half<T, TW, TH, H>(F, p, xs, bs, i0, j0, 1, 2, false);
+    ft_load<H>(F, p, xs, bs, i0, j0, nullptr);
+    ft_half<H>(F, p, xs, bs, i0, j0, 0, 5, true);
+    ft_half<H>(F, p, xs, bs, i0, j0, 1, 4, false);
+    ft_half<H>(F, p, xs, bs, i0, j0, 0, 3, false);
+    ft_half<H>(F, p, xs, bs, i0, j0, 1, 2, false);
     // residual on the tile grown by 1 (read by the restriction), in place of b
     {
-        const int ncol = TW + 2, nrow = TH + 2;
+        const int ncol = FT_W + 2, nrow = FT_H + 2;
         for (int k = threadIdx.x; k < ncol * nrow; k += FT_THREADS) {
             const int gi = i0 - 1 + k % ncol, gj = j0 - 1 + k / ncol;
             const int wi = mg_dom(gi, F.nx, p.per_x), wj = mg_dom(gj, F.ny, p.per_y);
             if (wi < 0 || wj < 0) continue;
             const int q = (gj - (j0 - H)) * W + (gi - (i0 - H));
-            T ax = F.diag[mg_bits(p, F.nx, F.ny, wi, wj)] * xs[q];
+            float ax = F.diag[mg_bits(p, F.nx, F.ny, wi, wj)] * xs[q];
             ax = mg_fma(F.ms, xs[q - 1], ax);
             ax = mg_fma(F.ms, xs[q + 1], ax);
             ax = mg_fma(F.ms, xs[q - W], ax);
@@ -856,71 +852,66 @@ __global__ void __launch_bounds__(FT_THREADS, FT_BLOCKS) k_mg_pre(MgLev<T> F, Mg
     }
     __syncthreads();
     // x on the tile, into the r array (read back by k_mg_post)
-    for (int k = threadIdx.x; k < TW * TH; k += FT_THREADS) {
-        const int gi = i0 + k % TW, gj = j0 + k / TW;
+    for (int k = threadIdx.x; k < FT_W * FT_H; k += FT_THREADS) {
+        const int gi = i0 + k % FT_W, gj = j0 + k / FT_W;
         if (gi < F.nx && gj < F.ny) F.r[(size_t)gj * F.pitch + gi] = xs[(gj - (j0 - H)) * W + (gi - (i0 - H))];
     }
     // restriction of the coarse cells under the tile
-    for (int k = threadIdx.x; k < (TW / 2) * (TH / 2); k += FT_THREADS) {
-        const int I = i0 / 2 + k % (TW / 2), J = j0 / 2 + k / (TW / 2);
+    for (int k = threadIdx.x; k < (FT_W / 2) * (FT_H / 2); k += FT_THREADS) {
+        const int I = i0 / 2 + k % (FT_W / 2), J = j0 / 2 + k / (FT_W / 2);
         if (I >= C.nx || J >= C.ny) continue;
-        T acc = T(0);
+        float acc = 0.f;
         for (int fy0 = 2 * J - 1; fy0 <= 2 * J + 2; ++fy0) {
             const int fy = mg_dom(fy0, F.ny, p.per_y);
             if (fy < 0) continue;
-            const T wy = (T)mg_pwq(fy, J, C.ny, p.per_y, p.bc[1], p.bc[3]) * T(0.25);
+            const float wy = (float)mg_pwq(fy, J, C.ny, p.per_y, p.bc[1], p.bc[3]) * 0.25f;
             const int rowq = (fy0 - (j0 - H)) * W - (i0 - H);
-            T rs = T(0);
+            float rs = 0.f;
             for (int fx0 = 2 * I - 1; fx0 <= 2 * I + 2; ++fx0) {
                 const int fx = mg_dom(fx0, F.nx, p.per_x);
                 if (fx < 0) continue;
-                const T wx = (T)mg_pwq(fx, I, C.nx, p.per_x, p.bc[0], p.bc[2]) * T(0.25);
+                const float wx = (float)mg_pwq(fx, I, C.nx, p.per_x, p.bc[0], p.bc[2]) * 0.25f;
                 rs = mg_fma(wx, bs[rowq + fx0], rs);
             }
             acc = mg_fma(wy, rs, acc);
         }
-        C.b[(size_t)J * C.pitch + I] = T(0.25) * acc;
+        C.b[(size_t)J * C.pitch + I] = 0.25f * acc;
     }
 }
 
-template <typename T, int TW, int TH>
-__global__ void __launch_bounds__(FT_THREADS, FT_BLOCKS) k_mg_post(MgLev<T> C, MgLev<T> F, MgBc p,
-                                                                         SolverState* S, int inner,
-                                                           StripMap m, RzEpi E) {
+__global__ void __launch_bounds__(FT_THREADS, FT_BLOCKS) k_mg_post(MgLev<float> C, MgLev<float> F, MgBc p,
+                                                                   SolverState* S, int inner, StripMap m, RzEpi E) {
     if (!block_live(S, inner)) return;
-    constexpr int H = 4, W = TW + 2 * H, HT = TH + 2 * H;
+    constexpr int H = 4, W = FT_W + 2 * H, HT = FT_H + 2 * H;
     // coarse cells read by the prolongation of an interior tile's array
-    constexpr int CW = TW / 2 + H + 2, CH = TH / 2 + H + 2;
-    constexpr bool STRIPS = sizeof(T) == 4 && TW == 64;
-    constexpr size_t TILE_B = sizeof(T) * (2 * W * HT + CW * CH);
-    constexpr size_t RING_B = STRIPS ? (FT_THREADS / 32) * SP_RING * SP_POST_SLOT * sizeof(float) : 0;
+    constexpr int CW = FT_W / 2 + H + 2, CH = FT_H / 2 + H + 2;
+    constexpr size_t TILE_B = sizeof(float) * (2 * W * HT + CW * CH);
+    constexpr size_t RING_B = (FT_THREADS / 32) * SP_RING * SP_POST_SLOT * sizeof(float);
     __shared__ __align__(16) unsigned char smem[TILE_B > RING_B ? TILE_B : RING_B];
     const int nparts = m.nframe + m.ns * m.nr;
-    if constexpr (STRIPS) {
-        if ((int)blockIdx.x >= m.nframe) {
-            const int warp = threadIdx.x >> 5;
-            const int k = ((int)blockIdx.x - m.nframe) * (FT_THREADS / 32) + warp;
-            float rz = 0.f;
-            if (k < m.ns * m.nr) {
-                const int sx = k % m.ns, sy = k / m.ns;
-                rz = strip_post(C, F, reinterpret_cast<float4*>(smem) + warp * SP_RING * (SP_POST_SLOT / 4),
-                                m.x0 + SP_POST_OUT * sx, m.y0 + m.rh * sy, m.rh);
-            }
-            if (E.on) {
-                const double d = warp_fold((double)rz);
-                if (k < m.ns * m.nr && (threadIdx.x & 31) == 0) E.part[m.nframe + k] = d;
-                rz_finish(E, S, nparts);
-            }
-            return;
+    if ((int)blockIdx.x >= m.nframe) {
+        const int warp = threadIdx.x >> 5;
+        const int k = ((int)blockIdx.x - m.nframe) * (FT_THREADS / 32) + warp;
+        float rz = 0.f;
+        if (k < m.ns * m.nr) {
+            const int sx = k % m.ns, sy = k / m.ns;
+            rz = strip_post(C, F, reinterpret_cast<float4*>(smem) + warp * SP_RING * (SP_POST_SLOT / 4),
+                            m.x0 + SP_POST_OUT * sx, m.y0 + m.rh * sy, m.rh);
         }
+        if (E.on) {
+            const double d = warp_fold((double)rz);
+            if (k < m.ns * m.nr && (threadIdx.x & 31) == 0) E.part[m.nframe + k] = d;
+            rz_finish(E, S, nparts);
+        }
+        return;
     }
-    T* xs = reinterpret_cast<T*>(smem);
-    T* bs = xs + W * HT;
-    T* cs = bs + W * HT;
+    float* xs = reinterpret_cast<float*>(smem);
+    float* bs = xs + W * HT;
+    float* cs = bs + W * HT;
     int tx, ty;
     frame_tile(m, blockIdx.x, tx, ty);
-    const int i0 = tx * TW, j0 = ty * TH;
-    if (ft_interior<TW, TH, H>(F.nx, F.ny, i0, j0, p)) {
+    const int i0 = tx * FT_W, j0 = ty * FT_H;
+    if (ft_interior<H>(F.nx, F.ny, i0, j0, p)) {
         // coarse block from (i0 - H) / 2 - 1, (j0 - H) / 2 - 1 (wrapped
         // along periodic axes)
         const int ci0 = (i0 - H) / 2 - 1, cj0 = (j0 - H) / 2 - 1;
@@ -935,33 +926,33 @@ __global__ void __launch_bounds__(FT_THREADS, FT_BLOCKS) k_mg_post(MgLev<T> C, M
         for (int lj = warp; lj < HT; lj += FT_THREADS / 32) {
             const int fy = j0 - H + lj;
             const int J = (fy >> 1) - cj0, NJ = J + ((fy & 1) ? 1 : -1);
-            const T* c0 = cs + J * CW;
-            const T* c1 = cs + NJ * CW;
+            const float* c0 = cs + J * CW;
+            const float* c1 = cs + NJ * CW;
             const size_t frow = (size_t)mg_wrap(fy, F.ny) * F.pitch;
             for (int li = lane; li < W; li += 32) {
                 const int fx = i0 - H + li;
                 const int I = (fx >> 1) - ci0, NI = I + ((fx & 1) ? 1 : -1);
-                T row0 = T(0.75) * c0[I];
-                row0 = mg_fma(T(0.25), c0[NI], row0);
-                T v = T(0.75) * row0;
-                T row1 = T(0.75) * c1[I];
-                row1 = mg_fma(T(0.25), c1[NI], row1);
-                v = mg_fma(T(0.25), row1, v);
+                float row0 = 0.75f * c0[I];
+                row0 = mg_fma(0.25f, c0[NI], row0);
+                float v = 0.75f * row0;
+                float row1 = 0.75f * c1[I];
+                row1 = mg_fma(0.25f, c1[NI], row1);
+                v = mg_fma(0.25f, row1, v);
                 const size_t k = frow + mg_wrap(fx, F.nx);
                 bs[lj * W + li] = F.b[k];
                 xs[lj * W + li] = F.r[k] + v;
             }
         }
         __syncthreads();
-        ft_half_int<T, TW, TH, H>(F, xs, bs, i0, j0, 1, 3, false);
-        ft_half_int<T, TW, TH, H>(F, xs, bs, i0, j0, 0, 2, false);
-        ft_half_int<T, TW, TH, H>(F, xs, bs, i0, j0, 1, 1, false);
-        ft_half_int<T, TW, TH, H>(F, xs, bs, i0, j0, 0, 0, false);
-        T rz = T(0);
-        for (int k = threadIdx.x; k < TW * TH; k += FT_THREADS) {
-            const int li = k % TW, lj = k / TW, gi = i0 + li, gj = j0 + lj;
+        ft_half_int<H>(F, xs, bs, i0, j0, 1, 3, false);
+        ft_half_int<H>(F, xs, bs, i0, j0, 0, 2, false);
+        ft_half_int<H>(F, xs, bs, i0, j0, 1, 1, false);
+        ft_half_int<H>(F, xs, bs, i0, j0, 0, 0, false);
+        float rz = 0.f;
+        for (int k = threadIdx.x; k < FT_W * FT_H; k += FT_THREADS) {
+            const int li = k % FT_W, lj = k / FT_W, gi = i0 + li, gj = j0 + lj;
             const int q = (lj + H) * W + li + H;
-            T* row = F.x + (size_t)gj * F.pitch;
+            float* row = F.x + (size_t)gj * F.pitch;
             row[gi] = xs[q];
             if (E.on) {
                 if (!in_strips(m, gi, gj)) rz = mg_fma(bs[q], xs[q], rz);
@@ -979,37 +970,37 @@ __global__ void __launch_bounds__(FT_THREADS, FT_BLOCKS) k_mg_post(MgLev<T> C, M
         if (E.on) post_epilogue(E, S, nparts, (double)rz);
         return;
     }
-    ft_load<T, TW, TH, H>(F, p, xs, bs, i0, j0, F.r);
+    ft_load<H>(F, p, xs, bs, i0, j0, F.r);
     // x += P x_coarse on every cell of the array inside the domain
     for (int q = threadIdx.x; q < W * HT; q += FT_THREADS) {
         const int fx = mg_dom(i0 - H + q % W, F.nx, p.per_x), fy = mg_dom(j0 - H + q / W, F.ny, p.per_y);
         if (fx < 0 || fy < 0) continue;
         int I, NI, J, NJ;
-        T wxI, wxN, wyJ, wyN;
-        mg_axis<T>(fx, C.nx, p.per_x, p.bc[0], p.bc[2], I, NI, wxI, wxN);
-        mg_axis<T>(fy, C.ny, p.per_y, p.bc[1], p.bc[3], J, NJ, wyJ, wyN);
-        T row0 = wxI * C.x[(size_t)J * C.pitch + I];
+        float wxI, wxN, wyJ, wyN;
+        mg_axis<float>(fx, C.nx, p.per_x, p.bc[0], p.bc[2], I, NI, wxI, wxN);
+        mg_axis<float>(fy, C.ny, p.per_y, p.bc[1], p.bc[3], J, NJ, wyJ, wyN);
+        float row0 = wxI * C.x[(size_t)J * C.pitch + I];
         if (NI >= 0) row0 = mg_fma(wxN, C.x[(size_t)J * C.pitch + NI], row0);
-        T v = wyJ * row0;
+        float v = wyJ * row0;
         if (NJ >= 0) {
-            T row1 = wxI * C.x[(size_t)NJ * C.pitch + I];
+            float row1 = wxI * C.x[(size_t)NJ * C.pitch + I];
             if (NI >= 0) row1 = mg_fma(wxN, C.x[(size_t)NJ * C.pitch + NI], row1);
             v = mg_fma(wyN, row1, v);
         }
         xs[q] = xs[q] + v;
     }
     __syncthreads();
-    ft_half<T, TW, TH, H>(F, p, xs, bs, i0, j0, 1, 3, false);
-    ft_half<T, TW, TH, H>(F, p, xs, bs, i0, j0, 0, 2, false);
-    ft_half<T, TW, TH, H>(F, p, xs, bs, i0, j0, 1, 1, false);
-    ft_half<T, TW, TH, H>(F, p, xs, bs, i0, j0, 0, 0, false);
-    T rz = T(0);
-    for (int k = threadIdx.x; k < TW * TH; k += FT_THREADS) {
-        const int gi = i0 + k % TW, gj = j0 + k / TW;
+    ft_half<H>(F, p, xs, bs, i0, j0, 1, 3, false);
+    ft_half<H>(F, p, xs, bs, i0, j0, 0, 2, false);
+    ft_half<H>(F, p, xs, bs, i0, j0, 1, 1, false);
+    ft_half<H>(F, p, xs, bs, i0, j0, 0, 0, false);
+    float rz = 0.f;
+    for (int k = threadIdx.x; k < FT_W * FT_H; k += FT_THREADS) {
+        const int gi = i0 + k % FT_W, gj = j0 + k / FT_W;
         if (gi < F.nx && gj < F.ny) {
             const int q = (gj - (j0 - H)) * W + (gi - (i0 - H));
-            const T v = xs[q];
-            T* row = F.x + (size_t)gj * F.pitch;
+            const float v = xs[q];
+            float* row = F.x + (size_t)gj * F.pitch;
             row[gi] = v;
             if (E.on) {
                 if (!in_strips(m, gi, gj)) rz = mg_fma(bs[q], v, rz);
@@ -1119,8 +1110,8 @@ static bool cluster_fits(int cluster, size_t smem) {
 
 // The first level of the cluster launch: the first of at most McMax::first
 // cells whose bands fit shared memory (with CF_MG_FUSED=0 the first of at
-// most 1024 cells).  The finest FP32 level stays a tile launch, whose epilogue
-// forms r.z.  No such launch when the coarsest level has more than 1024 cells.
+// most 1024 cells).  The finest FP32 level stays a launch of its own, whose
+// epilogue forms r.z.  No such launch when the coarsest level has more than 1024 cells.
 template <typename T>
 static int coarse_setup(cf_ctx* c, MgHierarchy* H, const MgLev<T>* lev) {
     const int nlev = H->nlev;
@@ -1317,8 +1308,7 @@ static int vcycle(cf_ctx* c, const MgHierarchy* H, MgLev<T>* lev, double scale0,
             if (big(lev[l])) {
                 if constexpr (sizeof(T) == 4) {
                     const StripMap m = strip_map(lev[l].nx, lev[l].ny, FT_W, FT_H, strip_rows, true);
-                    k_mg_pre<T, FT_W, FT_H><<<launch_blocks(m), FT_THREADS, 0, c->stream>>>(lev[l], lev[l + 1], p, c->S,
-                                                                                          inner, m);
+                    k_mg_pre<<<launch_blocks(m), FT_THREADS, 0, c->stream>>>(lev[l], lev[l + 1], p, c->S, inner, m);
                 }
             } else {
                 const MtGrid m = mt_grid<T>(lev[l].nx, lev[l].ny, c->sms, true);
@@ -1382,8 +1372,7 @@ static int vcycle(cf_ctx* c, const MgHierarchy* H, MgLev<T>* lev, double scale0,
             if (big(lev[l])) {
                 if constexpr (sizeof(T) == 4) {
                     const StripMap m = strip_map(lev[l].nx, lev[l].ny, FT_W, FT_H, strip_rows, false);
-                    k_mg_post<T, FT_W, FT_H><<<launch_blocks(m), FT_THREADS, 0, c->stream>>>(lev[l + 1], lev[l], p, c->S,
-                                                                                            inner, m, E);
+                    k_mg_post<<<launch_blocks(m), FT_THREADS, 0, c->stream>>>(lev[l + 1], lev[l], p, c->S, inner, m, E);
                 }
             } else {
                 const MtGrid m = mt_grid<T>(lev[l].nx, lev[l].ny, c->sms, false, E.on ? MT_RZ_ROWS : 0);
