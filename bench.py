@@ -44,11 +44,10 @@ KERNEL_BYTES_MIXED_ITER = 40.0
 FP64_ITERS_PER_STEP_4096 = 7890
 MG_NAMES = ("PFMG", "SMG", "MG")
 # DRAM bytes (read + write) of one mixed MG-PCG inner iteration at 4096^2:
-# dram__bytes_read.sum + dram__bytes_write.sum of this bench's kernels, one
-# kernel per ncu capture (K1, the fused x update and reliable update, the
-# V-cycle's pre- and post-smoothing per level, the coarse levels), summed over
-# one iteration
-MEASURED_TRAFFIC_MG_ITER_4096 = 1.234e9
+# dram__bytes_read.sum + dram__bytes_write.sum of its launches (K1, the fused x
+# update and reliable update, the V-cycle's pre- and post-smoothing per level,
+# the coarse levels) in an ncu capture, summed over one iteration
+MEASURED_TRAFFIC_MG_ITER_4096 = 1.203e9
 
 
 def mg_levels(nx, ny, periodic):
@@ -362,8 +361,8 @@ def bench_gb300(args, rank, world, dist, device):
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_source": f"hbm_gbs {peak_kind}",
                          "traffic": MEASURED_TRAFFIC_MG_ITER_4096 if (mg and w.nx == 4096) else None,
-                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, one kernel per "
-                                           "capture, summed over the kernels of one inner iteration"
+                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, summed over the "
+                                           "launches of one inner iteration"
                                            if (mg and w.nx == 4096) else None,
                          "algorithmic_bytes": it_bytes,
                          "algorithmic_bytes_per_cell": it_bytes / ncell, **kern_extra},

@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(kThreads, kCtas2)
 // iterations, a block keeping its tiles' r, x and A p in registers and p with its
 // halo in shared memory, the grid meeting at two barriers per iteration
 // (cf_grid.cuh).  The launches above cost 22 us per iteration at 501 x 333 (84
-// tiles), most of it launch, TMA and fold latency; this form 8.1 us, half of it
+// tiles), most of it launch, TMA and fold latency; this form 8.2 us, half of it
 // the two barriers and half the FP64 sums and divisions between them.  Every cell value, thread sum,
 // block sum and fold is formed as by those kernels (tile k of block b is tile
 // b + k gridDim; the thread sums of tiles that one of their blocks walks in turn

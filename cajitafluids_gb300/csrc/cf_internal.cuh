@@ -314,8 +314,9 @@ __device__ __forceinline__ double final_max(const double* partial, int n) {
 // warp (eight units, 8192 cells, on one SM) takes 25 us however small the grid.
 // Measured, unit per warp and unit per block: the direction and matvec kernel
 // 26.6 and 10.5 us at 192x160 (30 units), 33.3 and 25.8 us at 1024^2, the update
-// 17.9 and 9.0, 20.9 and 23.1 us; at 4096^2 246 and 269 us, 182 and 147 us (the
-// update without r.z under multigrid), bound by the FP64 pipe either way.
+// 17.9 and 9.0, 20.9 and 23.1 us; at 4096^2 246 and 269 us (239 since its products
+// run on the integer pipes), 182 and 147 us (the update without r.z under multigrid),
+// bound by the FP64 pipe either way.
 // Thread t owns column t % 64 of rows t / 64 + 4 m, m = 0 .. 3; the lane sums
 // of the canonical order are added by one warp from the factors staged in
 // shared memory.
