@@ -1602,18 +1602,20 @@ int cf_backward(cf_ctx* ctx, const double* dL_dq_T, const double* dL_du_T, const
     }
     int tally[3] = {0, 0, 0}, herr = 0;
     double rbar = 0.0;
+    cudaMemcpyAsync(&herr, A->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
     if (!rc) {
         cudaMemcpyAsync(tally, ctx->d_tally, sizeof(tally), cudaMemcpyDeviceToHost, ctx->stream);
-        cudaMemcpyAsync(&herr, A->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
         cudaMemcpyAsync(&rbar, A->d_rbar, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
     }
     const int rc1 = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "backward");
     ctx->adj_warm = 0;
-    if (rc) return rc;
-    if (rc1) return rc1;
-    if ((rc = check_tally(ctx, tally, "backward"))) return rc;
-    if (herr)
+    if (rc1) return rc ? rc : rc1;
+    if (!rc) rc = check_tally(ctx, tally, "backward");
+    // the adjoints that follow a trace the transpose does not cover mean nothing, and a
+    // solve of them may fail: the trace is what the caller has to know of
+    if (herr && (!rc || rc == CF_ERR_NUMERIC))
         return fail(ctx, CF_ERR_UNSUPPORTED, "adjoint: a trace moved more than one cell in a step (reduce dt)");
+    if (rc) return rc;
     double* outs[3] = {dL_dq0, dL_du0, dL_dv0};
     for (int k = 0; k < 3 && !rc; ++k)
         if (outs[k])
