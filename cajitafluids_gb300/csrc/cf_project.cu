@@ -1858,6 +1858,11 @@ static const int kResidentBatch = 16;    // Jacobi-PCG iterations per trip
 // to an SM); loading and storing the vectors costs about one iteration
 static const int kResidentBatchOnchip = 512;
 static const int kResidentBatchMG = 1;   // MG-PCG iterations per trip
+// A trip runs a whole batch of iterations, or fewer and (mixed) an outer refinement
+// after them, or ends the solve: the bound never cuts off a solve within its limits.
+static int trip_limit(const SolveOpts& o, bool mixed, bool mg) {
+    return o.max_iter / (mg ? kResidentBatchMG : kResidentBatch) + (mixed ? o.max_outer : 0) + 4;
+}
 
 // after each resident projection: count the solves that did not converge
 // (a solve still RUNNING stopped at the trip limit) and keep the worst status
@@ -2124,8 +2129,7 @@ static int project_resident(cf_ctx* c, double dt, const SolveOpts& o, SolveResul
         h->max_outer = o.max_outer;
         h->inner_tol2 = o.inner_tol * o.inner_tol;
         h->status = ST_RUNNING;
-        const int batch = mg ? kResidentBatchMG : kResidentBatch;
-        h->trip_limit = (o.max_iter + (mixed ? o.max_outer : 0)) / batch + 4;
+        h->trip_limit = trip_limit(o, mixed, mg);
         h->test_stall = c->test_stall;
     }
     cudaMemcpyAsync(c->S, h, sizeof(SolverState), cudaMemcpyHostToDevice, c->stream);
@@ -2191,8 +2195,7 @@ int step_resident(cf_ctx* c, double dt, int order, int fuse, const SolveOpts& o,
         h->max_outer = o.max_outer;
         h->inner_tol2 = o.inner_tol * o.inner_tol;
         h->status = ST_RUNNING;
-        const int batch = mg ? kResidentBatchMG : kResidentBatch;
-        h->trip_limit = (o.max_iter + (mixed ? o.max_outer : 0)) / batch + 4;
+        h->trip_limit = trip_limit(o, mixed, mg);
         h->test_stall = c->test_stall;
     }
     if ((rc = cuda_check(c, cudaGraphLaunch(c->sgx[s], c->stream), "step graph launch"))) return rc;
