@@ -11,8 +11,9 @@ BCS = [((False, False), (0, 0, 0, 0)), ((True, True), (0, 0, 0, 0)), ((False, Fa
        ((True, False), (0, 1, 0, 0))]
 # from hierarchies that one block solves alone (8 x 8 cells in one warp's registers,
 # 17 x 9: an odd row) to distributed levels of 2, 4 and 8 columns to a lane and
-# windows above them
-SIZES = {"mixed": [(16, 16), (32, 16), (34, 18), (64, 32), (48, 80), (128, 128), (192, 96), (320, 256), (600, 304)],
+# windows above them; the last mixed one has register strips
+SIZES = {"mixed": [(16, 16), (32, 16), (34, 18), (64, 32), (48, 80), (128, 128), (192, 96), (320, 256), (600, 304),
+                   (2048, 1024)],
          "fp64": [(16, 16), (32, 16), (34, 18), (48, 80), (64, 64), (112, 64), (256, 256)]}
 
 
